@@ -47,8 +47,8 @@ class CSite(C.Structure):
 
 
 class CModule(C.Structure):
-    _fields_ = [("layer", C.c_int32), ("r", C.c_int32), ("module", C.c_char_p), ("a", C.POINTER(C.c_float)),
-                ("b", C.POINTER(C.c_float)), ("a_len", C.c_uint64), ("b_len", C.c_uint64)]
+    _fields_ = [("layer", C.c_int32), ("r", C.c_int32), ("module", C.c_char_p), ("a", C.c_void_p),
+                ("b", C.c_void_p), ("a_len", C.c_uint64), ("b_len", C.c_uint64)]
 
 
 class Desc(C.Structure):
@@ -245,8 +245,7 @@ class Prep:
         for i, f in enumerate(modules):
             arr[i].layer, arr[i].r = f.layer, f.r
             arr[i].module = f.module.encode()
-            arr[i].a = f.a.ctypes.data_as(C.POINTER(C.c_float))
-            arr[i].b = f.b.ctypes.data_as(C.POINTER(C.c_float))
+            arr[i].a, arr[i].b = f.a.ctypes.data, f.b.ctypes.data
             arr[i].a_len, arr[i].b_len = f.a.size, f.b.size
             keep.append(f)
         out = _P()

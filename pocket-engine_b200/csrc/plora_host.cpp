@@ -3,9 +3,12 @@
 // Linear::forward puts around a layer's own matrix multiply (src/linear.rs:428-443,844-921).
 // Device work is launched through plora_kernels.cu; nothing here computes on the CPU.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <system_error>
+#include <thread>
 
 #include "plora_internal.h"
 
@@ -69,13 +72,57 @@ int next_mult(int x, int m) { return (x + m - 1) / m * m; }
 // so that the grouping output behind it (and with it every 32-word work item) starts on a 128-byte line
 size_t tile_words(const plora_t* h) { return (size_t)next_mult(1 + 3 * h->cap_tiles, 32); }
 
-// bf16 with round-to-nearest-even, as half::bf16::from_f32 does for finite values (src/lora.rs:141-145)
-inline uint16_t bf16_bits(float x) {
-    uint32_t u;
-    memcpy(&u, &x, 4);
-    if ((u & 0x7fffffffu) > 0x7f800000u) return 0x7fff;
-    u += 0x7fffu + ((u >> 16) & 1u);
-    return (uint16_t)(u >> 16);
+// bf16 with round-to-nearest-even, as half::bf16::from_f32 does for finite values (src/lora.rs:141-145). Free of
+// branches, one clone per vector width of the host.
+__attribute__((target_clones("arch=skylake-avx512", "avx2", "default"))) void bf16_fill(uint16_t* __restrict__ dst, const float* __restrict__ src,
+                                                                              size_t n) {
+    for (size_t i = 0; i < n; i++) {
+        uint32_t u;
+        memcpy(&u, src + i, 4);
+        const uint32_t r = (u + 0x7fffu + ((u >> 16) & 1u)) >> 16;
+        dst[i] = (uint16_t)((u & 0x7fffffffu) > 0x7f800000u ? 0x7fffu : r);
+    }
+}
+
+// One stretch of a slab: `rows` rows of `live` values, each followed by `pad` zeros, then `tail` zeros.
+struct FillJob {
+    uint16_t* dst;
+    const float* src;
+    size_t rows, live, pad, tail;
+};
+
+void run_job(const FillJob& j) {
+    if (j.pad == 0) {
+        bf16_fill(j.dst, j.src, j.rows * j.live);
+    } else {
+        for (size_t r = 0; r < j.rows; r++) {
+            uint16_t* d = j.dst + r * (j.live + j.pad);
+            bf16_fill(d, j.src + r * j.live, j.live);
+            memset(d + j.live, 0, j.pad * 2);
+        }
+    }
+    if (j.tail) memset(j.dst + j.rows * (j.live + j.pad), 0, j.tail * 2);
+}
+
+// Jobs of at most this many values, handed to the threads one after another
+constexpr size_t kJobValues = (size_t)128 << 10;
+
+// Fills a slab from its jobs, on as many threads as it has work for (about half a megabyte of factors each: starting a
+// thread costs what one converts in that time), at most 16.
+void run_jobs(const std::vector<FillJob>& jobs, size_t values) {
+    std::atomic<size_t> next{0};
+    auto work = [&] {
+        for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < jobs.size();) run_job(jobs[i]);
+    };
+    const size_t want = std::min<size_t>(std::min<size_t>(16, std::max(1u, std::thread::hardware_concurrency())), values / kJobValues + 1);
+    std::vector<std::thread> others;
+    try {
+        for (size_t t = 1; t < want; t++) others.emplace_back(work);
+    } catch (const std::system_error&) {
+        // no more threads to be had: the ones that run, this one among them, do the work
+    }
+    work();
+    for (auto& t : others) t.join();
 }
 
 // src/lora.rs:98-101
@@ -124,6 +171,59 @@ plora_desc desc_for(const SiteInfo& site, const SiteData& sd, uint64_t base) {
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
 
 }  // namespace
+
+void PinnedPool::release(const Buf& b) {
+    if (b.used) cudaEventDestroy(b.used);
+    if (b.p) cudaFreeHost(b.p);
+}
+
+PinnedPool::~PinnedPool() {
+    for (auto& b : idle) release(b);
+}
+
+cudaError_t PinnedPool::take(size_t bytes, Buf* out) {
+    Buf got;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        size_t best = idle.size();
+        for (size_t i = 0; i < idle.size(); i++)  // the smallest that holds it, unless most of it would lie idle
+            if (idle[i].cap >= bytes && idle[i].cap / 2 <= bytes + ((size_t)1 << 20) && (best == idle.size() || idle[i].cap < idle[best].cap))
+                best = i;
+        if (best < idle.size()) {
+            got = idle[best];
+            idle_bytes -= got.cap;
+            idle.erase(idle.begin() + (long)best);
+        }
+    }
+    if (got.p) {
+        // an upload of the adapter that left it may still be reading
+        const cudaError_t e = got.used ? cudaEventSynchronize(got.used) : cudaSuccess;
+        if (e != cudaSuccess) {
+            release(got);
+            return e;
+        }
+        *out = got;
+        return cudaSuccess;
+    }
+    const cudaError_t e = cudaMallocHost((void**)&got.p, bytes);
+    if (e != cudaSuccess) return e;
+    got.cap = bytes;
+    *out = got;
+    return cudaSuccess;
+}
+
+void PinnedPool::give(const Buf& b) {
+    if (!b.p) return;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (idle.size() < kMaxIdle && idle_bytes + b.cap <= kMaxBytes) {
+            idle.push_back(b);
+            idle_bytes += b.cap;
+            return;
+        }
+    }
+    release(b);
+}
 
 static_assert(sizeof(plora_desc) == 112, "Desc is 112 bytes (src/lora.rs:59-70)");
 
@@ -420,16 +520,30 @@ int plora_adapter_prepare(const plora_t* h, const char* name, const plora_module
     if (h->device >= 0) {
         // the Pinner of src/gpu.rs:85-110: make the device current on this (possibly worker) thread
         cudaError_t e = cudaSetDevice(h->device);
-        if (e == cudaSuccess) e = cudaMallocHost((void**)&a->data, alloc);
+        if (e == cudaSuccess) e = h->pinned->take(alloc, &a->buf);
         if (e != cudaSuccess) {
             delete a;
             return bad(PLORA_ERR_CUDA, std::string("pinned adapter buffer: ") + cudaGetErrorString(e));
         }
-        a->pinned = true;
+        a->home = h->pinned;
+        a->data = a->buf.p;
     } else {
         a->data = (uint8_t*)malloc(alloc);
     }
-    memset(a->data, 0, alloc);  // :375
+    // The slab is bound by the host's memory: 4 bytes in and 2 out per value, once (the zeros of :375 are written where
+    // padding is, not under everything). Jobs first, then several threads fill them: an adapter of 9.7 M values took 20
+    // ms on one thread behind a clearing pass over a freshly pinned buffer, and takes about 1 ms.
+    std::vector<FillJob> jobs;
+    std::vector<std::vector<float>> permuted;  // (the buffers stay where they are when the outer vector grows)
+    size_t values = 0;
+    auto add_rows = [&](uint16_t* dst, const float* src, size_t rows, size_t live, size_t pad, size_t tail) {
+        values += rows * (live + pad) + tail;
+        const size_t step = std::max<size_t>(1, kJobValues / (live + pad));
+        for (size_t r = 0; r < rows; r += step) {
+            const size_t n = std::min(step, rows - r);
+            jobs.push_back({dst + r * (live + pad), src + r * live, n, live, pad, r + n == rows ? tail : 0});
+        }
+    };
     for (size_t si = 0; si < h->sites.size(); si++) {  // :376-403 fill
         const SiteInfo& site = h->sites[si];
         const SiteData& sd = sds[si];
@@ -439,45 +553,41 @@ int plora_adapter_prepare(const plora_t* h, const char* name, const plora_module
             const plora_module* f = find_module(modules, n_modules, site.layer, site.parts[pi].module);
             const float* fa = f->a;
             const float* fb = f->b;
-            std::vector<float> pa, pb;
             if (!order.empty()) {  // Factors::permute, :115-135
                 const auto& part = site.parts[pi];
                 if (part.heads_start >= 0) {
-                    pb.assign(f->b, f->b + f->b_len);
+                    permuted.emplace_back(f->b, f->b + f->b_len);
+                    auto& pb = permuted.back();
                     permute_blocks(pb.data(), (size_t)part.heads_start * (size_t)f->r,
                                    (size_t)part.heads_block * (size_t)f->r, order, false);
                     fb = pb.data();
                 }
                 if (site.col_heads_start >= 0) {
-                    pa.assign(f->a, f->a + f->a_len);
+                    permuted.emplace_back(f->a, f->a + f->a_len);
+                    auto& pa = permuted.back();
                     for (int row = 0; row < f->r; row++)
                         permute_blocks(pa.data() + (size_t)row * (size_t)site.cols, (size_t)site.col_heads_start,
                                        (size_t)site.col_heads_block, order, false);
                     fa = pa.data();
                 }
             }
-            // A rows r_off .. r_off + r of the stacked A; padding rows stay zero (:388-393)
-            uint16_t* adst = (uint16_t*)(a->data + sd.a + (size_t)sd.r_off[pi] * (size_t)site.cols * 2);
-            size_t na = (size_t)f->r * (size_t)site.cols;
-            for (size_t i = 0; i < na; i++) adst[i] = bf16_bits(fa[i]);
+            // A rows r_off .. r_off + r of the stacked A; padding rows are zero (:388-393)
+            const size_t r = (size_t)f->r, cols = (size_t)site.cols;
+            add_rows((uint16_t*)(a->data + sd.a + (size_t)sd.r_off[pi] * cols * 2), fa, r, cols, 0, ((size_t)rp - r) * cols);
             // B [rows, rp], the last rp - r columns zero (:394-401)
-            for (int row = 0; row < site.parts[pi].rows; row++) {
-                uint16_t* bdst = (uint16_t*)(a->data + sd.b_off[pi] + (size_t)row * (size_t)rp * 2);
-                const float* src = fb + (size_t)row * (size_t)f->r;
-                for (int j = 0; j < f->r; j++) bdst[j] = bf16_bits(src[j]);
-            }
+            add_rows((uint16_t*)(a->data + sd.b_off[pi]), fb, (size_t)site.parts[pi].rows, r, (size_t)rp - r, 0);
         }
     }
+    run_jobs(jobs, values);
     *out = a;
     return PLORA_OK;
 }
 
 void plora_adapter_drop(plora_adapter_t* a) {
     if (!a) return;
-    if (a->data) {
-        if (a->pinned) cudaFreeHost(a->data);
-        else free(a->data);
-    }
+    if (!a->home) free(a->data);
+    else if (a->keep_out) PinnedPool::release(a->buf);
+    else a->home->give(a->buf);
     delete a;
 }
 
@@ -564,28 +674,46 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
     if (slot < 1 || slot > h->max_slots) return fail(h, PLORA_ERR_ARG, "slot " + std::to_string(slot) + " is out of range");
     auto it = h->adapters.find(id);
     if (it == h->adapters.end()) return fail(h, PLORA_ERR_UNKNOWN_ID, "adapter " + std::to_string(id) + " is not loaded");
-    const plora_adapter* a = it->second;
+    plora_adapter* a = it->second;
     if (a->len > h->slot_bytes) return fail(h, PLORA_ERR_CONFIG, "adapter is larger than a slot");
     CU(h, "cudaSetDevice", cudaSetDevice(h->device));
     cudaStream_t st = as_stream(stream);
     uint8_t* base = h->pool + (size_t)(slot - 1) * h->slot_bytes;
-    if (a->len > 0) CU(h, "upload slab", cudaMemcpyAsync(base, a->data, a->len, cudaMemcpyHostToDevice, st));
-    for (size_t si = 0; si < h->sites.size(); si++)
-        h->host_tables[si * (size_t)(h->max_slots + 1) + (size_t)slot] =
-            desc_for(h->sites[si], a->sites[si], (uint64_t)(uintptr_t)base);
-    // one copy per site's entry for this slot (:616-621)
-    for (size_t si = 0; si < h->sites.size(); si++) {
-        size_t at = si * (size_t)(h->max_slots + 1) + (size_t)slot;
-        CU(h, "upload descriptor",
-           cudaMemcpyAsync(h->tables + at, h->host_tables + at, sizeof(plora_desc), cudaMemcpyHostToDevice, st));
-        const plora_desc& d = h->host_tables[at];
-        if (h->mma_ok && d.rank > 0) {  // the tile path's view of the stacked A
-            CU(h, "encode slab tensor map",
-               plora_mma_encode_slab(&h->host_amaps[at], (const void*)(uintptr_t)d.a, h->sites[si].cols, d.rank));
-            CU(h, "upload slab tensor map",
-               cudaMemcpyAsync(h->amaps + at, h->host_amaps + at, sizeof(PloraTmap), cudaMemcpyHostToDevice, st));
+    if (a->len > 0) {
+        CU(h, "upload slab", cudaMemcpyAsync(base, a->data, a->len, cudaMemcpyHostToDevice, st));
+        // the buffer may be handed to another adapter once this copy is done; a second stream, or a graph that copies
+        // again on every replay, takes it out of that
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        CU(h, "capture status", cudaStreamIsCapturing(st, &cs));
+        if (cs != cudaStreamCaptureStatusNone || (a->uploaded && a->up_stream != stream)) a->keep_out = true;
+        if (!a->keep_out) {
+            if (!a->buf.used) CU(h, "event", cudaEventCreateWithFlags(&a->buf.used, cudaEventDisableTiming));
+            CU(h, "upload record", cudaEventRecord(a->buf.used, st));
+            a->up_stream = stream;
+            a->uploaded = true;
         }
     }
+    // The slot's column of the descriptor tables [sites][max_slots + 1], and of the tile path's views of the stacked A:
+    // one strided copy each (:616-621 copies entry by entry; at 4.6 us per 112-byte copy the 32 layers' entries of an
+    // eight-layer model took as long as 16 MB of slab).
+    const size_t stride = (size_t)h->max_slots + 1, n = h->sites.size();
+    bool maps = false;
+    for (size_t si = 0; si < n; si++) {
+        const size_t at = si * stride + (size_t)slot;
+        const plora_desc d = h->host_tables[at] = desc_for(h->sites[si], a->sites[si], (uint64_t)(uintptr_t)base);
+        if (h->mma_ok && d.rank > 0) {
+            CU(h, "encode slab tensor map",
+               plora_mma_encode_slab(&h->host_amaps[at], (const void*)(uintptr_t)d.a, h->sites[si].cols, d.rank));
+            maps = true;
+        }
+    }
+    CU(h, "upload descriptors",
+       cudaMemcpy2DAsync(h->tables + slot, stride * sizeof(plora_desc), h->host_tables + slot, stride * sizeof(plora_desc),
+                         sizeof(plora_desc), n, cudaMemcpyHostToDevice, st));
+    if (maps)
+        CU(h, "upload slab tensor maps",
+           cudaMemcpy2DAsync(h->amaps + slot, stride * sizeof(PloraTmap), h->host_amaps + slot, stride * sizeof(PloraTmap),
+                             sizeof(PloraTmap), n, cudaMemcpyHostToDevice, st));
     return PLORA_OK;
 }
 

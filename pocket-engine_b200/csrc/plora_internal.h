@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -107,13 +109,38 @@ struct SiteData {  // src/lora.rs:74-79
     int r[PLORA_MAX_PARTS] = {0, 0, 0, 0};
 };
 
+// Pinned host buffers that dropped adapters leave behind for the next ones prepared on the same handle. Page-locking
+// and unlocking the slab of an adapter costs several times what filling it does, and a program that swaps adapters in
+// and out asks for buffers of the same few sizes. Bounded (two buffers, 256 MB together), shared by the handle and
+// its adapters, safe from several threads; whatever is idle goes back to the system with the last of them.
+struct PinnedPool {
+    struct Buf {
+        uint8_t* p = nullptr;
+        size_t cap = 0;
+        cudaEvent_t used = nullptr;  // recorded behind the last upload that read the buffer
+    };
+    static constexpr size_t kMaxIdle = 2, kMaxBytes = (size_t)256 << 20;
+    std::mutex mu;
+    std::vector<Buf> idle;
+    size_t idle_bytes = 0;
+    cudaError_t take(size_t bytes, Buf* out);  // no copy still reads the buffer it returns
+    void give(const Buf& b);                   // keeps it or frees it
+    static void release(const Buf& b);
+    ~PinnedPool();
+};
+
 struct plora_adapter {  // src/lora.rs:82-88
     std::string name;
     int rank = 0;
     uint8_t* data = nullptr;  // pinned when a device is present, else plain host memory
-    bool pinned = false;
     size_t len = 0;
     std::vector<SiteData> sites;
+    // device handles only: where the buffer came from, and whether it may go back there (not once uploads on several
+    // streams or a captured graph may still read it)
+    std::shared_ptr<PinnedPool> home;
+    PinnedPool::Buf buf;
+    void* up_stream = nullptr;
+    bool uploaded = false, keep_out = false;
 };
 
 struct plora {
@@ -128,6 +155,7 @@ struct plora {
     size_t table_bytes = 0;
     PloraTmap* amaps = nullptr;       // device: per (layer, slot) tensor map of the stacked A (tile path)
     PloraTmap* host_amaps = nullptr;  // pinned mirror
+    std::shared_ptr<PinnedPool> pinned = std::make_shared<PinnedPool>();
     std::unordered_map<uint32_t, plora_adapter*> adapters;
     std::map<std::string, uint32_t> names;
     uint32_t next_id = 1;
