@@ -38,6 +38,8 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t saddr) {
 __global__ void __launch_bounds__(256) plora_fp8_quant_rows_kernel(const bf16* __restrict__ X, int ldx, int K,
                                                                     uint8_t* __restrict__ Xq, float* __restrict__ st) {
     __shared__ float red[8];
+    pdl_wait();
+    pdl_trigger();
     const int t = blockIdx.x;
     const bf16* x = X + (size_t)t * ldx;
     float amax = 0.f;
@@ -516,11 +518,9 @@ cudaError_t plora_fp8_init(int max_rank) {
     return plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_fused_kernel<true>), smem);
 }
 
-cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, cudaStream_t stream) {
-    if (rows == 0) return cudaSuccess;
-    plora_fp8_quant_rows_kernel<<<rows, 256, 0, stream>>>(reinterpret_cast<const bf16*>(x), ldx, K,
-                                                          reinterpret_cast<uint8_t*>(xq), st);
-    return cudaGetLastError();
+cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, bool pdl, cudaStream_t stream) {
+    return launch_pdl(plora_fp8_quant_rows_kernel, dim3((unsigned)rows), dim3(256), 0, stream, pdl, reinterpret_cast<const bf16*>(x), ldx, K,
+                      reinterpret_cast<uint8_t*>(xq), st);
 }
 
 cudaError_t plora_launch_s_reduce(float* S, size_t s_stride_elems, int lds, int nsplit, const int32_t* segs,

@@ -856,12 +856,16 @@ int plora_meta_build(plora_t* h, uint64_t cu_dev, uint64_t seq_slot_dev, int n_s
     if (!cu_dev || !seq_slot_dev) return fail(h, PLORA_ERR_ARG, "null device pointer");
     CUK(h, "meta_tiles", plora_launch_meta_tiles((const int32_t*)(uintptr_t)cu_dev, (const int32_t*)(uintptr_t)seq_slot_dev,
                                                 n_seqs, h->meta, h->cap_tiles, h->status, as_stream(stream)));
+    h->tiles_built = true;
+    h->pdl_armed = 0;
     return PLORA_OK;
 }
 
 int plora_meta_upload(plora_t* h, const int32_t* words, void* stream) {
     if (!h || !words) return PLORA_ERR_ARG;
     if (h->device < 0) return fail(h, PLORA_ERR_CUDA, "layout-only handle: no device");
+    h->tiles_built = false;
+    h->pdl_armed = 0;
     int count = words[0];
     if (count < 0 || count > h->cap_tiles) return fail(h, PLORA_ERR_CAPACITY, "more tiles than the metadata holds");
     CU(h, "upload tiles", cudaMemcpyAsync(h->meta, words, (size_t)(1 + 3 * count) * 4, cudaMemcpyHostToDevice,
@@ -874,11 +878,12 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
     if (h->device < 0) return fail(h, PLORA_ERR_CUDA, "layout-only handle: no device");
     if (max_tiles < 0) return fail(h, PLORA_ERR_ARG, "max_tiles is negative");
     int32_t* segs = h->meta + tile_words(h);
-    h->pdl_armed = false;
     SegLayout lay = h->seg;
     if (decode) lay.run_min = 1 << 30;
     CUK(h, "meta_group", plora_launch_meta_group(h->meta, segs, lay, h->status, h->tables, h->site_cols, (int)h->sites.size(),
-                                                 h->recs, h->rec_cap, as_stream(stream)));
+                                                 h->recs, h->rec_cap, h->pdl && h->tiles_built, as_stream(stream)));
+    h->tiles_built = false;
+    h->pdl_armed = 1;
     out->run_min = lay.run_min;
     out->pad_ = 0;
     out->tiles = (uint64_t)(uintptr_t)h->meta;
@@ -936,13 +941,13 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     // at most one per slot plus one per 16 tokens
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
+    h->pdl_armed = 2;
     CUK(h, "shrink",
        plora_launch_shrink((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
                            (float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.kchunk, site.nsplit,
                            work_cap, hook->parts * h->max_rank, bounds_of(h, hook, rows, 0), h->status, pdl, early, early_x,
-                           as_stream(stream)));
+                           late, as_stream(stream)));
     if (h->mma_ok && rows >= step->run_min)
         CUK(h, "shrink (tile path)",
            plora_launch_shrink_mma((const void*)(uintptr_t)x, rows, site.cols, site.cols, (const int32_t*)(uintptr_t)step->segs,
@@ -986,8 +991,8 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     if (!y || (y & (f32_out ? 7 : 3)) || (ldy & 1)) return fail(h, PLORA_ERR_ARG, "y must be aligned to two elements and ldy even");
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
+    h->pdl_armed = 2;
     int total = 0;
     for (auto& p : site.parts) total += p.rows;
     CUK(h, "site kernel",
@@ -995,7 +1000,7 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
                          hook->site + 1 < (int)h->sites.size() ? recs_of(h, hook->site + 1) : nullptr,
                          (void*)(uintptr_t)y, ldy, f32_out, (int)site.parts.size(), h->max_rank, total, work_cap,
                          site.max_clusters, (h->early_x ? 1 : 0) | ((h->site_release >= 0 && h->site_release <= 4 ? h->site_release : (h->early_x ? 0 : 1)) << 1) |
-                             (h->prefetch_next ? 16 : 0),
+                             (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
                          bounds_of(h, hook, rows, ldy), h->status, pdl, as_stream(stream)));
     if (h->mma_ok && rows >= step->run_min) {
         CUK(h, "shrink (tile path)",
@@ -1021,8 +1026,8 @@ int plora_s_reduce(plora_t* h, const plora_hook* hook, const plora_step* step, i
     if (rows < 0 || rows > h->max_tokens) return fail(h, PLORA_ERR_CAPACITY, "more rows than max_tokens");
     const SiteInfo& site = h->sites[(size_t)hook->site];
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool pdl = h->pdl && h->pdl_armed == 2;
+    h->pdl_armed = 2;
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
@@ -1042,8 +1047,8 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     const SiteInfo& site = h->sites[(size_t)hook->site];
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);  // src/linear.rs:900
     if (work_cap == 0) return PLORA_OK;
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool pdl = h->pdl && h->pdl_armed == 2;
+    h->pdl_armed = 2;
     CUK(h, "expand",
        plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds,
                            reduced ? 1 : site.nsplit, recs_of(h, hook->site), h->rec_cap,
@@ -1064,9 +1069,11 @@ int plora_fp8_quant_rows(plora_t* h, uint64_t x, int rows, int cols, uint64_t xq
     if (h->device < 0) return fail(h, PLORA_ERR_CUDA, "layout-only handle: no device");
     if (!x || !xq || !st || (x & 15) || (xq & 7) || cols <= 0 || (cols & 7) || rows < 0)
         return fail(h, PLORA_ERR_ARG, "x, xq, st must be aligned device addresses and cols a multiple of 8");
+    if (rows == 0) return PLORA_OK;
+    // (waits for the kernel before it reads or releases anything: what follows may read launch records at once)
     CUK(h, "fp8 quantise", plora_launch_fp8_quant((const void*)(uintptr_t)x, rows, cols, cols, (void*)(uintptr_t)xq,
-                                                 (float*)(uintptr_t)st, as_stream(stream)));
-    h->pdl_armed = false;
+                                                 (float*)(uintptr_t)st, h->pdl && h->pdl_armed != 0, as_stream(stream)));
+    h->pdl_armed = 2;
     return PLORA_OK;
 }
 
@@ -1076,8 +1083,8 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
                       uint64_t w, uint64_t sn, int rows, int width, uint64_t y, int ldy, int f32_out, int work_cap,
                       void* stream) {
     const SiteInfo& site = h->sites[(size_t)hook->site];
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool pdl = h->pdl && h->pdl_armed == 2;
+    h->pdl_armed = 2;
     // the kernel reads the long runs' S from plane 0: fold the tile path's planes (the gather tokens' K-split
     // planes are added by the gather expand itself)
     CUK(h, "S reduce (tiles)",
@@ -1151,8 +1158,8 @@ int plora_linear_fp8_fused(plora_t* h, const plora_hook* hook, const plora_step*
         plora_gemm_fits(0, (const void*)(uintptr_t)xq, (const void*)(uintptr_t)wq, (const void*)(uintptr_t)y, ldy, f32_out,
                         site.cols, (int)site.parts.size(), off))
         return gemm_layer(h, hook, step, 0, xq, st, wq, sn, rows, width, y, ldy, f32_out, work_cap, stream);
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool pdl = h->pdl && h->pdl_armed == 2;
+    h->pdl_armed = 2;
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
@@ -1376,8 +1383,8 @@ int plora_s_exchange(plora_t* h, const plora_hook* hook, const plora_step* step,
     int nblocks = 0;
     int rc = xchg_ctx(h, hook, step, rows, &c, &nblocks);
     if (rc != PLORA_OK) return rc;
-    const bool pdl = h->pdl && h->pdl_armed;
-    h->pdl_armed = true;
+    const bool pdl = h->pdl && h->pdl_armed == 2;
+    h->pdl_armed = 2;
     CUK(h, "S exchange", plora_launch_xchg(c, nblocks, pdl, as_stream(stream)));
     return PLORA_OK;
 }
@@ -1396,7 +1403,7 @@ int plora_s_exchange_all_ranks(plora_t* const* hs, const plora_hook* const* hook
         if (rc != PLORA_OK) return rc;
         if (r && nb != nblocks) return fail(h0, PLORA_ERR_ARG, "all-ranks exchange: ranks disagree on the step's shape");
         nblocks = nb;
-        hs[r]->pdl_armed = false;  // a cooperative launch: the next kernel of each rank starts plain
+        hs[r]->pdl_armed = 0;  // a cooperative launch: the next kernel of each rank starts plain
     }
     CU(h0, "cudaSetDevice", cudaSetDevice(h0->device));
     PloraXchgCtx* dev = (PloraXchgCtx*)(h0->xchg + h0->xchg_ctx_off);

@@ -193,7 +193,10 @@ struct plora {
     int fused_tile_rows = 1;  // steps with at least this many rows take it (plora_set_fused_tile_rows)
     bool tile_late = true;    // the tile shrink runs beside the gather shrink launched right before it (PLORA_TILE_LATE=0: behind it)
     bool mma_ok = false;    // the tensor-core tile kernels can run (max_rank <= 128 and the driver entry point exists)
-    bool pdl_armed = false;  // false right after the step's grouping kernel: the next launch is a plain one
+    // what the kernel before the next launch is: 0 = not one of ours (a plain launch), 1 = the step's grouping (its
+    // launch records must not be read before the dependency wait), 2 = a kernel of the step
+    int pdl_armed = 0;
+    bool tiles_built = false;  // plora_meta_build was the last call that touched the tile words
     // plora_profile_begin / _end: one pair of events per kernel launch while a profile is open
     struct ProfEntry {
         const char* what;
@@ -245,7 +248,7 @@ cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, 
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
 // site_info: per layer {input width, blocks that share a work item's output columns in the cluster kernel (0: none)}
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, cudaStream_t st);
+                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, bool pdl, cudaStream_t st);
 // Dynamic shared-memory limit of a kernel together with a request for the largest shared-memory split of the SM.
 // Kernels of this library overlap with their neighbours in the stream (programmatic dependent launch); an SM's
 // split between L1 and shared memory is fixed while any block runs on it, so kernels that each let the driver
@@ -265,7 +268,7 @@ cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* rec
                               int max_clusters, int mode, const PloraBounds& bnd, int* status, bool pdl, cudaStream_t st);
 cudaError_t plora_mma_init();
 cudaError_t plora_fp8_init(int max_rank);
-cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, cudaStream_t stream);
+cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, bool pdl, cudaStream_t stream);
 cudaError_t plora_launch_s_reduce(float* S, size_t s_stride_elems, int lds, int nsplit, const int32_t* segs,
                                   SegLayout lay, const plora_desc* table, int work_cap, int tile_cap, int tile_split,
                                   int K, bool pdl, cudaStream_t st);
@@ -290,10 +293,12 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
                                     int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
                                     int max_rows, int tile_cap, int* status, bool pdl, cudaStream_t st);
 // early: dependents are released at kernel start and slabs are requested ahead of the dependency wait (used by
-// plora_apply, whose kernels follow one another); early_x: x too may be read ahead of the wait
+// plora_apply, whose kernels follow one another); early_x: x too may be read ahead of the wait; late: the kernel before
+// is the step's grouping, so not even a launch record may be read ahead of it
 cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, float* S,
                                 size_t s_stride_elems, int lds, int kchunk, int nsplit, int work_cap, int max_rank_total,
-                                const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, cudaStream_t st);
+                                const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, bool late,
+                                cudaStream_t st);
 cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, int nsplit, const PloraRec* recs,
                                 int rec_cap, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
                                 const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st);

@@ -18,32 +18,32 @@ typedef __nv_bfloat16 bf16;
 
 namespace {
 
-// Exclusive scan of one int per thread over a block of 1024 threads. `sh` holds 33 ints.
-__device__ __forceinline__ int block_scan_excl(int v, int& total, int* sh) {
+// Exclusive scan of one 64-bit word per thread over a block of 1024 threads (several counts packed into one word are
+// scanned together). `sh` holds 33 words; it may be used again after the next __syncthreads().
+__device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long v, unsigned long long& total, unsigned long long* sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int incl = v;
+    unsigned long long incl = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        int u = __shfl_up_sync(0xffffffffu, incl, o);
+        const unsigned long long u = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += u;
     }
     if (lane == 31) sh[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        int t = sh[lane], ti = t;
+        const unsigned long long t = sh[lane];
+        unsigned long long ti = t;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            int u = __shfl_up_sync(0xffffffffu, ti, o);
+            const unsigned long long u = __shfl_up_sync(0xffffffffu, ti, o);
             if (lane >= o) ti += u;
         }
         sh[lane] = ti - t;
         if (lane == 31) sh[32] = ti;
     }
     __syncthreads();
-    const int r = incl - v + sh[warp];
     total = sh[32];
-    __syncthreads();
-    return r;
+    return incl - v + sh[warp];
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -53,9 +53,10 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
                                                                  const int* __restrict__ seq_slot, int n_seqs,
                                                                  int* __restrict__ tiles, int cap_tiles,
                                                                  int* __restrict__ status) {
-    __shared__ int sh[33];
+    __shared__ unsigned long long sh[33];
     __shared__ int s_first[1024], s_start[1024], s_n[1024], s_slot[1024];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    pdl_trigger();  // the grouping kernel waits for this grid before it reads a word
     int carry = 0;
     for (int base = 0; base < n_seqs; base += 1024) {
         const int i = base + tid;
@@ -67,8 +68,8 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
             if (n < 0) n = 0;
             nt = slot != 0 ? (n + PLORA_TILE - 1) / PLORA_TILE : 0;
         }
-        int total;
-        const int excl = block_scan_excl(nt, total, sh);
+        unsigned long long total;
+        const int excl = (int)block_scan_excl((unsigned long long)nt, total, sh);
         s_first[tid] = carry + excl;
         s_start[tid] = start;
         s_n[tid] = n;
@@ -89,7 +90,7 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
                 }
             }
         }
-        carry += total;
+        carry += (int)total;
         __syncthreads();
     }
     if (tid == 0) {
@@ -145,85 +146,123 @@ __device__ __forceinline__ void write_record(uint4* o, const int* segs, const Se
 // least lay.run_min tokens become tensor-core tiles; the rest are gathered by slot: perm lists their
 // token rows ordered by (slot, position in the tile list), cut into work items of <= 16 tokens.
 //
-// The same block then writes the step's launch records: every gather work item resolved against every layer's
-// descriptor table. The list of a layer ends with records whose cnt is 0.
+// Every block then writes the launch records of its layers (blockIdx.x, blockIdx.x + gridDim.x, ...): each gather work
+// item resolved against the layer's descriptor table. The list of a layer ends with records whose cnt is 0.
+//
+// The kernel is a chain of latencies (fetch, scans, fetch of the descriptors), not of bytes. So the blocks do not
+// share the grouping, which would take a grid-wide wait: each of them does all of it, with the same result, and writes
+// the regrouped rows and work items that it will read back itself (the same words from every block); block 0 also
+// writes what only later kernels read. Counts that are scanned together share one 64-bit scan. One block wrote the
+// records of all layers before: 9 us for a single token over 16 layers, 13 us for 64 tokens, 19-27 us for a prefill
+// step, against what bench.py reports as meta_us now.
 __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __restrict__ tiles, int* __restrict__ segs,
                                                                  SegLayout lay, int* __restrict__ status,
                                                                  const plora_desc* __restrict__ tables,
                                                                  const int* __restrict__ site_cols, int n_sites,
                                                                  PloraRec* __restrict__ recs, int rec_cap) {
     extern __shared__ int sm[];
-    __shared__ int sh[33];
+    __shared__ unsigned long long sh[4][33];  // a row per scan in flight: no barrier between one scan and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cap = lay.cap_tiles, S1 = lay.max_slots + 1;
-    int* run_start = sm;
-    int* run_len = run_start + cap;
-    int* run_slot = run_len + cap;
+    const bool first = blockIdx.x == 0;
+    int* run_tok = sm;  // [cap + 1]: tokens of the runs before; the length of run r is run_tok[r + 1] - run_tok[r]
+    int* run_start = run_tok + cap + 1;
+    int* run_slot = run_start + cap;
     int* run_pos = run_slot + cap;
     int* cnt = run_pos + cap;
     int* seg_base = cnt + S1;
     int* fill = seg_base + S1;
     int* whist = fill + S1;  // [32][S1]
 
+    // what needs no tile word, under the wait for the kernel before (the tile words, or the step before, which may
+    // still be reading the metadata)
+    for (int i = tid; i < S1; i += 1024) cnt[i] = fill[i] = seg_base[i] = 0;
+    for (int i = tid; i < 32 * S1; i += 1024) whist[i] = 0;
+    pdl_trigger();  // (the first kernel of the step waits for this grid before it reads a record)
+    pdl_wait();
+
+    // the first tile words are fetched together with their count
+    int w0 = 0, w1 = 0, w2 = 0;
+    if (tid < cap) {
+        w0 = tiles[1 + 3 * tid];
+        w1 = tiles[2 + 3 * tid];
+        w2 = tiles[3 + 3 * tid];
+    }
     int n_tiles = tiles[0];
     bool bad = false;
     if (n_tiles < 0 || n_tiles > cap) {
         n_tiles = 0;
         bad = true;
     }
-    for (int i = tid; i < n_tiles; i += 1024) run_len[i] = 0;
-    for (int i = tid; i < lay.max_tokens; i += 1024) segs[lay.tslot() + i] = 0;
-    for (int i = tid; i < S1; i += 1024) {
-        cnt[i] = 0;
-        fill[i] = 0;
-        seg_base[i] = 0;
-    }
+    if (first)
+        for (int i = tid; i < lay.max_tokens; i += 1024) segs[lay.tslot() + i] = 0;
     __syncthreads();
 
     // runs
-    int n_runs = 0;
+    int n_runs = 0, n_tok = 0;
     for (int base = 0; base < n_tiles; base += 1024) {
         const int i = base + tid;
         int head = 0, start = 0, len = 0, slot = 0;
         if (i < n_tiles) {
-            start = tiles[1 + 3 * i];
-            len = tiles[2 + 3 * i];
-            slot = tiles[3 + 3 * i];
+            if (base > 0) {
+                w0 = tiles[1 + 3 * i];
+                w1 = tiles[2 + 3 * i];
+                w2 = tiles[3 + 3 * i];
+            }
+            start = w0;
+            len = w1;
+            slot = w2;
+        }
+        // the tile before: a neighbour's, or fetched by the first lane of a warp
+        int ps = __shfl_up_sync(0xffffffffu, start, 1), pl = __shfl_up_sync(0xffffffffu, len, 1), pslot = __shfl_up_sync(0xffffffffu, slot, 1);
+        if (i < n_tiles) {
+            if (lane == 0 && i > 0) {
+                ps = tiles[1 + 3 * (i - 1)];
+                pl = tiles[2 + 3 * (i - 1)];
+                pslot = tiles[3 + 3 * (i - 1)];
+            }
             if (slot < 0 || slot > lay.max_slots || len < 1 || len > PLORA_TILE || start < 0 ||
                 start + len > lay.max_tokens) {
                 bad = true;
                 slot = 0;
                 len = 0;
                 start = 0;
+            } else if (recs != nullptr && blockIdx.x < (unsigned)n_sites) {
+                // the descriptor this block will resolve first
+                prefetch_l2(tables + (size_t)blockIdx.x * (size_t)S1 + slot);
             }
-            if (i == 0) head = 1;
-            else {
-                const int ps = tiles[1 + 3 * (i - 1)], pl = tiles[2 + 3 * (i - 1)], pslot = tiles[3 + 3 * (i - 1)];
-                head = !(pslot == slot && ps + pl == start);
-            }
+            head = i == 0 || !(pslot == slot && ps + pl == start);
         }
-        int total;
-        const int excl = block_scan_excl(head, total, sh);
-        const int rid = n_runs + excl + head - 1;
-        if (i < n_tiles) {
-            if (head) {
-                run_start[rid] = start;
-                run_slot[rid] = slot;
-            }
-            atomicAdd(&run_len[rid], len);
-            for (int k = 0; k < len; k++) segs[lay.tslot() + start + k] = slot;
+        unsigned long long total;
+        const unsigned long long excl = block_scan_excl(((unsigned long long)head << 32) | (unsigned)len, total, sh[(base >> 10) & 1]);
+        const int rid = n_runs + (int)(excl >> 32);
+        if (head) {
+            run_start[rid] = start;
+            run_slot[rid] = slot;
+            run_tok[rid] = n_tok + (int)(excl & 0xffffffffu);
         }
-        n_runs += total;
-        __syncthreads();
+        n_runs += (int)(total >> 32);
+        n_tok += (int)(total & 0xffffffffu);
     }
+    if (tid == 0) run_tok[n_runs] = n_tok;
+    __syncthreads();
+    // the slot of every token row: 16 lanes a tile
+    if (first)
+        for (int i = tid; i < 16 * n_tiles; i += 1024) {
+            const int t = i >> 4, k = i & 15;
+            const int start = tiles[1 + 3 * t], len = tiles[2 + 3 * t], slot = tiles[3 + 3 * t];
+            if (slot >= 0 && slot <= lay.max_slots && len >= 1 && len <= PLORA_TILE && start >= 0 && start + len <= lay.max_tokens && k < len)
+                segs[lay.tslot() + start + k] = slot;
+        }
 
-    // classify runs; tensor-core tiles
+    // classify runs; tensor-core tiles (none when every run stays under run_min)
+    const bool any_mma = lay.run_min <= n_tok;
     int n_mma = 0;
     for (int base = 0; base < n_runs; base += 1024) {
         const int r = base + tid;
         int nm = 0, len = 0, slot = 0, start = 0;
         if (r < n_runs) {
-            len = run_len[r];
+            len = run_tok[r + 1] - run_tok[r];
             slot = run_slot[r];
             start = run_start[r];
             if (slot == 0 || len == 0) run_pos[r] = -1;
@@ -235,107 +274,116 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                 atomicAdd(&cnt[slot], len);
             }
         }
-        int total;
-        const int excl = block_scan_excl(nm, total, sh);
-        int* mma = segs + lay.mma();
-        for (int q = 0; q < nm; q++) {
-            const int at = n_mma + excl + q;
-            if (at >= cap) break;  // tiles that overlap can add up to more rows than the step has: flagged below
-            mma[3 * at] = start + q * PLORA_MMA_TOKENS;
-            mma[3 * at + 1] = min(PLORA_MMA_TOKENS, len - q * PLORA_MMA_TOKENS);
-            mma[3 * at + 2] = slot;
+        if (any_mma) {
+            unsigned long long total;
+            const int excl = (int)block_scan_excl((unsigned long long)nm, total, sh[2 + ((base >> 10) & 1)]);
+            int* mma = segs + lay.mma();
+            for (int q = 0; first && q < nm; q++) {
+                const int at = n_mma + excl + q;
+                if (at >= cap) break;  // tiles that overlap can add up to more rows than the step has: flagged below
+                mma[3 * at] = start + q * PLORA_MMA_TOKENS;
+                mma[3 * at + 1] = min(PLORA_MMA_TOKENS, len - q * PLORA_MMA_TOKENS);
+                mma[3 * at + 2] = slot;
+            }
+            n_mma += (int)total;
         }
-        n_mma += total;
     }
     __syncthreads();
 
-    // slots with gather tokens, ascending; their offsets into perm; work items
+    // slots with gather tokens, ascending; their offsets into perm; work items. One scan of (slots, work items, tokens).
     int n_act, n_gather, n_work;
     {
         const int s = tid;
         const int c = (s >= 1 && s < S1) ? cnt[s] : 0;
         const int flag = c > 0;
         const int nw = (c + PLORA_WORK_TOKENS - 1) / PLORA_WORK_TOKENS;
-        const int aidx = block_scan_excl(flag, n_act, sh);
-        const int off = block_scan_excl(c, n_gather, sh);
-        const int woff = block_scan_excl(nw, n_work, sh);
+        unsigned long long total;
+        const unsigned long long excl =
+            block_scan_excl(((unsigned long long)flag << 53) | ((unsigned long long)nw << 29) | (unsigned long long)c, total, sh[0]);
+        const int aidx = (int)(excl >> 53), woff = (int)((excl >> 29) & 0xffffffu), off = (int)(excl & 0x1fffffffu);
+        n_act = (int)(total >> 53);
+        n_work = (int)((total >> 29) & 0xffffffu);
+        n_gather = (int)(total & 0x1fffffffu);
         // Tiles that overlap one another pass the per-tile checks but name more token rows than the step has: the
         // regrouped rows would not fit their region. Such a list is refused as a whole.
-        if (n_gather > lay.max_tokens || n_work > cap || n_mma > cap) bad = true;
         const bool over = n_gather > lay.max_tokens || n_work > cap || n_mma > cap;
+        if (over) bad = true;
         if (flag && !over) {
-            segs[lay.act() + aidx] = s;
-            segs[lay.seg_off() + aidx] = off;
+            if (first) {
+                segs[lay.act() + aidx] = s;
+                segs[lay.seg_off() + aidx] = off;
+            }
             seg_base[s] = off;
             int* work = segs + lay.work();
-            for (int q = 0; q < nw; q++) {
-                int* wi = work + PLORA_WORK_WORDS * (woff + q);
-                wi[0] = s;
-                wi[1] = off + q * PLORA_WORK_TOKENS;
-                wi[2] = min(PLORA_WORK_TOKENS, c - q * PLORA_WORK_TOKENS);
-                wi[3] = 0;
-            }
+            for (int q = 0; q < nw; q++)
+                *reinterpret_cast<int4*>(work + PLORA_WORK_WORDS * (woff + q)) =
+                    make_int4(s, off + q * PLORA_WORK_TOKENS, min(PLORA_WORK_TOKENS, c - q * PLORA_WORK_TOKENS), 0);
             cnt[s] = woff;  // from here on: the slot's first work item
         }
-        if (tid == 0 && !over) segs[lay.seg_off() + n_act] = n_gather;
+        if (first && tid == 0 && !over) segs[lay.seg_off() + n_act] = n_gather;
         if (over) n_act = n_gather = n_work = n_mma = n_runs = 0;
     }
-    __syncthreads();
 
-    // stable position of every gather run inside its slot's segment
+    // stable position of every gather run inside its slot's segment: the weights of the same slot in the lanes below,
+    // in the warps below (whist), and in the rounds of 1024 runs before (fill)
     for (int base = 0; base < n_runs; base += 1024) {
         const int r = base + tid;
         int key = 0, w = 0;
         if (r < n_runs && run_pos[r] == -2) {
             key = run_slot[r];
-            w = run_len[r];
+            w = run_tok[r + 1] - run_tok[r];
         }
-        for (int i = tid; i < 32 * S1; i += 1024) whist[i] = 0;
-        __syncthreads();
+        if (base > 0) {
+            for (int i = tid; i < 32 * S1; i += 1024) whist[i] = 0;
+            __syncthreads();
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, key);
+        const unsigned below = peers & ((1u << lane) - 1u);
         int sum = 0;
-        bool last = true;
+        if (__all_sync(0xffffffffu, w <= 1)) {
+            sum = key != 0 ? __popc(below) : 0;
+        } else {
 #pragma unroll 8
-        for (int j = 0; j < 32; j++) {
-            const int wj = __shfl_sync(0xffffffffu, w, j);
-            const int kj = __shfl_sync(0xffffffffu, key, j);
-            if (kj == key) {
-                if (j < lane) sum += wj;
-                if (j > lane) last = false;
+            for (int j = 0; j < 32; j++) {
+                const int wj = __shfl_sync(0xffffffffu, w, j);
+                if ((below >> j) & 1u) sum += wj;
             }
         }
-        if (key != 0 && last) whist[warp * S1 + key] = sum + w;
+        if (key != 0 && (peers >> lane) == 1u) whist[warp * S1 + key] = sum + w;  // the slot's last lane of the warp
         __syncthreads();
         if (key != 0) {
             int pre = 0;
             for (int q = 0; q < warp; q++) pre += whist[q * S1 + key];
             run_pos[r] = seg_base[key] + fill[key] + pre + sum;
         }
-        __syncthreads();
-        for (int s = tid; s < S1; s += 1024) {
-            int tot = 0;
-            for (int q = 0; q < 32; q++) tot += whist[q * S1 + s];
-            fill[s] += tot;
+        if (base + 1024 < n_runs) {
+            __syncthreads();
+            for (int s = tid; s < S1; s += 1024) {
+                int tot = 0;
+                for (int q = 0; q < 32; q++) tot += whist[q * S1 + s];
+                fill[s] += tot;
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 
-    // perm, and the same token rows inside the work items
+    // perm, and the same token rows inside the work items (each thread reads back the positions it wrote)
     int* perm = segs + lay.perm();
     int* work = segs + lay.work();
     for (int r = tid; r < n_runs; r += 1024) {
         const int pos = run_pos[r];
         if (pos < 0) continue;
-        const int start = run_start[r], len = run_len[r], slot = run_slot[r];
+        const int start = run_start[r], len = run_tok[r + 1] - run_tok[r], slot = run_slot[r];
         const int rel0 = pos - seg_base[slot], w0 = cnt[slot];
         for (int k = 0; k < len; k++) {
-            perm[pos + k] = start + k;
+            if (first) perm[pos + k] = start + k;
             const int rel = rel0 + k;
             work[PLORA_WORK_WORDS * (w0 + rel / PLORA_WORK_TOKENS) + 4 + rel % PLORA_WORK_TOKENS] = start + k;
         }
     }
     const int any_bad = __syncthreads_or(bad);
-    if (any_bad && tid == 0) atomicMax(status, PLORA_ERR_ARG);
-    if (tid == 0) {
+    if (first && tid == 0) {
+        if (any_bad) atomicMax(status, PLORA_ERR_ARG);
         segs[SEG_N_ACT] = n_act;
         segs[SEG_N_WORK] = n_work;
         segs[SEG_N_MMA] = n_mma;
@@ -346,12 +394,13 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     // launch records (the barrier above made the work items, written by other threads of this block, visible)
     if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
-        for (int i = tid; i < n_sites * end; i += 1024) {
-            const int site = i / end, w = i - site * end;
+        const int mine = ((int)blockIdx.x < n_sites) ? (n_sites - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+        for (int i = tid; i < mine * end; i += 1024) {
+            const int q = i / end, w = i - q * end, site = (int)blockIdx.x + q * (int)gridDim.x;
             uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
             const int cols = site_cols[2 * site];
             if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
-            else write_record(o, segs, lay, tables + (size_t)site * (size_t)(lay.max_slots + 1), w, cols, site_cols[2 * site + 1]);
+            else write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, site_cols[2 * site + 1]);
         }
     }
 }
@@ -366,7 +415,9 @@ __global__ void __launch_bounds__(128) plora_shrink_gather_kernel(const bf16* __
                                                                    const PloraRec* __restrict__ recs, int rec_cap,
                                                                    float* __restrict__ S, size_t s_stride, int lds,
                                                                    int kchunk, int rps, int rt_max, int early, int early_x,
-                                                                   int* __restrict__ status PLORA_BOUNDS_PARAM) {
+                                                                   int late, int* __restrict__ status PLORA_BOUNDS_PARAM) {
+    // late != 0: the kernel before is the step's grouping, which writes the records: nothing is read, and no dependent
+    // released, before the dependency wait. (The launch itself then overlaps the grouping.)
     // early != 0: dependents are released at kernel start (every store of the path comes after a wait).
     // early_x != 0: the caller vouches that x is older than every kernel still in flight, so x is fetched and
     // the partial sums computed before the dependency wait; only the stores into S (which the expand before may
@@ -375,13 +426,18 @@ __global__ void __launch_bounds__(128) plora_shrink_gather_kernel(const bf16* __
     __shared__ __align__(8) uint64_t bars[2];
     __shared__ PloraRec srec;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (early) pdl_trigger();
+    if (early && !late) pdl_trigger();
     if (threadIdx.x == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
         mbar_fence_init();
     }
     bool waited = false;
+    if (late) {
+        pdl_wait();
+        pdl_trigger();
+        waited = true;
+    }
     uint32_t phase = 0;
     const int split = blockIdx.x / rt_max, rt = blockIdx.x - split * rt_max;
     const int row0 = rt * rps;
@@ -666,6 +722,24 @@ __global__ void __launch_bounds__(256 / NH, 4 * NH) plora_expand_gather_kernel(c
 
 // ---------------------------------------------------------------------------------------------
 
+namespace {
+template <typename... Params, typename... Args>
+cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
+                       Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+}  // namespace
+
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st) {
     plora_meta_tiles_kernel<<<1, 1024, 0, st>>>(cu, seq_slot, n_seqs, tiles, cap_tiles, status);
@@ -673,7 +747,7 @@ cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, 
 }
 
 size_t plora_meta_group_smem(const SegLayout& lay) {
-    return (size_t)(4 * lay.cap_tiles + 3 * (lay.max_slots + 1) + 32 * (lay.max_slots + 1)) * sizeof(int);
+    return (size_t)(4 * lay.cap_tiles + 1 + 3 * (lay.max_slots + 1) + 32 * (lay.max_slots + 1)) * sizeof(int);
 }
 
 // One-time function attributes (dynamic shared memory above 48 KB). Called from plora_create, never from
@@ -703,29 +777,13 @@ cudaError_t plora_kernels_init(const SegLayout& lay) {
 }
 
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, cudaStream_t st) {
-    plora_meta_group_kernel<<<1, 1024, plora_meta_group_smem(lay), st>>>(tiles, segs, lay, status, tables, site_cols, n_sites, recs,
-                                                                         rec_cap);
-    return cudaGetLastError();
+                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, bool pdl, cudaStream_t st) {
+    // a block per layer, up to 64: past that a block has more than one layer's records to write, and every further
+    // block repeats the grouping
+    const int blocks = recs == nullptr ? 1 : n_sites < 64 ? n_sites : 64;
+    return launch_pdl(plora_meta_group_kernel, dim3((unsigned)blocks), dim3(1024), plora_meta_group_smem(lay), st, pdl, tiles, segs, lay,
+                      status, tables, site_cols, n_sites, recs, rec_cap);
 }
-
-namespace {
-template <typename... Params, typename... Args>
-cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
-                       Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
-}
-}  // namespace
 
 #define PLORA_GRID_Z_CAP 64  // blocks along the work-item axis; more work items are walked in a loop
 
@@ -738,14 +796,15 @@ int plora_shrink_rps(int kchunk) {
 
 cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, float* S,
                                 size_t s_stride_elems, int lds, int kchunk, int nsplit, int work_cap, int max_rank_total,
-                                const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, cudaStream_t st) {
+                                const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, bool late,
+                                cudaStream_t st) {
     (void)bnd;
     const int rps = plora_shrink_rps(kchunk);
     const int rt_max = (max_rank_total + rps - 1) / rps;
     dim3 grid((unsigned)(nsplit * rt_max), 1, (unsigned)(work_cap < PLORA_GRID_Z_CAP ? work_cap : PLORA_GRID_Z_CAP));
     const size_t smem = (size_t)(rps + PLORA_WORK_TOKENS) * (size_t)kchunk * 2;
     return launch_pdl(plora_shrink_gather_kernel, grid, dim3(128), smem, st, pdl, reinterpret_cast<const bf16*>(x), ldx,
-                      K, recs, rec_cap, S, s_stride_elems, lds, kchunk, rps, rt_max, early ? 1 : 0, early_x ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
+                      K, recs, rec_cap, S, s_stride_elems, lds, kchunk, rps, rt_max, early ? 1 : 0, early_x ? 1 : 0, pdl && late ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
 }
 
 // output columns per block (two per thread): 512 for wide layers so the grid stays near one wave, 256

@@ -176,7 +176,10 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
     // mode: bit 0 = the caller vouched for x; bits 1-3 = when the next kernel of the stream is released (0: at
     // once, 1: after the shrink, 2: after the exchange); bit 4 = ask L2 for the next layer's slabs too
     const int early_x = mode & 1, release_at = (mode >> 1) & 7;  // (3, 4: after the wait, after A and x landed)
-    bool triggered = release_at == 0;
+    // bit 5 = the kernel before is the step's grouping, which writes the records: nothing is read, and nothing
+    // released, before the dependency wait (the launch itself overlaps the grouping)
+    const bool late = (mode & 32) != 0;
+    bool triggered = release_at == 0 && !late;
     if (triggered) pdl_trigger();
     if (tid == 0) {
         mbar_init(&bars[0], 1);
@@ -186,7 +189,15 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
         mbar_fence_init();
     }
     cluster_arrive_relaxed();  // the barriers exist (published by the init fence); met before the first remote arrival
-    bool met = false, waited = false;
+    bool met = false, waited = false, hints = true;
+    if (late) {
+        pdl_wait();
+        waited = true;
+        if (release_at == 0) {
+            pdl_trigger();
+            triggered = true;
+        }
+    }
     uint32_t ph_ax = 0, ph_b = 0, ph_s = 0;  // barrier phases (each flips only when its barrier was used)
     bool alive = true;                       // false once a bounded wait ran out: keep meeting the cluster, do no more work
     const int k0 = (int)crank * sh.kchunk;
@@ -264,9 +275,9 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                                                      : Xs + (size_t)(r - R) * sh.kb_pad) + kbytes) = make_uint4(0u, 0u, 0u, 0u);
             __syncthreads();  // the share is known to every warp
             // ---- hints: the x and y lines this block will touch, and the next layer's slabs of this work item
-            if (!waited && warp >= 2) {
+            if (hints && warp >= 2) {
                 const int t1 = tid - 64, n1 = SITE_THREADS - 64;
-                if (klen > 0 && !early_x) {
+                if (klen > 0 && !early_x && !waited) {
                     const int lines = (int)((kbytes + 127) / 128);
                     for (int i = t1; i < cn * lines; i += n1) {
                         const int t = i / lines, l = i - t * lines;
@@ -304,6 +315,7 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                     }
                 }
             }
+            hints = false;
             if (!waited && !early_x) {
                 pdl_wait();
                 waited = true;
