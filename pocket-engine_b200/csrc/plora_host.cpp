@@ -331,12 +331,12 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             check("alloc pool", cudaMalloc((void**)&h->pool, h->slot_bytes * (size_t)max_slots));
             check("alloc tables", cudaMalloc((void**)&h->tables, h->table_bytes));
             check("pinned tables", cudaMallocHost((void**)&h->host_tables, h->table_bytes));
-            const size_t amap_bytes = sizeof(PloraTmap) * h->sites.size() * (size_t)(max_slots + 1);
-            check("alloc slab tensor maps", cudaMalloc((void**)&h->amaps, amap_bytes));
-            check("pinned slab tensor maps", cudaMallocHost((void**)&h->host_amaps, amap_bytes));
+            const size_t smap_bytes = sizeof(PloraSlabMaps) * h->sites.size() * (size_t)(max_slots + 1);
+            check("alloc slab tensor maps", cudaMalloc((void**)&h->smaps, smap_bytes));
+            check("pinned slab tensor maps", cudaMallocHost((void**)&h->host_smaps, smap_bytes));
             if (rc == PLORA_OK) {
-                memset(h->host_amaps, 0, amap_bytes);
-                check("zero slab tensor maps", cudaMemset(h->amaps, 0, amap_bytes));
+                memset(h->host_smaps, 0, smap_bytes);
+                check("zero slab tensor maps", cudaMemset(h->smaps, 0, smap_bytes));
             }
             check("alloc S", cudaMalloc((void**)&h->s, h->s_bytes));
             check("alloc meta", cudaMalloc((void**)&h->meta, meta_words * 4));
@@ -404,8 +404,8 @@ void plora_destroy(plora_t* h) {
         if (h->pool) cudaFree(h->pool);
         if (h->tables) cudaFree(h->tables);
         if (h->host_tables) cudaFreeHost(h->host_tables);
-        if (h->amaps) cudaFree(h->amaps);
-        if (h->host_amaps) cudaFreeHost(h->host_amaps);
+        if (h->smaps) cudaFree(h->smaps);
+        if (h->host_smaps) cudaFreeHost(h->host_smaps);
         if (h->s) cudaFree(h->s);
         if (h->meta) cudaFree(h->meta);
         if (h->recs) cudaFree(h->recs);
@@ -703,7 +703,7 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
         const plora_desc d = h->host_tables[at] = desc_for(h->sites[si], a->sites[si], (uint64_t)(uintptr_t)base);
         if (h->mma_ok && d.rank > 0) {
             CU(h, "encode slab tensor map",
-               plora_mma_encode_slab(&h->host_amaps[at], (const void*)(uintptr_t)d.a, h->sites[si].cols, d.rank));
+               plora_mma_encode_slab(&h->host_smaps[at], d, h->sites[si].cols));
             maps = true;
         }
     }
@@ -712,8 +712,8 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
                          sizeof(plora_desc), n, cudaMemcpyHostToDevice, st));
     if (maps)
         CU(h, "upload slab tensor maps",
-           cudaMemcpy2DAsync(h->amaps + slot, stride * sizeof(PloraTmap), h->host_amaps + slot, stride * sizeof(PloraTmap),
-                             sizeof(PloraTmap), n, cudaMemcpyHostToDevice, st));
+           cudaMemcpy2DAsync(h->smaps + slot, stride * sizeof(PloraSlabMaps), h->host_smaps + slot, stride * sizeof(PloraSlabMaps),
+                             sizeof(PloraSlabMaps), n, cudaMemcpyHostToDevice, st));
     return PLORA_OK;
 }
 
@@ -952,7 +952,7 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
         CUK(h, "shrink (tile path)",
            plora_launch_shrink_mma((const void*)(uintptr_t)x, rows, site.cols, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
-                                   h->amaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
+                                   h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
                                    tile_split(h, rows), h->status, h->pdl, h->tile_late && (!early || early_x),
                                    as_stream(stream)));
@@ -1006,13 +1006,14 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
         CUK(h, "shrink (tile path)",
            plora_launch_shrink_mma((const void*)(uintptr_t)x, rows, site.cols, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
-                                   h->amaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
+                                   h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
                                    tile_split(h, rows), h->status, h->pdl, false, as_stream(stream)));
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
                                    tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
-                                   (const plora_desc*)(uintptr_t)hook->table, (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
+                                   (const plora_desc*)(uintptr_t)hook->table,
+                                   h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
                                    h->pdl, as_stream(stream)));
     }
@@ -1058,7 +1059,8 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
                                    reduced ? 1 : tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
-                                   (const plora_desc*)(uintptr_t)hook->table, (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
+                                   (const plora_desc*)(uintptr_t)hook->table,
+                                   h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
                                    h->pdl, as_stream(stream)));
     return PLORA_OK;

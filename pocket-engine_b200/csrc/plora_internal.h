@@ -80,6 +80,10 @@ struct PloraBounds {
 struct alignas(64) PloraTmap {  // a CUtensorMap, opaque to the host registry
     unsigned char b[128];
 };
+// the tile path's views of one slot's slabs for one layer: the stacked A, and every targeted part's B
+struct PloraSlabMaps {
+    PloraTmap a, b[PLORA_MAX_PARTS];
+};
 
 struct SiteInfo {
     int layer = 0, cols = 0;
@@ -153,8 +157,8 @@ struct plora {
     plora_desc* tables = nullptr;       // device
     plora_desc* host_tables = nullptr;  // pinned mirror
     size_t table_bytes = 0;
-    PloraTmap* amaps = nullptr;       // device: per (layer, slot) tensor map of the stacked A (tile path)
-    PloraTmap* host_amaps = nullptr;  // pinned mirror
+    PloraSlabMaps* smaps = nullptr;       // device: per (layer, slot) tensor maps of the slabs (tile path)
+    PloraSlabMaps* host_smaps = nullptr;  // pinned mirror
     std::shared_ptr<PinnedPool> pinned = std::make_shared<PinnedPool>();
     std::unordered_map<uint32_t, plora_adapter*> adapters;
     std::map<std::string, uint32_t> names;
@@ -283,14 +287,14 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
                                     int K, const int32_t* segs, SegLayout lay, const plora_desc* table, int n_parts,
                                     const int* part_off, const int* part_rows, const float* S, int lds, void* y, int ldy,
                                     int f32_out, int* status, bool pdl, cudaStream_t stream);
-cudaError_t plora_mma_encode_slab(void* out128, const void* a, int K, int R);
+cudaError_t plora_mma_encode_slab(PloraSlabMaps* out, const plora_desc& d, int K);
 cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, const int32_t* segs, SegLayout lay,
-                                    const plora_desc* table, const PloraTmap* amaps, float* S, size_t s_stride_elems, int lds,
+                                    const plora_desc* table, const PloraSlabMaps* smaps, float* S, size_t s_stride_elems, int lds,
                                     int max_rank_total, int tile_cap, int tile_split, int* status, bool pdl, bool late,
                                     cudaStream_t st);
 cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int lds, int K, int tile_split,
-                                    const int32_t* segs, SegLayout lay, const plora_desc* table, void* y, int ldy,
-                                    int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
+                                    const int32_t* segs, SegLayout lay, const plora_desc* table, const PloraSlabMaps* smaps, void* y,
+                                    int ldy, int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
                                     int max_rows, int tile_cap, int* status, bool pdl, cudaStream_t st);
 // early: dependents are released at kernel start and slabs are requested ahead of the dependency wait (used by
 // plora_apply, whose kernels follow one another); early_x: x too may be read ahead of the wait; late: the kernel before

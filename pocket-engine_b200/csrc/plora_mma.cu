@@ -13,6 +13,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "plora_internal.h"
 #include "plora_device.cuh"
 #include "plora_tc.cuh"
@@ -22,6 +24,21 @@ typedef __nv_bfloat16 bf16;
 namespace {
 
 // ---- tcgen05 ----
+
+// D (tensor memory) (+)= A (tensor memory: lane = row, two bf16 per column) . B (shared), f32 accumulate
+__device__ __forceinline__ void umma_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+// 4 consecutive columns of this warp's 32 lanes; to be followed by tmem_st_wait
+__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 // 8 consecutive columns, without the wait (several loads, then one tmem_ld_wait)
 __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, float* v) {
@@ -83,7 +100,7 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
 #define SHR_MAX_STAGES 8
 
 __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                                const CUtensorMap* __restrict__ amaps, int K,
+                                                                const PloraSlabMaps* __restrict__ smaps, int K,
                                                                 const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table,
                                                                 float* __restrict__ S, size_t s_stride, int lds,
@@ -112,7 +129,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     const int s_eff = min(ksplit, n_chunks);
     if ((int)blockIdx.x >= s_eff) return pdl_exit_idle();
     const int n_acc = n_chunks / s_eff;  // accumulators (chunks) of this block
-    const CUtensorMap* amap = amaps + slot;
+    const CUtensorMap* amap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].a);
     const int tid = threadIdx.x, warp = tid >> 5;
     // 1024-byte aligned stage ring: [x tile 16 KB][slab rows R x 128 B]
     unsigned char* ring = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);
@@ -471,40 +488,56 @@ __global__ void __launch_bounds__(128) plora_expand_mma_kernel(const float* __re
 // ------------------------------------------------------------------------------------------------------
 // The same expand with y moved by tensor copies, for outputs whose base, row pitch and part offsets are
 // 16-byte aligned (every model width in practice; the kernel above stays for the rest). Eight adding warps and
-// one more (two blocks per SM; sixteen and one, one block per SM, where the operands of a high maximum rank leave
-// no room for two: measured slower at equal shared memory, 509 against 399 us on the widest prefill layer). The
-// last warp copies the blocks' rows of B and issues the MMAs, up to two column blocks ahead (mbarriers tell it when S is
-// staged and when an accumulator has been read); the other eight never meet at a block-wide barrier inside the
-// loop. Each of them owns the 32 token rows tensor memory gives it (two warps per 32 rows, taking alternate
-// slots of columns) and a private ring of 4 KB slots; a slot holds 32 rows x 128 bytes of y
-// (64 bf16 or 32 f32 columns, 128-byte swizzle). Lane 0 keeps the ring full of loads; a landed slot gets the
-// accumulator columns added in shared memory (thread = row: with the swizzle, eight rows cover all banks) and
-// goes back with a tensor store, whose completion frees the slot for the next load. So the read-modify-write
-// of y, which is most of the bytes of a prefill step, is asynchronous on both sides and many slots deep. The
-// accumulator is double-buffered in tensor memory: the MMAs of the next column block run during this block's
-// additions. Tensor maps are per part and end at the part's last column, so a box at the edge is clipped
+// one more, two blocks per SM. The last warp copies the blocks' rows of B and issues the MMAs of 64 output columns at a
+// time, up to two column blocks ahead (mbarriers tell it when S is staged and when an accumulator has been read); the
+// other eight never meet at a block-wide barrier inside the loop. Each of them owns the 32 token rows tensor memory
+// gives it (two warps per 32 rows, taking alternate slots of columns) and a private ring of 4 KB slots; a slot holds
+// 32 rows x 128 bytes of y (64 bf16 or 32 f32 columns, 128-byte swizzle). Lane 0 keeps the ring full of loads; a landed
+// slot gets the accumulator columns added in shared memory (thread = row: with the swizzle, eight rows cover all banks)
+// and goes back with a tensor store, whose completion frees the slot for the next load. So the read-modify-write
+// of y, which is most of the bytes of a prefill step, is asynchronous on both sides and several slots deep.
+//
+// S is the A operand in tensor memory (written there row by row by the threads that split it): in shared memory it left
+// room for one slot per warp at a rank of 64. B arrives by tensor copies of its own: copied by the lanes of the MMA
+// warp, 16 bytes each, it bounded the kernel (435 us for the widest prefill layer, 304 without those copies).
+// The accumulator is double-buffered in tensor memory and given back as soon as it is in registers: the MMAs of the next
+// column block run during this block's additions. Tensor memory: 2 x 64 accumulator columns, then S high and low
+// (r / 2 columns each). Tensor maps are per part and end at the part's last column, so a box at the edge is clipped
 // instead of touching the next part's columns. A warp whose 32 rows are not all inside the tile (the tail of
 // a run) loads the same way but writes its live rows with plain stores: the other rows belong to other tokens.
 struct ExpandYMaps {
     CUtensorMap m[PLORA_MAX_PARTS];
 };
-#define EXP_RING_MAX 8
+#ifndef EXP_RING_MAX
+#define EXP_RING_MAX 3
+#endif
 #define EXP_SLOT_BYTES 4096
+#define EXP_BN 64        // output columns per MMA
+#define EXP_TMEM_A 128   // first tensor-memory column of S
+#define EXP_WARPS 8      // adding warps
+#define EXP_B_STAGES 4
+// ranks per box of B: a swizzle span of 128, 64 or 32 bytes, whichever divides a row
+__host__ __device__ inline int exp_b_width(int r) { return r % 64 == 0 ? 64 : r % 32 == 0 ? 32 : 16; }
+#define EXP_TMA_SMEM (113 * 1024)  // two blocks per SM: half of 228 KB, less the 1 KB the system keeps per block
+struct ExpandBars {
+    uint64_t done[2], acc_free[2], a_full, b_full[EXP_B_STAGES], ybar[EXP_WARPS][EXP_RING_MAX];
+    uint32_t tmem_slot;
+};
 
 __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 
-template <bool F32, int WPQ>  // WPQ: warps per 32 rows (2 or 4)
-__global__ void __launch_bounds__(32 * (4 * WPQ + 1)) plora_expand_tma_kernel(const float* __restrict__ S, size_t s_stride, int lds, int K,
+template <bool F32>
+__global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kernel(const float* __restrict__ S, size_t s_stride, int lds, int K,
                                                                 int ksplit, const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table,
+                                                                const PloraSlabMaps* __restrict__ smaps,
                                                                 const __grid_constant__ ExpandYMaps ymaps, void* Y, int ldy,
-                                                                int nb_per_cta, int op_bytes, int nst,
+                                                                int nb_per_cta, int b_bytes, int nbs, int nst,
                                                                 int* __restrict__ status) {
-    extern __shared__ unsigned char dsm_raw[];
-    __shared__ __align__(8) uint64_t done[2], acc_free[2], a_full, ybar[4 * WPQ][EXP_RING_MAX];
-    __shared__ uint32_t tmem_slot;
-    constexpr int CW = F32 ? 32 : 64;  // y columns per slot
-    constexpr int CH = 128 / CW;       // slots per block of 128 columns
+    extern __shared__ __align__(1024) unsigned char dsm1k[];  // (no static shared memory: the ring starts 1024-byte aligned)
+    constexpr int CW = F32 ? 32 : 64;     // y columns per slot
+    constexpr int CH = EXP_BN / CW;       // slots per column block
+    constexpr int NW = EXP_WARPS, WPQ = NW / 4;
     const int tile = blockIdx.z;
     const int n_mma = segs[SEG_N_MMA];
     const int* mt = segs + lay.mma() + 3 * tile;
@@ -515,92 +548,90 @@ __global__ void __launch_bounds__(32 * (4 * WPQ + 1)) plora_expand_tma_kernel(co
     if (r == 0) return pdl_exit_idle();
     const int rows = d.rows[p];
     const int cb0 = blockIdx.x * nb_per_cta;
-    if (cb0 * 128 >= rows) return pdl_exit_idle();
-    const int nblk = min(nb_per_cta, (rows - cb0 * 128 + 127) / 128);
-    const int nchunks = min(nblk * CH, (rows - cb0 * 128 + CW - 1) / CW);  // slots this block fills, in column order
+    if (cb0 * EXP_BN >= rows) return pdl_exit_idle();
+    const int nblk = min(nb_per_cta, (rows - cb0 * EXP_BN + EXP_BN - 1) / EXP_BN);
+    const int nchunks = min(nblk * CH, (rows - cb0 * EXP_BN + CW - 1) / CW);  // slots this block fills, in column order
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    unsigned char* dsm = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);
-    unsigned char* ring = dsm + (size_t)warp * nst * EXP_SLOT_BYTES;  // this warp's slots
-    constexpr int NW = 4 * WPQ;  // warps that add; warp NW copies B and issues the MMAs
-    unsigned char* ops = dsm + (size_t)NW * nst * EXP_SLOT_BYTES;
-    // Eight warps: warps w and w + 4 read the same 32 lanes of tensor memory (rows 32 (w % 4) ...) and take
-    // the even and the odd slots of every column block.
+    unsigned char* ring = dsm1k + (size_t)warp * nst * EXP_SLOT_BYTES;  // this warp's slots
+    unsigned char* ops = dsm1k + (size_t)NW * nst * EXP_SLOT_BYTES;
+    ExpandBars& bars = *reinterpret_cast<ExpandBars*>(ops + nbs * (size_t)b_bytes);
+    // warps w and w + 4 read the same 32 lanes of tensor memory (rows 32 (w % 4) ...) and take the even and the odd
+    // slots of the block's columns
     const int wq = warp & 3, wh = warp >> 2;
-    unsigned char* Ahi = ops;
-    unsigned char* Alo = ops + op_bytes;
-    unsigned char* Bs[2] = {ops + 2 * (size_t)op_bytes, ops + 3 * (size_t)op_bytes};
-    const bf16* B = reinterpret_cast<const bf16*>(d.b[p]);
-    const uint32_t sbo = (uint32_t)r * 16u;  // 8-row group stride
     const int P = r >> 3;
     const CUtensorMap* ymap = &ymaps.m[p];
-
-    // warp 8 alone copies the blocks' rows of B (four rows of the block per lane) and issues the MMAs
-    auto load_b = [&](int cb, unsigned char* dst) {
-        for (int n = lane; n < 128; n += 32) {  // row of B = output column of the block
-            const bool valid = cb * 128 + n < rows;
-            const bf16* src = B + (size_t)(valid ? cb * 128 + n : 0) * r;
-            unsigned char* drow = dst + (size_t)(n >> 3) * sbo + (n & 7) * 16;
-            for (int j = 0; j < P; j++) cp_async16(drow + j * 128, src + j * 8, valid);
-        }
+    const CUtensorMap* bmap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].b[p]);
+    // the rows of B of column block nb: r / bw boxes of 64 rows by bw ranks, one after another in stage nb % nbs
+    const int bw = exp_b_width(r);
+    auto load_b = [&](int nb) {
+        const int stg = nb % nbs;
+        mbar_expect_tx(&bars.b_full[stg], (uint32_t)(EXP_BN * r * 2));
+        for (int q = 0; q < r; q += bw)
+            tma_load_2d(ops + (size_t)stg * b_bytes + (size_t)q * EXP_BN * 2, bmap, q, (cb0 + nb) * EXP_BN, &bars.b_full[stg]);
     };
-    // warps that have rows of the tile and a slot in every full column block
-    const int live_warps = (WPQ < CH ? WPQ : CH) * min(4, (len + 31) / 32);
 
     if (tid == 0) {
-        mbar_init(&done[0], 1);
-        mbar_init(&done[1], 1);
-        mbar_init(&acc_free[0], live_warps);
-        mbar_init(&acc_free[1], live_warps);
-        mbar_init(&a_full, 32 * NW);
+        mbar_init(&bars.done[0], 1);
+        mbar_init(&bars.done[1], 1);
+        // the warps that have rows of the tile and a slot in the accumulator's column blocks: the ones of one parity
+        // where a column block is one slot, all where it is two
+        const int live_warps = CH * min(4, (len + 31) / 32);
+        mbar_init(&bars.acc_free[0], live_warps);
+        mbar_init(&bars.acc_free[1], live_warps);
+        mbar_init(&bars.a_full, 32 * NW);
+        for (int i = 0; i < nbs; i++) mbar_init(&bars.b_full[i], 1);
         for (int w = 0; w < NW; w++)
-            for (int i = 0; i < nst; i++) mbar_init(&ybar[w][i], 1);
+            for (int i = 0; i < nst; i++) mbar_init(&bars.ybar[w][i], 1);
         mbar_fence_init();
     }
-    if (warp == NW) {
-        tmem_alloc(&tmem_slot, 256);
-        load_b(cb0, Bs[0]);  // B is a slab: it may be fetched before the kernels ahead have finished
-        cp_async_commit();
-    }
+    if (warp == NW) tmem_alloc(&bars.tmem_slot, 256);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = bars.tmem_slot;
+    const bool leader = warp == NW && elect_one();
+    if (leader) {
+        tmap_acquire(bmap);
+        for (int nb = 0; nb < nbs - 2 && nb < nblk; nb++) load_b(nb);  // a slab: it may be fetched before the kernels ahead have finished
+    }
     pdl_wait();
     pdl_trigger();
 
     if (warp == NW) {
-        // ---- B copies and MMAs, running up to two column blocks ahead of the additions
-        const uint32_t idesc = umma_idesc_bf16(MMA_M, 128);
-        bool ok = mbar_wait_long(&a_full, 0, status);  // S staged by the other warps
-        for (int nb = 0; ok && nb < nblk; nb++) {
-            cp_async_wait<0>();  // this warp's copies of block nb's rows of B
-            fence_async_smem();
-            __syncwarp();
-            // the accumulator this block goes to was last read for block nb - 2
-            if (nb >= 2) ok = mbar_wait_long(&acc_free[nb & 1], ((nb >> 1) - 1) & 1, status);
-            if (!ok) break;
-            if (elect_one()) {
+        // ---- B copies (nbs - 2 column blocks ahead) and MMAs (up to two column blocks ahead of the additions)
+        if (leader) {
+            const uint32_t idesc = umma_idesc_bf16(MMA_M, EXP_BN);
+            const uint32_t a_hi = tmem + EXP_TMEM_A, a_lo = a_hi + (uint32_t)(r >> 1);
+            const uint32_t sw = bw == 64 ? 2u : bw == 32 ? 4u : 6u;
+            const uint64_t b0 = umma_desc(smem_u32(ops), 16, (uint32_t)bw * 16u, sw);  // eight rows of a box are bw * 16 bytes
+            bool ok = mbar_wait_long(&bars.a_full, 0, status);  // S staged by the other warps
+            int stg = 0;
+            uint32_t bpar = 0;
+            for (int nb = 0; ok && nb < nblk; nb++) {
+                // the accumulator this block goes to was last read for block nb - 2, whose stage of B is therefore free too
+                if (nb >= 2) ok = mbar_wait_long(&bars.acc_free[nb & 1], ((nb >> 1) - 1) & 1, status);
+                if (!ok) break;
+                if (nb + nbs - 2 < nblk) load_b(nb + nbs - 2);
+                ok = mbar_wait_long(&bars.b_full[stg], bpar, status);
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_hi = smem_u32(Ahi), a_lo = smem_u32(Alo), b = smem_u32(Bs[nb & 1]);
-                const uint32_t acc = tmem + (uint32_t)(nb & 1) * 128u;
-                for (int kk = 0; kk < r / 16; kk++)
-                    umma<1>(acc, umma_desc(a_hi + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc, kk != 0);
-                for (int kk = 0; kk < r / 16; kk++)
-                    umma<1>(acc, umma_desc(a_lo + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc, 1);
-                umma_commit(&done[nb & 1]);
+                const uint64_t bd = b0 + (uint64_t)((uint32_t)stg * (uint32_t)b_bytes >> 4);
+                const uint32_t acc = tmem + (uint32_t)(nb & 1) * EXP_BN;
+                for (int half = 0; half < 2; half++)
+                    for (int k = 0; k < r; k += 16)
+                        umma_ta(acc, (half ? a_lo : a_hi) + (uint32_t)(k >> 1), bd + (uint64_t)((k / bw) * (EXP_BN * bw * 2 / 16) + (k % bw) / 8),
+                                idesc, (half | k) != 0);
+                umma_commit(&bars.done[nb & 1]);
+                if (++stg == nbs) {
+                    stg = 0;
+                    bpar ^= 1;
+                }
             }
-            __syncwarp();
-            if (nb + 1 < nblk) {
-                // the other B buffer was read by block nb - 1's MMAs
-                if (nb >= 1) ok = mbar_wait_long(&done[(nb - 1) & 1], ((nb - 1) >> 1) & 1, status);
-                if (ok) load_b(cb0 + nb + 1, Bs[(nb + 1) & 1]);
-            }
-            cp_async_commit();
+            // every MMA has completed before the tensor memory goes back
+            if (ok && nblk >= 1) mbar_wait_long(&bars.done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status);
+            if (ok && nblk >= 2) mbar_wait_long(&bars.done[(nblk - 2) & 1], ((nblk - 2) >> 1) & 1, status);
         }
-        // every MMA has completed before the tensor memory goes back
-        if (ok && nblk >= 1) mbar_wait_long(&done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status);
-        if (ok && nblk >= 2) mbar_wait_long(&done[(nblk - 2) & 1], ((nblk - 2) >> 1) & 1, status);
-        cp_async_wait<0>();
+        __syncwarp();
         tc_fence_before();
         __syncthreads();
         tmem_dealloc(tmem, 256);
@@ -610,27 +641,24 @@ __global__ void __launch_bounds__(32 * (4 * WPQ + 1)) plora_expand_tma_kernel(co
     const int wrow0 = wq * 32;
     const bool live = wrow0 < len;            // the warp has rows of the tile
     const bool whole = wrow0 + 32 <= len;     // all its 32 rows are: results go back by tensor store
-    const int ycol0 = d.off[p] + cb0 * 128;   // first y column of this block's range
-    // the warp's i-th slot is slot q of the block's column range
-    auto slot_of = [&](int i) { return wh + WPQ * i; };
-    int my_n = 0;  // slots this warp handles
-    while (slot_of(my_n) < nchunks) my_n++;
-    auto load_y = [&](int i) {                // lane 0 only
-        uint64_t* bar = &ybar[warp][i % nst];
+    const int ycol0 = d.off[p] + cb0 * EXP_BN;  // first y column of this block's range
+    const uint32_t lane_base = tmem + ((uint32_t)wrow0 << 16);
+    // the warp's i-th slot is slot wh + 2 i of the block's column range
+    const int my_n = (nchunks - wh + WPQ - 1) / WPQ;
+    auto load_y = [&](int i, int at) {        // lane 0 only; `at` = i % nst
+        uint64_t* bar = &bars.ybar[warp][at];
         mbar_expect_tx(bar, EXP_SLOT_BYTES);
-        tma_load_2d(ring + (size_t)(i % nst) * EXP_SLOT_BYTES, ymap, ycol0 + slot_of(i) * CW, start + wrow0, bar);
+        tma_load_2d(ring + (size_t)at * EXP_SLOT_BYTES, ymap, ycol0 + (wh + WPQ * i) * CW, start + wrow0, bar);
     };
     if (live && lane == 0)
-        for (int i = 0; i < nst && i < my_n; i++) load_y(i);
+        for (int i = 0; i < nst && i < my_n; i++) load_y(i, i);
 
-    // this thread's token row of S, split into a bf16 high part and the bf16 of what is left
+    // this thread's token row of S, split into a bf16 high part and the bf16 of what is left, into its lane of tensor memory
     {
         const int row = tid & 127;
         const bool valid = row < len;
         const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
         const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
-        unsigned char* ahi = Ahi + (size_t)(row >> 3) * sbo + (row & 7) * 16;
-        unsigned char* alo = Alo + (size_t)(row >> 3) * sbo + (row & 7) * 16;
         for (int j = tid >> 7; j < P; j += WPQ) {
             float f[8];
             if (valid && s_eff > 1) {
@@ -664,111 +692,107 @@ __global__ void __launch_bounds__(32 * (4 * WPQ + 1)) plora_expand_tma_kernel(co
                 hi[e] = *reinterpret_cast<const uint32_t*>(&h);
                 lo[e] = *reinterpret_cast<const uint32_t*>(&l);
             }
-            *reinterpret_cast<uint4*>(ahi + j * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-            *reinterpret_cast<uint4*>(alo + j * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            __syncwarp();
+            tmem_st4(lane_base + EXP_TMEM_A + 4 * j, hi);
+            tmem_st4(lane_base + EXP_TMEM_A + (r >> 1) + 4 * j, lo);
         }
+        tmem_st_wait();
+        tc_fence_before();
+        mbar_arrive(&bars.a_full);  // S is staged
     }
-    // S is staged: tell the MMA warp (the writes above, made visible to the tensor cores first)
-    fence_async_smem();
-    mbar_arrive(&a_full);
 
     bool ok = true;
+    int at = 0;             // i % nst
+    uint32_t ypar = 0;      // (i / nst) & 1
 #pragma unroll 1
     for (int i = 0; ok && live && i < my_n; i++) {  // the warp's slots, in column order
-        const int q = slot_of(i), nb = q / CH, ch = q % CH;
-        if (ch < WPQ) {  // the warp's first slot of column block nb: its MMAs must be complete
-            ok = mbar_wait_long(&done[nb & 1], (nb >> 1) & 1, status);
-            if (!ok) break;
-            tc_fence_after();
+        const int q = wh + WPQ * i, nb = q / CH, ch = q % CH;
+        ok = mbar_wait_long(&bars.done[nb & 1], (nb >> 1) & 1, status);
+        if (!ok) break;
+        tc_fence_after();
+        uint32_t v[CW];
+#pragma unroll
+        for (int h = 0; h < CW / 32; h++) tmem_ld32_nowait(lane_base + (uint32_t)(nb & 1) * EXP_BN + ch * CW + h * 32, v + 32 * h);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.acc_free[nb & 1]);
+        unsigned char* sl = ring + (size_t)at * EXP_SLOT_BYTES;
+        if (!mbar_wait(&bars.ybar[warp][at], ypar, status)) {
+            ok = false;
+            break;
         }
-        const uint32_t acc = tmem + ((uint32_t)wrow0 << 16) + (uint32_t)(nb & 1) * 128u;
-        {
-            unsigned char* sl = ring + (size_t)(i % nst) * EXP_SLOT_BYTES;
-            if (!mbar_wait(&ybar[warp][i % nst], (i / nst) & 1, status)) {
-                ok = false;
-                break;
-            }
-            unsigned char* myrow = sl + lane * 128;
-            const int col0 = (cb0 + nb) * 128 + ch * CW;  // first column of the slot within the part
-            const bool mine = wrow0 + lane < len;
-            if (F32) {
-                uint32_t v[32];
-                tmem_ld32(acc + ch * 32, v);
-                float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+        unsigned char* myrow = sl + lane * 128;
+        const int col0 = (cb0 + nb) * EXP_BN + ch * CW;  // first column of the slot within the part
+        const bool mine = wrow0 + lane < len;
+        if (F32) {
+            float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
 #pragma unroll
-                for (int c = 0; c < 8; c++) {
-                    float4* at = reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4));
-                    float4 y = *at;
-                    y.x += __uint_as_float(v[4 * c]), y.y += __uint_as_float(v[4 * c + 1]);
-                    y.z += __uint_as_float(v[4 * c + 2]), y.w += __uint_as_float(v[4 * c + 3]);
-                    if (whole) {
-                        *at = y;
-                    } else if (mine) {
-                        if (col0 + 4 * c + 4 <= rows) {
-                            *reinterpret_cast<float4*>(yrow + 4 * c) = y;
-                        } else {
-                            const float e[4] = {y.x, y.y, y.z, y.w};
-                            for (int i = 0; i < 4; i++)
-                                if (col0 + 4 * c + i < rows) yrow[4 * c + i] = e[i];
-                        }
-                    }
-                }
-            } else {
-                bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    uint32_t v[32];
-                    tmem_ld32(acc + ch * 64 + h * 32, v);
-#pragma unroll
-                    for (int c4 = 0; c4 < 4; c4++) {
-                        const int c = h * 4 + c4;
-                        uint4* at = reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4));
-                        const uint4 raw = *at;
-                        float f[8];
-                        unpack8(raw, f);
-                        uint32_t o[4];
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[8 * c4 + 2 * e]),
-                                                                            f[2 * e + 1] + __uint_as_float(v[8 * c4 + 2 * e + 1]));
-                            o[e] = *reinterpret_cast<const uint32_t*>(&b2);
-                        }
-                        if (whole) {
-                            *at = make_uint4(o[0], o[1], o[2], o[3]);
-                        } else if (mine) {
-                            if (col0 + 8 * c + 8 <= rows) {
-                                *reinterpret_cast<uint4*>(yrow + 8 * c) = make_uint4(o[0], o[1], o[2], o[3]);
-                            } else {
-                                const bf16* e = reinterpret_cast<const bf16*>(o);
-                                for (int i = 0; i < 8; i++)
-                                    if (col0 + 8 * c + i < rows) yrow[8 * c + i] = e[i];
-                            }
-                        }
-                    }
-                }
-            }
-            if (whole) fence_async_smem();  // the additions above, before the tensor store reads them
-            __syncwarp();
-            if (lane == 0) {
+            for (int c = 0; c < 8; c++) {
+                float4* yp = reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4));
+                float4 y = *yp;
+                y.x += __uint_as_float(v[4 * c]), y.y += __uint_as_float(v[4 * c + 1]);
+                y.z += __uint_as_float(v[4 * c + 2]), y.w += __uint_as_float(v[4 * c + 3]);
                 if (whole) {
-                    tma_store_2d(ymap, ycol0 + q * CW, start + wrow0, sl);
-                    bulk_commit();
-                    if (nst == 1) {  // one slot: wait for this store to have read it, then refill it
-                        bulk_wait_read();
-                        if (i + 1 < my_n) load_y(i + 1);
-                    } else {  // the store before this one has read its slot: refill that slot
-                        bulk_wait_read_1();
-                        if (i >= 1 && i - 1 + nst < my_n) load_y(i - 1 + nst);
+                    *yp = y;
+                } else if (mine) {
+                    if (col0 + 4 * c + 4 <= rows) {
+                        *reinterpret_cast<float4*>(yrow + 4 * c) = y;
+                    } else {
+                        const float e[4] = {y.x, y.y, y.z, y.w};
+                        for (int k = 0; k < 4; k++)
+                            if (col0 + 4 * c + k < rows) yrow[4 * c + k] = e[k];
                     }
-                } else if (i + nst < my_n) {
-                    load_y(i + nst);  // plain stores: the slot is free at once
+                }
+            }
+        } else {
+            bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+#pragma unroll
+            for (int c = 0; c < 8; c++) {
+                uint4* yp = reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4));
+                const uint4 raw = *yp;
+                float f[8];
+                unpack8(raw, f);
+                uint32_t o[4];
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[(8 * c + 2 * e) % CW]),
+                                                                    f[2 * e + 1] + __uint_as_float(v[(8 * c + 2 * e + 1) % CW]));
+                    o[e] = *reinterpret_cast<const uint32_t*>(&b2);
+                }
+                if (whole) {
+                    *yp = make_uint4(o[0], o[1], o[2], o[3]);
+                } else if (mine) {
+                    if (col0 + 8 * c + 8 <= rows) {
+                        *reinterpret_cast<uint4*>(yrow + 8 * c) = make_uint4(o[0], o[1], o[2], o[3]);
+                    } else {
+                        const bf16* e = reinterpret_cast<const bf16*>(o);
+                        for (int k = 0; k < 8; k++)
+                            if (col0 + 8 * c + k < rows) yrow[8 * c + k] = e[k];
+                    }
                 }
             }
         }
-        if (ch + WPQ >= CH) {  // the warp's last slot of column block nb: it is done with that accumulator
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_free[nb & 1]);
+        if (whole) fence_async_smem();  // the additions above, before the tensor store reads them
+        __syncwarp();
+        if (lane == 0) {
+            if (whole) {
+                tma_store_2d(ymap, ycol0 + q * CW, start + wrow0, sl);
+                bulk_commit();
+                if (nst == 1) {  // one slot: wait for this store to have read it, then refill it
+                    bulk_wait_read();
+                    if (i + 1 < my_n) load_y(i + 1, 0);
+                } else {  // the store before this one has read its slot: refill that slot
+                    bulk_wait_read_1();
+                    if (i >= 1 && i - 1 + nst < my_n) load_y(i - 1 + nst, at == 0 ? nst - 1 : at - 1);
+                }
+            } else if (i + nst < my_n) {
+                load_y(i + nst, at);  // plain stores: the slot is free at once
+            }
+        }
+        if (++at == nst) {
+            at = 0;
+            ypar ^= 1;
         }
     }
     if (lane == 0) bulk_wait_all();
@@ -799,10 +823,8 @@ cudaError_t plora_mma_init() {
     if (e != cudaSuccess) return e;
     e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_mma_kernel<true>), 172 * 1024);
     if (e != cudaSuccess) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false, 2>), 220 * 1024))) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true, 2>), 220 * 1024))) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false, 4>), 220 * 1024))) return e;
-    return plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true, 4>), 220 * 1024);
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false>), EXP_TMA_SMEM))) return e;
+    return plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true>), EXP_TMA_SMEM);
 }
 
 namespace {
@@ -823,24 +845,32 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
 }
 }  // namespace
 
-// The tensor map of one slot's stacked A for one layer: [R, K] bf16 row-major, boxes of 64 inputs by R rows
-// (R / 2 rows when R is over 256, the limit of a box), 128-byte swizzle.
-cudaError_t plora_mma_encode_slab(void* out128, const void* a, int K, int R) {
+// The tensor maps of one slot's slabs for one layer. Stacked A [R, K]: boxes of 64 inputs by R rows (R / 2 rows when R
+// is over 256, the limit of a box), 128-byte swizzle. B of a part [rows, r]: boxes of 64 output columns by as many ranks
+// as exp_b_width says, the swizzle as wide as the box.
+cudaError_t plora_mma_encode_slab(PloraSlabMaps* out, const plora_desc& d, int K) {
     static_assert(sizeof(CUtensorMap) == sizeof(PloraTmap), "tensor map size");
     if (!g_encode) return cudaErrorNotSupported;
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)R};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {SHR_KSTEP, (cuuint32_t)(R > 256 ? R / 2 : R)};
-    const cuuint32_t es[2] = {1, 1};
-    if (g_encode(reinterpret_cast<CUtensorMap*>(out128), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(a), dims,
-                 strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return cudaErrorInvalidValue;
-    return cudaSuccess;
+    auto encode = [](PloraTmap* m, uint64_t base, int inner, int outer, int box_inner, int box_outer) {
+        const cuuint64_t dims[2] = {(cuuint64_t)inner, (cuuint64_t)outer};
+        const cuuint64_t strides[1] = {(cuuint64_t)inner * 2};
+        const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer};
+        const cuuint32_t es[2] = {1, 1};
+        const CUtensorMapSwizzle sw = box_inner == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
+                                      : box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                                        : CU_TENSOR_MAP_SWIZZLE_32B;
+        return g_encode(reinterpret_cast<CUtensorMap*>(m), CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (void*)(uintptr_t)base, dims, strides, box,
+                        es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    bool ok = encode(&out->a, d.a, K, d.rank, SHR_KSTEP, d.rank > 256 ? d.rank / 2 : d.rank);
+    for (int p = 0; p < PLORA_MAX_PARTS; p++)
+        if (d.r[p] > 0) ok = ok && encode(&out->b[p], d.b[p], d.r[p], d.rows[p], exp_b_width(d.r[p]), EXP_BN);
+    return ok ? cudaSuccess : cudaErrorInvalidValue;
 }
 
 cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, const int32_t* segs, SegLayout lay,
-                                    const plora_desc* table, const PloraTmap* amaps, float* S, size_t s_stride_elems, int lds,
+                                    const plora_desc* table, const PloraSlabMaps* smaps, float* S, size_t s_stride_elems, int lds,
                                     int max_rank_total, int tile_cap, int tile_split, int* status, bool pdl, bool late,
                                     cudaStream_t st) {
     if (!g_encode) return cudaErrorNotSupported;
@@ -862,49 +892,44 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
     if (nstage < 2) return cudaErrorInvalidValue;
     const size_t smem = (size_t)nstage * stage_bytes + 1024;
     return launch_pdl(plora_shrink_mma_kernel, dim3((unsigned)tile_split, 1, (unsigned)tile_cap), dim3(128), smem, st, pdl,
-                      map, reinterpret_cast<const CUtensorMap*>(amaps), K, segs, lay, table, S, s_stride_elems, lds, tile_split,
+                      map, smaps, K, segs, lay, table, S, s_stride_elems, lds, tile_split,
                       nstage, stage_bytes, sub, late && pdl ? 1 : 0, status);
 }
 
 cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int lds, int K, int tile_split,
-                                    const int32_t* segs, SegLayout lay, const plora_desc* table, void* y, int ldy,
-                                    int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
+                                    const int32_t* segs, SegLayout lay, const plora_desc* table, const PloraSlabMaps* smaps, void* y,
+                                    int ldy, int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
                                     int max_rows, int tile_cap, int* status, bool pdl, cudaStream_t st) {
     const int max_rank = lds / PLORA_MAX_PARTS;
     const int op_bytes = MMA_M * max_rank * 2;
-    const int nblocks = (max_rows + 127) / 128;
-    // Column blocks per thread block (one staging of its S tile each): the count, up to 16, that minimises
-    // waves x (start-up + blocks walked) for the step's estimated tile count, two thread blocks per SM; start-up
-    // (tensor-memory allocation, staging S, the first MMAs) costs about as much as two and a half column blocks.
+    // Column blocks per thread block (one staging of its S tile each): the count that minimises waves x (start-up +
+    // blocks walked) for the step's estimated tile count, two thread blocks per SM; start-up (tensor-memory allocation,
+    // staging S, the first MMAs) costs about as much as walking 320 columns.
     const long long tiles_est = (tile_cap + 1) / 2;  // tile_cap counts 64-token halves
-    int nb_per_cta = 1;
-    double best = 1e30;
-    for (int nb = 1; nb <= 16; nb++) {
-        long long groups = 0;
-        for (int p = 0; p < parts; p++) groups += ((part_rows[p] + 127) / 128 + nb - 1) / nb;
-        const long long waves = (tiles_est * groups + 2 * 148 - 1) / (2 * 148);
-        const double cost = (double)waves * (2.5 + nb);
-        if (cost < best) {
-            best = cost;
-            nb_per_cta = nb;
+    auto per_cta = [&](int width, int most) {
+        int pick = 1;
+        double best = 1e30;
+        for (int nb = 1; nb <= most; nb++) {
+            long long groups = 0;
+            for (int p = 0; p < parts; p++) groups += ((part_rows[p] + width - 1) / width + nb - 1) / nb;
+            const long long waves = (tiles_est * groups + 2 * 148 - 1) / (2 * 148);
+            const double cost = (double)waves * (320.0 + (double)nb * width);
+            if (cost < best) {
+                best = cost;
+                pick = nb;
+            }
         }
-    }
-    if (nb_per_cta > nblocks) nb_per_cta = nblocks;
-    dim3 grid((unsigned)((nblocks + nb_per_cta - 1) / nb_per_cta), (unsigned)parts, (unsigned)tile_cap);
+        return std::min(pick, (max_rows + width - 1) / width);
+    };
     // y by tensor copies where its base, pitch and part offsets are 16-byte aligned
     const int elt = f32_out ? 4 : 2;
     bool aligned = g_encode && ((uintptr_t)y & 15) == 0 && ((size_t)ldy * elt) % 16 == 0 && rows_total > 0;
     for (int p = 0; p < parts; p++) aligned = aligned && ((size_t)part_off[p] * elt) % 16 == 0;
-    // Two blocks per SM of eight adding warps with the ring slots that leaves room for; where the operands are too
-    // large for that, one block per SM of sixteen adding warps.
-    int wpq = 2;
-    int nst = (111 * 1024 - 1024 - 4 * op_bytes) / (8 * EXP_SLOT_BYTES);
-    if (nst < 1) {
-        wpq = 4;
-        nst = (216 * 1024 - 1024 - 4 * op_bytes) / (16 * EXP_SLOT_BYTES);
-    }
-    nst = nst > 4 ? 4 : nst;
-    if (aligned && nst >= 1) {
+    if (aligned) {
+        // stages of B of 2 KB (rank 16) to 16 KB (rank 128); two slots per warp fit at every rank
+        const int b_bytes = EXP_BN * max_rank * 2, nbs = b_bytes <= 8192 ? EXP_B_STAGES : 3;
+        int nst = (int)((EXP_TMA_SMEM - nbs * b_bytes - (int)sizeof(ExpandBars)) / (EXP_WARPS * EXP_SLOT_BYTES));
+        nst = nst > EXP_RING_MAX ? EXP_RING_MAX : nst;
         ExpandYMaps maps;
         memset(&maps, 0, sizeof(maps));
         const cuuint32_t es[2] = {1, 1};
@@ -917,21 +942,17 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
                                dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
         }
-        if (aligned) {
-            const size_t smem_tma = 1024 + (size_t)4 * wpq * nst * EXP_SLOT_BYTES + (size_t)4 * op_bytes;
-            const dim3 block(32 * (4 * wpq + 1));
-#define PLORA_EXPAND_TMA(F32, WPQ)                                                                                      \
-    return launch_pdl(plora_expand_tma_kernel<F32, WPQ>, grid, block, smem_tma, st, pdl, S, s_stride_elems, lds, K, \
-                      tile_split, segs, lay, table, maps, y, ldy, nb_per_cta, op_bytes, nst, status)
-            if (wpq == 2) {
-                if (f32_out) PLORA_EXPAND_TMA(true, 2);
-                PLORA_EXPAND_TMA(false, 2);
-            }
-            if (f32_out) PLORA_EXPAND_TMA(true, 4);
-            PLORA_EXPAND_TMA(false, 4);
-#undef PLORA_EXPAND_TMA
+        if (aligned && nst >= 1) {
+            const size_t smem_tma = (size_t)EXP_WARPS * nst * EXP_SLOT_BYTES + nbs * (size_t)b_bytes + sizeof(ExpandBars);
+            const int nb_per_cta = per_cta(EXP_BN, 32);
+            const dim3 grid((unsigned)(((max_rows + EXP_BN - 1) / EXP_BN + nb_per_cta - 1) / nb_per_cta), (unsigned)parts, (unsigned)tile_cap);
+            return launch_pdl(f32_out ? plora_expand_tma_kernel<true> : plora_expand_tma_kernel<false>, grid, dim3(32 * (EXP_WARPS + 1)),
+                              smem_tma, st, pdl, S, s_stride_elems, lds, K, tile_split, segs, lay, table, smaps, maps, y, ldy,
+                              nb_per_cta, b_bytes, nbs, nst, status);
         }
     }
+    const int nb_per_cta = per_cta(128, 16);
+    const dim3 grid((unsigned)(((max_rows + 127) / 128 + nb_per_cta - 1) / nb_per_cta), (unsigned)parts, (unsigned)tile_cap);
     // at least 48 KB of shared memory per block: no more than four blocks, 128 tensor-memory columns each,
     // share an SM's 512 columns
     size_t smem = (size_t)4 * op_bytes + (size_t)4 * 32 * EXP_TPAD * sizeof(float);
