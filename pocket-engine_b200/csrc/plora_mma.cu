@@ -515,7 +515,7 @@ struct ExpandYMaps {
 #define EXP_BN 64        // output columns per MMA
 #define EXP_TMEM_A 128   // first tensor-memory column of S
 #define EXP_WARPS 8      // adding warps
-#define EXP_B_STAGES 4
+#define EXP_B_STAGES 6
 // ranks per box of B: a swizzle span of 128, 64 or 32 bytes, whichever divides a row
 __host__ __device__ inline int exp_b_width(int r) { return r % 64 == 0 ? 64 : r % 32 == 0 ? 32 : 16; }
 #define EXP_TMA_SMEM (113 * 1024)  // two blocks per SM: half of 228 KB, less the 1 KB the system keeps per block
@@ -538,17 +538,17 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
     constexpr int CW = F32 ? 32 : 64;     // y columns per slot
     constexpr int CH = EXP_BN / CW;       // slots per column block
     constexpr int NW = EXP_WARPS, WPQ = NW / 4;
-    const int tile = blockIdx.z;
-    const int n_mma = segs[SEG_N_MMA];
+    const int n_mma = segs[SEG_N_MMA], p = blockIdx.y, cb0 = blockIdx.x * nb_per_cta;
+    bool begun = false;  // the block has waited for the kernels before it and holds tensor memory
+    // The grid is as deep as a step of full tiles needs; a step of many short runs has more tiles, which the blocks then
+    // walk in turn. (Sized for the most tiles a step can have, half of the blocks of a prefill step found none and
+    // cost 15 us of 780.)
+    for (int tile = blockIdx.z; tile < n_mma; tile += gridDim.z) {
     const int* mt = segs + lay.mma() + 3 * tile;
     const int start = mt[0], len = mt[1], slot = mt[2];
-    if (tile >= n_mma) return pdl_exit_idle();
     const plora_desc& d = table[slot];
-    const int p = blockIdx.y, r = d.r[p];
-    if (r == 0) return pdl_exit_idle();
-    const int rows = d.rows[p];
-    const int cb0 = blockIdx.x * nb_per_cta;
-    if (cb0 * EXP_BN >= rows) return pdl_exit_idle();
+    const int r = d.r[p], rows = d.rows[p];
+    if (r == 0 || cb0 * EXP_BN >= rows) continue;
     const int nblk = min(nb_per_cta, (rows - cb0 * EXP_BN + EXP_BN - 1) / EXP_BN);
     const int nchunks = min(nblk * CH, (rows - cb0 * EXP_BN + CW - 1) / CW);  // slots this block fills, in column order
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -571,20 +571,24 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
     };
 
     if (tid == 0) {
-        mbar_init(&bars.done[0], 1);
-        mbar_init(&bars.done[1], 1);
+        auto start_bar = [&](uint64_t* bar, uint32_t count) {
+            if (begun) mbar_inval(bar);
+            mbar_init(bar, count);
+        };
+        start_bar(&bars.done[0], 1);
+        start_bar(&bars.done[1], 1);
         // the warps that have rows of the tile and a slot in the accumulator's column blocks: the ones of one parity
         // where a column block is one slot, all where it is two
         const int live_warps = CH * min(4, (len + 31) / 32);
-        mbar_init(&bars.acc_free[0], live_warps);
-        mbar_init(&bars.acc_free[1], live_warps);
-        mbar_init(&bars.a_full, 32 * NW);
-        for (int i = 0; i < nbs; i++) mbar_init(&bars.b_full[i], 1);
+        start_bar(&bars.acc_free[0], live_warps);
+        start_bar(&bars.acc_free[1], live_warps);
+        start_bar(&bars.a_full, 32 * NW);
+        for (int i = 0; i < nbs; i++) start_bar(&bars.b_full[i], 1);
         for (int w = 0; w < NW; w++)
-            for (int i = 0; i < nst; i++) mbar_init(&bars.ybar[w][i], 1);
+            for (int i = 0; i < nst; i++) start_bar(&bars.ybar[w][i], 1);
         mbar_fence_init();
     }
-    if (warp == NW) tmem_alloc(&bars.tmem_slot, 256);
+    if (warp == NW && !begun) tmem_alloc(&bars.tmem_slot, 256);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -594,8 +598,11 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         tmap_acquire(bmap);
         for (int nb = 0; nb < nbs - 2 && nb < nblk; nb++) load_b(nb);  // a slab: it may be fetched before the kernels ahead have finished
     }
-    pdl_wait();
-    pdl_trigger();
+    if (!begun) {
+        pdl_wait();
+        pdl_trigger();
+        begun = true;
+    }
 
     if (warp == NW) {
         // ---- B copies (nbs - 2 column blocks ahead) and MMAs (up to two column blocks ahead of the additions)
@@ -632,12 +639,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             if (ok && nblk >= 2) mbar_wait_long(&bars.done[(nblk - 2) & 1], ((nblk - 2) >> 1) & 1, status);
         }
         __syncwarp();
-        tc_fence_before();
-        __syncthreads();
-        tmem_dealloc(tmem, 256);
-        return;
-    }
-
+    } else {
     const int wrow0 = wq * 32;
     const bool live = wrow0 < len;            // the warp has rows of the tile
     const bool whole = wrow0 + 32 <= len;     // all its 32 rows are: results go back by tensor store
@@ -659,30 +661,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         const bool valid = row < len;
         const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
         const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
-        for (int j = tid >> 7; j < P; j += WPQ) {
-            float f[8];
-            if (valid && s_eff > 1) {
-                float v[PLORA_TILE_SPLIT_MAX][8];
-#pragma unroll
-                for (int s = 0; s < PLORA_TILE_SPLIT_MAX; s++)
-                    if (s < s_eff) {
-                        const float* q = sp + (size_t)s * s_stride + j * 8;
-                        const float4 a = __ldcg(reinterpret_cast<const float4*>(q));
-                        const float4 b = __ldcg(reinterpret_cast<const float4*>(q + 4));
-                        v[s][0] = a.x, v[s][1] = a.y, v[s][2] = a.z, v[s][3] = a.w;
-                        v[s][4] = b.x, v[s][5] = b.y, v[s][6] = b.z, v[s][7] = b.w;
-                    }
-                tree_sum<8>(v, s_eff);
-#pragma unroll
-                for (int e = 0; e < 8; e++) f[e] = v[0][e];
-            } else if (valid) {
-                const float4 a = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
-                const float4 b = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
-                f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; e++) f[e] = 0.f;
-            }
+        auto put = [&](int j, const float* f) {
             uint32_t hi[4], lo[4];
 #pragma unroll
             for (int e = 0; e < 4; e++) {
@@ -695,6 +674,43 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             __syncwarp();
             tmem_st4(lane_base + EXP_TMEM_A + 4 * j, hi);
             tmem_st4(lane_base + EXP_TMEM_A + (r >> 1) + 4 * j, lo);
+        };
+        if (s_eff > 1) {
+#pragma unroll 1
+            for (int j = tid >> 7; j < P; j += WPQ) {
+                float v[PLORA_TILE_SPLIT_MAX][8];
+#pragma unroll
+                for (int s = 0; s < PLORA_TILE_SPLIT_MAX; s++) {
+                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+                    if (valid && s < s_eff) {
+                        const float* q = sp + (size_t)s * s_stride + j * 8;
+                        a = __ldcg(reinterpret_cast<const float4*>(q));
+                        b = __ldcg(reinterpret_cast<const float4*>(q + 4));
+                    }
+                    v[s][0] = a.x, v[s][1] = a.y, v[s][2] = a.z, v[s][3] = a.w;
+                    v[s][4] = b.x, v[s][5] = b.y, v[s][6] = b.z, v[s][7] = b.w;
+                }
+                tree_sum<8>(v, s_eff);
+                put(j, v[0]);
+            }
+        } else {
+            // four pieces of eight values per round trip
+#pragma unroll 1
+            for (int j0 = tid >> 7; j0 < P; j0 += 4 * WPQ) {
+                float4 f[4][2];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const int j = j0 + q * WPQ;
+                    f[q][0] = f[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (valid && j < P) {
+                        f[q][0] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
+                        f[q][1] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (j0 + q * WPQ < P) put(j0 + q * WPQ, reinterpret_cast<const float*>(f[q]));
+            }
         }
         tmem_st_wait();
         tc_fence_before();
@@ -710,13 +726,19 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         ok = mbar_wait_long(&bars.done[nb & 1], (nb >> 1) & 1, status);
         if (!ok) break;
         tc_fence_after();
-        uint32_t v[CW];
-#pragma unroll
-        for (int h = 0; h < CW / 32; h++) tmem_ld32_nowait(lane_base + (uint32_t)(nb & 1) * EXP_BN + ch * CW + h * 32, v + 32 * h);
-        tmem_ld_wait();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.acc_free[nb & 1]);
+        // 32 accumulator columns at a time: 64 at once leave too few registers, and what spills goes through to L2 beside y;
+        // the accumulator is given back once the last ones are in registers
+        uint32_t v[32];
+        const uint32_t acc = lane_base + (uint32_t)(nb & 1) * EXP_BN + ch * CW;
+        auto fetch = [&](int h) {
+            tmem_ld32(acc + h * 32, v);
+            if (h + 1 == CW / 32) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars.acc_free[nb & 1]);
+            }
+        };
+        fetch(0);
         unsigned char* sl = ring + (size_t)at * EXP_SLOT_BYTES;
         if (!mbar_wait(&bars.ybar[warp][at], ypar, status)) {
             ok = false;
@@ -740,6 +762,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                         *reinterpret_cast<float4*>(yrow + 4 * c) = y;
                     } else {
                         const float e[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
                         for (int k = 0; k < 4; k++)
                             if (col0 + 4 * c + k < rows) yrow[4 * c + k] = e[k];
                     }
@@ -749,6 +772,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
 #pragma unroll
             for (int c = 0; c < 8; c++) {
+                if (c == 4) fetch(1);
                 uint4* yp = reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4));
                 const uint4 raw = *yp;
                 float f[8];
@@ -756,8 +780,8 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                 uint32_t o[4];
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[(8 * c + 2 * e) % CW]),
-                                                                    f[2 * e + 1] + __uint_as_float(v[(8 * c + 2 * e + 1) % CW]));
+                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[8 * (c & 3) + 2 * e]),
+                                                                    f[2 * e + 1] + __uint_as_float(v[8 * (c & 3) + 2 * e + 1]));
                     o[e] = *reinterpret_cast<const uint32_t*>(&b2);
                 }
                 if (whole) {
@@ -766,9 +790,9 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                     if (col0 + 8 * c + 8 <= rows) {
                         *reinterpret_cast<uint4*>(yrow + 8 * c) = make_uint4(o[0], o[1], o[2], o[3]);
                     } else {
-                        const bf16* e = reinterpret_cast<const bf16*>(o);
-                        for (int k = 0; k < 8; k++)
-                            if (col0 + 8 * c + k < rows) yrow[8 * c + k] = e[k];
+#pragma unroll
+                        for (int k = 0; k < 4; k++)  // (a part's width is even)
+                            if (col0 + 8 * c + 2 * k < rows) *reinterpret_cast<uint32_t*>(yrow + 8 * c + 2 * k) = o[k];
                     }
                 }
             }
@@ -796,8 +820,12 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         }
     }
     if (lane == 0) bulk_wait_all();
+    }
     tc_fence_before();
     __syncthreads();
+    }
+    if (!begun) return pdl_exit_idle();
+    if ((threadIdx.x >> 5) == NW) tmem_dealloc(reinterpret_cast<ExpandBars*>(dsm1k + (size_t)NW * nst * EXP_SLOT_BYTES + nbs * (size_t)b_bytes)->tmem_slot, 256);
 }
 
 // cuTensorMapEncodeTiled, fetched from the driver once (no link-time dependency on libcuda)
@@ -945,7 +973,8 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
         if (aligned && nst >= 1) {
             const size_t smem_tma = (size_t)EXP_WARPS * nst * EXP_SLOT_BYTES + nbs * (size_t)b_bytes + sizeof(ExpandBars);
             const int nb_per_cta = per_cta(EXP_BN, 32);
-            const dim3 grid((unsigned)(((max_rows + EXP_BN - 1) / EXP_BN + nb_per_cta - 1) / nb_per_cta), (unsigned)parts, (unsigned)tile_cap);
+            const dim3 grid((unsigned)(((max_rows + EXP_BN - 1) / EXP_BN + nb_per_cta - 1) / nb_per_cta), (unsigned)parts,
+                            (unsigned)std::min(tile_cap, (rows_total + MMA_M - 1) / MMA_M + 4));
             return launch_pdl(f32_out ? plora_expand_tma_kernel<true> : plora_expand_tma_kernel<false>, grid, dim3(32 * (EXP_WARPS + 1)),
                               smem_tma, st, pdl, S, s_stride_elems, lds, K, tile_split, segs, lay, table, smaps, maps, y, ldy,
                               nb_per_cta, b_bytes, nbs, nst, status);
