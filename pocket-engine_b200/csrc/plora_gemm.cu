@@ -3,23 +3,32 @@
 // tcgen05 with accumulators in tensor memory, y written once (no read-modify-write). No counterpart in
 // pocket-engine, whose expand is always a separate kernel after the layer's own GEMM (src/linear.rs:889-921).
 //
-// Block = 128 tokens x 256 output columns, 192 threads:
-//   warp 0      producer: per step of 128 bytes of K, the x tile (16 KB) and the W tile (32 KB) as tensor copies
-//               into a ring of three stages (128-byte swizzle)
-//   warp 1      issues the MMAs: the base product into tensor-memory columns 0..255; after the last step, the
-//               adapter passes into columns 256..511
-//   warps 2..5  stage the adapter passes while the main loop runs, then the epilogue. A pass = one tensor-core
-//               tile of the step's grouping (a run of one slot's tokens) that meets the block's rows x 64 columns
-//               of the slot's rank: S rows (plane 0, other rows zero) split into bf16 high and low parts, and the
-//               block's 256 rows of B_p, in the unswizzled core-matrix layout. Epilogue: y = s_t s_n acc + adapter
-//               (or acc + adapter), staged in the idle ring in 128-byte-swizzled slots and written by tensor stores.
+// A pair of blocks (a cluster of two, cta_group::2) computes tiles of 256 tokens x BN output columns (256, or 128 where
+// that fills the device better); as many pairs as fit walk the tiles. Each block holds half of the tile's tokens and
+// half of its rows of W; the MMAs of the leading block read both, so a byte that enters an SM is used twice as often
+// as in a tile of one block's own: the single-block 128 x 256 kernel before this one moved 48 KB per SM and step of 128
+// bytes of K where this one moves 32. 320 threads per block:
+//   warp 0      producer: per step of 128 bytes of K, the block's x rows (16 KB) and W rows (BN / 2 x 128 bytes) as tensor
+//               copies into a ring of four stages (128-byte swizzle); both blocks' copies report to the leader
+//   warp 1      (leader) issues the MMAs and tells both blocks when a stage, an accumulator or the adapter operands are free
+//   warps 2..9  stage the adapter passes of the next tile, then run its epilogue. A pass = one tensor-core tile of the
+//               step's grouping (a run of one slot's tokens) that meets the pair's rows x 64 columns of the slot's rank:
+//               S rows (plane 0, other rows zero) split into bf16 high and low parts, and the block's rows of B_p, in
+//               the unswizzled core-matrix layout. The MMA warp takes a pass as soon as it is staged, in the middle of
+//               the main loop.
+// bf16: the adapter products accumulate onto the base product; two accumulators of BN columns, so the epilogue of a tile
+// runs under the next tile's main loop. FP8: the base product has to be scaled first, so the adapter term has an
+// accumulator of its own (columns BN ..), and the next tile starts when both have been read into registers.
+// Epilogue: y = s_t s_n acc + adapter (or acc), staged in 128-byte-swizzled slots and written by tensor stores.
 //
 // Tokens outside long runs (decode tokens, short prompts) get only the base product here; the gather expand
 // kernel adds their adapter term afterwards. Needs y 16-byte aligned with a 16-byte multiple pitch, and part
-// boundaries at multiples of 256 columns (a block lies in one part). Every wait is bounded.
+// boundaries at multiples of 256 columns (a tile lies in one part). Every wait is bounded.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 
 #include "plora_internal.h"
 #include "plora_device.cuh"
@@ -35,16 +44,85 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool vali
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-#define G_BM 128
-#define G_BN 256
+// ---- the two blocks of a pair ----
+__device__ __forceinline__ uint32_t pair_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// the address, in the cluster's shared memory, of the leading block's copy of a shared variable
+__device__ __forceinline__ uint32_t at_leader(const void* p) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+    return a;
+}
+__device__ __forceinline__ void arrive_at(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// tiled load into this block's shared memory whose bytes are counted on a barrier of either block of the pair
+__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+            smem_u32(dst)),
+        "l"(map), "r"(c0), "r"(c1), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void pair_tmem_alloc(uint32_t* slot) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void pair_tmem_dealloc(uint32_t taddr) {
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(taddr) : "memory");
+}
+template <int KIND>
+__device__ __forceinline__ void pair_umma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    if (KIND == 0)
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(acc)
+            : "memory");
+    else
+        asm volatile(
+            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+            "l"(a), "l"(b), "r"(idesc), "r"(acc)
+            : "memory");
+}
+// arrives on the barrier at this address in both blocks once this thread's earlier MMAs are complete
+__device__ __forceinline__ void pair_commit(uint64_t* bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)),
+                 "h"((uint16_t)3)
+                 : "memory");
+}
+
+#define G_BM 128   // token rows per block
 #define G_BKB 128  // bytes of K per stage row
-#define G_STAGES 3
-#define G_STAGE_BYTES (G_BM * G_BKB + G_BN * G_BKB)
+#define G_STAGES 4
 #define G_RC 64  // rank columns per adapter pass
 #define G_AOP (G_BM * G_RC * 2)
-#define G_BOP (G_BN * G_RC * 2)
 #define G_MAX_PASS 16
 #define G_SLOT 4096  // 32 rows x 128 bytes of y
+#define G_EPI_WARPS 8
+#define G_EPI (32 * G_EPI_WARPS)
+#define G_GROUP_M 8  // tiles of tokens that are walked together: neighbouring pairs share rows of x and of W in L2
+
+__device__ __forceinline__ void epi_sync_all() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 struct GemmParts {
     int n;
@@ -52,224 +130,293 @@ struct GemmParts {
     int rows[PLORA_MAX_PARTS];
 };
 
-template <int KIND, bool F32>
-__global__ void __launch_bounds__(192) plora_gemm_fused_kernel(const __grid_constant__ CUtensorMap xmap,
-                                                                const __grid_constant__ CUtensorMap wmap,
-                                                                const __grid_constant__ CUtensorMap ymap,
-                                                                const float* __restrict__ st, const float* __restrict__ sn,
-                                                                int T, int N, int K, const int* __restrict__ segs,
-                                                                SegLayout lay, const plora_desc* __restrict__ table,
-                                                                GemmParts parts, const float* __restrict__ S, int lds,
-                                                                int* __restrict__ status) {
+struct GemmShared {
+    uint64_t full[G_STAGES], empty[G_STAGES], acc_full[2], acc_empty[2], meta, ad_full, ad_empty;
+    uint32_t tmem_slot;
+    int npass, row0[G_MAX_PASS], row1[G_MAX_PASS], slot[G_MAX_PASS], rc0[G_MAX_PASS], rw[G_MAX_PASS];
+};
+
+__host__ __device__ constexpr size_t gemm_stage_bytes(int bn) { return G_BM * G_BKB + bn / 2 * G_BKB; }
+constexpr size_t gemm_smem(int bn) {
+    return 1024 + G_STAGES * gemm_stage_bytes(bn) + 2 * G_AOP + (size_t)bn / 2 * G_RC * 2 + G_EPI_WARPS * G_SLOT + bn * sizeof(float);
+}
+
+template <int KIND, bool F32, int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
+    plora_gemm_fused_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+                            const __grid_constant__ CUtensorMap ymap, const float* __restrict__ st, const float* __restrict__ sn, int T,
+                            int N, int K, const int* __restrict__ segs, SegLayout lay, const plora_desc* __restrict__ table,
+                            GemmParts parts, const float* __restrict__ S, int lds, int* __restrict__ status) {
     extern __shared__ unsigned char dsm_raw[];
-    __shared__ __align__(8) uint64_t full[G_STAGES], empty[G_STAGES], acc_bar, meta_bar, ad_full, ad_empty;
-    __shared__ uint32_t tmem_slot;
-    __shared__ int s_npass, p_row0[G_MAX_PASS], p_row1[G_MAX_PASS], p_slot[G_MAX_PASS], p_rc0[G_MAX_PASS], p_rw[G_MAX_PASS];
+    __shared__ __align__(8) GemmShared sh;
+    constexpr uint32_t STAGE = (uint32_t)gemm_stage_bytes(BN);
+    constexpr int NBUF = KIND == 0 ? 1 : 2;               // accumulators of the base product
+    constexpr int KEL = KIND == 0 ? G_BKB : G_BKB / 2;    // elements of K per step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int n0 = blockIdx.x * G_BN, m0 = blockIdx.y * G_BM;
+    const uint32_t rank = pair_rank();
     unsigned char* ring = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);
-    unsigned char* Ahi = ring + G_STAGES * G_STAGE_BYTES;
+    unsigned char* Ahi = ring + G_STAGES * STAGE;
     unsigned char* Alo = Ahi + G_AOP;
     unsigned char* Bop = Alo + G_AOP;
-    float* sn_s = reinterpret_cast<float*>(Bop + G_BOP);  // the block's 256 column scales
+    unsigned char* slots = Bop + BN / 2 * G_RC * 2;
+    float* sn_s = reinterpret_cast<float*>(slots + G_EPI_WARPS * G_SLOT);  // the tile's column scales
     if (tid == 0) {
         for (int i = 0; i < G_STAGES; i++) {
-            mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 1);
+            mbar_init(&sh.full[i], 1);
+            mbar_init(&sh.empty[i], 1);
         }
-        mbar_init(&acc_bar, 1);
-        mbar_init(&meta_bar, 1);
-        mbar_init(&ad_full, 1);
-        mbar_init(&ad_empty, 1);
+        for (int i = 0; i < 2; i++) {
+            mbar_init(&sh.acc_full[i], 1);
+            mbar_init(&sh.acc_empty[i], 2 * G_EPI_WARPS);
+        }
+        mbar_init(&sh.meta, 1);
+        mbar_init(&sh.ad_full, 2);
+        mbar_init(&sh.ad_empty, 1);
         mbar_fence_init();
     }
-    if (warp == 1) tmem_alloc(&tmem_slot, 512);
+    if (warp == 1) pair_tmem_alloc(&sh.tmem_slot);
     tc_fence_before();
     __syncthreads();
+    pair_sync();  // the other block's barriers exist
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
-    const int kbytes = KIND == 0 ? K : 2 * K;
-    const int nk = (kbytes + G_BKB - 1) / G_BKB;
-    constexpr int KEL = KIND == 0 ? G_BKB : G_BKB / 2;  // elements of K per step
+    const uint32_t tmem = sh.tmem_slot;
+    const int nk = ((KIND == 0 ? K : 2 * K) + G_BKB - 1) / G_BKB;
+    // tiles in groups of G_GROUP_M tiles of tokens; within a group, tokens first
+    const int mt = (T + 2 * G_BM - 1) / (2 * G_BM), nt = (N + BN - 1) / BN, tiles = mt * nt;
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    auto place = [&](int t, int& m0, int& n0) {
+        const int per = G_GROUP_M * nt, g = t / per, in = t - g * per, gm = min(G_GROUP_M, mt - g * G_GROUP_M);
+        m0 = (g * G_GROUP_M + in % gm) * 2 * G_BM;
+        n0 = in / gm * BN;
+    };
     pdl_wait();  // S, x and the scales come from the kernels before
     pdl_trigger();
-    // the part this block's columns lie in
-    int part = 0;
-#pragma unroll
-    for (int q = 1; q < PLORA_MAX_PARTS; q++)
-        if (q < parts.n && n0 >= parts.off[q]) part = q;
-    const int n_local = n0 - parts.off[part];  // first row of B_p for this block
 
     if (warp == 0) {
         if (elect_one()) {
-            for (int ks = 0; ks < nk; ks++) {
-                const int stg = ks % G_STAGES;
-                if (ks >= G_STAGES && !mbar_wait(&empty[stg], ((ks / G_STAGES) - 1) & 1, status)) break;
-                unsigned char* xs = ring + (size_t)stg * G_STAGE_BYTES;
-                mbar_expect_tx(&full[stg], G_STAGE_BYTES);
-                tma_load_2d(xs, &xmap, ks * KEL, m0, &full[stg]);
-                tma_load_2d(xs + G_BM * G_BKB, &wmap, ks * KEL, n0, &full[stg]);
+            int stg = 0;
+            uint32_t par = 0;
+            bool ok = true, round2 = false;
+            for (int t = pair; ok && t < tiles; t += pairs) {
+                int m0, n0;
+                place(t, m0, n0);
+                for (int ks = 0; ks < nk; ks++) {
+                    if (round2) ok = mbar_wait_long(&sh.empty[stg], par ^ 1, status);
+                    if (!ok) break;
+                    unsigned char* xs = ring + (size_t)stg * STAGE;
+                    if (rank == 0) mbar_expect_tx(&sh.full[stg], 2 * STAGE);
+                    const uint32_t bar = at_leader(&sh.full[stg]);
+                    tma_load_2d_pair(xs, &xmap, ks * KEL, m0 + (int)rank * G_BM, bar);
+                    tma_load_2d_pair(xs + G_BM * G_BKB, &wmap, ks * KEL, n0 + (int)rank * (BN / 2), bar);
+                    if (++stg == G_STAGES) {
+                        stg = 0;
+                        par ^= 1;
+                        round2 = true;
+                    }
+                }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (elect_one()) {
-            // M 128, N 256, f32 accumulator, K-major operands; kind::f16 carries the bf16 formats in bits 7 and 10
-            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(G_BN >> 3) << 17) | ((uint32_t)(G_BM >> 4) << 24);
-            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(G_BN >> 3) << 17) | ((uint32_t)(G_BM >> 4) << 24) : idesc_ad;
+        if (rank == 0 && elect_one()) {
+            // M 256, N BN, f32 accumulator, K-major operands; kind::f16 carries the bf16 formats in bits 7 and 10
+            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24);
+            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24) : idesc_ad;
+            const uint64_t dx0 = umma_desc(smem_u32(ring), 16, 1024, 2), dw0 = umma_desc(smem_u32(ring) + G_BM * G_BKB, 16, 1024, 2);
+            int stg = 0, i = 0;
+            uint32_t par = 0, apar = 0;  // parities of the stages and of the adapter operands
             bool ok = true;
-            for (int ks = 0; ok && ks < nk; ks++) {
-                const int stg = ks % G_STAGES;
-                ok = mbar_wait(&full[stg], (ks / G_STAGES) & 1, status);
-                if (!ok) break;
+            for (int t = pair; ok && t < tiles; t += pairs, i++) {
+                const int buf = KIND == 0 ? 0 : i & 1;
+                const uint32_t acc = tmem + (uint32_t)buf * BN, ad = KIND == 0 ? tmem + BN : acc;
+                if (i >= NBUF) ok = mbar_wait_long(&sh.acc_empty[buf], (i / NBUF - 1) & 1, status);
                 tc_fence_after();
-                const uint32_t xs = smem_u32(ring + (size_t)stg * G_STAGE_BYTES);
-                const uint32_t ws = xs + G_BM * G_BKB;
+                int npass = -1, ps = 0;  // npass: not known before the other warps have written the list
+                auto pass = [&]() {
+                    tc_fence_after();
+                    const int rw = sh.rw[ps];
+                    const uint32_t sbo = (uint32_t)rw * 16u;
+                    const uint32_t a_hi = smem_u32(Ahi), a_lo = smem_u32(Alo), b = smem_u32(Bop);
+                    for (int kk = 0; kk < rw / 16; kk++)
+                        pair_umma<1>(ad, umma_desc(a_hi + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad,
+                                     KIND == 1 || (ps | kk) != 0);
+                    for (int kk = 0; kk < rw / 16; kk++)
+                        pair_umma<1>(ad, umma_desc(a_lo + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad, 1);
+                    pair_commit(&sh.ad_empty);
+                    ps++;
+                    apar ^= 1;
+                };
+                for (int ks = 0; ok && ks < nk; ks++) {
+                    ok = mbar_wait_long(&sh.full[stg], par, status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t dx = dx0 + (uint64_t)((uint32_t)stg * STAGE >> 4), dw = dw0 + (uint64_t)((uint32_t)stg * STAGE >> 4);
 #pragma unroll
-                for (int kk = 0; kk < G_BKB / 32; kk++)
-                    umma<KIND>(tmem, umma_desc(xs + kk * 32, 16, 1024, 2), umma_desc(ws + kk * 32, 16, 1024, 2), idesc,
-                               (ks | kk) != 0);
-                umma_commit(&empty[stg]);
+                    for (int kk = 0; kk < G_BKB / 32; kk++) pair_umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
+                    pair_commit(&sh.empty[stg]);
+                    if (++stg == G_STAGES) {
+                        stg = 0;
+                        par ^= 1;
+                    }
+                    if (npass < 0 && mbar_test(&sh.meta, i & 1)) npass = sh.npass;
+                    if (ps < npass && mbar_test(&sh.ad_full, apar)) pass();
+                }
+                if (ok && npass < 0) {
+                    ok = mbar_wait_long(&sh.meta, i & 1, status);
+                    npass = ok ? sh.npass : 0;
+                }
+                while (ok && ps < npass) {
+                    ok = mbar_wait_long(&sh.ad_full, apar, status);
+                    if (ok) pass();
+                }
+                if (ok) pair_commit(&sh.acc_full[buf]);
             }
-            // the adapter passes, staged by warps 2..5 while the loop above ran
-            if (ok) ok = mbar_wait_long(&meta_bar, 0, status);
-            const int npass = ok ? s_npass : 0;
-            for (int ps = 0; ok && ps < npass; ps++) {
-                ok = mbar_wait_long(&ad_full, ps & 1, status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t sbo = (uint32_t)p_rw[ps] * 16u;
-                const uint32_t a_hi = smem_u32(Ahi), a_lo = smem_u32(Alo), b = smem_u32(Bop);
-                for (int kk = 0; kk < p_rw[ps] / 16; kk++)
-                    umma<1>(tmem + 256, umma_desc(a_hi + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad,
-                            (ps | kk) != 0);
-                for (int kk = 0; kk < p_rw[ps] / 16; kk++)
-                    umma<1>(tmem + 256, umma_desc(a_lo + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad, 1);
-                umma_commit(&ad_empty);
-            }
-            umma_commit(&acc_bar);
         }
         __syncwarp();
     } else {
-        const int e = tid - 64;  // 0..127: token row of the block, and (twice) a row of B
-        // ---- the block's adapter passes: tensor-core tiles of the grouping that meet its rows
-        if (e == 0) {
-            int np = 0;
-            const int n_mma = segs[SEG_N_MMA];
-            const int* mt = segs + lay.mma();
-            int lo = 0, hi = n_mma;  // first tile that ends after the block's first row
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (mt[3 * mid] + mt[3 * mid + 1] > m0) hi = mid;
-                else lo = mid + 1;
-            }
-            for (int t = lo; t < n_mma && mt[3 * t] < m0 + G_BM; t++) {
-                const int start = mt[3 * t], len = mt[3 * t + 1], slot = mt[3 * t + 2];
-                const int r = table[slot].r[part];
-                for (int rc0 = 0; rc0 < r; rc0 += G_RC) {
-                    if (np == G_MAX_PASS) {
-                        atomicMax(status, PLORA_ERR_CAPACITY);
-                        break;
-                    }
-                    p_row0[np] = max(start, m0) - m0;
-                    p_row1[np] = min(start + len, m0 + G_BM) - m0;
-                    p_slot[np] = slot;
-                    p_rc0[np] = rc0;
-                    p_rw[np] = min(G_RC, r - rc0);
-                    np++;
-                }
-            }
-            s_npass = np;
-        }
-        if (KIND == 0)
-            for (int i = e; i < G_BN; i += 128) sn_s[i] = n0 + i < N ? sn[n0 + i] : 0.f;
-        epi_sync();
-        const int npass = s_npass;
-        if (e == 0) mbar_arrive(&meta_bar);
+        const int e = tid - 64;                  // 0..255
+        const int ew = warp - 2, wq = warp & 3;  // tensor-memory lanes 32 wq .. 32 wq + 31, columns of half ew / 4
+        unsigned char* slot = slots + ew * G_SLOT;
+        const uint32_t ad_full = at_leader(&sh.ad_full);
+        uint32_t apar = 0;
+        bool staged = false;  // the adapter operands have been used before
         bool ok = true;
-        for (int ps = 0; ok && ps < npass; ps++) {
-            if (ps > 0) {  // the operands of the pass before are still being read until its MMAs complete
-                ok = mbar_wait_long(&ad_empty, (ps - 1) & 1, status);
-                if (!ok) break;
-            }
-            const plora_desc& d = table[p_slot[ps]];
-            const int rw = p_rw[ps], rc0 = p_rc0[ps], r = d.r[part], P = rw >> 3;
-            const uint32_t sbo = (uint32_t)rw * 16u;
-            // rows of B_p for the block's columns: thread e copies rows e and e + 128
-            const bf16* B = reinterpret_cast<const bf16*>(d.b[part]);
-            for (int h = 0; h < 2; h++) {
-                const int n = e + 128 * h;
-                const bool valid = n_local + n < d.rows[part];
-                const bf16* src = B + (size_t)(valid ? n_local + n : 0) * r + rc0;
-                unsigned char* drow = Bop + (size_t)(n >> 3) * sbo + (n & 7) * 16;
-                for (int j = 0; j < P; j++) cp_async16(drow + j * 128, src + j * 8, valid);
-            }
-            // this thread's token row of S (zero outside the pass's rows), as bf16 high and low parts
-            {
-                const bool valid = e >= p_row0[ps] && e < p_row1[ps];
-                const float* sp = S + (size_t)(m0 + (valid ? e : 0)) * lds + d.r_off[part] + rc0;
-                unsigned char* ahi = Ahi + (size_t)(e >> 3) * sbo + (e & 7) * 16;
-                unsigned char* alo = Alo + (size_t)(e >> 3) * sbo + (e & 7) * 16;
-                for (int j = 0; j < P; j++) {
-                    float f[8];
-                    if (valid) {
-                        const float4 a = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
-                        const float4 b = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
-                        f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-                    } else {
+        int i = 0;
+        for (int t = pair; ok && t < tiles; t += pairs, i++) {
+            int m0, n0;
+            place(t, m0, n0);
+            int part = 0;  // the part the tile's columns lie in
 #pragma unroll
-                        for (int q = 0; q < 8; q++) f[q] = 0.f;
-                    }
-                    uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
-                        const float2 hf = __bfloat1622float2(h2);
-                        const __nv_bfloat162 l2 = __floats2bfloat162_rn(f[2 * q] - hf.x, f[2 * q + 1] - hf.y);
-                        hi[q] = *reinterpret_cast<const uint32_t*>(&h2);
-                        lo[q] = *reinterpret_cast<const uint32_t*>(&l2);
-                    }
-                    *reinterpret_cast<uint4*>(ahi + j * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                    *reinterpret_cast<uint4*>(alo + j * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            for (int q = 1; q < PLORA_MAX_PARTS; q++)
+                if (q < parts.n && n0 >= parts.off[q]) part = q;
+            const int n_local = n0 - parts.off[part] + (int)rank * (BN / 2);  // this block's first row of B_p
+            // ---- the tile's adapter passes: tensor-core tiles of the grouping that meet the pair's rows
+            if (e == 0) {
+                int np = 0;
+                const int n_mma = segs[SEG_N_MMA];
+                const int* ml = segs + lay.mma();
+                int lo = 0, hi = n_mma;  // first tile that ends after the first row
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    if (ml[3 * mid] + ml[3 * mid + 1] > m0) hi = mid;
+                    else lo = mid + 1;
                 }
+                for (int q = lo; q < n_mma && ml[3 * q] < m0 + 2 * G_BM; q++) {
+                    const int start = ml[3 * q], len = ml[3 * q + 1], slot_id = ml[3 * q + 2];
+                    const int r = table[slot_id].r[part];
+                    for (int rc0 = 0; rc0 < r; rc0 += G_RC) {
+                        if (np == G_MAX_PASS) {
+                            atomicMax(status, PLORA_ERR_CAPACITY);
+                            break;
+                        }
+                        sh.row0[np] = max(start, m0) - m0;
+                        sh.row1[np] = min(start + len, m0 + 2 * G_BM) - m0;
+                        sh.slot[np] = slot_id;
+                        sh.rc0[np] = rc0;
+                        sh.rw[np] = min(G_RC, r - rc0);
+                        np++;
+                    }
+                }
+                sh.npass = np;
             }
-            cp_async_wait_all();
-            fence_async_smem();
-            epi_sync();
-            if (e == 0) mbar_arrive(&ad_full);
-        }
-        // ---- epilogue: the warp's 32 rows of both accumulators, scaled and added, into swizzled slots of the
-        // idle ring, then tensor stores (clipped at the edges of y by the tensor map)
-        if (ok) ok = mbar_wait_long(&acc_bar, 0, status);
-        if (ok) {
+            if (KIND == 0)
+                for (int c = e; c < BN; c += G_EPI) sn_s[c] = n0 + c < N ? sn[n0 + c] : 0.f;
+            epi_sync_all();
+            const int npass = sh.npass;
+            if (e == 0) mbar_arrive(&sh.meta);
+            for (int ps = 0; ok && ps < npass; ps++) {
+                if (staged) {  // the operands of the pass before are still being read until its MMAs complete
+                    ok = mbar_wait_long(&sh.ad_empty, apar, status);
+                    apar ^= 1;
+                    if (!ok) break;
+                }
+                staged = true;
+                const plora_desc& d = table[sh.slot[ps]];
+                const int rw = sh.rw[ps], rc0 = sh.rc0[ps], r = d.r[part], P = rw >> 3;
+                const uint32_t sbo = (uint32_t)rw * 16u;
+                // rows of B_p for the block's half of the columns
+                const bf16* B = reinterpret_cast<const bf16*>(d.b[part]);
+                for (int q = e; q < BN / 2 * P; q += G_EPI) {
+                    const int n = q / P, j = q - n * P;
+                    const bool valid = n_local + n < d.rows[part];
+                    cp_async16(Bop + (size_t)(n >> 3) * sbo + (n & 7) * 16 + j * 128,
+                               B + (size_t)(valid ? n_local + n : 0) * r + rc0 + j * 8, valid);
+                }
+                // this block's token rows of S (zero outside the pass's rows), as bf16 high and low parts
+                {
+                    const int row = e & (G_BM - 1), rel = row + (int)rank * G_BM;
+                    const bool valid = rel >= sh.row0[ps] && rel < sh.row1[ps];
+                    const float* sp = S + (size_t)(m0 + (valid ? rel : 0)) * lds + d.r_off[part] + rc0;
+                    unsigned char* ahi = Ahi + (size_t)(row >> 3) * sbo + (row & 7) * 16;
+                    unsigned char* alo = Alo + (size_t)(row >> 3) * sbo + (row & 7) * 16;
+#pragma unroll 4
+                    for (int j = e / G_BM; j < P; j += G_EPI / G_BM) {
+                        float f[8];
+                        if (valid) {
+                            const float4 a = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
+                            const float4 b = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
+                            f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+                        } else {
+#pragma unroll
+                            for (int q = 0; q < 8; q++) f[q] = 0.f;
+                        }
+                        uint32_t hi[4], lo[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
+                            const float2 hf = __bfloat1622float2(h2);
+                            const __nv_bfloat162 l2 = __floats2bfloat162_rn(f[2 * q] - hf.x, f[2 * q + 1] - hf.y);
+                            hi[q] = *reinterpret_cast<const uint32_t*>(&h2);
+                            lo[q] = *reinterpret_cast<const uint32_t*>(&l2);
+                        }
+                        *reinterpret_cast<uint4*>(ahi + j * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *reinterpret_cast<uint4*>(alo + j * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                    }
+                }
+                cp_async_wait_all();
+                fence_async_smem();
+                epi_sync_all();
+                if (e == 0) arrive_at(ad_full);
+            }
+            // ---- epilogue: the warp's 32 rows of its half of the columns, scaled and added, into a swizzled slot of 128
+            // bytes a row, then a tensor store (clipped at the edges of y by the tensor map)
+            const int buf = KIND == 0 ? 0 : i & 1;
+            if (ok) ok = mbar_wait_long(&sh.acc_full[buf], (i / NBUF) & 1, status);
+            if (!ok) break;
             tc_fence_after();
-            const int wq = warp & 3;  // tensor-memory lanes 32 wq .. 32 wq + 31
-            const int row = m0 + wq * 32 + lane;
-            constexpr int CW = F32 ? 32 : 64;     // y columns per slot
-            constexpr int NSL = G_BN / CW;        // slots per warp
-            unsigned char* slots = ring + (size_t)wq * NSL * G_SLOT;
+            const int row = m0 + (int)rank * G_BM + wq * 32 + lane;
+            constexpr int CW = F32 ? 32 : 64;  // y columns per slot
+            const int c0 = (ew >> 2) * (BN / 2);
             const float srow = KIND == 0 ? (row < T ? st[row] : 0.f) : 1.f;
-            const uint32_t lane_base = tmem + ((uint32_t)(wq * 32) << 16);
+            const uint32_t base = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)buf * BN + (uint32_t)c0;
 #pragma unroll 1
-            for (int g = 0; g < G_BN / 32; g++) {  // 32 accumulator columns at a time
+            for (int g = 0; g < BN / 64; g++) {  // 32 accumulator columns at a time
                 uint32_t vb[32], va[32];
-                tmem_ld32_nowait(lane_base + g * 32, vb);
-                if (npass > 0) tmem_ld32_nowait(lane_base + 256 + g * 32, va);
+                tmem_ld32_nowait(base + g * 32, vb);
+                if (KIND == 0 && npass > 0) tmem_ld32_nowait(base + BN + g * 32, va);
                 tmem_ld_wait();
+                if (g == BN / 64 - 1) {  // everything this warp reads is in registers: the accumulator is free
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) arrive_at(at_leader(&sh.acc_empty[buf]));
+                }
                 float o[32];
 #pragma unroll
                 for (int q = 0; q < 32; q++) {
-                    const float base = KIND == 0 ? __uint_as_float(vb[q]) * (srow * sn_s[g * 32 + q]) : __uint_as_float(vb[q]);
-                    o[q] = npass > 0 ? base + __uint_as_float(va[q]) : base;
+                    const float v = KIND == 0 ? __uint_as_float(vb[q]) * (srow * sn_s[c0 + g * 32 + q]) : __uint_as_float(vb[q]);
+                    o[q] = KIND == 0 && npass > 0 ? v + __uint_as_float(va[q]) : v;
                 }
+                if (F32 || (g & 1) == 0) {  // a new slot: the store before has to have read it
+                    if (lane == 0) bulk_wait_read();
+                    __syncwarp();
+                }
+                unsigned char* myrow = slot + lane * 128;
                 if (F32) {
-                    unsigned char* myrow = slots + (size_t)g * G_SLOT + lane * 128;
 #pragma unroll
                     for (int c = 0; c < 8; c++)
                         *reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4)) =
                             make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
                 } else {
-                    unsigned char* myrow = slots + (size_t)(g >> 1) * G_SLOT + lane * 128;
 #pragma unroll
                     for (int c4 = 0; c4 < 4; c4++) {
                         uint32_t w[4];
@@ -282,20 +429,24 @@ __global__ void __launch_bounds__(192) plora_gemm_fused_kernel(const __grid_cons
                         *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
                     }
                 }
+                if (F32 || (g & 1) == 1) {
+                    fence_async_smem();
+                    __syncwarp();
+                    const int col = n0 + c0 + (F32 ? g : g >> 1) * CW;
+                    if (lane == 0) {
+                        if (col < N && m0 + (int)rank * G_BM + wq * 32 < T) tma_store_2d(&ymap, col, m0 + (int)rank * G_BM + wq * 32, slot);
+                        bulk_commit();
+                    }
+                }
             }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-                for (int s = 0; s < NSL; s++)
-                    if (n0 + s * CW < N) tma_store_2d(&ymap, n0 + s * CW, m0 + wq * 32, slots + (size_t)s * G_SLOT);
-                bulk_commit();
-                bulk_wait_all();
-            }
+            epi_sync_all();  // the list of passes and the column scales are overwritten for the next tile
         }
+        if (lane == 0) bulk_wait_all();
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem, 512);
+    pair_sync();  // neither block leaves while the other may still signal it or read its operands
+    if (warp == 1) pair_tmem_dealloc(tmem);
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -303,7 +454,7 @@ typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 encode_tiled_fn g_encode = nullptr;
 
-size_t gemm_smem() { return 1024 + (size_t)G_STAGES * G_STAGE_BYTES + 2 * G_AOP + G_BOP + G_BN * sizeof(float); }
+int g_pairs = 74;  // pairs of blocks the device runs at once
 
 template <typename... Params, typename... Args>
 cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool pdl,
@@ -328,7 +479,7 @@ bool encode2d(CUtensorMap* m, CUtensorMapDataType dt, const void* base, uint64_t
     const cuuint32_t box[2] = {box_inner, box_outer};
     const cuuint32_t es[2] = {1, 1};
     return g_encode(m, dt, 2, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -344,11 +495,24 @@ cudaError_t plora_gemm_init() {
         g_encode = reinterpret_cast<encode_tiled_fn>(fn);
     }
     cudaError_t e;
-    const int smem = (int)gemm_smem();
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<0, false>), smem))) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<0, true>), smem))) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<1, false>), smem))) return e;
-    return plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<1, true>), smem);
+#define PLORA_GEMM_INIT(KIND, F32)                                                                                                         \
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<KIND, F32, 256>), (int)gemm_smem(256)))) return e; \
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<KIND, F32, 128>), (int)gemm_smem(128)))) return e
+    PLORA_GEMM_INIT(0, false);
+    PLORA_GEMM_INIT(0, true);
+    PLORA_GEMM_INIT(1, false);
+    PLORA_GEMM_INIT(1, true);
+#undef PLORA_GEMM_INIT
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(148);
+    cfg.blockDim = dim3(64 + G_EPI);
+    cfg.dynamicSmemBytes = gemm_smem(256);
+    int n = 0;
+    e = cudaOccupancyMaxActiveClusters(&n, plora_gemm_fused_kernel<0, false, 256>, &cfg);
+    if (e != cudaSuccess) return e;
+    if (n < 1) return cudaErrorInvalidConfiguration;
+    g_pairs = n;
+    return cudaSuccess;
 }
 
 // Whether a layer's shapes fit the kernel: parts starting at multiples of 256 columns (so does every block),
@@ -360,7 +524,7 @@ bool plora_gemm_fits(int kind, const void* x, const void* w, const void* y, int 
     if (((uintptr_t)x & 15) || ((uintptr_t)w & 15) || ((uintptr_t)y & 15)) return false;
     if (((size_t)K * el) % 16 || ((size_t)ldy * yel) % 16) return false;
     for (int p = 0; p < n_parts; p++)
-        if (part_off[p] % G_BN) return false;
+        if (part_off[p] % 256) return false;
     return true;
 }
 
@@ -372,8 +536,17 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
     CUtensorMap xmap, wmap, ymap;
     const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int el = kind == 0 ? 1 : 2;
+    // 256 output columns per tile, or 128 where that leaves fewer columns' worth of rounds: a step of few tokens has few
+    // tiles, and a round of one tile per pair that is nearly empty costs as much as a full one (96 tiles of 256 on 74
+    // pairs: 2 rounds; 192 of 128: 3 rounds of half the length). A tile of 128 moves 1.5 times the bytes per product, so
+    // it has to save more than a tenth.
+    auto rounds = [&](int width) {
+        const long long tiles = (long long)((T + 2 * G_BM - 1) / (2 * G_BM)) * ((N + width - 1) / width);
+        return (double)((tiles + g_pairs - 1) / g_pairs) * width;
+    };
+    const int bn = rounds(128) < 0.9 * rounds(256) ? 128 : 256;
     if (!encode2d(&xmap, dt, x, (uint64_t)K, (uint64_t)T, (uint64_t)K * el, G_BKB / el, G_BM)) return cudaErrorInvalidValue;
-    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, G_BN)) return cudaErrorInvalidValue;
+    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)bn / 2)) return cudaErrorInvalidValue;
     if (!encode2d(&ymap, f32_out ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, (uint64_t)N,
                   (uint64_t)T, (uint64_t)ldy * (f32_out ? 4 : 2), f32_out ? 32 : 64, 32))
         return cudaErrorInvalidValue;
@@ -383,11 +556,13 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
         parts.off[p] = p < n_parts ? part_off[p] : 0;
         parts.rows[p] = p < n_parts ? part_rows[p] : 0;
     }
-    dim3 grid((unsigned)((N + G_BN - 1) / G_BN), (unsigned)((T + G_BM - 1) / G_BM));
-    const size_t smem = gemm_smem();
-#define PLORA_GEMM_LAUNCH(KIND, F32)                                                                                        \
-    return launch_pdl(plora_gemm_fused_kernel<KIND, F32>, grid, dim3(192), smem, stream, pdl, xmap, wmap, ymap, st_, sn, T, \
-                      N, K, segs, lay, table, parts, S, lds, status)
+    const long long tiles = (long long)((T + 2 * G_BM - 1) / (2 * G_BM)) * ((N + bn - 1) / bn);
+    const dim3 grid(2u * (unsigned)std::min<long long>(tiles, g_pairs)), block(64 + G_EPI);
+#define PLORA_GEMM_LAUNCH(KIND, F32)                                                                                                          \
+    return bn == 256 ? launch_pdl(plora_gemm_fused_kernel<KIND, F32, 256>, grid, block, gemm_smem(256), stream, pdl, xmap, wmap, ymap, st_,   \
+                                  sn, T, N, K, segs, lay, table, parts, S, lds, status)                                                      \
+                     : launch_pdl(plora_gemm_fused_kernel<KIND, F32, 128>, grid, block, gemm_smem(128), stream, pdl, xmap, wmap, ymap, st_,   \
+                                  sn, T, N, K, segs, lay, table, parts, S, lds, status)
     if (kind == 0) {
         if (f32_out) PLORA_GEMM_LAUNCH(0, true);
         PLORA_GEMM_LAUNCH(0, false);
