@@ -14,7 +14,8 @@
 //   warps 2..9  stage the adapter passes of the next tile, then run its epilogue. A pass = one tensor-core tile of the
 //               step's grouping (a run of one slot's tokens) that meets the pair's rows x 64 columns of the slot's rank:
 //               S rows (plane 0, other rows zero) split into bf16 high and low parts, and the block's rows of B_p, in
-//               the unswizzled core-matrix layout. The MMA warp takes a pass as soon as it is staged, in the middle of
+//               rows of 128 bytes with the 128-byte swizzle (the same products from unswizzled operands, whose rows
+//               collide in shared memory, took a fifth of the FP8 layer's time). The MMA warp takes a pass as soon as it is staged, in the middle of
 //               the main loop.
 // bf16: the adapter products accumulate onto the base product; two accumulators of BN columns, so the epilogue of a tile
 // runs under the next tile's main loop. FP8: the base product has to be scaled first, so the adapter term has an
@@ -235,13 +236,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                 auto pass = [&]() {
                     tc_fence_after();
                     const int rw = sh.rw[ps];
-                    const uint32_t sbo = (uint32_t)rw * 16u;
-                    const uint32_t a_hi = smem_u32(Ahi), a_lo = smem_u32(Alo), b = smem_u32(Bop);
-                    for (int kk = 0; kk < rw / 16; kk++)
-                        pair_umma<1>(ad, umma_desc(a_hi + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad,
-                                     KIND == 1 || (ps | kk) != 0);
-                    for (int kk = 0; kk < rw / 16; kk++)
-                        pair_umma<1>(ad, umma_desc(a_lo + kk * 256, 128, sbo, 0), umma_desc(b + kk * 256, 128, sbo, 0), idesc_ad, 1);
+                    const uint64_t a_hi = umma_desc(smem_u32(Ahi), 16, 1024, 2), a_lo = umma_desc(smem_u32(Alo), 16, 1024, 2);
+                    const uint64_t b = umma_desc(smem_u32(Bop), 16, 1024, 2);
+                    for (int kk = 0; kk < rw / 16; kk++) pair_umma<1>(ad, a_hi + 2 * kk, b + 2 * kk, idesc_ad, KIND == 1 || (ps | kk) != 0);
+                    for (int kk = 0; kk < rw / 16; kk++) pair_umma<1>(ad, a_lo + 2 * kk, b + 2 * kk, idesc_ad, 1);
                     pair_commit(&sh.ad_empty);
                     ps++;
                     apar ^= 1;
@@ -291,33 +289,41 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                 if (q < parts.n && n0 >= parts.off[q]) part = q;
             const int n_local = n0 - parts.off[part] + (int)rank * (BN / 2);  // this block's first row of B_p
             // ---- the tile's adapter passes: tensor-core tiles of the grouping that meet the pair's rows
-            if (e == 0) {
-                int np = 0;
+            if (ew == 0) {
                 const int n_mma = segs[SEG_N_MMA];
                 const int* ml = segs + lay.mma();
-                int lo = 0, hi = n_mma;  // first tile that ends after the first row
-                while (lo < hi) {
-                    const int mid = (lo + hi) >> 1;
-                    if (ml[3 * mid] + ml[3 * mid + 1] > m0) hi = mid;
-                    else lo = mid + 1;
+                // the first tile that ends after the first row: 32 probes a round
+                int lo = 0, n = n_mma;
+                while (n > 0) {
+                    const int step = (n + 31) >> 5, at = lo + lane * step;
+                    const unsigned past = __ballot_sync(0xffffffffu, lane * step >= n || ml[3 * at] + ml[3 * at + 1] > m0);
+                    const int q = past ? __ffs(past) - 1 : 32;  // tile lo + q * step is past, the one a step before is not
+                    if (q == 0) break;
+                    const int from = (q - 1) * step + 1, to = min(n, q * step);
+                    lo += from;
+                    n = to - from;
                 }
-                for (int q = lo; q < n_mma && ml[3 * q] < m0 + 2 * G_BM; q++) {
-                    const int start = ml[3 * q], len = ml[3 * q + 1], slot_id = ml[3 * q + 2];
-                    const int r = table[slot_id].r[part];
-                    for (int rc0 = 0; rc0 < r; rc0 += G_RC) {
-                        if (np == G_MAX_PASS) {
-                            atomicMax(status, PLORA_ERR_CAPACITY);
-                            break;
+                if (lane == 0) {
+                    int np = 0;
+                    for (int q = lo; q < n_mma && ml[3 * q] < m0 + 2 * G_BM; q++) {
+                        const int start = ml[3 * q], len = ml[3 * q + 1], slot_id = ml[3 * q + 2];
+                        const int r = table[slot_id].r[part];
+                        for (int rc0 = 0; rc0 < r; rc0 += G_RC) {
+                            if (np == G_MAX_PASS) {
+                                atomicMax(status, PLORA_ERR_CAPACITY);
+                                break;
+                            }
+                            sh.row0[np] = max(start, m0) - m0;
+                            sh.row1[np] = min(start + len, m0 + 2 * G_BM) - m0;
+                            sh.slot[np] = slot_id;
+                            sh.rc0[np] = rc0;
+                            sh.rw[np] = min(G_RC, r - rc0);
+                            np++;
                         }
-                        sh.row0[np] = max(start, m0) - m0;
-                        sh.row1[np] = min(start + len, m0 + 2 * G_BM) - m0;
-                        sh.slot[np] = slot_id;
-                        sh.rc0[np] = rc0;
-                        sh.rw[np] = min(G_RC, r - rc0);
-                        np++;
                     }
+                    sh.npass = np;
                 }
-                sh.npass = np;
+                __syncwarp();
             }
             if (KIND == 0)
                 for (int c = e; c < BN; c += G_EPI) sn_s[c] = n0 + c < N ? sn[n0 + c] : 0.f;
@@ -332,45 +338,45 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                 }
                 staged = true;
                 const plora_desc& d = table[sh.slot[ps]];
-                const int rw = sh.rw[ps], rc0 = sh.rc0[ps], r = d.r[part], P = rw >> 3;
-                const uint32_t sbo = (uint32_t)rw * 16u;
-                // rows of B_p for the block's half of the columns
-                const bf16* B = reinterpret_cast<const bf16*>(d.b[part]);
-                for (int q = e; q < BN / 2 * P; q += G_EPI) {
-                    const int n = q / P, j = q - n * P;
+                const int rc0 = sh.rc0[ps], r = d.r[part], P = sh.rw[ps] >> 3;
+                // eight threads a row, one 16-byte piece of 8 ranks each: rows of B_p for the block's half of the columns
+                const int j = e & 7;
+                const bf16* B = reinterpret_cast<const bf16*>(d.b[part]) + rc0 + j * 8;
+#pragma unroll
+                for (int h = 0; h < BN / 64; h++) {
+                    const int n = (e >> 3) + 32 * h;
                     const bool valid = n_local + n < d.rows[part];
-                    cp_async16(Bop + (size_t)(n >> 3) * sbo + (n & 7) * 16 + j * 128,
-                               B + (size_t)(valid ? n_local + n : 0) * r + rc0 + j * 8, valid);
+                    if (j < P) cp_async16(Bop + (size_t)n * 128 + ((j ^ (n & 7)) << 4), B + (size_t)(valid ? n_local + n : 0) * r, valid);
                 }
-                // this block's token rows of S (zero outside the pass's rows), as bf16 high and low parts
-                {
-                    const int row = e & (G_BM - 1), rel = row + (int)rank * G_BM;
-                    const bool valid = rel >= sh.row0[ps] && rel < sh.row1[ps];
-                    const float* sp = S + (size_t)(m0 + (valid ? rel : 0)) * lds + d.r_off[part] + rc0;
-                    unsigned char* ahi = Ahi + (size_t)(row >> 3) * sbo + (row & 7) * 16;
-                    unsigned char* alo = Alo + (size_t)(row >> 3) * sbo + (row & 7) * 16;
-#pragma unroll 4
-                    for (int j = e / G_BM; j < P; j += G_EPI / G_BM) {
-                        float f[8];
-                        if (valid) {
-                            const float4 a = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
-                            const float4 b = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
-                            f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w, f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
-                        } else {
+                // ... and this block's token rows of S (zero outside the pass's rows), as bf16 high and low parts
+                const float* sp = S + d.r_off[part] + rc0 + j * 8;
+                float4 f[4][2];
 #pragma unroll
-                            for (int q = 0; q < 8; q++) f[q] = 0.f;
-                        }
-                        uint32_t hi[4], lo[4];
+                for (int h = 0; h < 4; h++) {
+                    const int rel = (e >> 3) + 32 * h + (int)rank * G_BM;
+                    f[h][0] = f[h][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (j < P && rel >= sh.row0[ps] && rel < sh.row1[ps]) {
+                        f[h][0] = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)(m0 + rel) * lds));
+                        f[h][1] = __ldcg(reinterpret_cast<const float4*>(sp + (size_t)(m0 + rel) * lds + 4));
+                    }
+                }
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const __nv_bfloat162 h2 = __floats2bfloat162_rn(f[2 * q], f[2 * q + 1]);
-                            const float2 hf = __bfloat1622float2(h2);
-                            const __nv_bfloat162 l2 = __floats2bfloat162_rn(f[2 * q] - hf.x, f[2 * q + 1] - hf.y);
-                            hi[q] = *reinterpret_cast<const uint32_t*>(&h2);
-                            lo[q] = *reinterpret_cast<const uint32_t*>(&l2);
-                        }
-                        *reinterpret_cast<uint4*>(ahi + j * 128) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                        *reinterpret_cast<uint4*>(alo + j * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                for (int h = 0; h < 4; h++) {
+                    const int row = (e >> 3) + 32 * h;
+                    const float v[8] = {f[h][0].x, f[h][0].y, f[h][0].z, f[h][0].w, f[h][1].x, f[h][1].y, f[h][1].z, f[h][1].w};
+                    uint32_t hi[4], lo[4];
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const __nv_bfloat162 h2 = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+                        const float2 hf = __bfloat1622float2(h2);
+                        const __nv_bfloat162 l2 = __floats2bfloat162_rn(v[2 * q] - hf.x, v[2 * q + 1] - hf.y);
+                        hi[q] = *reinterpret_cast<const uint32_t*>(&h2);
+                        lo[q] = *reinterpret_cast<const uint32_t*>(&l2);
+                    }
+                    const uint32_t at = (uint32_t)row * 128u + (uint32_t)((j ^ (row & 7)) << 4);
+                    if (j < P) {
+                        *reinterpret_cast<uint4*>(Ahi + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+                        *reinterpret_cast<uint4*>(Alo + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
                     }
                 }
                 cp_async_wait_all();
@@ -536,15 +542,14 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
     CUtensorMap xmap, wmap, ymap;
     const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int el = kind == 0 ? 1 : 2;
-    // 256 output columns per tile, or 128 where that leaves fewer columns' worth of rounds: a step of few tokens has few
-    // tiles, and a round of one tile per pair that is nearly empty costs as much as a full one (96 tiles of 256 on 74
-    // pairs: 2 rounds; 192 of 128: 3 rounds of half the length). A tile of 128 moves 1.5 times the bytes per product, so
-    // it has to save more than a tenth.
-    auto rounds = [&](int width) {
+    // 256 output columns per tile, or 128 where that makes the rounds of the pairs shorter: a step of few tokens has few
+    // tiles, and a round that is nearly empty costs as much as a full one. A step of K costs what it moves into an SM,
+    // G_BM + bn / 2 rows of 128 bytes.
+    auto cost = [&](int width) {
         const long long tiles = (long long)((T + 2 * G_BM - 1) / (2 * G_BM)) * ((N + width - 1) / width);
-        return (double)((tiles + g_pairs - 1) / g_pairs) * width;
+        return ((tiles + g_pairs - 1) / g_pairs) * (G_BM + width / 2);
     };
-    const int bn = rounds(128) < 0.9 * rounds(256) ? 128 : 256;
+    const int bn = cost(128) < cost(256) ? 128 : 256;
     if (!encode2d(&xmap, dt, x, (uint64_t)K, (uint64_t)T, (uint64_t)K * el, G_BKB / el, G_BM)) return cudaErrorInvalidValue;
     if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)bn / 2)) return cudaErrorInvalidValue;
     if (!encode2d(&ymap, f32_out ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, (uint64_t)N,
