@@ -297,7 +297,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
     h->seg.max_tokens = max_tokens;
     h->seg.cap_tiles = h->cap_tiles;
     h->seg.run_min = 1 << 30;  // every run takes the gather path unless the tile path can run (set below)
-    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 200 * 1024) {
+    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024) {
         delete h;
         return fail(nullptr, PLORA_ERR_CAPACITY,
                     "limits: max_slots <= 1023, max_rank <= 512, and max_tokens/16 + max_seqs tiles must fit the "

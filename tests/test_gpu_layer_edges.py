@@ -28,6 +28,31 @@ def test_row_quantisation_of_every_row_length(pe, oracle, cols):
     loras.close()
 
 
+def test_row_quantisation_of_every_mantissa(pe, oracle):
+    """Every eight-bit mantissa of an input under every one of a row's maximum, at three scales; inputs of all exponents that
+    give a normal, a subnormal and a zero e4m3."""
+    import torch
+    x = np.zeros((3 * 128, 128 * 20 + 8), np.float32)
+    m = (128 + np.arange(128, dtype=np.float32)) / 128
+    for i, scale in enumerate([1.0, 2.0 ** 40, 2.0 ** -40]):
+        for k in range(128):
+            row = np.concatenate([m * np.float32(2.0 ** -e) for e in range(1, 21)]).astype(np.float32)
+            row[1::2] *= -1
+            x[128 * i + k, :len(row)] = row * np.float32(scale)
+            x[128 * i + k, -1] = m[k] * np.float32(scale)  # the maximum
+    xb = pe.bf16_bits(x).reshape(x.shape)
+    loras = pe.Loras([pe.Site.fused(0, x.shape[1], [("a", 64)])], 1, 16, 384, device=0)
+    xd = harness.to_dev_bf16(xb, 0)
+    xq = torch.zeros(x.shape, dtype=torch.uint8, device="cuda")
+    st = torch.zeros(len(x), dtype=torch.float32, device="cuda")
+    loras.fp8_quant_rows(xd.data_ptr(), len(x), x.shape[1], xq.data_ptr(), st.data_ptr())
+    torch.cuda.synchronize()
+    want_q, want_s = oracle.fp8_quant_rows(xb)
+    assert np.array_equal(st.cpu().numpy(), want_s)
+    assert np.array_equal(xq.cpu().numpy(), want_q)
+    loras.close()
+
+
 LAYERS = [
     # name, rows of the sequences, ranks, input width, part widths
     ("one-row", [1], [16], 64, [256]),
