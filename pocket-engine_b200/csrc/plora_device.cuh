@@ -119,6 +119,12 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     return v;
 }
 
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+
 // Programmatic dependent launch. Every kernel of the path waits for the kernels before it and only then
 // lets the next one start its prologue, so a prologue may read anything written two or more kernels back
 // (slabs, descriptors, the step's grouping) but nothing the kernel right before it writes.
@@ -130,36 +136,6 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // "the kernel before me is done" keeps meaning "everything before me is done".
 __device__ __forceinline__ void pdl_exit_idle() {
     if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
-}
-
-__device__ __forceinline__ uint4 lds16(const void* p) { return *reinterpret_cast<const uint4*>(p); }
-
-// 16 values per lane -> their 16 warp-wide sums in 16 shuffles; returns the sum of value (lane >> 1) & 15.
-__device__ __forceinline__ float reduce16(float (&v)[16], int lane) {
-#pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const float send = (lane & 16) ? v[i] : v[i + 8];
-        const float keep = (lane & 16) ? v[i + 8] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        const float send = (lane & 8) ? v[i] : v[i + 4];
-        const float keep = (lane & 8) ? v[i + 4] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++) {
-        const float send = (lane & 4) ? v[i] : v[i + 2];
-        const float keep = (lane & 4) ? v[i + 2] : v[i];
-        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, 4);
-    }
-    {
-        const float send = (lane & 2) ? v[0] : v[1];
-        const float keep = (lane & 2) ? v[1] : v[0];
-        v[0] = keep + __shfl_xor_sync(0xffffffffu, send, 2);
-    }
-    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 // Hints that the 128-byte line holding `p` will be read soon: the line is brought into L2, no value is bound,

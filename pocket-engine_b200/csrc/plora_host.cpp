@@ -275,10 +275,10 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             }
             si.parts.push_back(part);
         }
-        // K-split of the shrink, a function of the site alone: chunks of at least 512 inputs, at most 16
-        // of them, but never wider than 2048 (what one block stages in shared memory).
-        int want = std::max((si.cols + 2047) / 2048, std::min(16, std::max(1, (si.cols + 511) / 512)));
-        si.kchunk = next_mult((si.cols + want - 1) / want, 256);
+        // K-split of the shrink, a function of the site alone: about 2048 inputs each, at most eight of them, in multiples
+        // of the 1024 inputs of the gather shrink's pieces
+        const int want = std::min(8, std::max(1, (si.cols + 2047) / 2048));
+        si.kchunk = next_mult((si.cols + want - 1) / want, 1024);
         si.nsplit = (si.cols + si.kchunk - 1) / si.kchunk;
         h->nsplit_max = std::max(h->nsplit_max, si.nsplit);
         for (size_t p = 0; p < si.parts.size() && p < PLORA_MAX_PARTS; p++) {
@@ -345,7 +345,10 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             h->rec_cap = std::min(h->cap_tiles, max_slots + max_tokens / PLORA_WORK_TOKENS) + 1;
             const size_t rec_bytes = sizeof(PloraRec) * h->sites.size() * (size_t)h->rec_cap;
             check("alloc launch records", cudaMalloc((void**)&h->recs, rec_bytes));
-            check("alloc layer widths", cudaMalloc((void**)&h->site_cols, 2 * h->sites.size() * sizeof(int32_t)));
+            check("alloc layer widths", cudaMalloc((void**)&h->site_cols, 4 * h->sites.size() * sizeof(int32_t)));
+            const size_t prefix_bytes = h->sites.size() * 2 * (size_t)(h->rec_cap + 2) * sizeof(int32_t);
+            check("alloc unit counts", cudaMalloc((void**)&h->prefix, prefix_bytes));
+            if (rc == PLORA_OK) check("zero unit counts", cudaMemset(h->prefix, 0, prefix_bytes));
             if (rc == PLORA_OK) check("zero launch records", cudaMemset(h->recs, 0, rec_bytes));
             check("alloc status", cudaMalloc((void**)&h->status, 64));
             check("kernel attributes", plora_kernels_init(h->seg));
@@ -362,6 +365,8 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
                 }
                 info.push_back(s.cols);
                 info.push_back(s.cluster_ok ? 8 * nsub : 0);
+                info.push_back(s.nsplit);
+                info.push_back(0);
             }
             if (rc == PLORA_OK)
                 check("upload layer widths", cudaMemcpy(h->site_cols, info.data(), info.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -410,6 +415,7 @@ void plora_destroy(plora_t* h) {
         if (h->meta) cudaFree(h->meta);
         if (h->recs) cudaFree(h->recs);
         if (h->site_cols) cudaFree(h->site_cols);
+        if (h->prefix) cudaFree(h->prefix);
         if (h->host_meta) cudaFreeHost(h->host_meta);
         if (h->status) cudaFree(h->status);
         for (int p = 0; p < PLORA_XCHG_MAX_WORLD; p++)
@@ -881,7 +887,7 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
     SegLayout lay = h->seg;
     if (decode) lay.run_min = 1 << 30;
     CUK(h, "meta_group", plora_launch_meta_group(h->meta, segs, lay, h->status, h->tables, h->site_cols, (int)h->sites.size(),
-                                                 h->recs, h->rec_cap, h->pdl && h->tiles_built, as_stream(stream)));
+                                                 h->recs, h->rec_cap, h->prefix, h->pdl && h->tiles_built, as_stream(stream)));
     h->tiles_built = false;
     h->pdl_armed = 1;
     out->run_min = lay.run_min;
@@ -927,6 +933,8 @@ static PloraBounds bounds_of(const plora_t* h, const plora_hook* hook, int rows,
 }
 
 // the launch records of a layer for this step
+static const int32_t* shrink_units(const plora_t* h, int site) { return h->prefix + (size_t)site * 2 * (size_t)(h->rec_cap + 2); }
+static const int32_t* expand_units(const plora_t* h, int site) { return shrink_units(h, site) + h->rec_cap + 2; }
 static const PloraRec* recs_of(const plora_t* h, int site) { return h->recs + (size_t)site * (size_t)h->rec_cap; }
 
 static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* step, uint64_t x, int rows, bool early,
@@ -945,7 +953,7 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     h->pdl_armed = 2;
     CUK(h, "shrink",
        plora_launch_shrink((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
-                           (float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.kchunk, site.nsplit,
+                           shrink_units(h, hook->site), (float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.kchunk, site.nsplit,
                            work_cap, hook->parts * h->max_rank, bounds_of(h, hook, rows, 0), h->status, pdl, early, early_x,
                            late, as_stream(stream)));
     if (h->mma_ok && rows >= step->run_min)
@@ -1052,7 +1060,7 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     h->pdl_armed = 2;
     CUK(h, "expand",
        plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds,
-                           reduced ? 1 : site.nsplit, recs_of(h, hook->site), h->rec_cap,
+                           reduced ? 1 : site.nsplit, recs_of(h, hook->site), h->rec_cap, expand_units(h, hook->site),
                            (void*)(uintptr_t)y, ldy, f32_out, hook->parts, hook->max_rows, work_cap,
                            bounds_of(h, hook, rows, ldy), h->status, pdl, early, as_stream(stream)));
     if (h->mma_ok && rows >= step->run_min)
@@ -1103,7 +1111,7 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
     if (work_cap > 0)
         CUK(h, "expand (tokens outside long runs)",
            plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
-                               recs_of(h, hook->site), h->rec_cap, (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
+                               recs_of(h, hook->site), h->rec_cap, expand_units(h, hook->site), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                hook->max_rows, work_cap, bounds_of(h, hook, rows, ldy), h->status, h->pdl, false,
                                as_stream(stream)));
     return PLORA_OK;

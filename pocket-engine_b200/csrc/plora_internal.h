@@ -169,8 +169,9 @@ struct plora {
     int32_t* meta = nullptr;  // device: tile words, then segs
     PloraRec* recs = nullptr;  // device: [sites][rec_cap] launch records of the step
     int rec_cap = 0;
+    int32_t* prefix = nullptr;  // device: [sites][2][rec_cap + 2] units of the gather kernels before every work item of the step
     int32_t* host_meta = nullptr;  // pinned staging for plora_meta_upload
-    int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel} (for the launch records)
+    int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel, K-splits, 0} (for the launch records)
     int cap_tiles = 0;
     SegLayout seg;
     int* status = nullptr;  // device status word
@@ -250,9 +251,11 @@ __host__ __device__ inline int plora_tile_chunks(int K, int R) {
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st);
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
-// site_info: per layer {input width, blocks that share a work item's output columns in the cluster kernel (0: none)}
+// site_info: per layer {input width, blocks that share a work item's output columns in the cluster kernel (0: none),
+// K-splits of the gather shrink, 0}; prefix: per layer the unit counts of the gather shrink and expand before every item
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, bool pdl, cudaStream_t st);
+                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
+                                    cudaStream_t st);
 // Dynamic shared-memory limit of a kernel together with a request for the largest shared-memory split of the SM.
 // Kernels of this library overlap with their neighbours in the stream (programmatic dependent launch); an SM's
 // split between L1 and shared memory is fixed while any block runs on it, so kernels that each let the driver
@@ -299,10 +302,10 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
 // early: dependents are released at kernel start and slabs are requested ahead of the dependency wait (used by
 // plora_apply, whose kernels follow one another); early_x: x too may be read ahead of the wait; late: the kernel before
 // is the step's grouping, so not even a launch record may be read ahead of it
-cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, float* S,
+cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, const int* prefix, float* S,
                                 size_t s_stride_elems, int lds, int kchunk, int nsplit, int work_cap, int max_rank_total,
                                 const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, bool late,
                                 cudaStream_t st);
 cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, int nsplit, const PloraRec* recs,
-                                int rec_cap, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
+                                int rec_cap, const int* prefix, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
                                 const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st);

@@ -12,8 +12,8 @@
 
 #include "plora_internal.h"
 #include "plora_device.cuh"
-
-typedef __nv_bfloat16 bf16;
+#include "plora_tc.cuh"
+#include "plora_tiles.cuh"
 
 
 namespace {
@@ -104,10 +104,22 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 }
 
 // ---------------------------------------------------------------------------------------------
+// Units of an item. Shrink: rows of the stacked A. Expand: output columns whose rows of B (2 r bytes each) and y of the
+// item's tokens (4 bytes each, counted twice: it is read, written and scattered) come to about 32 KB, in whole steps of a
+// block's eight warps. (With columns by rank alone, the blocks with the popular slots' items of 16 tokens took three
+// times as long as the rest.)
+#define SHR_ROWS 16
+#define SHR_PAD 20  // floats between the token rows of a warp's partial
+__host__ __device__ __forceinline__ int expand_unit_cols(int r, int cnt) {
+    const int step = r <= 64 ? 256 : 128, cols = 32768 / (2 * r + 8 * cnt) / step * step;
+    return cols > step ? cols : step;
+}
+
 // One launch record: gather work item w resolved against one layer's descriptor table, so that the kernels of
 // that layer make one metadata fetch per block. `o` is the record's 16 uint4.
-__device__ __forceinline__ void write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
-                                             int cols, int pieces) {
+// Returns the item's units of the few-token kernels: (expand << 32) | shrink.
+__device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
+                                             int cols, int pieces, int nsplit) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
     const uint4 head = work[0];  // slot, perm start, count, 0
     const int slot = (int)head.x;
@@ -139,6 +151,16 @@ __device__ __forceinline__ void write_record(uint4* o, const int* segs, const Se
     o[10] = work[3];
     o[11] = work[4];
     o[12] = make_uint4(cat[0], cat[1], cat[2], cat[3]);
+    unsigned long long ue = 0;
+#pragma unroll
+    for (int p = 0; p < PLORA_MAX_PARTS; p++) {
+        const int r = (int)dw[11 + p], rows = (int)dw[23 + p];
+        if (r > 0 && rows > 0) {
+            const int uc = expand_unit_cols(r, (int)head.z);
+            ue += (unsigned)((rows + uc - 1) / uc);
+        }
+    }
+    return (ue << 32) | (unsigned)(((int)dw[10] + SHR_ROWS - 1) / SHR_ROWS * nsplit);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -159,7 +181,8 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                                                                  SegLayout lay, int* __restrict__ status,
                                                                  const plora_desc* __restrict__ tables,
                                                                  const int* __restrict__ site_cols, int n_sites,
-                                                                 PloraRec* __restrict__ recs, int rec_cap) {
+                                                                 PloraRec* __restrict__ recs, int rec_cap,
+                                                                 int* __restrict__ prefix) {
     extern __shared__ int sm[];
     __shared__ unsigned long long sh[4][33];  // a row per scan in flight: no barrier between one scan and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -394,42 +417,104 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     // launch records (the barrier above made the work items, written by other threads of this block, visible)
     if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
-        const int mine = ((int)blockIdx.x < n_sites) ? (n_sites - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-        for (int i = tid; i < mine * end; i += 1024) {
-            const int q = i / end, w = i - q * end, site = (int)blockIdx.x + q * (int)gridDim.x;
-            uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
-            const int cols = site_cols[2 * site];
-            if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
-            else write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, site_cols[2 * site + 1]);
+        for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
+            const int cols = site_cols[4 * site], pieces = site_cols[4 * site + 1], nsplit = site_cols[4 * site + 2];
+            // a layer's prefix counts: [items, units before item 0, 1, ..., all] for the shrink, then for the expand
+            int* ps = prefix + (size_t)site * 2 * (size_t)(rec_cap + 2);
+            int* pe = ps + rec_cap + 2;
+            unsigned long long before = 0;
+            for (int base = 0; base < end; base += 1024) {
+                const int w = base + tid;
+                unsigned long long units = 0, total = 0;
+                if (w < end) {
+                    uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
+                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, pieces, nsplit);
+                }
+                const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
+                if (w < nw) {
+                    ps[1 + w] = (int)(at & 0xffffffffu);
+                    pe[1 + w] = (int)(at >> 32);
+                }
+                before += total;
+            }
+            if (tid == 0) {
+                ps[0] = pe[0] = nw;
+                ps[1 + nw] = (int)(before & 0xffffffffu);
+                pe[1 + nw] = (int)(before >> 32);
+            }
+            __syncthreads();
         }
     }
 }
 
-// Shrink over gather work items. Grid (K-splits x row tiles, 1, work items); 128 threads. A work item is up
-// to 16 tokens of one slot, described by one launch record. The block's rows of the slot's stacked A (one
-// K-chunk wide) arrive in shared memory by bulk async copies issued before the dependency wait; the tokens'
-// x chunks follow right after it. Each warp takes 4 of every 16 rows and 4 tokens at a time, its lanes 8
-// inputs each per 256-wide step; sums cross the warp by shuffles. Every (token, row, split) is written
-// exactly once.
-__global__ void __launch_bounds__(128) plora_shrink_gather_kernel(const bf16* __restrict__ X, int ldx, int K,
-                                                                   const PloraRec* __restrict__ recs, int rec_cap,
-                                                                   float* __restrict__ S, size_t s_stride, int lds,
-                                                                   int kchunk, int rps, int rt_max, int early, int early_x,
-                                                                   int late, int* __restrict__ status PLORA_BOUNDS_PARAM) {
+// ---------------------------------------------------------------------------------------------
+// The few-token kernels below share a form. Their work is a list of equal units over all work items of the layer, found
+// through a prefix count per item that the grouping kernel wrote: a step's slots differ up to 8-fold in rank and its
+// layers in width, so a grid of (items x most tiles an item can have) is mostly idle blocks next to a few long ones. Two
+// blocks per SM take an equal, contiguous range of units each. In a block, a producer warp walks the units ahead of the
+// eight computing warps and keeps a ring of three 32 KB pieces full of slab rows by bulk copies, beginning before the
+// dependency wait: 190 KB in flight per SM, where two steps' worth of operand registers per warp were not enough (25 us for
+// 52 MB of A, 80 us for 157 MB of B). The products are tiles of the warp-level tensor instruction (m16n8k16; a 128-row tcgen05
+// tile would spend 7/8 or more of its rows on tokens that are not there; on the CUDA cores both kernels were bound by
+// instructions). Its 16 input slots may be permuted freely as long as both operands agree, so lane t of four holds inputs
+// 8 t .. 8 t + 7 of a row's 32 (two multiplies), and operands move in 16-byte pieces.
+
+// The prefix counts of a layer in shared memory: pre[0] = items, pre[1 + w] = units before item w, pre[1 + items] = all
+__device__ __forceinline__ int load_prefix(int* pre, const int* __restrict__ src, int rec_cap) {
+    for (int i = threadIdx.x; i < min(rec_cap + 2, (int)blockDim.x); i += blockDim.x) pre[i] = __ldcg(src + i);
+    __syncthreads();
+    const int n = min(pre[0], rec_cap);
+    for (int i = (int)blockDim.x + threadIdx.x; i < n + 2; i += blockDim.x) pre[i] = __ldcg(src + i);
+    if (n + 2 > (int)blockDim.x) __syncthreads();
+    return pre[1 + n];
+}
+// the item that unit u belongs to
+__device__ __forceinline__ int find_item(const int* pre, int u) {
+    int lo = 0, hi = pre[0];
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[1 + mid] <= u) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+// barrier among the eight warps that compute (the producer warp does not take part)
+__device__ __forceinline__ void gather_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+
+#define GATHER_STAGES 3
+#define GATHER_THREADS 288  // eight computing warps and the producer
+
+// Shrink: unit = (item, one of the layer's K-splits, 16 rows of the slot's stacked A), in pieces of 1024 inputs. Every warp
+// multiplies the item's tokens (16 rows of the tile) by the 16 rows of A over its 128 inputs of each piece, the
+// eight partials are added in warp order in shared memory, and every (token, row, split) is written exactly once.
+// Bound by the slabs' bytes (A of every slot present once).
+#define SHR_PIECE 1024
+#define SHR_PITCH (SHR_PIECE * 2 + 64)  // bytes between rows of a piece: eight lanes' 16-byte reads then meet all banks
+#define SHR_STAGE (SHR_ROWS * SHR_PITCH)
+__global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(const bf16* __restrict__ X, int ldx, int K,
+                                                                      const PloraRec* __restrict__ recs, int rec_cap,
+                                                                      const int* __restrict__ prefix, float* __restrict__ S,
+                                                                      size_t s_stride, int lds, int kchunk, int nsplit, int early,
+                                                                      int early_x, int late, int* __restrict__ status PLORA_BOUNDS_PARAM) {
     // late != 0: the kernel before is the step's grouping, which writes the records: nothing is read, and no dependent
     // released, before the dependency wait. (The launch itself then overlaps the grouping.)
     // early != 0: dependents are released at kernel start (every store of the path comes after a wait).
     // early_x != 0: the caller vouches that x is older than every kernel still in flight, so x is fetched and
     // the partial sums computed before the dependency wait; only the stores into S (which the expand before may
     // still be reading) come after it.
-    extern __shared__ __align__(128) unsigned char dsm[];
-    __shared__ __align__(8) uint64_t bars[2];
-    __shared__ PloraRec srec;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    extern __shared__ __align__(128) unsigned char gsm[];
+    __shared__ __align__(16) PloraRec srec[2];
+    __shared__ __align__(8) uint64_t full[GATHER_STAGES], empty[GATHER_STAGES];
+    float* red = reinterpret_cast<float*>(gsm + GATHER_STAGES * SHR_STAGE);  // [8 warps][16][SHR_PAD]
+    int* pre = reinterpret_cast<int*>(red + 8 * 16 * SHR_PAD);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     if (early && !late) pdl_trigger();
-    if (threadIdx.x == 0) {
-        mbar_init(&bars[0], 1);
-        mbar_init(&bars[1], 1);
+    if (tid == 0) {
+        for (int i = 0; i < GATHER_STAGES; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 8);
+        }
         mbar_fence_init();
     }
     bool waited = false;
@@ -438,284 +523,544 @@ __global__ void __launch_bounds__(128) plora_shrink_gather_kernel(const bf16* __
         pdl_trigger();
         waited = true;
     }
-    uint32_t phase = 0;
-    const int split = blockIdx.x / rt_max, rt = blockIdx.x - split * rt_max;
-    const int row0 = rt * rps;
-    const int k0 = split * kchunk, klen = min(kchunk, K - k0);
-    const uint32_t kbytes = (uint32_t)klen * 2u;
-    // the grid's z extent is capped: a block walks the work items z, z + gridDim.z, ...
-    for (int w = blockIdx.z; w < rec_cap; w += gridDim.z) {
-    if (threadIdx.x < 12) reinterpret_cast<uint4*>(&srec)[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(recs + w) + threadIdx.x);
-    __syncthreads();
-    const int cnt = srec.cnt, rank = srec.rank;
-    if (cnt == 0) break;
+    const int total = load_prefix(pre, prefix, rec_cap);  // (its barrier publishes the ring's as well)
+    const int u0 = (int)((long long)total * blockIdx.x / gridDim.x), u1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+    if (u0 >= u1) {
+        if (!waited) pdl_exit_idle();
+        return;
+    }
+    // a unit's place: its item, its split and first row (units of an item go split by split, so that the rows of A of a split
+    // find the tokens' x in L2)
+    struct Place {
+        int item, k0, split, row0;
+    };
+    auto place = [&](int u, int item) {
+        Place q;
+        while (pre[2 + item] <= u) item++;  // (items without units are passed over)
+        q.item = item;
+        const int n = (pre[2 + item] - pre[1 + item]) / nsplit, local = u - pre[1 + item];
+        q.split = local / n;
+        q.k0 = q.split * kchunk;
+        q.row0 = (local - q.split * n) * SHR_ROWS;
+        return q;
+    };
+    auto fine = [&](const PloraRec& rec, const Place& q) {
 #ifdef PLORA_BOUNDS
-    if (!rec_in_bounds(srec, bnd, K)) {
-        if (threadIdx.x == 0) atomicMax(status, PLORA_ERR_ARG);
-        __syncthreads();
-        continue;
-    }
+        return rec_in_bounds(rec, bnd, K) && q.row0 + SHR_ROWS <= rec.rank;
+#else
+        (void)rec, (void)q;
+        return true;
 #endif
-    if (row0 >= rank) {
-        __syncthreads();
-        continue;
-    }
-    const int rows = min(rps, rank - row0);
-    unsigned char* As = dsm;
-    unsigned char* Xs = dsm + (size_t)rps * kchunk * 2;
-    if (warp == 0) {
-        const bf16* A = reinterpret_cast<const bf16*>(srec.a) + (size_t)row0 * K + k0;
-        if (lane == 0) mbar_expect_tx(&bars[0], (uint32_t)rows * kbytes);
-        __syncwarp();
-        for (int r = lane; r < rows; r += 32) bulk_g2s(As + (size_t)r * kbytes, A + (size_t)r * K, kbytes, &bars[0]);
-    } else if (!waited && !early_x) {
-        // hint only: the x lines this block will copy once the kernel before is done
-        const int lines = (int)((kbytes + 127) / 128);
-        for (int i = threadIdx.x - 32; i < cnt * lines; i += 96) {
-            const int t = i / lines, l = i - t * lines;
-            prefetch_l2(reinterpret_cast<const unsigned char*>(X + (size_t)srec.tok[t] * ldx + k0) + (size_t)l * 128);
+    };
+    int item = find_item(pre, u0);
+    if (warp == 8) {
+        int stg = 0, n = 0;
+        uint32_t par = 1;
+        bool ok = true;
+        for (int u = u0; ok && u < u1; u++) {
+            const Place q = place(u, item);
+            item = q.item;
+            if (!fine(recs[q.item], q)) continue;
+            const bf16* A = reinterpret_cast<const bf16*>(__ldcg(&recs[q.item].a)) + (size_t)(q.row0 + (lane & 15)) * K;
+            const int kend = min(K, q.k0 + kchunk);
+            for (int k = q.k0; k < kend; k += SHR_PIECE, n++) {
+                if (n >= GATHER_STAGES) ok = mbar_wait_long(&empty[stg], par, status);
+                if (!ok) break;
+                const uint32_t bytes = (uint32_t)min(SHR_PIECE, kend - k) * 2u;
+                if (lane == 0) mbar_expect_tx(&full[stg], bytes * SHR_ROWS);
+                __syncwarp();
+                if (lane < SHR_ROWS) bulk_g2s(gsm + (size_t)stg * SHR_STAGE + (size_t)lane * SHR_PITCH, A + k, bytes, &full[stg]);
+                if (++stg == GATHER_STAGES) {
+                    stg = 0;
+                    par ^= 1;
+                }
+            }
         }
+        if (!waited) pdl_wait();
+        return;
     }
+    // ---- computing warps
+    auto fetch = [&](int w, int at) {
+        if (tid < 12) reinterpret_cast<uint4*>(&srec[at])[tid] = __ldcg(reinterpret_cast<const uint4*>(recs + w) + tid);
+    };
+    const bf16 *x0 = nullptr, *x1 = nullptr;
+    bool two = false;
+    uint4 xv[4][2];
+    auto aim = [&](const PloraRec& rec) {
+        x0 = X + (size_t)rec.tok[g < rec.cnt ? g : 0] * ldx + warp * 128 + 8 * t4;
+        x1 = X + (size_t)rec.tok[g + 8 < rec.cnt ? g + 8 : 0] * ldx + warp * 128 + 8 * t4;
+        two = rec.cnt > 8;  // (else rows 8 to 15 of the tile hold zeros, and their results are dropped)
+    };
+    auto load_x = [&](int k, int kend) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const bool in = k + warp * 128 + 32 * q + 8 * t4 < kend;
+            xv[q][0] = in ? __ldcg(reinterpret_cast<const uint4*>(x0 + k + 32 * q)) : make_uint4(0u, 0u, 0u, 0u);
+            xv[q][1] = in && two ? __ldcg(reinterpret_cast<const uint4*>(x1 + k + 32 * q)) : make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    Place here = place(u0, item);
+    fetch(here.item, 0);
+    gather_sync();
+    bool good = fine(srec[0], here);
+    if (!good && tid == 0) atomicMax(status, PLORA_ERR_ARG);
+    aim(srec[0]);
     if (!early_x && !waited) {
         pdl_wait();
         if (!early) pdl_trigger();
         waited = true;
     }
-    if (warp == 0) {
-        if (lane == 0) mbar_expect_tx(&bars[1], (uint32_t)cnt * kbytes);
-        __syncwarp();
-        if (lane < cnt) bulk_g2s(Xs + (size_t)lane * kbytes, X + (size_t)srec.tok[lane] * ldx + k0, kbytes, &bars[1]);
-    }
-    if (!mbar_wait(&bars[0], phase, status)) return;
-    if (!mbar_wait(&bars[1], phase, status)) return;
-    phase ^= 1;
-    float* Sout = S + (size_t)split * s_stride;
-    float res[PLORA_WORK_TOKENS / 4];  // rows == 16: one 4-row group per warp, one value per token pass
+    if (good) load_x(here.k0, min(K, here.k0 + kchunk));
+    int stg = 0;
+    uint32_t par = 0;
+    bool ok = true;
+    for (int u = u0, at = 0; ok && u < u1; u++, at ^= 1) {
+        Place next = here;
+        if (u + 1 < u1) {
+            next = place(u + 1, here.item);
+            fetch(next.item, at ^ 1);
+        }
+        float acc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+        const int kend = min(K, here.k0 + kchunk);
+#pragma unroll 1
+        for (int k = here.k0; good && k < kend; k += SHR_PIECE) {
+            ok = mbar_wait_long(&full[stg], par, status);
+            if (!ok) break;
+            const uint32_t a = smem_u32(gsm) + (uint32_t)stg * SHR_STAGE + (uint32_t)g * SHR_PITCH + (uint32_t)(warp * 256 + 16 * t4);
 #pragma unroll
-    for (int tq = 0; tq < PLORA_WORK_TOKENS / 4; tq++) {
-        const int tp = 4 * tq;
-        res[tq] = 0.f;
-        if (tp >= cnt) continue;
-        const int nt = min(4, cnt - tp);
-        {
-            const int n0 = warp * 4;
-            float acc[16];
+            for (int q = 0; q < 4; q++) {
+                if (k + warp * 128 + 32 * q < kend) {
+                    const uint4 &x = xv[q][0], &z = xv[q][1];
+                    const uint32_t f0[4] = {x.x, z.x, x.y, z.y}, f1[4] = {x.z, z.z, x.w, z.w};
+                    const bool in = k + warp * 128 + 32 * q + 8 * t4 < kend;
 #pragma unroll
-            for (int i = 0; i < 16; i++) acc[i] = 0.f;
-            for (int k = lane * 8; k < klen; k += 256) {
-                float xf[4][8];
-#pragma unroll
-                for (int t = 0; t < 4; t++) unpack8(lds16(Xs + (size_t)(tp + min(t, nt - 1)) * kbytes + k * 2), xf[t]);
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    float af[8];
-                    unpack8(lds16(As + (size_t)(n0 + r) * kbytes + k * 2), af);
-#pragma unroll
-                    for (int t = 0; t < 4; t++)
-#pragma unroll
-                        for (int e = 0; e < 8; e++) acc[r * 4 + t] = fmaf(xf[t][e], af[e], acc[r * 4 + t]);
+                    for (int i = 0; i < 2; i++) {
+                        uint4 b = make_uint4(0u, 0u, 0u, 0u);
+                        if (in) b = lds128(a + (uint32_t)(8 * i) * SHR_PITCH + 64u * q);
+                        mma_16816(acc[i], f0, b.x, b.y);
+                        mma_16816(acc[i], f1, b.z, b.w);
+                    }
                 }
             }
-            res[tq] = reduce16(acc, lane);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty[stg]);
+            if (++stg == GATHER_STAGES) {
+                stg = 0;
+                par ^= 1;
+            }
+            if (k + SHR_PIECE < kend) load_x(k + SHR_PIECE, kend);
         }
-    }
-    if (!waited) {
-        pdl_wait();
-        if (!early) pdl_trigger();
-        waited = true;
-    }
-    if ((lane & 1) == 0) {
-        const int i = lane >> 1, r = i >> 2, t = i & 3;
+        float* mine = red + (size_t)warp * 16 * SHR_PAD + g * SHR_PAD + 2 * t4;
 #pragma unroll
-        for (int tq = 0; tq < PLORA_WORK_TOKENS / 4; tq++)
-            if (4 * tq + t < cnt) Sout[(size_t)srec.tok[4 * tq + t] * lds + row0 + warp * 4 + r] = res[tq];
+        for (int i = 0; i < 2; i++) {
+            *reinterpret_cast<float2*>(mine + 8 * i) = make_float2(acc[i][0], acc[i][1]);
+            if (two) *reinterpret_cast<float2*>(mine + 8 * SHR_PAD + 8 * i) = make_float2(acc[i][2], acc[i][3]);
+        }
+        gather_sync();  // the partials and the next record are there
+        const bool was = good && ok;
+        if (u + 1 < u1) {
+            good = fine(srec[at ^ 1], next);
+            if (!good && tid == 0) atomicMax(status, PLORA_ERR_ARG);
+            aim(srec[at ^ 1]);
+            if (good && (waited || early_x)) load_x(next.k0, min(K, next.k0 + kchunk));
+        }
+        if (!waited) {
+            pdl_wait();
+            if (!early) pdl_trigger();
+            waited = true;
+        }
+        const int t = tid >> 4, c = tid & 15;
+        if (was && t < srec[at].cnt) {
+            float sum = red[t * SHR_PAD + c];
+#pragma unroll
+            for (int q = 1; q < 8; q++) sum += red[q * 16 * SHR_PAD + t * SHR_PAD + c];
+            S[(size_t)here.split * s_stride + (size_t)srec[at].tok[t] * lds + here.row0 + c] = sum;
+        }
+        here = next;
+        gather_sync();  // shared memory is reused by the next unit
     }
-    __syncthreads();  // shared memory is reused by the next work item
-    }
-    if (!waited) pdl_exit_idle();
+    if (!waited) pdl_wait();
 }
 
-// Expand over gather work items. Grid (column blocks, parts, work items); 128 threads, two adjacent output
-// columns each. The block's rows of B arrive in shared memory by one bulk async copy issued before the
-// dependency wait, together with L2 prefetch hints for its y lines. After the wait, the work item's S rows
-// (K-split partials, all in flight together, added in split order) go to shared memory while the y values are
-// on their way; every thread then walks its two rows of B once per group of 4 tokens and writes y back.
-#define EXP_SPAD 12  // floats per 8-wide piece of an S row in shared memory (conflict-free for rotated reads)
+// Expand: unit = (item, part, some 32 KB worth of output columns), so that a block's range is a few stretches of columns of
+// one part for one item's tokens. The producer copies their rows of B (contiguous) and hints the lines of y that go with
+// them to L2. At the start of a stretch the computing warps put the item's S rows (K-split partials, added in split order)
+// into shared memory as three bf16 terms (high, middle, low part, whose products with bf16 B are exact in f32, so no
+// precision is given up against an f32 multiply-add chain); then each takes its groups of columns of every piece. An item's
+// tokens are taken 8 at a time, whatever their number, so that a token's result does not depend on the others: rows 0-7 of
+// the token tile carry one term of S and rows 8-15 another, two multiplies per 8 x 16 ranks ([low | zero], then
+// [high | middle]), and a lane adds its two rows. The rows of B go to the tiles of a group in an order that leaves every
+// lane with 8 (above 64 ranks: 4) adjacent columns of its token: y moves in pieces of 16 (8) bytes.
+// Bound by the bytes of B and y.
+#define EXP_PIECE 32768
+struct ExpandUnit {
+    int r, r_off;          // rank, first column of S
+    int c0, c1;            // the stretch of the part's columns
+    size_t ybase;          // column of y where the part starts
+};
+__device__ __forceinline__ int expand_piece_cols(int r) { return r <= 16 ? 1024 : r <= 32 ? 512 : r <= 64 ? 256 : 128; }
 
-// PASSES: whether the tile buffer is smaller than a block's columns at the maximum rank. NH: column pairs per
-// thread, half a block's width apart (2 for the 512-column blocks of wide layers: 128 threads instead of 256
-// hold the block's registers, so more blocks, and more bytes in flight, share an SM).
-template <bool PASSES, int NH>
-__global__ void __launch_bounds__(256 / NH, 4 * NH) plora_expand_gather_kernel(const float* __restrict__ S, size_t s_stride,
-                                                                      int lds, int nsplit,
+// Where the stretch at unit `local` of an item lies, at most `left` units of it; returns its units
+__device__ __forceinline__ int expand_stretch_at(const int* r, const int* rows, int cnt, int local, int left, int& part, int& c0, int& c1) {
+    for (part = 0; part < PLORA_MAX_PARTS; part++) {
+        if (r[part] <= 0 || rows[part] <= 0) continue;
+        const int uc = expand_unit_cols(r[part], cnt), n = (rows[part] + uc - 1) / uc;
+        if (local < n) {
+            const int take = min(left, n - local);
+            c0 = local * uc;
+            c1 = min(rows[part], (local + take) * uc);
+            return take;
+        }
+        local -= n;
+    }
+    part = c0 = c1 = 0;
+    return 1;
+}
+
+// The products of 8 tokens (row g of the planes at `sp`) with one group of NT tiles of 8 columns, whose rows of B start at
+// `rows` in shared memory. NARROW: a rank of 16; else up to 128, 32 ranks at a time.
+template <int NT, bool NARROW>
+__device__ __forceinline__ void expand_multiply(float (&d)[NT][4], uint32_t rows, int ncols, int r, uint32_t sp, uint32_t plane, int g, int t4) {
+    uint32_t col[NT];  // this lane's row of every tile (past the last column: any row, its products are dropped)
+#pragma unroll
+    for (int i = 0; i < NT; i++) col[i] = rows + (uint32_t)min(2 * NT * (g >> 1) + 2 * i + (g & 1), ncols - 1) * (uint32_t)r * 2u;
+    if (NARROW) {
+        const uint2 h = lds64(sp + 8u * t4), m = lds64(sp + plane + 8u * t4), l = lds64(sp + 2 * plane + 8u * t4);
+        const uint32_t al[4] = {l.x, 0u, l.y, 0u}, ah[4] = {h.x, m.x, h.y, m.y};
+#pragma unroll
+        for (int i = 0; i < NT; i++) {
+            const uint2 b = lds64(col[i] + 8u * t4);
+            mma_16816(d[i], al, b.x, b.y);
+            mma_16816(d[i], ah, b.x, b.y);
+        }
+    } else {
+#pragma unroll 1
+        for (int k = 0; k < r; k += 32) {
+            const uint32_t o = 2u * k + 16u * t4;
+            const bool in = k + 8 * t4 < r;  // (the second half of the last 32 ranks may lie outside)
+            const uint4 h = lds128(sp + o), m = lds128(sp + plane + o), l = lds128(sp + 2 * plane + o);
+            const uint32_t al0[4] = {l.x, 0u, l.y, 0u}, ah0[4] = {h.x, m.x, h.y, m.y}, al1[4] = {l.z, 0u, l.w, 0u}, ah1[4] = {h.z, m.z, h.w, m.w};
+#pragma unroll
+            for (int i = 0; i < NT; i++) {
+                uint4 b = make_uint4(0u, 0u, 0u, 0u);
+                if (in) b = lds128(col[i] + o);
+                mma_16816(d[i], al0, b.x, b.y);
+                mma_16816(d[i], ah0, b.x, b.y);
+                mma_16816(d[i], al1, b.z, b.w);
+                mma_16816(d[i], ah1, b.z, b.w);
+            }
+        }
+    }
+}
+
+// A lane's 2 NT adjacent columns of one token of y, in one or two pieces where the row allows it
+template <bool F32, int NT>
+struct YPiece {
+    uint32_t w[F32 ? 2 * NT : NT];
+};
+template <bool F32, int NT>
+__device__ __forceinline__ void y_load(YPiece<F32, NT>& q, const unsigned char* y, int cols, bool wide) {
+    constexpr int NW = F32 ? 2 * NT : NT;  // words
+    if (cols <= 0) return;
+    if (wide && cols >= 2 * NT) {
+        if (NW == 2) {
+            const uint2 v = __ldcg(reinterpret_cast<const uint2*>(y));
+            q.w[0] = v.x, q.w[1] = v.y;
+        } else {
+#pragma unroll
+            for (int i = 0; i < NW / 4; i++) {
+                const uint4 v = __ldcg(reinterpret_cast<const uint4*>(y) + i);
+                q.w[(4 * i) % NW] = v.x, q.w[(4 * i + 1) % NW] = v.y, q.w[(4 * i + 2) % NW] = v.z, q.w[(4 * i + 3) % NW] = v.w;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < NW; c++)  // (widths, offsets and pitches are even)
+            if (c * (F32 ? 1 : 2) < cols) q.w[c] = __ldcg(reinterpret_cast<const uint32_t*>(y) + c);
+    }
+}
+template <bool F32, int NT>
+__device__ __forceinline__ void y_store(const YPiece<F32, NT>& q, const float (&d)[NT][4], unsigned char* y, int cols, bool wide) {
+    constexpr int NW = F32 ? 2 * NT : NT;
+    if (cols <= 0) return;
+    uint32_t o[NW];
+#pragma unroll
+    for (int i = 0; i < NT; i++) {
+        const float a = d[i][0] + d[i][2], b = d[i][1] + d[i][3];
+        if (F32) {
+            o[(2 * i) % NW] = __float_as_uint(__uint_as_float(q.w[(2 * i) % NW]) + a);
+            o[(2 * i + 1) % NW] = __float_as_uint(__uint_as_float(q.w[(2 * i + 1) % NW]) + b);
+        } else {
+            const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.w[i]));
+            const __nv_bfloat162 s = __floats2bfloat162_rn(f.x + a, f.y + b);
+            o[i] = *reinterpret_cast<const uint32_t*>(&s);
+        }
+    }
+    if (wide && cols >= 2 * NT) {
+        if (NW == 2) {
+            *reinterpret_cast<uint2*>(y) = make_uint2(o[0], o[1]);
+        } else {
+#pragma unroll
+            for (int i = 0; i < NW / 4; i++)
+                reinterpret_cast<uint4*>(y)[i] = make_uint4(o[(4 * i) % NW], o[(4 * i + 1) % NW], o[(4 * i + 2) % NW], o[(4 * i + 3) % NW]);
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < NW; c++)
+            if (c * (F32 ? 1 : 2) < cols) reinterpret_cast<uint32_t*>(y)[c] = o[c];
+    }
+}
+
+// What a stretch needs besides its B: S of the item as planes in shared memory, and y
+struct ExpandStep {
+    const float* S;
+    size_t s_stride;
+    int lds, nsplit;
+    unsigned char* planes;  // three bf16 planes [16 tokens][s_pad bytes]
+    uint32_t s_pad;
+    unsigned char* Y;
+    int ldy;
+};
+
+// One piece of B (its rows in shared memory at `rows`, the part's columns [p0, p1)) for the item's tokens, by one warp
+template <int NT, bool NARROW, bool F32>
+__device__ __forceinline__ void expand_piece(uint32_t rows, int p0, int p1, const ExpandUnit& un, const ExpandStep& st,
+                                             const PloraRec& rec, int warp, int g, int t4) {
+    constexpr int ES = F32 ? 4 : 2, GC = 8 * NT;
+    const bool wide = ((reinterpret_cast<uintptr_t>(st.Y) | ((size_t)st.ldy * ES) | (un.ybase * ES)) & 15) == 0;
+#pragma unroll 1
+    for (int t0 = 0; t0 < rec.cnt; t0 += 8) {
+        const int t = min(t0 + g, rec.cnt - 1);
+        unsigned char* yrow = st.Y + ((size_t)rec.tok[t] * st.ldy + un.ybase) * ES;
+        const uint32_t sp = smem_u32(st.planes) + (uint32_t)t * st.s_pad;
+        const int end = t0 + g < rec.cnt ? p1 : 0;
+        int c = p0 + warp * GC;
+        YPiece<F32, NT> y, next;
+        y_load<F32, NT>(y, yrow + (size_t)(c + 2 * NT * t4) * ES, end - c - 2 * NT * t4, wide);
+#pragma unroll 1
+        for (; c < p1; c += 8 * GC) {
+            const int mine = c + 2 * NT * t4;
+            y_load<F32, NT>(next, yrow + (size_t)(mine + 8 * GC) * ES, end - mine - 8 * GC, wide);
+            float d[NT][4];
+#pragma unroll
+            for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+            expand_multiply<NT, NARROW>(d, rows + (uint32_t)(c - p0) * (uint32_t)un.r * 2u, p1 - c, un.r, sp, 16u * st.s_pad, g, t4);
+            y_store<F32, NT>(y, d, yrow + (size_t)mine * ES, end - mine, wide);
+            y = next;
+        }
+    }
+}
+
+// The same for ranks above 128, which no piece holds: the rows of B from global memory, 32 ranks at a time
+template <bool F32>
+__device__ __forceinline__ void expand_wide_rank(const bf16* B, const ExpandUnit& un, const ExpandStep& st, const PloraRec& rec, int warp, int g, int t4) {
+    constexpr int ES = F32 ? 4 : 2, NT = 2;
+    const bool wide = ((reinterpret_cast<uintptr_t>(st.Y) | ((size_t)st.ldy * ES) | (un.ybase * ES)) & 15) == 0;
+    const uint32_t plane = 16u * st.s_pad;
+#pragma unroll 1
+    for (int t0 = 0; t0 < rec.cnt; t0 += 8) {
+        const int t = min(t0 + g, rec.cnt - 1);
+        unsigned char* yrow = st.Y + ((size_t)rec.tok[t] * st.ldy + un.ybase) * ES;
+        const uint32_t sp = smem_u32(st.planes) + (uint32_t)t * st.s_pad;
+#pragma unroll 1
+        for (int c = un.c0 + warp * 8 * NT; c < un.c1; c += 64 * NT) {
+            const int mine = c + 2 * NT * t4, cols = t0 + g < rec.cnt ? un.c1 - mine : 0;
+            YPiece<F32, NT> y;
+            y_load<F32, NT>(y, yrow + (size_t)mine * ES, cols, wide);
+            float d[NT][4];
+#pragma unroll
+            for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < un.r; k += 32) {
+                const uint32_t o = 2u * k + 16u * t4;
+                const uint4 h = lds128(sp + o), m = lds128(sp + plane + o), l = lds128(sp + 2 * plane + o);
+                const uint32_t al0[4] = {l.x, 0u, l.y, 0u}, ah0[4] = {h.x, m.x, h.y, m.y}, al1[4] = {l.z, 0u, l.w, 0u}, ah1[4] = {h.z, m.z, h.w, m.w};
+#pragma unroll
+                for (int i = 0; i < NT; i++) {
+                    const int col = min(c + 2 * NT * (g >> 1) + 2 * i + (g & 1), un.c1 - 1);
+                    uint4 b = make_uint4(0u, 0u, 0u, 0u);
+                    if (k + 8 * t4 < un.r) b = __ldg(reinterpret_cast<const uint4*>(B + (size_t)col * un.r + k + 8 * t4));
+                    mma_16816(d[i], al0, b.x, b.y);
+                    mma_16816(d[i], ah0, b.x, b.y);
+                    mma_16816(d[i], al1, b.z, b.w);
+                    mma_16816(d[i], ah1, b.z, b.w);
+                }
+            }
+            y_store<F32, NT>(y, d, yrow + (size_t)mine * ES, cols, wide);
+        }
+    }
+}
+
+// S of an item's part, four values a thread and step: all planes on their way together, added in split order; the bf16
+// planes are filled up with zeros to a multiple of 32 ranks
+__device__ __forceinline__ void expand_stage_s(const ExpandUnit& un, const ExpandStep& st, const PloraRec& rec, int tid) {
+    const uint32_t plane = 16u * st.s_pad;
+    const int r4 = ((un.r + 31) & ~31) >> 2;
+    for (int i = tid; i < rec.cnt * r4; i += 256) {
+        const int t = i / r4, j = (i - t * r4) * 4;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (j < un.r) {
+            const float* sp = st.S + (size_t)rec.tok[t] * st.lds + un.r_off + j;
+            for (int s0 = 0; s0 < st.nsplit; s0 += 4) {
+                float4 v[4];
+#pragma unroll
+                for (int s = 0; s < 4; s++)
+                    v[s] = s0 + s < st.nsplit ? __ldcg(reinterpret_cast<const float4*>(sp + (size_t)(s0 + s) * st.s_stride)) : a;
+#pragma unroll
+                for (int s = 0; s < 4; s++) {
+                    if (s0 + s == 0) a = v[0];
+                    else if (s0 + s < st.nsplit) a.x += v[s].x, a.y += v[s].y, a.z += v[s].z, a.w += v[s].w;
+                }
+            }
+        }
+        const float f[4] = {a.x, a.y, a.z, a.w};
+        uint32_t w[3][2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+            const float2 hf = __bfloat1622float2(h);
+            const float m0 = f[2 * e] - hf.x, m1 = f[2 * e + 1] - hf.y;
+            const __nv_bfloat162 m = __floats2bfloat162_rn(m0, m1);
+            const float2 mf = __bfloat1622float2(m);
+            const __nv_bfloat162 l = __floats2bfloat162_rn(m0 - mf.x, m1 - mf.y);
+            w[0][e] = *reinterpret_cast<const uint32_t*>(&h);
+            w[1][e] = *reinterpret_cast<const uint32_t*>(&m);
+            w[2][e] = *reinterpret_cast<const uint32_t*>(&l);
+        }
+#pragma unroll
+        for (int q = 0; q < 3; q++) *reinterpret_cast<uint2*>(st.planes + q * plane + (size_t)t * st.s_pad + j * 2) = make_uint2(w[q][0], w[q][1]);
+    }
+}
+
+template <bool F32>
+__global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(const float* __restrict__ S, size_t s_stride, int lds, int nsplit,
                                                                       const PloraRec* __restrict__ recs, int rec_cap,
-                                                                      void* Y, int ldy, int f32_out, int nc, int bs_bytes,
+                                                                      const int* __restrict__ prefix, void* Y, int ldy, int s_pad,
                                                                       int early, int* __restrict__ status PLORA_BOUNDS_PARAM) {
     // early != 0: dependents are released at kernel start. No value of y is bound before the dependency wait
     // (the kernel before, the layer's matrix multiply, may still be writing it): only L2 prefetch hints.
-    extern __shared__ __align__(128) unsigned char dsm[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ PloraRec srec;
+    extern __shared__ __align__(128) unsigned char gsm[];
+    __shared__ __align__(16) PloraRec srec;
+    __shared__ __align__(8) uint64_t full[GATHER_STAGES], empty[GATHER_STAGES];
+    unsigned char* planes = gsm + GATHER_STAGES * EXP_PIECE;
+    int* pre = reinterpret_cast<int*>(planes + 3 * 16 * (size_t)s_pad);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
+    constexpr int ES = F32 ? 4 : 2;
     if (early) pdl_trigger();
-    if (threadIdx.x == 0) {
-        mbar_init(&bar, 1);
+    if (tid == 0) {
+        for (int i = 0; i < GATHER_STAGES; i++) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 8);
+        }
         mbar_fence_init();
     }
-    bool waited = false;
-    uint32_t phase = 0;
-    const int esize = f32_out ? 4 : 2;
-    // the grid's z extent is capped: a block walks the work items z, z + gridDim.z, ...
-    for (int w = blockIdx.z; w < rec_cap; w += gridDim.z) {
-    if (threadIdx.x < 12) reinterpret_cast<uint4*>(&srec)[threadIdx.x] = __ldg(reinterpret_cast<const uint4*>(recs + w) + threadIdx.x);
-    __syncthreads();
-    const int cnt = srec.cnt;
-    if (cnt == 0) break;
+    const int total = load_prefix(pre, prefix, rec_cap);  // (its barrier publishes the ring's as well)
+    const int u0 = (int)((long long)total * blockIdx.x / gridDim.x), u1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
+    if (u0 >= u1) return pdl_exit_idle();
+    const int w0 = find_item(pre, u0);
+    if (warp == 8) {
+        // ---- copies of B, and hints for y
+        int stg = 0, n = 0;
+        uint32_t par = 1;
+        bool ok = true;
+        for (int u = u0, w = w0; ok && u < u1;) {
+            while (pre[2 + w] <= u) w++;  // (items without units are passed over)
+            const PloraRec& rec = recs[w];
+            int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS], part, c0, c1;
+            const int cnt = __ldcg(&rec.cnt), tok = lane < PLORA_WORK_TOKENS ? __ldcg(&rec.tok[lane]) : 0;
+#pragma unroll
+            for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = __ldcg(&rec.r[p]), rows[p] = __ldcg(&rec.rows[p]);
 #ifdef PLORA_BOUNDS
-    if (!rec_in_bounds(srec, bnd, srec.cols)) {
-        if (threadIdx.x == 0) atomicMax(status, PLORA_ERR_ARG);
-        __syncthreads();
-        continue;
-    }
+            if (!rec_in_bounds(rec, bnd, rec.cols)) {
+                u = pre[2 + w];
+                continue;
+            }
 #endif
-    const int p = blockIdx.y, r = srec.r[p];
-    const int rows = srec.rows[p], c0 = blockIdx.x * nc;
-    if (r == 0 || c0 >= rows) {
-        __syncthreads();
-        continue;
-    }
-    const int ncols_all = min(nc, rows - c0);
-    // The tile buffer holds bs_bytes of B: all the block's columns for ranks up to bs_bytes / (2 nc), fewer
-    // columns per pass (a multiple of 32) for higher ranks, so that a high maximum rank does not cost every
-    // block, whatever its slot's rank, the shared memory that limits how many blocks share an SM.
-    const int sub = PASSES ? min(nc, max(32, (bs_bytes / (2 * r)) & ~31)) : nc;
-    int ncols = min(sub, ncols_all);
-    unsigned char* Bs = dsm;
-    float* ss = reinterpret_cast<float*>(dsm + bs_bytes);
-    const bf16* Bp = reinterpret_cast<const bf16*>(srec.b[p]);
-    if (threadIdx.x == 0) {
-        const uint32_t bytes = (uint32_t)ncols * (uint32_t)r * 2u;
-        mbar_expect_tx(&bar, bytes);
-        bulk_g2s(Bs, Bp + (size_t)c0 * r, bytes, &bar);
-    }
-    const int r_off = srec.r_off[p];
-    const int c = 2 * threadIdx.x;       // the thread's first column pair; pair h is h * HALF columns further
-    const int HALF = 2 * blockDim.x;
-    size_t ycol = (size_t)srec.off[p] + c0 + c;
-    if (!waited) {
-        // hints for the block's y lines, then the dependency wait
-        const size_t len = (size_t)ncols_all * esize;
-        const int lines = (int)((len + 127) / 128) + 1;
-        for (int i = threadIdx.x; i < cnt * lines; i += blockDim.x) {
-            const int t = i / lines, l = i - t * lines;
-            const size_t start = ((size_t)srec.tok[t] * ldy + srec.off[p] + c0) * esize;
-            const size_t at = (start & ~(size_t)127) + (size_t)l * 128;
-            if (at < start + len) prefetch_l2(reinterpret_cast<const unsigned char*>(Y) + at);
+            u += expand_stretch_at(r, rows, cnt, u - pre[1 + w], u1 - u, part, c0, c1);
+            const int rp = __ldcg(&rec.r[part]);
+            if (c0 >= c1 || rp > 128) continue;  // (ranks above 128 are read from global memory)
+            const bf16* B = reinterpret_cast<const bf16*>(__ldcg(&rec.b[part]));
+            const size_t off = (size_t)__ldcg(&rec.off[part]);
+            const int pc = expand_piece_cols(rp);
+            for (int p0 = c0; p0 < c1; p0 += pc, n++) {
+                const int p1 = min(c1, p0 + pc);
+                if (n >= GATHER_STAGES) ok = mbar_wait_long(&empty[stg], par, status);
+                if (!ok) break;
+                if (lane == 0) {
+                    const uint32_t bytes = (uint32_t)(p1 - p0) * (uint32_t)rp * 2u;
+                    mbar_expect_tx(&full[stg], bytes);
+                    bulk_g2s(gsm + (size_t)stg * EXP_PIECE, B + (size_t)p0 * rp, bytes, &full[stg]);
+                }
+                if (++stg == GATHER_STAGES) {
+                    stg = 0;
+                    par ^= 1;
+                }
+                const size_t len = (size_t)(p1 - p0) * ES;
+                const int lines = (int)((len + 127) / 128) + 1;
+                for (int i = lane; i < ((cnt * lines + 31) & ~31); i += 32) {
+                    const int t = i / lines, l = i - t * lines;
+                    const int tk = __shfl_sync(0xffffffffu, tok, t & 15);
+                    const size_t start = ((size_t)tk * ldy + off + p0) * ES, at = (start & ~(size_t)127) + (size_t)l * 128;
+                    if (t < cnt && at < start + len) prefetch_l2(reinterpret_cast<const unsigned char*>(Y) + at);
+                }
+            }
         }
         pdl_wait();
-        if (!early) pdl_trigger();
-        waited = true;
+        return;
     }
-    // y of a group of 4 tokens, all of the thread's pairs
-    float2 yv[4][NH];
-    auto load_y = [&](int tg) {
-#pragma unroll
-        for (int h = 0; h < NH; h++) {
-            if (c + h * HALF < ncols) {
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    if (tg + t < cnt) {
-                        const size_t at = (size_t)srec.tok[tg + t] * ldy + ycol + h * HALF;
-                        if (f32_out) yv[t][h] = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(Y) + at);
-                        else yv[t][h] = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(reinterpret_cast<const bf16*>(Y) + at));
+    const ExpandStep st = {S, s_stride, lds, nsplit, planes, (uint32_t)s_pad, reinterpret_cast<unsigned char*>(Y), ldy};
+    bool waited = false, ok = true;
+    int stg = 0;
+    uint32_t par = 0;
+    for (int u = u0, w = w0; ok && u < u1;) {
+        while (pre[2 + w] <= u) w++;
+        if (tid < 12) reinterpret_cast<uint4*>(&srec)[tid] = __ldcg(reinterpret_cast<const uint4*>(recs + w) + tid);
+        gather_sync();
+        if (!waited) {
+            pdl_wait();
+            if (!early) pdl_trigger();
+            waited = true;
+        }
+#ifdef PLORA_BOUNDS
+        if (!rec_in_bounds(srec, bnd, srec.cols)) {
+            if (tid == 0) atomicMax(status, PLORA_ERR_ARG);
+            u = pre[2 + w];
+            gather_sync();
+            continue;
+        }
+#endif
+        ExpandUnit un;
+        int part;
+        u += expand_stretch_at(srec.r, srec.rows, srec.cnt, u - pre[1 + w], u1 - u, part, un.c0, un.c1);
+        if (un.c0 < un.c1) {
+            un.r = srec.r[part], un.r_off = srec.r_off[part];
+            un.ybase = (size_t)srec.off[part];
+            expand_stage_s(un, st, srec, tid);
+            gather_sync();
+            if (un.r > 128) {
+                expand_wide_rank<F32>(reinterpret_cast<const bf16*>(srec.b[part]), un, st, srec, warp, g, t4);
+            } else {
+                const int pc = expand_piece_cols(un.r);
+                for (int p0 = un.c0; p0 < un.c1; p0 += pc) {
+                    const int p1 = min(un.c1, p0 + pc);
+                    ok = mbar_wait_long(&full[stg], par, status);
+                    if (!ok) break;
+                    const uint32_t rows = smem_u32(gsm) + (uint32_t)stg * EXP_PIECE;
+                    if (un.r <= 16) expand_piece<4, true, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
+                    else if (un.r <= 64) expand_piece<4, false, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
+                    else expand_piece<2, false, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&empty[stg]);
+                    if (++stg == GATHER_STAGES) {
+                        stg = 0;
+                        par ^= 1;
                     }
                 }
             }
         }
-    };
-    // y of the first token group: on its way before anything else is waited for
-    load_y(0);
-    const int P = r >> 3;  // 16-byte pieces per row of B
-    for (int i = threadIdx.x; i < cnt * r; i += blockDim.x) {
-        const int t = i / r, j = i - t * r;
-        const float* sp = S + (size_t)srec.tok[t] * lds + r_off + j;
-        float acc = 0.f;
-        for (int s0 = 0; s0 < nsplit; s0 += 8) {
-            float v[8];
-#pragma unroll
-            for (int s = 0; s < 8; s++) v[s] = s0 + s < nsplit ? __ldcg(sp + (size_t)(s0 + s) * s_stride) : 0.f;
-#pragma unroll
-            for (int s = 0; s < 8; s++)
-                if (s0 + s < nsplit) acc = s0 + s == 0 ? v[s] : acc + v[s];
-        }
-        ss[t * P * EXP_SPAD + (j >> 3) * EXP_SPAD + (j & 7)] = acc;
+        gather_sync();  // S and the record are replaced for the next stretch
     }
-    __syncthreads();
-    for (int cs = 0; cs < ncols_all; cs += sub) {
-    if (cs > 0) {
-        // the next columns of the block: the tile buffer is free once every thread is through the pass before
-        __syncthreads();
-        ncols = min(sub, ncols_all - cs);
-        if (threadIdx.x == 0) {
-            const uint32_t bytes = (uint32_t)ncols * (uint32_t)r * 2u;
-            mbar_expect_tx(&bar, bytes);
-            bulk_g2s(Bs, Bp + (size_t)(c0 + cs) * r, bytes, &bar);
-        }
-        ycol = (size_t)srec.off[p] + c0 + cs + c;
-        load_y(0);
-    }
-    if (!mbar_wait(&bar, phase, status)) return;
-    phase ^= 1;
-    const int rot = (P >= 8 ? threadIdx.x : threadIdx.x >> 1) % P;
-    const int sstride = P * EXP_SPAD;
-    for (int tg = 0; tg < cnt; tg += 4) {
-        if (tg > 0) load_y(tg);
-#pragma unroll
-        for (int h = 0; h < NH; h++) {
-            if (c + h * HALF >= ncols) continue;
-            const unsigned char* b0 = Bs + (size_t)(c + h * HALF) * r * 2;
-            const unsigned char* b1 = b0 + (size_t)r * 2;
-            float acc[4][2];
-#pragma unroll
-            for (int t = 0; t < 4; t++) acc[t][0] = acc[t][1] = 0.f;
-            int jp = rot;
-            for (int q = 0; q < P; q++) {
-                float f0[8], f1[8];
-                unpack8(lds16(b0 + jp * 16), f0);
-                unpack8(lds16(b1 + jp * 16), f1);
-#pragma unroll
-                for (int t = 0; t < 4; t++) {
-                    if (tg + t < cnt) {
-                        const float* sp = ss + (tg + t) * sstride + jp * EXP_SPAD;
-                        const float4 s0 = *reinterpret_cast<const float4*>(sp);
-                        const float4 s1 = *reinterpret_cast<const float4*>(sp + 4);
-                        const float sv[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-                        for (int e = 0; e < 8; e++) {
-                            acc[t][0] = fmaf(sv[e], f0[e], acc[t][0]);
-                            acc[t][1] = fmaf(sv[e], f1[e], acc[t][1]);
-                        }
-                    }
-                }
-                jp = jp + 1 == P ? 0 : jp + 1;
-            }
-#pragma unroll
-            for (int t = 0; t < 4; t++) {
-                if (tg + t < cnt) {
-                    const size_t at = (size_t)srec.tok[tg + t] * ldy + ycol + h * HALF;
-                    if (f32_out)
-                        *reinterpret_cast<float2*>(reinterpret_cast<float*>(Y) + at) =
-                            make_float2(yv[t][h].x + acc[t][0], yv[t][h].y + acc[t][1]);
-                    else
-                        *reinterpret_cast<__nv_bfloat162*>(reinterpret_cast<bf16*>(Y) + at) =
-                            __floats2bfloat162_rn(yv[t][h].x + acc[t][0], yv[t][h].y + acc[t][1]);
-                }
-            }
-        }
-    }
-    }
-    __syncthreads();  // shared memory is reused by the next work item
-    }
-    if (!waited) pdl_exit_idle();
+    if (!waited) pdl_wait();
 }
 
 }  // namespace
@@ -764,83 +1109,46 @@ cudaError_t plora_kernels_init(const SegLayout& lay) {
     // The few-token kernels overlap with their neighbours in the stream (programmatic dependent launch), and an SM's
     // split between L1 and shared memory is fixed while any block runs on it: all of them ask for the largest
     // split, so that a block of the next kernel finds room beside the blocks of this one.
-    const void* fns[5] = {reinterpret_cast<const void*>(plora_shrink_gather_kernel),
-                          reinterpret_cast<const void*>(plora_expand_gather_kernel<false, 1>),
-                          reinterpret_cast<const void*>(plora_expand_gather_kernel<true, 1>),
-                          reinterpret_cast<const void*>(plora_expand_gather_kernel<false, 2>),
-                          reinterpret_cast<const void*>(plora_expand_gather_kernel<true, 2>)};
-    for (int i = 0; i < 5 && e == cudaSuccess; i++) {
-        e = cudaFuncSetAttribute(fns[i], cudaFuncAttributeMaxDynamicSharedMemorySize, i == 0 ? 136 * 1024 : 112 * 1024);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(fns[i], cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    }
+    const void* fns[3] = {reinterpret_cast<const void*>(plora_shrink_gather_kernel), reinterpret_cast<const void*>(plora_expand_gather_kernel<false>),
+                          reinterpret_cast<const void*>(plora_expand_gather_kernel<true>)};
+    for (int i = 0; i < 3 && e == cudaSuccess; i++) e = plora_kernel_shared(fns[i], 220 * 1024);
     return e;
 }
 
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, bool pdl, cudaStream_t st) {
+                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
+                                    cudaStream_t st) {
     // a block per layer, up to 64: past that a block has more than one layer's records to write, and every further
     // block repeats the grouping
     const int blocks = recs == nullptr ? 1 : n_sites < 64 ? n_sites : 64;
     return launch_pdl(plora_meta_group_kernel, dim3((unsigned)blocks), dim3(1024), plora_meta_group_smem(lay), st, pdl, tiles, segs, lay,
-                      status, tables, site_cols, n_sites, recs, rec_cap);
+                      status, tables, site_cols, n_sites, recs, rec_cap, prefix);
 }
 
-#define PLORA_GRID_Z_CAP 64  // blocks along the work-item axis; more work items are walked in a loop
+// Two blocks per SM walk the units; `bound` is the most units a step of this size can have
+static unsigned unit_grid(long long bound) { return (unsigned)(bound < 2 * g_sms ? bound : 2 * g_sms); }
 
-// rows of A per block: 16 (one 4-row group per warp), so that a slot's rows spread over many blocks and
-// each block's copies are issued and consumed quickly
-int plora_shrink_rps(int kchunk) {
-    (void)kchunk;
-    return 16;
-}
-
-cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, float* S,
+cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, const int* prefix, float* S,
                                 size_t s_stride_elems, int lds, int kchunk, int nsplit, int work_cap, int max_rank_total,
                                 const PloraBounds& bnd, int* status, bool pdl, bool early, bool early_x, bool late,
                                 cudaStream_t st) {
     (void)bnd;
-    const int rps = plora_shrink_rps(kchunk);
-    const int rt_max = (max_rank_total + rps - 1) / rps;
-    dim3 grid((unsigned)(nsplit * rt_max), 1, (unsigned)(work_cap < PLORA_GRID_Z_CAP ? work_cap : PLORA_GRID_Z_CAP));
-    const size_t smem = (size_t)(rps + PLORA_WORK_TOKENS) * (size_t)kchunk * 2;
-    return launch_pdl(plora_shrink_gather_kernel, grid, dim3(128), smem, st, pdl, reinterpret_cast<const bf16*>(x), ldx,
-                      K, recs, rec_cap, S, s_stride_elems, lds, kchunk, rps, rt_max, early ? 1 : 0, early_x ? 1 : 0, pdl && late ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
-}
-
-// output columns per block (two per thread): 512 for wide layers so the grid stays near one wave, 256
-// otherwise, fewer when a row of B is so long that the block's rows would pass 64 KB of shared memory
-int plora_expand_nc(int max_rank, int max_rows) {
-    int nc = max_rows >= 8192 ? 512 : 256;
-    while (nc > 32 && nc * max_rank * 2 > 64 * 1024) nc >>= 1;
-    return nc;
+    const unsigned grid = unit_grid((long long)work_cap * ((max_rank_total + SHR_ROWS - 1) / SHR_ROWS) * nsplit);
+    const size_t smem = (size_t)GATHER_STAGES * SHR_STAGE + (size_t)8 * 16 * SHR_PAD * sizeof(float) + (size_t)(rec_cap + 2) * sizeof(int);
+    return launch_pdl(plora_shrink_gather_kernel, dim3(grid), dim3(GATHER_THREADS), smem, st, pdl, reinterpret_cast<const bf16*>(x), ldx, K, recs,
+                      rec_cap, prefix, S, s_stride_elems, lds, kchunk, nsplit, early ? 1 : 0, early_x ? 1 : 0, pdl && late ? 1 : 0,
+                      status PLORA_BOUNDS_ARG(bnd));
 }
 
 cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, int nsplit, const PloraRec* recs,
-                                int rec_cap, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
+                                int rec_cap, const int* prefix, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
                                 const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st) {
     (void)bnd;
     const int max_rank = lds / PLORA_MAX_PARTS;
-    const int nc = plora_expand_nc(max_rank, max_rows);
-    // tile buffer: all of a block's columns at the maximum rank, up to 32 KB; blocks of higher-rank slots take
-    // their columns in passes
-    const int bs_bytes = nc * max_rank * 2 < 32 * 1024 ? nc * max_rank * 2 : 32 * 1024;
-    dim3 grid((unsigned)((max_rows + nc - 1) / nc), (unsigned)parts,
-              (unsigned)(work_cap < PLORA_GRID_Z_CAP ? work_cap : PLORA_GRID_Z_CAP));
-    const size_t smem = (size_t)bs_bytes + (size_t)PLORA_WORK_TOKENS * (size_t)(max_rank / 8) * EXP_SPAD * sizeof(float);
-    // 512-column blocks take two column pairs per thread (128 threads instead of 256) where that makes the whole
-    // launch resident at once (8 such blocks of 64 registers per thread share an SM, shared memory permitting):
-    // a launch this small is a chain of dependent fetches per block, and a second wave of blocks pays it again.
-    // Larger launches are bound by their arithmetic and keep one pair per thread.
-    const bool passes = bs_bytes < nc * max_rank * 2;
-    int per_sm = (int)((size_t)(227 * 1024) / (smem + 1024));
-    if (per_sm > 8) per_sm = 8;
-    const int nh = nc >= 512 && (long long)grid.x * grid.y * grid.z <= (long long)per_sm * g_sms ? 2 : 1;
-    const dim3 block((unsigned)(nc / (2 * nh)));
-#define PLORA_EXPAND_ARGS S, s_stride_elems, lds, nsplit, recs, rec_cap, y, ldy, f32_out, nc, bs_bytes, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd)
-    if (nh == 2)
-        return passes ? launch_pdl(plora_expand_gather_kernel<true, 2>, grid, block, smem, st, pdl, PLORA_EXPAND_ARGS)
-                      : launch_pdl(plora_expand_gather_kernel<false, 2>, grid, block, smem, st, pdl, PLORA_EXPAND_ARGS);
-    return passes ? launch_pdl(plora_expand_gather_kernel<true, 1>, grid, block, smem, st, pdl, PLORA_EXPAND_ARGS)
-                  : launch_pdl(plora_expand_gather_kernel<false, 1>, grid, block, smem, st, pdl, PLORA_EXPAND_ARGS);
-#undef PLORA_EXPAND_ARGS
+    const int s_pad = ((max_rank + 31) & ~31) * 2 + 16;  // an odd number of 16-byte pieces between the rows of a plane
+    const int uc = expand_unit_cols(max_rank, PLORA_WORK_TOKENS);  // (lower ranks and fewer tokens have wider units)
+    const unsigned grid = unit_grid((long long)work_cap * parts * ((max_rows + uc - 1) / uc));
+    const size_t smem = (size_t)GATHER_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)(rec_cap + 2) * sizeof(int);
+    return launch_pdl(f32_out ? plora_expand_gather_kernel<true> : plora_expand_gather_kernel<false>, dim3(grid), dim3(GATHER_THREADS), smem, st,
+                      pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
 }
