@@ -104,15 +104,16 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// Units of an item. Shrink: rows of the stacked A. Expand: output columns whose rows of B (2 r bytes each) and y of the
-// item's tokens (4 bytes each, counted twice: it is read, written and scattered) come to about 32 KB, in whole steps of a
-// block's eight warps. (With columns by rank alone, the blocks with the popular slots' items of 16 tokens took three
-// times as long as the rest.)
+// Units of an item. Shrink: SHR_ROWS rows of the stacked A over one K-split. Expand: what an output column costs. Blocks get
+// equal shares of the sum, cut at multiples of 32 columns. The costs are times measured on stretches of every kind, in
+// 0.35 us per 1000 columns with two blocks per SM: what a column of B and y takes is not in proportion to its bytes. (With a
+// fixed number of columns per unit the slowest blocks took three times as long as the rest, with bytes twice as long.)
 #define SHR_ROWS 16
 #define SHR_PAD 20  // floats between the token rows of a warp's partial
-__host__ __device__ __forceinline__ int expand_unit_cols(int r, int cnt) {
-    const int step = r <= 64 ? 256 : 128, cols = 32768 / (2 * r + 8 * cnt) / step * step;
-    return cols > step ? cols : step;
+#define EXP_GRAIN 32
+__host__ __device__ __forceinline__ int expand_cost(int r, int cnt) {
+    const int b = r <= 32 ? 12 : r <= 64 ? 21 : 21 + 11 * (r - 64) / 64;
+    return (cnt > 8 ? 2 * b : b) + (cnt >> 2);
 }
 
 // One launch record: gather work item w resolved against one layer's descriptor table, so that the kernels of
@@ -155,10 +156,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
 #pragma unroll
     for (int p = 0; p < PLORA_MAX_PARTS; p++) {
         const int r = (int)dw[11 + p], rows = (int)dw[23 + p];
-        if (r > 0 && rows > 0) {
-            const int uc = expand_unit_cols(r, (int)head.z);
-            ue += (unsigned)((rows + uc - 1) / uc);
-        }
+        if (r > 0 && rows > 0) ue += (unsigned)(rows * expand_cost(r, (int)head.z));
     }
     return (ue << 32) | (unsigned)(((int)dw[10] + SHR_ROWS - 1) / SHR_ROWS * nsplit);
 }
@@ -682,15 +680,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
     if (!waited) pdl_wait();
 }
 
-// Expand: unit = (item, part, some 32 KB worth of output columns), so that a block's range is a few stretches of columns of
-// one part for one item's tokens. The producer copies their rows of B (contiguous) and hints the lines of y that go with
+// Expand: the units are what the columns cost, so that a block's range is a few stretches of columns of one part for one
+// item's tokens, as long as any other block's. The producer copies their rows of B (contiguous) and hints the lines of y that go with
 // them to L2. At the start of a stretch the computing warps put the item's S rows (K-split partials, added in split order)
 // into shared memory as three bf16 terms (high, middle, low part, whose products with bf16 B are exact in f32, so no
 // precision is given up against an f32 multiply-add chain); then each takes its groups of columns of every piece. An item's
 // tokens are taken 8 at a time, whatever their number, so that a token's result does not depend on the others: rows 0-7 of
 // the token tile carry one term of S and rows 8-15 another, two multiplies per 8 x 16 ranks ([low | zero], then
 // [high | middle]), and a lane adds its two rows. The rows of B go to the tiles of a group in an order that leaves every
-// lane with 8 (above 64 ranks: 4) adjacent columns of its token: y moves in pieces of 16 (8) bytes.
+// lane with 8 adjacent columns of its token: y moves in pieces of 16 bytes.
 // Bound by the bytes of B and y.
 #define EXP_PIECE 32768
 struct ExpandUnit {
@@ -700,56 +698,74 @@ struct ExpandUnit {
 };
 __device__ __forceinline__ int expand_piece_cols(int r) { return r <= 16 ? 1024 : r <= 32 ? 512 : r <= 64 ? 256 : 128; }
 
-// Where the stretch at unit `local` of an item lies, at most `left` units of it; returns its units
+// The block's next stretch: the part of the item that the sum reaches at `local` (into the item), and its columns up to
+// `left` further. Returns how much of the sum that is. Both blocks at a cut round it the same way.
 __device__ __forceinline__ int expand_stretch_at(const int* r, const int* rows, int cnt, int local, int left, int& part, int& c0, int& c1) {
     for (part = 0; part < PLORA_MAX_PARTS; part++) {
         if (r[part] <= 0 || rows[part] <= 0) continue;
-        const int uc = expand_unit_cols(r[part], cnt), n = (rows[part] + uc - 1) / uc;
-        if (local < n) {
-            const int take = min(left, n - local);
-            c0 = local * uc;
-            c1 = min(rows[part], (local + take) * uc);
+        const int each = expand_cost(r[part], cnt), all = rows[part] * each;
+        if (local < all) {
+            const int take = min(left, all - local), grain = EXP_GRAIN * each;
+            c0 = min(rows[part], (local + grain - 1) / grain * EXP_GRAIN);
+            c1 = take == all - local ? rows[part] : min(rows[part], (local + take + grain - 1) / grain * EXP_GRAIN);
             return take;
         }
-        local -= n;
+        local -= all;
     }
     part = c0 = c1 = 0;
-    return 1;
+    return left;
 }
 
-// The products of 8 tokens (row g of the planes at `sp`) with one group of NT tiles of 8 columns, whose rows of B start at
-// `rows` in shared memory. NARROW: a rank of 16; else up to 128, 32 ranks at a time.
+// 8 tokens' three terms of S over 32 ranks (16 where NARROW), as this lane's operands of a step
+template <bool NARROW>
+struct SFrag {
+    uint32_t h[NARROW ? 2 : 4], m[NARROW ? 2 : 4], l[NARROW ? 2 : 4];
+    __device__ __forceinline__ void load(uint32_t sp, uint32_t plane, int k, int t4) {  // (row g of the planes at `sp`, from rank k)
+        if (NARROW) {
+            const uint2 a = lds64(sp + 8u * t4), b = lds64(sp + plane + 8u * t4), c = lds64(sp + 2 * plane + 8u * t4);
+            h[0] = a.x, h[1] = a.y, m[0] = b.x, m[1] = b.y, l[0] = c.x, l[1] = c.y;
+        } else {
+            constexpr int Z = NARROW ? 0 : 2, W = NARROW ? 1 : 3;
+            const uint32_t o = sp + 2u * k + 16u * t4;
+            const uint4 a = lds128(o), b = lds128(o + plane), c = lds128(o + 2 * plane);
+            h[0] = a.x, h[1] = a.y, h[Z] = a.z, h[W] = a.w;
+            m[0] = b.x, m[1] = b.y, m[Z] = b.z, m[W] = b.w;
+            l[0] = c.x, l[1] = c.y, l[Z] = c.z, l[W] = c.w;
+        }
+    }
+};
+
+// The products with one group of NT tiles of 8 columns over the same ranks: `col` = this lane's row of B in every tile. Loads
+// first, then one term after another over all tiles: a tile's products depend on one another.
 template <int NT, bool NARROW>
-__device__ __forceinline__ void expand_multiply(float (&d)[NT][4], uint32_t rows, int ncols, int r, uint32_t sp, uint32_t plane, int g, int t4) {
-    uint32_t col[NT];  // this lane's row of every tile (past the last column: any row, its products are dropped)
-#pragma unroll
-    for (int i = 0; i < NT; i++) col[i] = rows + (uint32_t)min(2 * NT * (g >> 1) + 2 * i + (g & 1), ncols - 1) * (uint32_t)r * 2u;
+__device__ __forceinline__ void expand_step(float (&d)[NT][4], const SFrag<NARROW>& s, const uint32_t (&col)[NT], int k, int r, int t4) {
+    const uint32_t al[4] = {s.l[0], 0u, s.l[1], 0u}, ah[4] = {s.h[0], s.m[0], s.h[1], s.m[1]};
     if (NARROW) {
-        const uint2 h = lds64(sp + 8u * t4), m = lds64(sp + plane + 8u * t4), l = lds64(sp + 2 * plane + 8u * t4);
-        const uint32_t al[4] = {l.x, 0u, l.y, 0u}, ah[4] = {h.x, m.x, h.y, m.y};
+        uint2 b[NT];
+#pragma unroll
+        for (int i = 0; i < NT; i++) b[i] = lds64(col[i] + 8u * t4);
+#pragma unroll
+        for (int i = 0; i < NT; i++) mma_16816(d[i], al, b[i].x, b[i].y);
+#pragma unroll
+        for (int i = 0; i < NT; i++) mma_16816(d[i], ah, b[i].x, b[i].y);
+    } else {
+        constexpr int Z = NARROW ? 0 : 2, W = NARROW ? 1 : 3;
+        const bool in = k + 8 * t4 < r;  // (the second half of the last 32 ranks may lie outside)
+        uint4 b[NT];
 #pragma unroll
         for (int i = 0; i < NT; i++) {
-            const uint2 b = lds64(col[i] + 8u * t4);
-            mma_16816(d[i], al, b.x, b.y);
-            mma_16816(d[i], ah, b.x, b.y);
+            b[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (in) b[i] = lds128(col[i] + 2u * k + 16u * t4);
         }
-    } else {
-#pragma unroll 1
-        for (int k = 0; k < r; k += 32) {
-            const uint32_t o = 2u * k + 16u * t4;
-            const bool in = k + 8 * t4 < r;  // (the second half of the last 32 ranks may lie outside)
-            const uint4 h = lds128(sp + o), m = lds128(sp + plane + o), l = lds128(sp + 2 * plane + o);
-            const uint32_t al0[4] = {l.x, 0u, l.y, 0u}, ah0[4] = {h.x, m.x, h.y, m.y}, al1[4] = {l.z, 0u, l.w, 0u}, ah1[4] = {h.z, m.z, h.w, m.w};
+        const uint32_t bl[4] = {s.l[Z], 0u, s.l[W], 0u}, bh[4] = {s.h[Z], s.m[Z], s.h[W], s.m[W]};
 #pragma unroll
-            for (int i = 0; i < NT; i++) {
-                uint4 b = make_uint4(0u, 0u, 0u, 0u);
-                if (in) b = lds128(col[i] + o);
-                mma_16816(d[i], al0, b.x, b.y);
-                mma_16816(d[i], ah0, b.x, b.y);
-                mma_16816(d[i], al1, b.z, b.w);
-                mma_16816(d[i], ah1, b.z, b.w);
-            }
-        }
+        for (int i = 0; i < NT; i++) mma_16816(d[i], al, b[i].x, b[i].y);
+#pragma unroll
+        for (int i = 0; i < NT; i++) mma_16816(d[i], bl, b[i].z, b[i].w);
+#pragma unroll
+        for (int i = 0; i < NT; i++) mma_16816(d[i], ah, b[i].x, b[i].y);
+#pragma unroll
+        for (int i = 0; i < NT; i++) mma_16816(d[i], bh, b[i].z, b[i].w);
     }
 }
 
@@ -822,38 +838,99 @@ struct ExpandStep {
     int ldy;
 };
 
-// One piece of B (its rows in shared memory at `rows`, the part's columns [p0, p1)) for the item's tokens, by one warp
-template <int NT, bool NARROW, bool F32>
-__device__ __forceinline__ void expand_piece(uint32_t rows, int p0, int p1, const ExpandUnit& un, const ExpandStep& st,
-                                             const PloraRec& rec, int warp, int g, int t4) {
-    constexpr int ES = F32 ? 4 : 2, GC = 8 * NT;
+// One stretch by one warp: every eighth group of 32 columns, wherever the pieces of B end. The y of the warp's next group is
+// asked for before this group's products. Up to 8 tokens keep their operands of S in registers (KEEP steps of 32 ranks, as
+// many as there is room for); the rest reads them again for every group. `at` = the ring's stage and, from bit 8 on, the parity
+// of its barriers; returns where the ring then stands, or -1 when a wait ran out. (Not inlined: eight of these share a
+// kernel, and each has its own use for 96 registers.)
+template <bool NARROW, int KEEP, bool TWO, bool F32>
+__device__ __noinline__ int expand_stretch(unsigned char* pieces, uint64_t* full, uint64_t* empty, int at, ExpandUnit un, ExpandStep st,
+                                           const PloraRec& rec, int* status) {
+    constexpr int NT = 4, ES = F32 ? 4 : 2, GC = 8 * NT, H = TWO ? 2 : 1;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
+    int stg = at & 0xff;
+    uint32_t par = (uint32_t)at >> 8;
     const bool wide = ((reinterpret_cast<uintptr_t>(st.Y) | ((size_t)st.ldy * ES) | (un.ybase * ES)) & 15) == 0;
+    const int cnt = rec.cnt, pc = expand_piece_cols(un.r);
+    const uint32_t plane = 16u * st.s_pad, planes = smem_u32(st.planes);
+    unsigned char* yrow[H];
+    uint32_t sp[H];
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        const int t = min(8 * h + g, cnt - 1);
+        yrow[h] = st.Y + ((size_t)rec.tok[t] * st.ldy + un.ybase) * ES;
+        sp[h] = planes + (uint32_t)t * st.s_pad;
+    }
+    constexpr int NK = TWO || KEEP == 0 ? 1 : KEEP;
+    SFrag<NARROW> keep[NK];
+    if (!TWO && KEEP > 0)
+#pragma unroll
+        for (int q = 0; q < NK; q++)
+            if (32 * q < un.r) keep[q].load(sp[0], plane, 32 * q, t4);
+    int p0 = un.c0;        // first column of the ring's current piece
+    bool landed = false;   // ... which this warp has waited for
+    auto wait = [&]() {
+        if (!landed) landed = mbar_wait_long(&full[stg], par, status);
+        return landed;
+    };
+    auto release = [&]() {  // this warp is through with the current piece
+        if (!wait()) return false;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[stg]);
+        if (++stg == GATHER_STAGES) {
+            stg = 0;
+            par ^= 1;
+        }
+        p0 += pc;
+        landed = false;
+        return true;
+    };
+    int c = un.c0 + warp * GC;  // this warp's group
+    YPiece<F32, NT> y, next;
+    y_load<F32, NT>(y, yrow[0] + (size_t)(c + 2 * NT * t4) * ES, g < cnt ? un.c1 - c - 2 * NT * t4 : 0, wide);
 #pragma unroll 1
-    for (int t0 = 0; t0 < rec.cnt; t0 += 8) {
-        const int t = min(t0 + g, rec.cnt - 1);
-        unsigned char* yrow = st.Y + ((size_t)rec.tok[t] * st.ldy + un.ybase) * ES;
-        const uint32_t sp = smem_u32(st.planes) + (uint32_t)t * st.s_pad;
-        const int end = t0 + g < rec.cnt ? p1 : 0;
-        int c = p0 + warp * GC;
-        YPiece<F32, NT> y, next;
-        y_load<F32, NT>(y, yrow + (size_t)(c + 2 * NT * t4) * ES, end - c - 2 * NT * t4, wide);
-#pragma unroll 1
-        for (; c < p1; c += 8 * GC) {
-            const int mine = c + 2 * NT * t4;
-            y_load<F32, NT>(next, yrow + (size_t)(mine + 8 * GC) * ES, end - mine - 8 * GC, wide);
+    for (; c < un.c1; c += 8 * GC) {
+        const int mine = c + 2 * NT * t4;
+        y_load<F32, NT>(next, yrow[0] + (size_t)(mine + 8 * GC) * ES, g < cnt ? un.c1 - mine - 8 * GC : 0, wide);
+        YPiece<F32, NT> other;
+        if (TWO) y_load<F32, NT>(other, yrow[H - 1] + (size_t)mine * ES, 8 + g < cnt ? un.c1 - mine : 0, wide);
+        while (c >= p0 + pc)
+            if (!release()) return -1;
+        if (!wait()) return -1;
+        uint32_t col[NT];  // (past the last column: any row, its products are dropped)
+#pragma unroll
+        for (int i = 0; i < NT; i++)
+            col[i] = smem_u32(pieces) + (uint32_t)stg * EXP_PIECE +
+                     (uint32_t)(c - p0 + min(2 * NT * (g >> 1) + 2 * i + (g & 1), un.c1 - c - 1)) * (uint32_t)un.r * 2u;
+#pragma unroll
+        for (int h = 0; h < H; h++) {
             float d[NT][4];
 #pragma unroll
             for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
-            expand_multiply<NT, NARROW>(d, rows + (uint32_t)(c - p0) * (uint32_t)un.r * 2u, p1 - c, un.r, sp, 16u * st.s_pad, g, t4);
-            y_store<F32, NT>(y, d, yrow + (size_t)mine * ES, end - mine, wide);
-            y = next;
+            if (TWO || KEEP == 0) {
+#pragma unroll 1
+                for (int k = 0; k < un.r; k += 32) {
+                    SFrag<NARROW> s;
+                    s.load(sp[h], plane, k, t4);
+                    expand_step<NT, NARROW>(d, s, col, k, un.r, t4);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < NK; q++)
+                    if (32 * q < un.r) expand_step<NT, NARROW>(d, keep[q], col, 32 * q, un.r, t4);
+            }
+            y_store<F32, NT>(h ? other : y, d, yrow[h] + (size_t)mine * ES, 8 * h + g < cnt ? un.c1 - mine : 0, wide);
         }
+        y = next;
     }
+    while (p0 < un.c1)
+        if (!release()) return -1;
+    return stg | (int)(par << 8);
 }
 
 // The same for ranks above 128, which no piece holds: the rows of B from global memory, 32 ranks at a time
 template <bool F32>
-__device__ __forceinline__ void expand_wide_rank(const bf16* B, const ExpandUnit& un, const ExpandStep& st, const PloraRec& rec, int warp, int g, int t4) {
+__device__ __noinline__ void expand_wide_rank(const bf16* B, ExpandUnit un, ExpandStep st, const PloraRec& rec, int warp, int g, int t4) {
     constexpr int ES = F32 ? 4 : 2, NT = 2;
     const bool wide = ((reinterpret_cast<uintptr_t>(st.Y) | ((size_t)st.ldy * ES) | (un.ybase * ES)) & 15) == 0;
     const uint32_t plane = 16u * st.s_pad;
@@ -955,8 +1032,10 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
         mbar_fence_init();
     }
     const int total = load_prefix(pre, prefix, rec_cap);  // (its barrier publishes the ring's as well)
-    const int u0 = (int)((long long)total * blockIdx.x / gridDim.x), u1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
-    if (u0 >= u1) return pdl_exit_idle();
+    // no less than about 200 columns per block
+    const int blocks = min((int)gridDim.x, max(1, total / 2048));
+    if ((int)blockIdx.x >= blocks || total == 0) return pdl_exit_idle();
+    const int u0 = (int)((long long)total * blockIdx.x / blocks), u1 = (int)((long long)total * (blockIdx.x + 1) / blocks);
     const int w0 = find_item(pre, u0);
     if (warp == 8) {
         // ---- copies of B, and hints for y
@@ -1010,8 +1089,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
     }
     const ExpandStep st = {S, s_stride, lds, nsplit, planes, (uint32_t)s_pad, reinterpret_cast<unsigned char*>(Y), ldy};
     bool waited = false, ok = true;
-    int stg = 0;
-    uint32_t par = 0;
+    int at = 0;  // the ring's position, see expand_stretch
     for (int u = u0, w = w0; ok && u < u1;) {
         while (pre[2 + w] <= u) w++;
         if (tid < 12) reinterpret_cast<uint4*>(&srec)[tid] = __ldcg(reinterpret_cast<const uint4*>(recs + w) + tid);
@@ -1040,22 +1118,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
             if (un.r > 128) {
                 expand_wide_rank<F32>(reinterpret_cast<const bf16*>(srec.b[part]), un, st, srec, warp, g, t4);
             } else {
-                const int pc = expand_piece_cols(un.r);
-                for (int p0 = un.c0; p0 < un.c1; p0 += pc) {
-                    const int p1 = min(un.c1, p0 + pc);
-                    ok = mbar_wait_long(&full[stg], par, status);
-                    if (!ok) break;
-                    const uint32_t rows = smem_u32(gsm) + (uint32_t)stg * EXP_PIECE;
-                    if (un.r <= 16) expand_piece<4, true, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
-                    else if (un.r <= 64) expand_piece<4, false, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
-                    else expand_piece<2, false, F32>(rows, p0, p1, un, st, srec, warp, g, t4);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&empty[stg]);
-                    if (++stg == GATHER_STAGES) {
-                        stg = 0;
-                        par ^= 1;
-                    }
-                }
+#define PLORA_STRETCH(NARROW, KEEP)                                                                                     \
+    at = srec.cnt > 8 ? expand_stretch<NARROW, KEEP, true, F32>(gsm, full, empty, at, un, st, srec, status)              \
+                      : expand_stretch<NARROW, KEEP, false, F32>(gsm, full, empty, at, un, st, srec, status)
+                if (un.r <= 16) PLORA_STRETCH(true, 1);
+                else if (un.r <= 32) PLORA_STRETCH(false, 1);
+                else if (un.r <= 64) PLORA_STRETCH(false, 2);
+                else PLORA_STRETCH(false, 0);
+#undef PLORA_STRETCH
+                ok = at >= 0;
             }
         }
         gather_sync();  // S and the record are replaced for the next stretch
@@ -1146,8 +1217,7 @@ cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, 
     (void)bnd;
     const int max_rank = lds / PLORA_MAX_PARTS;
     const int s_pad = ((max_rank + 31) & ~31) * 2 + 16;  // an odd number of 16-byte pieces between the rows of a plane
-    const int uc = expand_unit_cols(max_rank, PLORA_WORK_TOKENS);  // (lower ranks and fewer tokens have wider units)
-    const unsigned grid = unit_grid((long long)work_cap * parts * ((max_rows + uc - 1) / uc));
+    const unsigned grid = unit_grid(1 + (long long)work_cap * parts * max_rows * expand_cost(max_rank, PLORA_WORK_TOKENS) / 2048);
     const size_t smem = (size_t)GATHER_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)(rec_cap + 2) * sizeof(int);
     return launch_pdl(f32_out ? plora_expand_gather_kernel<true> : plora_expand_gather_kernel<false>, dim3(grid), dim3(GATHER_THREADS), smem, st,
                       pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
