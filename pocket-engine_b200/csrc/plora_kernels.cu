@@ -451,8 +451,8 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
 // through a prefix count per item that the grouping kernel wrote: a step's slots differ up to 8-fold in rank and its
 // layers in width, so a grid of (items x most tiles an item can have) is mostly idle blocks next to a few long ones. Two
 // blocks per SM take an equal, contiguous range of units each. In a block, a producer warp walks the units ahead of the
-// eight computing warps and keeps a ring of three 32 KB pieces full of slab rows by bulk copies, beginning before the
-// dependency wait: 190 KB in flight per SM, where two steps' worth of operand registers per warp were not enough (25 us for
+// eight computing warps and keeps a ring of pieces full of slab rows by bulk copies, beginning before the
+// dependency wait: 130 to 190 KB in flight per SM, where two steps' worth of operand registers per warp were not enough (25 us for
 // 52 MB of A, 80 us for 157 MB of B). The products are tiles of the warp-level tensor instruction (m16n8k16; a 128-row tcgen05
 // tile would spend 7/8 or more of its rows on tokens that are not there; on the CUDA cores both kernels were bound by
 // instructions). Its 16 input slots may be permuted freely as long as both operands agree, so lane t of four holds inputs
@@ -690,13 +690,16 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
 // [high | middle]), and a lane adds its two rows. The rows of B go to the tiles of a group in an order that leaves every
 // lane with 8 adjacent columns of its token: y moves in pieces of 16 bytes.
 // Bound by the bytes of B and y.
-#define EXP_PIECE 32768
+#define EXP_PIECE 16384
+#define EXP_STAGES 4
+#define EXP_AHEAD 4     // groups of columns whose y a warp has on its way
+#define EXP_Y_BYTES 1024 // ... each: two pieces of 16 bytes per lane (16 tokens of bf16, or 8 of f32)
 struct ExpandUnit {
     int r, r_off;          // rank, first column of S
     int c0, c1;            // the stretch of the part's columns
     size_t ybase;          // column of y where the part starts
 };
-__device__ __forceinline__ int expand_piece_cols(int r) { return r <= 16 ? 1024 : r <= 32 ? 512 : r <= 64 ? 256 : 128; }
+__device__ __forceinline__ int expand_piece_cols(int r) { return r <= 16 ? 512 : r <= 32 ? 256 : r <= 64 ? 128 : 64; }
 
 // The block's next stretch: the part of the item that the sum reaches at `local` (into the item), and its columns up to
 // `left` further. Returns how much of the sum that is. Both blocks at a cut round it the same way.
@@ -838,15 +841,25 @@ struct ExpandStep {
     int ldy;
 };
 
-// One stretch by one warp: every eighth group of 32 columns, wherever the pieces of B end. The y of the warp's next group is
-// asked for before this group's products. Up to 8 tokens keep their operands of S in registers (KEEP steps of 32 ranks, as
-// many as there is room for); the rest reads them again for every group. `at` = the ring's stage and, from bit 8 on, the parity
-// of its barriers; returns where the ring then stands, or -1 when a wait ran out. (Not inlined: eight of these share a
-// kernel, and each has its own use for 96 registers.)
+// One stretch by one warp: every eighth group of 32 columns, wherever the pieces of B end. Full groups of rows that move in
+// 16-byte pieces find their y in shared memory, where each lane has asked for its own pieces EXP_AHEAD groups before (in
+// registers, one group ahead was all that fitted, and the round trips to L2 were a third of the time). Up to 8 tokens
+// keep their operands of S in registers (KEEP steps of 32 ranks, as many as there is room for); the rest reads them again
+// for every group. `at` = the ring's stage and, from bit 8 on, the parity of its barriers; returns where the ring then
+// stands, or -1 when a wait ran out. (Not inlined: eight of these share a kernel, and each has its own use for 96 registers.)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 template <bool NARROW, int KEEP, bool TWO, bool F32>
 __device__ __noinline__ int expand_stretch(unsigned char* pieces, uint64_t* full, uint64_t* empty, int at, ExpandUnit un, ExpandStep st,
                                            const PloraRec& rec, int* status) {
-    constexpr int NT = 4, ES = F32 ? 4 : 2, GC = 8 * NT, H = TWO ? 2 : 1;
+    constexpr int NT = 4, ES = F32 ? 4 : 2, GC = 8 * NT, H = TWO ? 2 : 1, NW = F32 ? 2 * NT : NT, STEP = 8 * GC;
+    constexpr bool RING = !(TWO && F32);  // (16 tokens of f32 would take twice the space)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t4 = lane & 3;
     int stg = at & 0xff;
     uint32_t par = (uint32_t)at >> 8;
@@ -877,7 +890,7 @@ __device__ __noinline__ int expand_stretch(unsigned char* pieces, uint64_t* full
         if (!wait()) return false;
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stg]);
-        if (++stg == GATHER_STAGES) {
+        if (++stg == EXP_STAGES) {
             stg = 0;
             par ^= 1;
         }
@@ -885,43 +898,73 @@ __device__ __noinline__ int expand_stretch(unsigned char* pieces, uint64_t* full
         landed = false;
         return true;
     };
-    int c = un.c0 + warp * GC;  // this warp's group
-    YPiece<F32, NT> y, next;
-    y_load<F32, NT>(y, yrow[0] + (size_t)(c + 2 * NT * t4) * ES, g < cnt ? un.c1 - c - 2 * NT * t4 : 0, wide);
+    const uint32_t r2 = 2u * (uint32_t)un.r, brow = (uint32_t)(2 * NT * (g >> 1) + (g & 1)) * r2;
+    const uint32_t ybuf = planes + 3 * plane + (uint32_t)(warp * EXP_AHEAD * EXP_Y_BYTES + lane * 16);
+#pragma unroll
+    for (int h = 0; h < H; h++) yrow[h] += (un.c0 + warp * GC + 2 * NT * t4) * ES;  // this lane's columns of the warp's first group
+    const int full_end = RING && wide ? un.c1 - GC : un.c0 - 1;  // groups that start up to here go through shared memory
+    auto ask = [&](int c, int slot, int ahead) {
+        if (c <= full_end) {
+#pragma unroll
+            for (int h = 0; h < H; h++)
+                if (8 * h + g < cnt)
+#pragma unroll
+                    for (int i = 0; i < NW / 4; i++)
+                        cp_async16(ybuf + (uint32_t)(slot * EXP_Y_BYTES + (h * (NW / 4) + i) * 512), yrow[h] + (size_t)ahead * ES + 16 * i);
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int q = 0; q < EXP_AHEAD; q++) ask(un.c0 + warp * GC + q * STEP, q, q * STEP);
+    int slot = 0;
 #pragma unroll 1
-    for (; c < un.c1; c += 8 * GC) {
-        const int mine = c + 2 * NT * t4;
-        y_load<F32, NT>(next, yrow[0] + (size_t)(mine + 8 * GC) * ES, g < cnt ? un.c1 - mine - 8 * GC : 0, wide);
-        YPiece<F32, NT> other;
-        if (TWO) y_load<F32, NT>(other, yrow[H - 1] + (size_t)mine * ES, 8 + g < cnt ? un.c1 - mine : 0, wide);
+    for (int c = un.c0 + warp * GC; c < un.c1; c += STEP) {
         while (c >= p0 + pc)
             if (!release()) return -1;
         if (!wait()) return -1;
-        uint32_t col[NT];  // (past the last column: any row, its products are dropped)
-#pragma unroll
-        for (int i = 0; i < NT; i++)
-            col[i] = smem_u32(pieces) + (uint32_t)stg * EXP_PIECE +
-                     (uint32_t)(c - p0 + min(2 * NT * (g >> 1) + 2 * i + (g & 1), un.c1 - c - 1)) * (uint32_t)un.r * 2u;
+        // (rows past the last column are whatever the stage holds: their products are dropped)
+        const uint32_t rows = smem_u32(pieces) + (uint32_t)stg * EXP_PIECE + (uint32_t)(c - p0) * r2 + brow;
+        const uint32_t col[NT] = {rows, rows + 2 * r2, rows + 4 * r2, rows + 6 * r2};
+        const int left = un.c1 - c - 2 * NT * t4;  // this lane's columns and those after them
+        const bool ringed = c <= full_end;
+        cp_async_wait<EXP_AHEAD - 1>();
 #pragma unroll
         for (int h = 0; h < H; h++) {
+            const bool live = 8 * h + g < cnt;
+            YPiece<F32, NT> y;
+            if (!ringed) y_load<F32, NT>(y, yrow[h], live ? left : 0, wide);
             float d[NT][4];
 #pragma unroll
             for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
             if (TWO || KEEP == 0) {
 #pragma unroll 1
                 for (int k = 0; k < un.r; k += 32) {
-                    SFrag<NARROW> s;
-                    s.load(sp[h], plane, k, t4);
-                    expand_step<NT, NARROW>(d, s, col, k, un.r, t4);
+                    SFrag<NARROW> f;
+                    f.load(sp[h], plane, k, t4);
+                    expand_step<NT, NARROW>(d, f, col, k, un.r, t4);
                 }
             } else {
 #pragma unroll
-                for (int q = 0; q < NK; q++)
-                    if (32 * q < un.r) expand_step<NT, NARROW>(d, keep[q], col, 32 * q, un.r, t4);
+                for (int k = 0; k < NK; k++)
+                    if (32 * k < un.r) expand_step<NT, NARROW>(d, keep[k], col, 32 * k, un.r, t4);
             }
-            y_store<F32, NT>(h ? other : y, d, yrow[h] + (size_t)mine * ES, 8 * h + g < cnt ? un.c1 - mine : 0, wide);
+            if (ringed) {
+                if (live) {
+#pragma unroll
+                    for (int i = 0; i < NW / 4; i++) {
+                        const uint4 z = lds128(ybuf + (uint32_t)(slot * EXP_Y_BYTES + (h * (NW / 4) + i) * 512));
+                        y.w[4 * i] = z.x, y.w[4 * i + 1] = z.y, y.w[4 * i + 2] = z.z, y.w[4 * i + 3] = z.w;
+                    }
+                    y_store<F32, NT>(y, d, yrow[h], 2 * NT, true);
+                }
+            } else {
+                y_store<F32, NT>(y, d, yrow[h], live ? left : 0, wide);
+            }
         }
-        y = next;
+        ask(c + EXP_AHEAD * STEP, slot, EXP_AHEAD * STEP);
+        slot = slot + 1 == EXP_AHEAD ? 0 : slot + 1;
+#pragma unroll
+        for (int h = 0; h < H; h++) yrow[h] += STEP * ES;
     }
     while (p0 < un.c1)
         if (!release()) return -1;
@@ -1018,14 +1061,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
     // (the kernel before, the layer's matrix multiply, may still be writing it): only L2 prefetch hints.
     extern __shared__ __align__(128) unsigned char gsm[];
     __shared__ __align__(16) PloraRec srec;
-    __shared__ __align__(8) uint64_t full[GATHER_STAGES], empty[GATHER_STAGES];
-    unsigned char* planes = gsm + GATHER_STAGES * EXP_PIECE;
-    int* pre = reinterpret_cast<int*>(planes + 3 * 16 * (size_t)s_pad);
+    __shared__ __align__(8) uint64_t full[EXP_STAGES], empty[EXP_STAGES];
+    unsigned char* planes = gsm + EXP_STAGES * EXP_PIECE;
+    int* pre = reinterpret_cast<int*>(planes + 3 * 16 * (size_t)s_pad + 8 * EXP_AHEAD * EXP_Y_BYTES);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
     constexpr int ES = F32 ? 4 : 2;
     if (early) pdl_trigger();
     if (tid == 0) {
-        for (int i = 0; i < GATHER_STAGES; i++) {
+        for (int i = 0; i < EXP_STAGES; i++) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 8);
         }
@@ -1063,14 +1106,14 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
             const int pc = expand_piece_cols(rp);
             for (int p0 = c0; p0 < c1; p0 += pc, n++) {
                 const int p1 = min(c1, p0 + pc);
-                if (n >= GATHER_STAGES) ok = mbar_wait_long(&empty[stg], par, status);
+                if (n >= EXP_STAGES) ok = mbar_wait_long(&empty[stg], par, status);
                 if (!ok) break;
                 if (lane == 0) {
                     const uint32_t bytes = (uint32_t)(p1 - p0) * (uint32_t)rp * 2u;
                     mbar_expect_tx(&full[stg], bytes);
                     bulk_g2s(gsm + (size_t)stg * EXP_PIECE, B + (size_t)p0 * rp, bytes, &full[stg]);
                 }
-                if (++stg == GATHER_STAGES) {
+                if (++stg == EXP_STAGES) {
                     stg = 0;
                     par ^= 1;
                 }
@@ -1218,7 +1261,7 @@ cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, 
     const int max_rank = lds / PLORA_MAX_PARTS;
     const int s_pad = ((max_rank + 31) & ~31) * 2 + 16;  // an odd number of 16-byte pieces between the rows of a plane
     const unsigned grid = unit_grid(1 + (long long)work_cap * parts * max_rows * expand_cost(max_rank, PLORA_WORK_TOKENS) / 2048);
-    const size_t smem = (size_t)GATHER_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)(rec_cap + 2) * sizeof(int);
+    const size_t smem = (size_t)EXP_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)8 * EXP_AHEAD * EXP_Y_BYTES + (size_t)(rec_cap + 2) * sizeof(int);
     return launch_pdl(f32_out ? plora_expand_gather_kernel<true> : plora_expand_gather_kernel<false>, dim3(grid), dim3(GATHER_THREADS), smem, st,
                       pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
 }
