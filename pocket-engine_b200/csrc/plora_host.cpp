@@ -361,7 +361,11 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
                 s.cluster_ok = h->site_ok && plora_site_plan(s.cols, (int)s.parts.size(), h->max_rank, total, &nsub) > 0;
                 if (s.cluster_ok) {
                     s.max_clusters = plora_site_max_clusters(s.cols, (int)s.parts.size(), h->max_rank, total);
-                    if (s.max_clusters < nsub) s.cluster_ok = false;
+                    // One work item per slot, in no more than a round and a quarter of the clusters that run at once: past that
+                    // the pair of kernels, whose blocks share all items' work evenly, is faster (128 tokens of 48 rank-16
+                    // adapters, four layers: 295 us in clusters, 261 as pairs; of 32 adapters 181 and 216). The rule looks at
+                    // the registry and not at the step, so that a token's result does not depend on its batch.
+                    if (s.max_clusters < nsub || 4 * max_slots * nsub > 5 * s.max_clusters) s.cluster_ok = false;
                 }
                 info.push_back(s.cols);
                 info.push_back(s.cluster_ok ? 8 * nsub : 0);

@@ -691,8 +691,8 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
 // lane with 8 adjacent columns of its token: y moves in pieces of 16 bytes.
 // Bound by the bytes of B and y.
 #define EXP_PIECE 16384
-#define EXP_STAGES 4
-#define EXP_AHEAD 4     // groups of columns whose y a warp has on its way
+#define EXP_STAGES 5
+#define EXP_AHEAD 2     // groups of columns whose y a warp has on its way
 #define EXP_Y_BYTES 1024 // ... each: two pieces of 16 bytes per lane (16 tokens of bf16, or 8 of f32)
 struct ExpandUnit {
     int r, r_off;          // rank, first column of S
