@@ -955,12 +955,15 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     if (work_cap == 0) return PLORA_OK;
     const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
     h->pdl_armed = 2;
+    // a tile kernel behind the gather kernel runs beside it, provided that the gather kernel releases it only after its own wait
+    const bool tiles = h->mma_ok && rows >= step->run_min;
+    if (tiles && !early_x) early = false;
     CUK(h, "shrink",
        plora_launch_shrink((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
                            shrink_units(h, hook->site), (float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.kchunk, site.nsplit,
                            work_cap, hook->parts * h->max_rank, bounds_of(h, hook, rows, 0), h->status, pdl, early, early_x,
                            late, as_stream(stream)));
-    if (h->mma_ok && rows >= step->run_min)
+    if (tiles)
         CUK(h, "shrink (tile path)",
            plora_launch_shrink_mma((const void*)(uintptr_t)x, rows, site.cols, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
@@ -1020,14 +1023,14 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
-                                   tile_split(h, rows), h->status, h->pdl, false, as_stream(stream)));
+                                   tile_split(h, rows), h->status, h->pdl, h->tile_late, as_stream(stream)));
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
                                    tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
                                    (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
-                                   h->pdl, as_stream(stream)));
+                                   h->pdl, false, as_stream(stream)));
     }
     return PLORA_OK;
 }
@@ -1062,19 +1065,21 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     if (work_cap == 0) return PLORA_OK;
     const bool pdl = h->pdl && h->pdl_armed == 2;
     h->pdl_armed = 2;
+    const bool tiles = h->mma_ok && rows >= step->run_min;
+    if (tiles) early = false;  // (as in the shrink)
     CUK(h, "expand",
        plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds,
                            reduced ? 1 : site.nsplit, recs_of(h, hook->site), h->rec_cap, expand_units(h, hook->site),
                            (void*)(uintptr_t)y, ldy, f32_out, hook->parts, hook->max_rows, work_cap,
                            bounds_of(h, hook, rows, ldy), h->status, pdl, early, as_stream(stream)));
-    if (h->mma_ok && rows >= step->run_min)
+    if (tiles)
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
                                    reduced ? 1 : tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
                                    (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
-                                   h->pdl, as_stream(stream)));
+                                   h->pdl, h->tile_late, as_stream(stream)));
     return PLORA_OK;
 }
 

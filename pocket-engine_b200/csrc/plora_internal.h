@@ -196,7 +196,7 @@ struct plora {
     bool fp8_ok = false;    // the fused FP8 layer can run
     bool gemm_ok = false;   // the one-kernel layer for prefill-sized steps can run
     int fused_tile_rows = 1;  // steps with at least this many rows take it (plora_set_fused_tile_rows)
-    bool tile_late = true;    // the tile shrink runs beside the gather shrink launched right before it (PLORA_TILE_LATE=0: behind it)
+    bool tile_late = true;    // tile kernels run beside the gather kernel launched right before them (PLORA_TILE_LATE=0: behind it)
     bool mma_ok = false;    // the tensor-core tile kernels can run (max_rank <= 128 and the driver entry point exists)
     // what the kernel before the next launch is: 0 = not one of ours (a plain launch), 1 = the step's grouping (its
     // launch records must not be read before the dependency wait), 2 = a kernel of the step
@@ -298,7 +298,7 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
 cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int lds, int K, int tile_split,
                                     const int32_t* segs, SegLayout lay, const plora_desc* table, const PloraSlabMaps* smaps, void* y,
                                     int ldy, int f32_out, int parts, const int* part_off, const int* part_rows, int rows_total,
-                                    int max_rows, int tile_cap, int* status, bool pdl, cudaStream_t st);
+                                    int max_rows, int tile_cap, int* status, bool pdl, bool late, cudaStream_t st);
 // early: dependents are released at kernel start and slabs are requested ahead of the dependency wait (used by
 // plora_apply, whose kernels follow one another); early_x: x too may be read ahead of the wait; late: the kernel before
 // is the step's grouping, so not even a launch record may be read ahead of it
