@@ -296,6 +296,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
     h->seg.max_slots = max_slots;
     h->seg.max_tokens = max_tokens;
     h->seg.cap_tiles = h->cap_tiles;
+    h->seg.step_min = 0;
     h->seg.run_min = 1 << 30;  // every run takes the gather path unless the tile path can run (set below)
     if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024) {
         delete h;
@@ -377,7 +378,10 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             if (rc == PLORA_OK && h->max_rank <= 128) h->fp8_ok = plora_fp8_init(h->max_rank) == cudaSuccess;
             if (rc == PLORA_OK && h->mma_ok) h->gemm_ok = plora_gemm_init() == cudaSuccess;
             // runs of 64 or more contiguous tokens of one slot take the tensor-core tile kernels
-            if (h->mma_ok) h->seg.run_min = PLORA_RUN_MIN_DEFAULT;
+            if (h->mma_ok) {
+                h->seg.run_min = PLORA_RUN_MIN_DEFAULT;
+                h->seg.step_min = PLORA_STEP_MIN_DEFAULT;
+            }
             if (const char* e = getenv("PLORA_PDL")) h->pdl = e[0] != '0';
             if (const char* e = getenv("PLORA_FUSED_TILE_ROWS")) h->fused_tile_rows = std::max(1, atoi(e));
             if (const char* e = getenv("PLORA_TILE_LATE")) h->tile_late = e[0] != '0';
@@ -907,6 +911,11 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
 
 // ------------------------------------------------------------------ bracket
 
+// whether a step over `rows` token rows can have tensor-core tiles (its adapter tokens are at most its rows)
+static bool has_tiles(const plora_t* h, const plora_step* step, int rows) {
+    return h->mma_ok && rows >= step->run_min && rows > h->seg.step_min;
+}
+
 // How many blocks share the K chunks of one tensor-core tile: enough to fill the SMs when a step has few
 // tiles (prompt chunks inside a decode batch), one when there are plenty. Any value gives the same bits.
 static int tile_split(const plora_t* h, int rows) {
@@ -956,7 +965,7 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
     h->pdl_armed = 2;
     // a tile kernel behind the gather kernel runs beside it, provided that the gather kernel releases it only after its own wait
-    const bool tiles = h->mma_ok && rows >= step->run_min;
+    const bool tiles = has_tiles(h, step, rows);
     if (tiles && !early_x) early = false;
     CUK(h, "shrink",
        plora_launch_shrink((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
@@ -1017,7 +1026,7 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
                          site.max_clusters, (h->early_x ? 1 : 0) | ((h->site_release >= 0 && h->site_release <= 4 ? h->site_release : (h->early_x ? 0 : 1)) << 1) |
                              (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
                          bounds_of(h, hook, rows, ldy), h->status, pdl, as_stream(stream)));
-    if (h->mma_ok && rows >= step->run_min) {
+    if (has_tiles(h, step, rows)) {
         CUK(h, "shrink (tile path)",
            plora_launch_shrink_mma((const void*)(uintptr_t)x, rows, site.cols, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
@@ -1047,7 +1056,7 @@ int plora_s_reduce(plora_t* h, const plora_hook* hook, const plora_step* step, i
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
-                                            h->mma_ok && rows >= step->run_min ? std::max(1, rows / 64) : 0,
+                                            has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0,
                                             tile_split(h, rows), site.cols, pdl, as_stream(stream)));
     return PLORA_OK;
 }
@@ -1065,7 +1074,7 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     if (work_cap == 0) return PLORA_OK;
     const bool pdl = h->pdl && h->pdl_armed == 2;
     h->pdl_armed = 2;
-    const bool tiles = h->mma_ok && rows >= step->run_min;
+    const bool tiles = has_tiles(h, step, rows);
     if (tiles) early = false;  // (as in the shrink)
     CUK(h, "expand",
        plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds,
@@ -1109,7 +1118,7 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
     CUK(h, "S reduce (tiles)",
        plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, 1,
                              (const int32_t*)(uintptr_t)step->segs, h->seg, (const plora_desc*)(uintptr_t)hook->table, 0,
-                             h->mma_ok && rows >= step->run_min ? std::max(1, rows / 64) : 0, tile_split(h, rows),
+                             has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0, tile_split(h, rows),
                              site.cols, pdl, as_stream(stream)));
     CUK(h, "fused layer (tensor-core adapter term)",
        plora_launch_gemm_fused(kind, (const void*)(uintptr_t)x, (const float*)(uintptr_t)st, (const void*)(uintptr_t)w,
@@ -1182,7 +1191,7 @@ int plora_linear_fp8_fused(plora_t* h, const plora_hook* hook, const plora_step*
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
-                                            h->mma_ok && rows >= step->run_min ? std::max(1, rows / 64) : 0,
+                                            has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0,
                                             tile_split(h, rows), site.cols, pdl, as_stream(stream)));
     CUK(h, "fused fp8 layer",
        plora_launch_fp8_fused((const void*)(uintptr_t)xq, (const float*)(uintptr_t)st, (const void*)(uintptr_t)wq,
@@ -1276,6 +1285,7 @@ int plora_set_run_min(plora_t* h, int tokens) {
     if (!h->mma_ok && tokens < (1 << 30))
         return fail(h, PLORA_ERR_CONFIG, "the tile path needs a device handle and max_rank <= 128");
     h->seg.run_min = tokens;
+    h->seg.step_min = 0;  // the caller's line holds in steps of every size
     return PLORA_OK;
 }
 
@@ -1370,7 +1380,7 @@ static int xchg_ctx(plora_t* h, const plora_hook* hook, const plora_step* step, 
         if (!h->xchg_peer[p]) return fail(h, PLORA_ERR_ARG, "exchange: rank " + std::to_string(p) + " was not imported");
     const SiteInfo& site = h->sites[(size_t)hook->site];
     const int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
-    const int tile_cap = h->mma_ok && rows >= step->run_min ? std::max(1, rows / 64) : 0;
+    const int tile_cap = has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0;
     *nblocks = work_cap + tile_cap;
     if (*nblocks > h->xchg_max_blocks) return fail(h, PLORA_ERR_CAPACITY, "exchange: more blocks than flags");
     c->S = (float*)(uintptr_t)step->s;
