@@ -137,29 +137,38 @@ struct GemmShared {
     int npass, row0[G_MAX_PASS], row1[G_MAX_PASS], slot[G_MAX_PASS], rc0[G_MAX_PASS], rw[G_MAX_PASS];
 };
 
-__host__ __device__ constexpr size_t gemm_stage_bytes(int bn) { return G_BM * G_BKB + bn / 2 * G_BKB; }
-constexpr size_t gemm_smem(int bn) {
-    return 1024 + G_STAGES * gemm_stage_bytes(bn) + 2 * G_AOP + (size_t)bn / 2 * G_RC * 2 + G_EPI_WARPS * G_SLOT + bn * sizeof(float);
+// rows of W per block; the adapter operands are the pairs' only
+__host__ __device__ constexpr int gemm_w_rows(int bn, bool two) { return two ? bn / 2 : bn; }
+__host__ __device__ constexpr size_t gemm_stage_bytes(int bn, bool two) { return G_BM * G_BKB + gemm_w_rows(bn, two) * G_BKB; }
+__host__ __device__ constexpr size_t gemm_operands(int bn, bool two) { return two ? 2 * G_AOP + (size_t)bn / 2 * G_RC * 2 : 0; }
+constexpr size_t gemm_smem(int bn, bool two) {
+    return 1024 + G_STAGES * gemm_stage_bytes(bn, two) + gemm_operands(bn, two) + G_EPI_WARPS * G_SLOT + bn * sizeof(float);
 }
 
-template <int KIND, bool F32, int BN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
+// TWO: a pair of blocks per tile (above). Otherwise a block has a tile of 128 tokens x BN columns to itself and there are no
+// adapter passes: for steps of up to 128 tokens without long runs, in which the second block of a pair would have no tokens
+// and its MMAs no use.
+template <int KIND, bool F32, int BN, bool TWO>
+__global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI, 1)
     plora_gemm_fused_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                             const __grid_constant__ CUtensorMap ymap, const float* __restrict__ st, const float* __restrict__ sn, int T,
                             int N, int K, const int* __restrict__ segs, SegLayout lay, const plora_desc* __restrict__ table,
                             GemmParts parts, const float* __restrict__ S, int lds, int* __restrict__ status) {
     extern __shared__ unsigned char dsm_raw[];
     __shared__ __align__(8) GemmShared sh;
-    constexpr uint32_t STAGE = (uint32_t)gemm_stage_bytes(BN);
+    constexpr uint32_t STAGE = (uint32_t)gemm_stage_bytes(BN, TWO);
+    constexpr int BLOCKS = TWO ? 2 : 1, TM = BLOCKS * G_BM;  // blocks and tokens of a tile
+    constexpr int WR = gemm_w_rows(BN, TWO);
+    constexpr int HALF = BN == 192 ? 128 : BN / 2;  // columns of the first four epilogue warps (whole slots of 64)
     constexpr int NBUF = KIND == 0 ? 1 : 2;               // accumulators of the base product
     constexpr int KEL = KIND == 0 ? G_BKB : G_BKB / 2;    // elements of K per step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t rank = pair_rank();
+    const uint32_t rank = TWO ? pair_rank() : 0;
     unsigned char* ring = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);
     unsigned char* Ahi = ring + G_STAGES * STAGE;
     unsigned char* Alo = Ahi + G_AOP;
     unsigned char* Bop = Alo + G_AOP;
-    unsigned char* slots = Bop + BN / 2 * G_RC * 2;
+    unsigned char* slots = ring + G_STAGES * STAGE + gemm_operands(BN, TWO);
     float* sn_s = reinterpret_cast<float*>(slots + G_EPI_WARPS * G_SLOT);  // the tile's column scales
     if (tid == 0) {
         for (int i = 0; i < G_STAGES; i++) {
@@ -168,26 +177,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
         }
         for (int i = 0; i < 2; i++) {
             mbar_init(&sh.acc_full[i], 1);
-            mbar_init(&sh.acc_empty[i], 2 * G_EPI_WARPS);
+            mbar_init(&sh.acc_empty[i], BLOCKS * G_EPI_WARPS);
         }
         mbar_init(&sh.meta, 1);
         mbar_init(&sh.ad_full, 2);
         mbar_init(&sh.ad_empty, 1);
         mbar_fence_init();
     }
-    if (warp == 1) pair_tmem_alloc(&sh.tmem_slot);
+    if (warp == 1) {
+        if (TWO) pair_tmem_alloc(&sh.tmem_slot);
+        else tmem_alloc(&sh.tmem_slot, 512);
+    }
     tc_fence_before();
     __syncthreads();
-    pair_sync();  // the other block's barriers exist
+    if (TWO) pair_sync();  // the other block's barriers exist
     tc_fence_after();
     const uint32_t tmem = sh.tmem_slot;
     const int nk = ((KIND == 0 ? K : 2 * K) + G_BKB - 1) / G_BKB;
     // tiles in groups of G_GROUP_M tiles of tokens; within a group, tokens first
-    const int mt = (T + 2 * G_BM - 1) / (2 * G_BM), nt = (N + BN - 1) / BN, tiles = mt * nt;
-    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    const int mt = (T + TM - 1) / TM, nt = (N + BN - 1) / BN, tiles = mt * nt;
+    const int pair = blockIdx.x / BLOCKS, pairs = gridDim.x / BLOCKS;
     auto place = [&](int t, int& m0, int& n0) {
         const int per = G_GROUP_M * nt, g = t / per, in = t - g * per, gm = min(G_GROUP_M, mt - g * G_GROUP_M);
-        m0 = (g * G_GROUP_M + in % gm) * 2 * G_BM;
+        m0 = (g * G_GROUP_M + in % gm) * TM;
         n0 = in / gm * BN;
     };
     pdl_wait();  // S, x and the scales come from the kernels before
@@ -205,10 +217,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                     if (round2) ok = mbar_wait_long(&sh.empty[stg], par ^ 1, status);
                     if (!ok) break;
                     unsigned char* xs = ring + (size_t)stg * STAGE;
-                    if (rank == 0) mbar_expect_tx(&sh.full[stg], 2 * STAGE);
-                    const uint32_t bar = at_leader(&sh.full[stg]);
-                    tma_load_2d_pair(xs, &xmap, ks * KEL, m0 + (int)rank * G_BM, bar);
-                    tma_load_2d_pair(xs + G_BM * G_BKB, &wmap, ks * KEL, n0 + (int)rank * (BN / 2), bar);
+                    if (rank == 0) mbar_expect_tx(&sh.full[stg], BLOCKS * STAGE);
+                    if (TWO) {
+                        const uint32_t bar = at_leader(&sh.full[stg]);
+                        tma_load_2d_pair(xs, &xmap, ks * KEL, m0 + (int)rank * G_BM, bar);
+                        tma_load_2d_pair(xs + G_BM * G_BKB, &wmap, ks * KEL, n0 + (int)rank * WR, bar);
+                    } else {
+                        tma_load_2d(xs, &xmap, ks * KEL, m0, &sh.full[stg]);
+                        tma_load_2d(xs + G_BM * G_BKB, &wmap, ks * KEL, n0, &sh.full[stg]);
+                    }
                     if (++stg == G_STAGES) {
                         stg = 0;
                         par ^= 1;
@@ -220,9 +237,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
         __syncwarp();
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
-            // M 256, N BN, f32 accumulator, K-major operands; kind::f16 carries the bf16 formats in bits 7 and 10
-            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24);
-            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * G_BM >> 4) << 24) : idesc_ad;
+            // M TM, N BN, f32 accumulator, K-major operands; kind::f16 carries the bf16 formats in bits 7 and 10
+            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24) : idesc_ad;
             const uint64_t dx0 = umma_desc(smem_u32(ring), 16, 1024, 2), dw0 = umma_desc(smem_u32(ring) + G_BM * G_BKB, 16, 1024, 2);
             int stg = 0, i = 0;
             uint32_t par = 0, apar = 0;  // parities of the stages and of the adapter operands
@@ -232,7 +249,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                 const uint32_t acc = tmem + (uint32_t)buf * BN, ad = KIND == 0 ? tmem + BN : acc;
                 if (i >= NBUF) ok = mbar_wait_long(&sh.acc_empty[buf], (i / NBUF - 1) & 1, status);
                 tc_fence_after();
-                int npass = -1, ps = 0;  // npass: not known before the other warps have written the list
+                int npass = TWO ? -1 : 0, ps = 0;  // npass: not known before the other warps have written the list
                 auto pass = [&]() {
                     tc_fence_after();
                     const int rw = sh.rw[ps];
@@ -250,24 +267,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                     tc_fence_after();
                     const uint64_t dx = dx0 + (uint64_t)((uint32_t)stg * STAGE >> 4), dw = dw0 + (uint64_t)((uint32_t)stg * STAGE >> 4);
 #pragma unroll
-                    for (int kk = 0; kk < G_BKB / 32; kk++) pair_umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
-                    pair_commit(&sh.empty[stg]);
+                    for (int kk = 0; kk < G_BKB / 32; kk++) {
+                        if (TWO) pair_umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
+                        else umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
+                    }
+                    if (TWO) pair_commit(&sh.empty[stg]);
+                    else umma_commit(&sh.empty[stg]);
                     if (++stg == G_STAGES) {
                         stg = 0;
                         par ^= 1;
                     }
-                    if (npass < 0 && mbar_test(&sh.meta, i & 1)) npass = sh.npass;
-                    if (ps < npass && mbar_test(&sh.ad_full, apar)) pass();
+                    if (TWO && npass < 0 && mbar_test(&sh.meta, i & 1)) npass = sh.npass;
+                    if (TWO && ps < npass && mbar_test(&sh.ad_full, apar)) pass();
                 }
-                if (ok && npass < 0) {
+                if (TWO && ok && npass < 0) {
                     ok = mbar_wait_long(&sh.meta, i & 1, status);
                     npass = ok ? sh.npass : 0;
                 }
-                while (ok && ps < npass) {
+                while (TWO && ok && ps < npass) {
                     ok = mbar_wait_long(&sh.ad_full, apar, status);
                     if (ok) pass();
                 }
-                if (ok) pair_commit(&sh.acc_full[buf]);
+                if (ok && TWO) pair_commit(&sh.acc_full[buf]);
+                if (ok && !TWO) umma_commit(&sh.acc_full[buf]);
             }
         }
         __syncwarp();
@@ -287,9 +309,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
 #pragma unroll
             for (int q = 1; q < PLORA_MAX_PARTS; q++)
                 if (q < parts.n && n0 >= parts.off[q]) part = q;
-            const int n_local = n0 - parts.off[part] + (int)rank * (BN / 2);  // this block's first row of B_p
+            const int n_local = n0 - parts.off[part] + (int)rank * WR;  // this block's first row of B_p
             // ---- the tile's adapter passes: tensor-core tiles of the grouping that meet the pair's rows
-            if (ew == 0) {
+            if (TWO && ew == 0) {
                 const int n_mma = segs[SEG_N_MMA];
                 const int* ml = segs + lay.mma();
                 // the first tile that ends after the first row: 32 probes a round
@@ -305,7 +327,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                 }
                 if (lane == 0) {
                     int np = 0;
-                    for (int q = lo; q < n_mma && ml[3 * q] < m0 + 2 * G_BM; q++) {
+                    for (int q = lo; q < n_mma && ml[3 * q] < m0 + TM; q++) {
                         const int start = ml[3 * q], len = ml[3 * q + 1], slot_id = ml[3 * q + 2];
                         const int r = table[slot_id].r[part];
                         for (int rc0 = 0; rc0 < r; rc0 += G_RC) {
@@ -314,7 +336,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
                                 break;
                             }
                             sh.row0[np] = max(start, m0) - m0;
-                            sh.row1[np] = min(start + len, m0 + 2 * G_BM) - m0;
+                            sh.row1[np] = min(start + len, m0 + TM) - m0;
                             sh.slot[np] = slot_id;
                             sh.rc0[np] = rc0;
                             sh.rw[np] = min(G_RC, r - rc0);
@@ -328,8 +350,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
             if (KIND == 0)
                 for (int c = e; c < BN; c += G_EPI) sn_s[c] = n0 + c < N ? sn[n0 + c] : 0.f;
             epi_sync_all();
-            const int npass = sh.npass;
-            if (e == 0) mbar_arrive(&sh.meta);
+            const int npass = TWO ? sh.npass : 0;
+            if (TWO && e == 0) mbar_arrive(&sh.meta);
             for (int ps = 0; ok && ps < npass; ps++) {
                 if (staged) {  // the operands of the pass before are still being read until its MMAs complete
                     ok = mbar_wait_long(&sh.ad_empty, apar, status);
@@ -392,19 +414,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
             tc_fence_after();
             const int row = m0 + (int)rank * G_BM + wq * 32 + lane;
             constexpr int CW = F32 ? 32 : 64;  // y columns per slot
-            const int c0 = (ew >> 2) * (BN / 2);
+            const int c0 = (ew >> 2) * HALF, groups = (ew >> 2 ? BN - HALF : HALF) / 32;
             const float srow = KIND == 0 ? (row < T ? st[row] : 0.f) : 1.f;
             const uint32_t base = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)buf * BN + (uint32_t)c0;
 #pragma unroll 1
-            for (int g = 0; g < BN / 64; g++) {  // 32 accumulator columns at a time
+            for (int g = 0; g < groups; g++) {  // 32 accumulator columns at a time
                 uint32_t vb[32], va[32];
                 tmem_ld32_nowait(base + g * 32, vb);
                 if (KIND == 0 && npass > 0) tmem_ld32_nowait(base + BN + g * 32, va);
                 tmem_ld_wait();
-                if (g == BN / 64 - 1) {  // everything this warp reads is in registers: the accumulator is free
+                if (g == groups - 1) {  // everything this warp reads is in registers: the accumulator is free
                     tc_fence_before();
                     __syncwarp();
-                    if (lane == 0) arrive_at(at_leader(&sh.acc_empty[buf]));
+                    if (lane == 0) {
+                        if (TWO) arrive_at(at_leader(&sh.acc_empty[buf]));
+                        else mbar_arrive(&sh.acc_empty[buf]);
+                    }
                 }
                 float o[32];
 #pragma unroll
@@ -451,8 +476,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(64 + G_EPI, 1)
     }
     tc_fence_before();
     __syncthreads();
-    pair_sync();  // neither block leaves while the other may still signal it or read its operands
-    if (warp == 1) pair_tmem_dealloc(tmem);
+    if (TWO) pair_sync();  // neither block leaves while the other may still signal it or read its operands
+    if (warp == 1) {
+        if (TWO) pair_tmem_dealloc(tmem);
+        else tmem_dealloc(tmem, 512);
+    }
 }
 
 typedef CUresult (*encode_tiled_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -501,9 +529,12 @@ cudaError_t plora_gemm_init() {
         g_encode = reinterpret_cast<encode_tiled_fn>(fn);
     }
     cudaError_t e;
+    auto init = [](auto* kernel, size_t smem) { return plora_kernel_shared(reinterpret_cast<const void*>(kernel), (int)smem); };
 #define PLORA_GEMM_INIT(KIND, F32)                                                                                                         \
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<KIND, F32, 256>), (int)gemm_smem(256)))) return e; \
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_gemm_fused_kernel<KIND, F32, 128>), (int)gemm_smem(128)))) return e
+    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 256, true>, gemm_smem(256, true)))) return e;   \
+    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 128, true>, gemm_smem(128, true)))) return e;   \
+    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 256, false>, gemm_smem(256, false)))) return e; \
+    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 192, false>, gemm_smem(192, false)))) return e
     PLORA_GEMM_INIT(0, false);
     PLORA_GEMM_INIT(0, true);
     PLORA_GEMM_INIT(1, false);
@@ -512,9 +543,9 @@ cudaError_t plora_gemm_init() {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(148);
     cfg.blockDim = dim3(64 + G_EPI);
-    cfg.dynamicSmemBytes = gemm_smem(256);
+    cfg.dynamicSmemBytes = gemm_smem(256, true);
     int n = 0;
-    e = cudaOccupancyMaxActiveClusters(&n, plora_gemm_fused_kernel<0, false, 256>, &cfg);
+    e = cudaOccupancyMaxActiveClusters(&n, plora_gemm_fused_kernel<0, false, 256, true>, &cfg);
     if (e != cudaSuccess) return e;
     if (n < 1) return cudaErrorInvalidConfiguration;
     g_pairs = n;
@@ -537,21 +568,34 @@ bool plora_gemm_fits(int kind, const void* x, const void* w, const void* y, int 
 cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, const void* w, const float* sn, int T, int N,
                                     int K, const int32_t* segs, SegLayout lay, const plora_desc* table, int n_parts,
                                     const int* part_off, const int* part_rows, const float* S, int lds, void* y, int ldy,
-                                    int f32_out, int* status, bool pdl, cudaStream_t stream) {
+                                    int f32_out, bool tiles, int* status, bool pdl, cudaStream_t stream) {
     if (!g_encode) return cudaErrorNotSupported;
     CUtensorMap xmap, wmap, ymap;
     const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int el = kind == 0 ? 1 : 2;
     // 256 output columns per tile, or 128 where that makes the rounds of the pairs shorter: a step of few tokens has few
     // tiles, and a round that is nearly empty costs as much as a full one. A step of K costs what it moves into an SM,
-    // G_BM + bn / 2 rows of 128 bytes.
-    auto cost = [&](int width) {
-        const long long tiles = (long long)((T + 2 * G_BM - 1) / (2 * G_BM)) * ((N + width - 1) / width);
-        return ((tiles + g_pairs - 1) / g_pairs) * (G_BM + width / 2);
+    // G_BM rows of x and the block's rows of W, of 128 bytes each. Up to 128 tokens without long runs, blocks on their own
+    // take tiles of 256 or 192 columns where that costs less: layers too wide for one round of pairs. FP8, 24,576 columns: 36
+    // us in two rounds of pairs, 24 in one round of blocks (shrink and layer at 70 tokens: 65 -> 53 us, at 128: 69 -> 57);
+    // the bf16 layers of a block at 70 tokens: 238 -> 218 us.
+    const int blocks = 2 * g_pairs;
+    auto cost = [&](int width, bool two) {
+        const int tm = two ? 2 * G_BM : G_BM, places = two ? g_pairs : blocks;
+        const long long n = (long long)((T + tm - 1) / tm) * ((N + width - 1) / width);
+        return (n + places - 1) / places * (G_BM + gemm_w_rows(width, two));
     };
-    const int bn = cost(128) < cost(256) ? 128 : 256;
+    int bn = cost(128, true) < cost(256, true) ? 128 : 256;
+    bool two = true;
+    if (!tiles && T <= G_BM) {
+        const int one = cost(192, false) < cost(256, false) ? 192 : 256;
+        if (cost(one, false) < cost(bn, true)) {
+            bn = one;
+            two = false;
+        }
+    }
     if (!encode2d(&xmap, dt, x, (uint64_t)K, (uint64_t)T, (uint64_t)K * el, G_BKB / el, G_BM)) return cudaErrorInvalidValue;
-    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)bn / 2)) return cudaErrorInvalidValue;
+    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)gemm_w_rows(bn, two))) return cudaErrorInvalidValue;
     if (!encode2d(&ymap, f32_out ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, (uint64_t)N,
                   (uint64_t)T, (uint64_t)ldy * (f32_out ? 4 : 2), f32_out ? 32 : 64, 32))
         return cudaErrorInvalidValue;
@@ -561,13 +605,18 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
         parts.off[p] = p < n_parts ? part_off[p] : 0;
         parts.rows[p] = p < n_parts ? part_rows[p] : 0;
     }
-    const long long tiles = (long long)((T + 2 * G_BM - 1) / (2 * G_BM)) * ((N + bn - 1) / bn);
-    const dim3 grid(2u * (unsigned)std::min<long long>(tiles, g_pairs)), block(64 + G_EPI);
-#define PLORA_GEMM_LAUNCH(KIND, F32)                                                                                                          \
-    return bn == 256 ? launch_pdl(plora_gemm_fused_kernel<KIND, F32, 256>, grid, block, gemm_smem(256), stream, pdl, xmap, wmap, ymap, st_,   \
-                                  sn, T, N, K, segs, lay, table, parts, S, lds, status)                                                      \
-                     : launch_pdl(plora_gemm_fused_kernel<KIND, F32, 128>, grid, block, gemm_smem(128), stream, pdl, xmap, wmap, ymap, st_,   \
-                                  sn, T, N, K, segs, lay, table, parts, S, lds, status)
+    const int tm = two ? 2 * G_BM : G_BM;
+    const long long n_tiles = (long long)((T + tm - 1) / tm) * ((N + bn - 1) / bn);
+    const dim3 grid(two ? 2u * (unsigned)std::min<long long>(n_tiles, g_pairs) : (unsigned)std::min<long long>(n_tiles, blocks)), block(64 + G_EPI);
+    auto launch = [&](auto* kernel) {
+        return launch_pdl(kernel, grid, block, gemm_smem(bn, two), stream, pdl, xmap, wmap, ymap, st_, sn, T, N, K, segs, lay, table, parts, S, lds,
+                          status);
+    };
+#define PLORA_GEMM_LAUNCH(KIND, F32)                                                  \
+    return two ? launch(bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, true>     \
+                                  : plora_gemm_fused_kernel<KIND, F32, 128, true>)    \
+               : launch(bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, false>    \
+                                  : plora_gemm_fused_kernel<KIND, F32, 192, false>)
     if (kind == 0) {
         if (f32_out) PLORA_GEMM_LAUNCH(0, true);
         PLORA_GEMM_LAUNCH(0, false);

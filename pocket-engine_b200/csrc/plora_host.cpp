@@ -1125,7 +1125,7 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
                                (const float*)(uintptr_t)sn, rows, width, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                h->seg, (const plora_desc*)(uintptr_t)hook->table, (int)site.parts.size(), site.part_off,
                                site.part_rows, (const float*)(uintptr_t)step->s, step->lds, (void*)(uintptr_t)y, ldy, f32_out,
-                               h->status, h->pdl, as_stream(stream)));
+                               has_tiles(h, step, rows), h->status, h->pdl, as_stream(stream)));
     if (work_cap > 0)
         CUK(h, "expand (tokens outside long runs)",
            plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,

@@ -306,7 +306,7 @@ bool plora_gemm_fits(int kind, const void* x, const void* w, const void* y, int 
 cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, const void* w, const float* sn, int T, int N,
                                     int K, const int32_t* segs, SegLayout lay, const plora_desc* table, int n_parts,
                                     const int* part_off, const int* part_rows, const float* S, int lds, void* y, int ldy,
-                                    int f32_out, int* status, bool pdl, cudaStream_t stream);
+                                    int f32_out, bool tiles, int* status, bool pdl, cudaStream_t stream);
 cudaError_t plora_mma_encode_slab(PloraSlabMaps* out, const plora_desc& d, int K);
 cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, const int32_t* segs, SegLayout lay,
                                     const plora_desc* table, const PloraSlabMaps* smaps, float* S, size_t s_stride_elems, int lds,

@@ -90,3 +90,45 @@ def test_bf16_layer_edges(pe, case, f32_out):
     mx, mn = harness.tolerance(got, want)
     assert (mx <= 1e-3 and mn <= 1e-4) if f32_out else (mx <= 4e-2 and mn <= 4e-3), (mx, mn)
     loras.close()
+
+
+@pytest.mark.parametrize("f32_out", [True, False])
+@pytest.mark.parametrize("kind", ["bf16", "fp8"])
+@pytest.mark.parametrize("rows,widths", [([1], [19456]), ([70], [9728, 9720]), ([100, 1, 27], [28416]), ([128], [14336, 14344]), ([1] * 65, [37896])])
+def test_few_tokens_over_a_wide_layer(pe, kind, rows, widths, f32_out):
+    """Blocks on their own, with tiles of 192 and of 256 columns, in one round and in more."""
+    import torch
+    from pocket_engine_b200 import workloads
+    cols = 272 if kind == "fp8" else 264
+    wl = workloads.Workload("wide", [pe.Site.fused(0, cols, [("p%d" % i, w) for i, w in enumerate(widths)])], [16, 40], 1.0, rows,
+                            [1 + i % 2 for i in range(len(rows))], 41)
+    table, _ = harness.oracle_registry(wl)
+    loras = harness.product_registry(pe, wl)
+    T, N = wl.tokens, wl.sites[0].width()
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = harness.to_dev_bf16(wl.x_bits(0), 0)
+    w = torch.randn(N, cols, device="cuda", generator=g) / cols ** 0.5
+    if kind == "fp8":
+        w, xq = w.to(torch.float8_e4m3fn), x.float().to(torch.float8_e4m3fn)
+        st = 0.9 + 0.2 * torch.rand(T, device="cuda", generator=g)
+        sn = 0.9 + 0.2 * torch.rand(N, device="cuda", generator=g)
+        base = (xq.float().double() @ w.float().double().t()) * st.double()[:, None] * sn.double()
+    else:
+        w = w.bfloat16()
+        base = x.double() @ w.double().t()
+    want = harness.oracle_f64(wl, table, harness.tiles_of(pe, wl), y_base=[base.cpu().numpy().astype(np.float32)])[0]
+    y = torch.full((T, N), float("nan"), dtype=torch.float32 if f32_out else torch.bfloat16, device="cuda")
+    loras.meta_upload(harness.tiles_of(pe, wl, loras.max_lora_tiles()))
+    step = loras.lora_step(loras.max_lora_tiles())
+    for _ in range(2):
+        loras.shrink(loras.hook(0), step, x.data_ptr(), T)
+        if kind == "fp8":
+            loras.linear_fp8_fused(loras.hook(0), step, xq.data_ptr(), st.data_ptr(), w.data_ptr(), sn.data_ptr(), T, y.data_ptr(), N, f32_out)
+        else:
+            loras.linear_bf16_fused(loras.hook(0), step, x.data_ptr(), w.data_ptr(), T, y.data_ptr(), N, f32_out)
+    torch.cuda.synchronize()
+    loras.device_status()
+    got = y.float().cpu().numpy()
+    mx, mn = harness.tolerance(got, want)
+    assert (mx <= 1e-3 and mn <= 1e-4) if f32_out else (mx <= 4e-2 and mn <= 4e-3), (mx, mn)
+    loras.close()
