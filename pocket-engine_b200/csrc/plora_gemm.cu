@@ -3,8 +3,8 @@
 // tcgen05 with accumulators in tensor memory, y written once (no read-modify-write). No counterpart in
 // pocket-engine, whose expand is always a separate kernel after the layer's own GEMM (src/linear.rs:889-921).
 //
-// A pair of blocks (a cluster of two, cta_group::2) computes tiles of 256 tokens x BN output columns (256, or 128 where
-// that fills the device better); as many pairs as fit walk the tiles. Each block holds half of the tile's tokens and
+// A pair of blocks (a cluster of two, cta_group::2) computes tiles of 256 tokens x BN output columns (256, or 192 or 128
+// where that fills the device better); as many pairs as fit walk the tiles. Each block holds half of the tile's tokens and
 // half of its rows of W; the MMAs of the leading block read both, so a byte that enters an SM is used twice as often
 // as in a tile of one block's own: the single-block 128 x 256 kernel before this one moved 48 KB per SM and step of 128
 // bytes of K where this one moves 32. 320 threads per block:
@@ -532,6 +532,7 @@ cudaError_t plora_gemm_init() {
     auto init = [](auto* kernel, size_t smem) { return plora_kernel_shared(reinterpret_cast<const void*>(kernel), (int)smem); };
 #define PLORA_GEMM_INIT(KIND, F32)                                                                                                         \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 256, true>, gemm_smem(256, true)))) return e;   \
+    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 192, true>, gemm_smem(192, true)))) return e;   \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 128, true>, gemm_smem(128, true)))) return e;   \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 256, false>, gemm_smem(256, false)))) return e; \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 192, false>, gemm_smem(192, false)))) return e
@@ -573,26 +574,32 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
     CUtensorMap xmap, wmap, ymap;
     const CUtensorMapDataType dt = kind == 0 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int el = kind == 0 ? 1 : 2;
-    // 256 output columns per tile, or 128 where that makes the rounds of the pairs shorter: a step of few tokens has few
+    // 256 output columns per tile, or fewer where that makes the rounds of the pairs shorter: a step of few tokens has few
     // tiles, and a round that is nearly empty costs as much as a full one. A step of K costs what it moves into an SM,
-    // G_BM rows of x and the block's rows of W, of 128 bytes each. Up to 128 tokens without long runs, blocks on their own
-    // take tiles of 256 or 192 columns where that costs less: layers too wide for one round of pairs. FP8, 24,576 columns: 36
-    // us in two rounds of pairs, 24 in one round of blocks (shrink and layer at 70 tokens: 65 -> 53 us, at 128: 69 -> 57);
-    // the bf16 layers of a block at 70 tokens: 238 -> 218 us.
+    // G_BM rows of x and the block's rows of W, of 128 bytes each. Tiles of 192 columns may span two parts, which adapter
+    // passes do not, so they are for steps without long runs (FP8, 256 tokens, 24,576 columns, shrink and layer: 77.3 -> 74.9 us). Up to 128
+    // tokens of such a step, blocks on their own take tiles of 256 or 192 columns where that costs less: layers too wide for
+    // one round of pairs. FP8, 24,576 columns: 36 us in two rounds of pairs, 24 in one round of blocks (shrink and layer at
+    // 70 tokens: 65 -> 53 us, at 128: 69 -> 57); the bf16 layers of a block at 70 tokens: 238 -> 218 us.
     const int blocks = 2 * g_pairs;
-    auto cost = [&](int width, bool two) {
-        const int tm = two ? 2 * G_BM : G_BM, places = two ? g_pairs : blocks;
-        const long long n = (long long)((T + tm - 1) / tm) * ((N + width - 1) / width);
-        return (n + places - 1) / places * (G_BM + gemm_w_rows(width, two));
-    };
-    int bn = cost(128, true) < cost(256, true) ? 128 : 256;
+    int bn = 0;
     bool two = true;
+    long long best = 0;
+    auto consider = [&](int width, bool pair) {
+        const int tm = pair ? 2 * G_BM : G_BM, places = pair ? g_pairs : blocks;
+        const long long n = (long long)((T + tm - 1) / tm) * ((N + width - 1) / width);
+        const long long cost = (n + places - 1) / places * (G_BM + gemm_w_rows(width, pair));
+        if (bn != 0 && cost >= best) return;
+        bn = width;
+        two = pair;
+        best = cost;
+    };
+    consider(256, true);
+    if (!tiles) consider(192, true);
+    consider(128, true);
     if (!tiles && T <= G_BM) {
-        const int one = cost(192, false) < cost(256, false) ? 192 : 256;
-        if (cost(one, false) < cost(bn, true)) {
-            bn = one;
-            two = false;
-        }
+        consider(256, false);
+        consider(192, false);
     }
     if (!encode2d(&xmap, dt, x, (uint64_t)K, (uint64_t)T, (uint64_t)K * el, G_BKB / el, G_BM)) return cudaErrorInvalidValue;
     if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)gemm_w_rows(bn, two))) return cudaErrorInvalidValue;
@@ -613,8 +620,9 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
                           status);
     };
 #define PLORA_GEMM_LAUNCH(KIND, F32)                                                  \
-    return two ? launch(bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, true>     \
-                                  : plora_gemm_fused_kernel<KIND, F32, 128, true>)    \
+    return two ? launch(bn == 256   ? plora_gemm_fused_kernel<KIND, F32, 256, true>   \
+                        : bn == 192 ? plora_gemm_fused_kernel<KIND, F32, 192, true>   \
+                                    : plora_gemm_fused_kernel<KIND, F32, 128, true>)  \
                : launch(bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, false>    \
                                   : plora_gemm_fused_kernel<KIND, F32, 192, false>)
     if (kind == 0) {

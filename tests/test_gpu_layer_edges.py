@@ -94,9 +94,10 @@ def test_bf16_layer_edges(pe, case, f32_out):
 
 @pytest.mark.parametrize("f32_out", [True, False])
 @pytest.mark.parametrize("kind", ["bf16", "fp8"])
-@pytest.mark.parametrize("rows,widths", [([1], [19456]), ([70], [9728, 9720]), ([100, 1, 27], [28416]), ([128], [14336, 14344]), ([1] * 65, [37896])])
+@pytest.mark.parametrize("rows,widths", [([1], [19456]), ([70], [9728, 9720]), ([100, 1, 27], [28416]), ([128], [14336, 14344]), ([1] * 65, [37896]),
+                                          ([60, 60, 50, 31], [9728, 9720]), ([200, 56], [512, 1000])])
 def test_few_tokens_over_a_wide_layer(pe, kind, rows, widths, f32_out):
-    """Blocks on their own, with tiles of 192 and of 256 columns, in one round and in more."""
+    """Blocks on their own, with tiles of 192 and of 256 columns, in one round and in more; pairs with tiles of 192 that span parts."""
     import torch
     from pocket_engine_b200 import workloads
     cols = 272 if kind == "fp8" else 264
