@@ -22,7 +22,7 @@
 #define PLORA_MMA_TOKENS 128
 #define PLORA_RUN_MIN_DEFAULT 64
 // A step of few tokens has too few tiles to fill the chip: a tile's shrink is a chain of copies along K that at most 8
-// blocks share (2 at a total rank of 192, 1 at 384), and two more kernels per layer have to be launched and waited for.
+// blocks share (1 at a total rank over 128), and two more kernels per layer have to be launched and waited for.
 // The gather kernels cut the same tokens into items of 16, each over many blocks, and read the slab again for each item
 // (from L2), so their time grows with the tokens. Gather against tile path, us per step of 4 layers (hidden 4096):
 //   tokens            128        199        256        320        384        448        768
@@ -99,7 +99,7 @@ struct alignas(64) PloraTmap {  // a CUtensorMap, opaque to the host registry
 };
 // the tile path's views of one slot's slabs for one layer: the stacked A, and every targeted part's B
 struct PloraSlabMaps {
-    PloraTmap a, b[PLORA_MAX_PARTS];
+    PloraTmap a, a64, b[PLORA_MAX_PARTS];  // a64: A in boxes of 64 rows
 };
 
 struct SiteInfo {

@@ -87,7 +87,7 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
 #define EXP_TPAD 66  // floats per row of the epilogue's transpose tile (64 columns + 2 of padding)
 
 // ------------------------------------------------------------------------------------------------------
-// Shrink of one 128-token tile. Grid (split, 1, tiles); 128 threads. The slot's K chunks (plora_tile_chunks) are
+// Shrink of one 128-token tile. Grid (split, rank groups, tiles); 128 threads. The slot's K chunks (plora_tile_chunks) are
 // shared evenly by min(split, chunks) blocks; each block accumulates its chunks in separate accumulators, adds
 // them as a tree and writes plane blockIdx.x of S. K is walked in steps of 64 inputs through a ring of stages
 // with two roles and no block-wide synchronisation in the loop: one thread of warp 0 issues, per step, the x
@@ -98,7 +98,16 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
 #define SHR_KSTEP 64
 #define SHR_X_BYTES (MMA_M * SHR_KSTEP * 2)
 #define SHR_MAX_STAGES 8
+// A block walks its K ranges at the rate at which copies of 128-byte rows arrive at one SM (0.3 us per 64 inputs for x and 64
+// rows of A, 0.5 us with 192 rows, 0.9 with 384), and a total rank over 128 leaves K a single range, since accumulators
+// share tensor memory. So where a step's tiles leave SMs idle, the rows of A go to one block for each SHR_GROUP of them
+// (RSPLIT); x is then read again for each group, from L2, which a step with tiles for every SM could not afford. The sums of
+// an element stay the same. 300 tokens, 4 layers: rank 64 169 -> 149 us, rank 128 262 -> 183 us; 2,000 tokens of one
+// adapter: rank 64 228 -> 213 us, rank 128 327 -> 259 us. (More K ranges instead, in 512 accumulator columns where 256 are
+// allowed: the expand's blocks then wait for tensor memory, 1-20% slower than with groups alone.)
+#define SHR_GROUP 64
 
+template <bool RSPLIT>
 __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_constant__ CUtensorMap xmap,
                                                                 const PloraSlabMaps* __restrict__ smaps, int K,
                                                                 const int* __restrict__ segs, SegLayout lay,
@@ -123,13 +132,16 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     const int start = mt[0], len = mt[1], slot = mt[2];
     if (tile >= n_mma) return pdl_exit_idle();
     const plora_desc& d = table[slot];
-    const int R = d.rank;
-    if (R == 0) return pdl_exit_idle();
-    const int n_chunks = plora_tile_chunks(K, R);
+    const int R_all = d.rank;
+    // this block's rows of the stacked A: all of them, or SHR_GROUP from r0 on
+    const int r0 = RSPLIT ? (int)blockIdx.y * SHR_GROUP : 0, R = RSPLIT ? SHR_GROUP : R_all;
+    const int R_out = RSPLIT ? min(SHR_GROUP, R_all - r0) : R_all;
+    if (R_out <= 0) return pdl_exit_idle();
+    const int n_chunks = plora_tile_chunks(K, R_all);
     const int s_eff = min(ksplit, n_chunks);
     if ((int)blockIdx.x >= s_eff) return pdl_exit_idle();
     const int n_acc = n_chunks / s_eff;  // accumulators (chunks) of this block
-    const CUtensorMap* amap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].a);
+    const CUtensorMap* amap = reinterpret_cast<const CUtensorMap*>(RSPLIT ? &smaps[slot].a64 : &smaps[slot].a);
     const int tid = threadIdx.x, warp = tid >> 5;
     // 1024-byte aligned stage ring: [x tile 16 KB][slab rows R x 128 B]
     unsigned char* ring = dsm_raw + ((1024u - (smem_u32(dsm_raw) & 1023u)) & 1023u);
@@ -184,7 +196,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
                 for (int u = 0; u < sub; u++)
                     for (int b = 0; b < nbox; b++)
                         tma_load_2d(as + (size_t)u * a_box_bytes + (size_t)b * box_rows * 128, amap, k0 + u * SHR_KSTEP,
-                                    b * box_rows, &full[st]);
+                                    r0 + b * box_rows, &full[st]);
                 k0 += sub * SHR_KSTEP;
                 if (++st == nstage) {
                     st = 0;
@@ -245,9 +257,9 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     if (ok && !s_fail) {
         tc_fence_after();
         const int row = tid;
-        float* out = S + (size_t)blockIdx.x * s_stride + (size_t)(start + row) * lds;
+        float* out = S + (size_t)blockIdx.x * s_stride + (size_t)(start + row) * lds + r0;
         const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-        for (int c = 0; n_acc > 1 && c < R; c += 8) {
+        for (int c = 0; n_acc > 1 && c < R_out; c += 8) {
             float v[PLORA_TILE_SPLIT_MAX][8];
 #pragma unroll
             for (int a = 0; a < PLORA_TILE_SPLIT_MAX; a++)
@@ -259,13 +271,13 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
                 *reinterpret_cast<float4*>(out + c + 4) = make_float4(v[0][4], v[0][5], v[0][6], v[0][7]);
             }
         }
-        for (int c = 0; n_acc == 1 && c < R; c += 32) {
+        for (int c = 0; n_acc == 1 && c < R_out; c += 32) {
             uint32_t v[32];
             tmem_ld32(lane_base + c, v);
             if (row < len) {
 #pragma unroll
                 for (int q = 0; q < 32; q += 4)
-                    if (c + q < R)
+                    if (c + q < R_out)
                         *reinterpret_cast<float4*>(out + c + q) =
                             make_float4(__uint_as_float(v[q]), __uint_as_float(v[q + 1]), __uint_as_float(v[q + 2]),
                                         __uint_as_float(v[q + 3]));
@@ -842,6 +854,8 @@ encode_tiled_fn g_encode = nullptr;
 
 }  // namespace
 
+static int g_sms = 148;
+
 cudaError_t plora_mma_init() {
     if (!g_encode) {
         void* fn = nullptr;
@@ -851,8 +865,12 @@ cudaError_t plora_mma_init() {
         if (!fn || q != cudaDriverEntryPointSuccess) return cudaErrorNotSupported;
         g_encode = reinterpret_cast<encode_tiled_fn>(fn);
     }
-    cudaError_t e = plora_kernel_shared(reinterpret_cast<const void*>(plora_shrink_mma_kernel), 200 * 1024);
-    if (e != cudaSuccess) return e;
+    cudaError_t e;
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_shrink_mma_kernel<false>), 200 * 1024)) != cudaSuccess) return e;
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_shrink_mma_kernel<true>), 200 * 1024)) != cudaSuccess) return e;
+    int dev = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_mma_kernel<false>), 172 * 1024);
     if (e != cudaSuccess) return e;
     e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_mma_kernel<true>), 172 * 1024);
@@ -898,6 +916,7 @@ cudaError_t plora_mma_encode_slab(PloraSlabMaps* out, const plora_desc& d, int K
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
     };
     bool ok = encode(&out->a, d.a, K, d.rank, SHR_KSTEP, d.rank > 256 ? d.rank / 2 : d.rank);
+    ok = ok && encode(&out->a64, d.a, K, d.rank, SHR_KSTEP, SHR_GROUP);  // (rows past the last one arrive as zeros)
     for (int p = 0; p < PLORA_MAX_PARTS; p++)
         if (d.r[p] > 0) ok = ok && encode(&out->b[p], d.b[p], d.r[p], d.rows[p], exp_b_width(d.r[p]), EXP_BN);
     return ok ? cudaSuccess : cudaErrorInvalidValue;
@@ -917,7 +936,10 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
-    int stage_bytes = SHR_X_BYTES + ((max_rank_total * 128 + 1023) / 1024) * 1024;
+    const int groups = (max_rank_total + SHR_GROUP - 1) / SHR_GROUP;
+    const int blocks = std::max(1, rows / MMA_M) * std::min(tile_split, plora_tile_chunks(K, max_rank_total));
+    const bool rsplit = groups > 1 && blocks * groups <= g_sms;
+    int stage_bytes = SHR_X_BYTES + (((rsplit ? SHR_GROUP : max_rank_total) * 128 + 1023) / 1024) * 1024;
     // two steps of 64 inputs per stage where at least three such stages fit
     const int sub = 3 * 2 * stage_bytes <= 190 * 1024 ? 2 : 1;
     stage_bytes *= sub;
@@ -925,8 +947,8 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
     nstage = nstage > SHR_MAX_STAGES ? SHR_MAX_STAGES : nstage;
     if (nstage < 2) return cudaErrorInvalidValue;
     const size_t smem = (size_t)nstage * stage_bytes + 1024;
-    return launch_pdl(plora_shrink_mma_kernel, dim3((unsigned)tile_split, 1, (unsigned)tile_cap), dim3(128), smem, st, pdl,
-                      map, smaps, K, segs, lay, table, S, s_stride_elems, lds, tile_split,
+    return launch_pdl(rsplit ? plora_shrink_mma_kernel<true> : plora_shrink_mma_kernel<false>,
+                      dim3((unsigned)tile_split, rsplit ? (unsigned)groups : 1, (unsigned)tile_cap), dim3(128), smem, st, pdl, map, smaps, K, segs, lay, table, S, s_stride_elems, lds, tile_split,
                       nstage, stage_bytes, sub, late && pdl ? 1 : 0, status);
 }
 

@@ -12,6 +12,9 @@ CASES = [
     ("rank-64-and-untargeted", [130, 64, 257], [64, 16], 520, [("a", 72), ("b", 1000)]),
     ("ranks-of-every-box", [200, 70, 64, 128, 129, 91], [16, 32, 48, 64, 96, 128], 1024, [("a", 130)]),
     ("one-column-block", [64], [80], 64, [("a", 8)]),
+    # total ranks of 384 and 144 whose rows of A go to several blocks, the last of which has 16; and too many tiles for that
+    ("rank-groups", [300, 70], [128, 48], 1032, [("a", 64), ("b", 40), ("c", 8)]),
+    ("rank-groups-no-room", [128] * 60, [96, 16], 520, [("a", 64), ("b", 40)]),
 ]
 
 
