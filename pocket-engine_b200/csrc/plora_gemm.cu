@@ -17,9 +17,11 @@
 //               rows of 128 bytes with the 128-byte swizzle (the same products from unswizzled operands, whose rows
 //               collide in shared memory, took a fifth of the FP8 layer's time). The MMA warp takes a pass as soon as it is staged, in the middle of
 //               the main loop.
-// bf16: the adapter products accumulate onto the base product; two accumulators of BN columns, so the epilogue of a tile
-// runs under the next tile's main loop. FP8: the base product has to be scaled first, so the adapter term has an
-// accumulator of its own (columns BN ..), and the next tile starts when both have been read into registers.
+// The adapter term has an accumulator of its own, added once in the epilogue: when a pass is taken depends on timing, so in
+// the base product's accumulator the order of the sums, and with it the last bits of y, would differ from run to run.
+// bf16: two accumulators of BN columns, so the epilogue of a tile without passes runs under the next tile's main loop. A
+// tile with passes has them in the other one (BN over 128; with 128 columns there is room for two of each), and the next
+// tile starts when both have been read into registers. FP8: base product in columns 0 .., adapter term in columns BN ..
 // Epilogue: y = s_t s_n acc + adapter (or acc), staged in 128-byte-swizzled slots and written by tensor stores.
 //
 // Tokens outside long runs (decode tokens, short prompts) get only the base product here; the gather expand
@@ -161,6 +163,9 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
     constexpr int WR = gemm_w_rows(BN, TWO);
     constexpr int HALF = BN == 192 ? 128 : BN / 2;  // columns of the first four epilogue warps (whole slots of 64)
     constexpr int NBUF = KIND == 0 ? 1 : 2;               // accumulators of the base product
+    constexpr bool SHARED = KIND == 1 && BN > 128;        // the adapter term uses the other one of them
+    // first column of the adapter term of a tile whose base product is in accumulator `buf`
+    auto ad_col = [](int buf) { return (uint32_t)(KIND == 0 ? BN : SHARED ? (buf ^ 1) * BN : (2 + buf) * BN); };
     constexpr int KEL = KIND == 0 ? G_BKB : G_BKB / 2;    // elements of K per step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = TWO ? pair_rank() : 0;
@@ -243,11 +248,16 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             const uint64_t dx0 = umma_desc(smem_u32(ring), 16, 1024, 2), dw0 = umma_desc(smem_u32(ring) + G_BM * G_BKB, 16, 1024, 2);
             int stg = 0, i = 0;
             uint32_t par = 0, apar = 0;  // parities of the stages and of the adapter operands
+            int before = 0;              // passes of the tile before
             bool ok = true;
             for (int t = pair; ok && t < tiles; t += pairs, i++) {
                 const int buf = KIND == 0 ? 0 : i & 1;
-                const uint32_t acc = tmem + (uint32_t)buf * BN, ad = KIND == 0 ? tmem + BN : acc;
-                if (i >= NBUF) ok = mbar_wait_long(&sh.acc_empty[buf], (i / NBUF - 1) & 1, status);
+                const uint32_t acc = tmem + (uint32_t)buf * BN, ad = tmem + ad_col(buf);
+                // Whoever last had this tile's accumulator has been read: the tile NBUF before, or the one before, whose
+                // adapter term was in it (its warps have then read the earlier tile too). The adapter term's needs no wait of
+                // its own: the warps that stage a pass have finished the tile before.
+                if (SHARED && before > 0) ok = mbar_wait_long(&sh.acc_empty[buf ^ 1], (i - 1) / NBUF & 1, status);
+                else if (i >= NBUF) ok = mbar_wait_long(&sh.acc_empty[buf], (i / NBUF - 1) & 1, status);
                 tc_fence_after();
                 int npass = TWO ? -1 : 0, ps = 0;  // npass: not known before the other warps have written the list
                 auto pass = [&]() {
@@ -255,7 +265,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                     const int rw = sh.rw[ps];
                     const uint64_t a_hi = umma_desc(smem_u32(Ahi), 16, 1024, 2), a_lo = umma_desc(smem_u32(Alo), 16, 1024, 2);
                     const uint64_t b = umma_desc(smem_u32(Bop), 16, 1024, 2);
-                    for (int kk = 0; kk < rw / 16; kk++) pair_umma<1>(ad, a_hi + 2 * kk, b + 2 * kk, idesc_ad, KIND == 1 || (ps | kk) != 0);
+                    for (int kk = 0; kk < rw / 16; kk++) pair_umma<1>(ad, a_hi + 2 * kk, b + 2 * kk, idesc_ad, (ps | kk) != 0);
                     for (int kk = 0; kk < rw / 16; kk++) pair_umma<1>(ad, a_lo + 2 * kk, b + 2 * kk, idesc_ad, 1);
                     pair_commit(&sh.ad_empty);
                     ps++;
@@ -288,6 +298,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                     ok = mbar_wait_long(&sh.ad_full, apar, status);
                     if (ok) pass();
                 }
+                before = ps;
                 if (ok && TWO) pair_commit(&sh.acc_full[buf]);
                 if (ok && !TWO) umma_commit(&sh.acc_full[buf]);
             }
@@ -416,49 +427,44 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             constexpr int CW = F32 ? 32 : 64;  // y columns per slot
             const int c0 = (ew >> 2) * HALF, groups = (ew >> 2 ? BN - HALF : HALF) / 32;
             const float srow = KIND == 0 ? (row < T ? st[row] : 0.f) : 1.f;
-            const uint32_t base = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)buf * BN + (uint32_t)c0;
-#pragma unroll 1
-            for (int g = 0; g < groups; g++) {  // 32 accumulator columns at a time
+            const uint32_t lanes = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)c0;
+            const uint32_t base = lanes + (uint32_t)buf * BN, ad = lanes + ad_col(buf);
+            constexpr int NW = F32 ? 32 : 16;  // words of 32 columns
+            auto fetch = [&](int g, uint32_t (&w)[NW]) {  // 32 accumulator columns, as they go to y
                 uint32_t vb[32], va[32];
                 tmem_ld32_nowait(base + g * 32, vb);
-                if (KIND == 0 && npass > 0) tmem_ld32_nowait(base + BN + g * 32, va);
+                if (npass > 0) tmem_ld32_nowait(ad + g * 32, va);
                 tmem_ld_wait();
-                if (g == groups - 1) {  // everything this warp reads is in registers: the accumulator is free
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        if (TWO) arrive_at(at_leader(&sh.acc_empty[buf]));
-                        else mbar_arrive(&sh.acc_empty[buf]);
-                    }
-                }
                 float o[32];
 #pragma unroll
                 for (int q = 0; q < 32; q++) {
                     const float v = KIND == 0 ? __uint_as_float(vb[q]) * (srow * sn_s[c0 + g * 32 + q]) : __uint_as_float(vb[q]);
-                    o[q] = KIND == 0 && npass > 0 ? v + __uint_as_float(va[q]) : v;
+                    o[q] = npass > 0 ? v + __uint_as_float(va[q]) : v;
                 }
+#pragma unroll
+                for (int q = 0; q < NW; q++) {
+                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(o[(2 * q) % 32], o[(2 * q + 1) % 32]);
+                    w[q] = F32 ? __float_as_uint(o[q]) : *reinterpret_cast<const uint32_t*>(&b2);
+                }
+            };
+            auto release = [&]() {  // everything this warp reads is in registers: the accumulator is free
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (TWO) arrive_at(at_leader(&sh.acc_empty[buf]));
+                    else mbar_arrive(&sh.acc_empty[buf]);
+                }
+            };
+            auto put = [&](int g, const uint32_t (&w)[NW]) {
                 if (F32 || (g & 1) == 0) {  // a new slot: the store before has to have read it
                     if (lane == 0) bulk_wait_read();
                     __syncwarp();
                 }
                 unsigned char* myrow = slot + lane * 128;
-                if (F32) {
 #pragma unroll
-                    for (int c = 0; c < 8; c++)
-                        *reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4)) =
-                            make_float4(o[4 * c], o[4 * c + 1], o[4 * c + 2], o[4 * c + 3]);
-                } else {
-#pragma unroll
-                    for (int c4 = 0; c4 < 4; c4++) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const __nv_bfloat162 b2 = __floats2bfloat162_rn(o[8 * c4 + 2 * q], o[8 * c4 + 2 * q + 1]);
-                            w[q] = *reinterpret_cast<const uint32_t*>(&b2);
-                        }
-                        const int c = (g & 1) * 4 + c4;
-                        *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-                    }
+                for (int q = 0; q < NW / 4; q++) {
+                    const int c = F32 ? q : (g & 1) * 4 + q;
+                    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
                 }
                 if (F32 || (g & 1) == 1) {
                     fence_async_smem();
@@ -468,6 +474,26 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                         if (col < N && m0 + (int)rank * G_BM + wq * 32 < T) tma_store_2d(&ymap, col, m0 + (int)rank * G_BM + wq * 32, slot);
                         bulk_commit();
                     }
+                }
+            };
+            // Where the next tile waits for both accumulators, all columns come to registers (as bf16 they fit) before any goes on
+            if (SHARED && TWO && !F32) {
+                constexpr int NG = SHARED && TWO && !F32 ? HALF / 32 : 1;
+                uint32_t w[NG][NW];
+#pragma unroll
+                for (int g = 0; g < NG; g++)
+                    if (g < groups) fetch(g, w[g]);
+                release();
+#pragma unroll
+                for (int g = 0; g < NG; g++)
+                    if (g < groups) put(g, w[g]);
+            } else {
+#pragma unroll 1
+                for (int g = 0; g < groups; g++) {
+                    uint32_t w[NW];
+                    fetch(g, w);
+                    if (g == groups - 1) release();
+                    put(g, w);
                 }
             }
             epi_sync_all();  // the list of passes and the column scales are overwritten for the next tile

@@ -79,13 +79,15 @@ def test_bf16_layer_edges(pe, case, f32_out):
     base = (x.double() @ w.double().t()).cpu().numpy()
     want = harness.oracle_f64(wl, table, harness.tiles_of(pe, wl), y_base=[base.astype(np.float32)])[0]
     y = torch.full((wl.tokens, wl.sites[0].width()), float("nan"), dtype=torch.float32 if f32_out else torch.bfloat16, device="cuda")
+    first = torch.empty_like(y)
     loras.meta_upload(harness.tiles_of(pe, wl, loras.max_lora_tiles()))
     step = loras.lora_step(loras.max_lora_tiles())
-    for _ in range(2):  # the second pass finds its barriers and accumulators as the first one left them
+    for out in (first, y):  # the second pass finds its barriers and accumulators as the first one left them
         loras.shrink(loras.hook(0), step, x.data_ptr(), wl.tokens)
-        loras.linear_bf16_fused(loras.hook(0), step, x.data_ptr(), w.data_ptr(), wl.tokens, y.data_ptr(), y.shape[1], f32_out)
+        loras.linear_bf16_fused(loras.hook(0), step, x.data_ptr(), w.data_ptr(), wl.tokens, out.data_ptr(), y.shape[1], f32_out)
     torch.cuda.synchronize()
     loras.device_status()
+    assert torch.equal(first, y)
     got = y.float().cpu().numpy()
     mx, mn = harness.tolerance(got, want)
     assert (mx <= 1e-3 and mn <= 1e-4) if f32_out else (mx <= 4e-2 and mn <= 4e-3), (mx, mn)
