@@ -347,7 +347,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             const size_t rec_bytes = sizeof(PloraRec) * h->sites.size() * (size_t)h->rec_cap;
             check("alloc launch records", cudaMalloc((void**)&h->recs, rec_bytes));
             check("alloc layer widths", cudaMalloc((void**)&h->site_cols, 4 * h->sites.size() * sizeof(int32_t)));
-            const size_t prefix_bytes = h->sites.size() * 2 * (size_t)(h->rec_cap + 2) * sizeof(int32_t);
+            const size_t prefix_bytes = h->sites.size() * (size_t)unit_words(h->rec_cap) * sizeof(int32_t);
             check("alloc unit counts", cudaMalloc((void**)&h->prefix, prefix_bytes));
             if (rc == PLORA_OK) check("zero unit counts", cudaMemset(h->prefix, 0, prefix_bytes));
             if (rc == PLORA_OK) check("zero launch records", cudaMemset(h->recs, 0, rec_bytes));
@@ -946,8 +946,8 @@ static PloraBounds bounds_of(const plora_t* h, const plora_hook* hook, int rows,
 }
 
 // the launch records of a layer for this step
-static const int32_t* shrink_units(const plora_t* h, int site) { return h->prefix + (size_t)site * 2 * (size_t)(h->rec_cap + 2); }
-static const int32_t* expand_units(const plora_t* h, int site) { return shrink_units(h, site) + h->rec_cap + 2; }
+static const int32_t* shrink_units(const plora_t* h, int site) { return h->prefix + (size_t)site * (size_t)unit_words(h->rec_cap); }
+static const int32_t* expand_units(const plora_t* h, int site) { return shrink_units(h, site) + unit_expand(h->rec_cap); }
 static const PloraRec* recs_of(const plora_t* h, int site) { return h->recs + (size_t)site * (size_t)h->rec_cap; }
 
 static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* step, uint64_t x, int rows, bool early,

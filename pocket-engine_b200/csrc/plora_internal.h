@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/plora.h"
+#include "plora_units.h"
 
 // ---- device metadata produced once per step by the grouping kernel ("segs") ----
 // All int32 words. Gather path: tokens of short runs regrouped by slot and cut into work items of at
@@ -186,7 +187,7 @@ struct plora {
     int32_t* meta = nullptr;  // device: tile words, then segs
     PloraRec* recs = nullptr;  // device: [sites][rec_cap] launch records of the step
     int rec_cap = 0;
-    int32_t* prefix = nullptr;  // device: [sites][2][rec_cap + 2] units of the gather kernels before every work item of the step
+    int32_t* prefix = nullptr;  // device: [sites][unit_words(rec_cap)] units of the gather kernels before every work item of the step
     int32_t* host_meta = nullptr;  // pinned staging for plora_meta_upload
     int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel, K-splits, 0} (for the launch records)
     int cap_tiles = 0;

@@ -104,21 +104,11 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 }
 
 // ---------------------------------------------------------------------------------------------
-// Units of an item. Shrink: SHR_ROWS rows of the stacked A over one K-split. Expand: what an output column costs. Blocks get
-// equal shares of the sum, cut at multiples of 32 columns. The costs are times measured on stretches of every kind, in
-// 0.35 us per 1000 columns with two blocks per SM: what a column of B and y takes is not in proportion to its bytes. (With a
-// fixed number of columns per unit the slowest blocks took three times as long as the rest, with bytes twice as long.)
-#define SHR_ROWS 16
 #define SHR_PAD 20  // floats between the token rows of a warp's partial
-#define EXP_GRAIN 32
-__host__ __device__ __forceinline__ int expand_cost(int r, int cnt) {
-    const int b = r <= 32 ? 12 : r <= 64 ? 21 : 21 + 11 * (r - 64) / 64;
-    return (cnt > 8 ? 2 * b : b) + (cnt >> 2);
-}
 
 // One launch record: gather work item w resolved against one layer's descriptor table, so that the kernels of
 // that layer make one metadata fetch per block. `o` is the record's 16 uint4.
-// Returns the item's units of the few-token kernels: (expand << 32) | shrink.
+// Returns the item's units of the few-token kernels (pack_units).
 __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
                                              int cols, int pieces, int nsplit) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
@@ -152,13 +142,10 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     o[10] = work[3];
     o[11] = work[4];
     o[12] = make_uint4(cat[0], cat[1], cat[2], cat[3]);
-    unsigned long long ue = 0;
+    int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
 #pragma unroll
-    for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-        const int r = (int)dw[11 + p], rows = (int)dw[23 + p];
-        if (r > 0 && rows > 0) ue += (unsigned)(rows * expand_cost(r, (int)head.z));
-    }
-    return (ue << 32) | (unsigned)(((int)dw[10] + SHR_ROWS - 1) / SHR_ROWS * nsplit);
+    for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = (int)dw[11 + p], rows[p] = (int)dw[23 + p];
+    return pack_units(expand_item_units(r, rows, (int)head.z), shrink_item_units((int)dw[10], nsplit));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -418,9 +405,8 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
         for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
             const int cols = site_cols[4 * site], pieces = site_cols[4 * site + 1], nsplit = site_cols[4 * site + 2];
-            // a layer's prefix counts: [items, units before item 0, 1, ..., all] for the shrink, then for the expand
-            int* ps = prefix + (size_t)site * 2 * (size_t)(rec_cap + 2);
-            int* pe = ps + rec_cap + 2;
+            int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
+            long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
             for (int base = 0; base < end; base += 1024) {
                 const int w = base + tid;
@@ -432,15 +418,16 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                 }
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
                 if (w < nw) {
-                    ps[1 + w] = (int)(at & 0xffffffffu);
-                    pe[1 + w] = (int)(at >> 32);
+                    ps[1 + w] = packed_shrink(at);
+                    pe[2 + w] = packed_expand(at);
                 }
                 before += total;
             }
             if (tid == 0) {
-                ps[0] = pe[0] = nw;
-                ps[1 + nw] = (int)(before & 0xffffffffu);
-                pe[1 + nw] = (int)(before >> 32);
+                ps[0] = nw;
+                pe[0] = nw;
+                ps[1 + nw] = packed_shrink(before);
+                pe[1] = pe[2 + nw] = packed_expand(before);
             }
             __syncthreads();
         }
@@ -459,7 +446,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
 // instructions). Its 16 input slots may be permuted freely as long as both operands agree, so lane t of four holds inputs
 // 8 t .. 8 t + 7 of a row's 32 (two multiplies), and operands move in 16-byte pieces.
 
-// The prefix counts of a layer in shared memory: pre[0] = items, pre[1 + w] = units before item w, pre[1 + items] = all
+// The shrink's unit counts of a layer in shared memory: pre[0] = items, pre[1 + w] = units before item w, pre[1 + items] = all
 __device__ __forceinline__ int load_prefix(int* pre, const int* __restrict__ src, int rec_cap) {
     for (int i = threadIdx.x; i < min(rec_cap + 2, (int)blockDim.x); i += blockDim.x) pre[i] = __ldcg(src + i);
     __syncthreads();
@@ -467,6 +454,24 @@ __device__ __forceinline__ int load_prefix(int* pre, const int* __restrict__ src
     for (int i = (int)blockDim.x + threadIdx.x; i < n + 2; i += blockDim.x) pre[i] = __ldcg(src + i);
     if (n + 2 > (int)blockDim.x) __syncthreads();
     return pre[1 + n];
+}
+// The same for the expand, and the block's share [u0, u1) of all units. In shared memory the units before an item are
+// counted from u0. False where the block has no share (no less than about 200 columns per block).
+__device__ __forceinline__ bool load_share(int* pre, const int* __restrict__ src, int rec_cap, int& share) {
+    const long long* pe = reinterpret_cast<const long long*>(src);
+    const int n = min((int)__ldcg(pe), rec_cap);
+    const long long total = __ldcg(pe + 1);
+    long long mine = 0;  // (fetched beside the counts that say how many there are)
+    if ((int)threadIdx.x <= rec_cap) mine = __ldcg(pe + 2 + threadIdx.x);
+    const long long most = total / 2048;
+    const int blocks = most < 1 ? 1 : most < (long long)gridDim.x ? (int)most : (int)gridDim.x;
+    if ((int)blockIdx.x >= blocks || total == 0) return false;
+    const long long u0 = share_at(total, blockIdx.x, blocks);
+    share = (int)(share_at(total, blockIdx.x + 1, blocks) - u0);
+    if (threadIdx.x == 0) pre[0] = n;
+    for (int i = threadIdx.x; i <= n; i += blockDim.x) pre[1 + i] = units_from(i == (int)threadIdx.x ? mine : __ldcg(pe + 2 + i), u0);
+    __syncthreads();
+    return true;
 }
 // the item that unit u belongs to
 __device__ __forceinline__ int find_item(const int* pre, int u) {
@@ -701,24 +706,6 @@ struct ExpandUnit {
     size_t ybase;          // column of y where the part starts
 };
 __device__ __forceinline__ int expand_piece_cols(int r) { return r <= 16 ? 512 : r <= 32 ? 256 : r <= 64 ? 128 : 64; }
-
-// The block's next stretch: the part of the item that the sum reaches at `local` (into the item), and its columns up to
-// `left` further. Returns how much of the sum that is. Both blocks at a cut round it the same way.
-__device__ __forceinline__ int expand_stretch_at(const int* r, const int* rows, int cnt, int local, int left, int& part, int& c0, int& c1) {
-    for (part = 0; part < PLORA_MAX_PARTS; part++) {
-        if (r[part] <= 0 || rows[part] <= 0) continue;
-        const int each = expand_cost(r[part], cnt), all = rows[part] * each;
-        if (local < all) {
-            const int take = min(left, all - local), grain = EXP_GRAIN * each;
-            c0 = min(rows[part], (local + grain - 1) / grain * EXP_GRAIN);
-            c1 = take == all - local ? rows[part] : min(rows[part], (local + take + grain - 1) / grain * EXP_GRAIN);
-            return take;
-        }
-        local -= all;
-    }
-    part = c0 = c1 = 0;
-    return left;
-}
 
 // 8 tokens' three terms of S over 32 ranks (16 where NARROW), as this lane's operands of a step
 template <bool NARROW>
@@ -1075,18 +1062,15 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
         }
         mbar_fence_init();
     }
-    const int total = load_prefix(pre, prefix, rec_cap);  // (its barrier publishes the ring's as well)
-    // no less than about 200 columns per block
-    const int blocks = min((int)gridDim.x, max(1, total / 2048));
-    if ((int)blockIdx.x >= blocks || total == 0) return pdl_exit_idle();
-    const int u0 = (int)((long long)total * blockIdx.x / blocks), u1 = (int)((long long)total * (blockIdx.x + 1) / blocks);
-    const int w0 = find_item(pre, u0);
+    int u1;  // the block's share is the units 0 .. u1
+    if (!load_share(pre, prefix, rec_cap, u1)) return pdl_exit_idle();  // (its barrier publishes the ring's as well)
+    const int w0 = find_item(pre, 0);
     if (warp == 8) {
         // ---- copies of B, and hints for y
         int stg = 0, n = 0;
         uint32_t par = 1;
         bool ok = true;
-        for (int u = u0, w = w0; ok && u < u1;) {
+        for (int u = 0, w = w0; ok && u < u1;) {
             while (pre[2 + w] <= u) w++;  // (items without units are passed over)
             const PloraRec& rec = recs[w];
             int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS], part, c0, c1;
@@ -1134,7 +1118,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
     const ExpandStep st = {S, s_stride, lds, nsplit, planes, (uint32_t)s_pad, reinterpret_cast<unsigned char*>(Y), ldy};
     bool waited = false, ok = true;
     int at = 0;  // the ring's position, see expand_stretch
-    for (int u = u0, w = w0; ok && u < u1;) {
+    for (int u = 0, w = w0; ok && u < u1;) {
         while (pre[2 + w] <= u) w++;
         if (tid < 12) reinterpret_cast<uint4*>(&srec)[tid] = __ldcg(reinterpret_cast<const uint4*>(recs + w) + tid);
         gather_sync();
