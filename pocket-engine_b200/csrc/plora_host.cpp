@@ -46,7 +46,10 @@ int cuda_fail(const plora_t* h, const char* what, cudaError_t e) {
             cudaEventRecord(pb_, as_stream(stream));                              \
             (h)->prof.push_back({what, pa_, pb_});                                \
         }                                                                         \
-        if (e_ != cudaSuccess) return cuda_fail(h, what, e_);                     \
+        if (e_ != cudaSuccess) {                                                  \
+            (h)->order.reset();                                                   \
+            return cuda_fail(h, what, e_);                                        \
+        }                                                                         \
     } while (0)
 
 // a pair of timing events for one launch, or false when no profile is open, the stream is capturing, or the
@@ -169,6 +172,24 @@ plora_desc desc_for(const SiteInfo& site, const SiteData& sd, uint64_t base) {
 }
 
 cudaStream_t as_stream(void* s) { return reinterpret_cast<cudaStream_t>(s); }
+
+// The stream as LaunchOrder knows it; false where the runtime cannot tell
+bool stream_key(void* stream, LaunchOrder::Stream* out) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(as_stream(stream), &cs, &id) != cudaSuccess) return false;
+    *out = {(uint64_t)(uintptr_t)stream, cs == cudaStreamCaptureStatusNone ? 0 : id + 1};
+    return true;
+}
+
+// How the next kernel on a stream is launched (see LaunchOrder)
+LaunchOrder::Launch next_launch(plora_t* h, void* stream, bool can_wait) {
+    LaunchOrder::Stream key;
+    if (!h->pdl || !stream_key(stream, &key)) return {false, false};
+    const LaunchOrder::Launch l = h->order.next(key, can_wait);
+    h->order.launched(key);
+    return l;
+}
 
 }  // namespace
 
@@ -870,16 +891,16 @@ int plora_meta_build(plora_t* h, uint64_t cu_dev, uint64_t seq_slot_dev, int n_s
     if (!cu_dev || !seq_slot_dev) return fail(h, PLORA_ERR_ARG, "null device pointer");
     CUK(h, "meta_tiles", plora_launch_meta_tiles((const int32_t*)(uintptr_t)cu_dev, (const int32_t*)(uintptr_t)seq_slot_dev,
                                                 n_seqs, h->meta, h->cap_tiles, h->status, as_stream(stream)));
-    h->tiles_built = true;
-    h->pdl_armed = 0;
+    h->order.reset();
+    h->tiles_built = stream_key(stream, &h->tiles_stream);
     return PLORA_OK;
 }
 
 int plora_meta_upload(plora_t* h, const int32_t* words, void* stream) {
     if (!h || !words) return PLORA_ERR_ARG;
     if (h->device < 0) return fail(h, PLORA_ERR_CUDA, "layout-only handle: no device");
+    h->order.reset();
     h->tiles_built = false;
-    h->pdl_armed = 0;
     int count = words[0];
     if (count < 0 || count > h->cap_tiles) return fail(h, PLORA_ERR_CAPACITY, "more tiles than the metadata holds");
     CU(h, "upload tiles", cudaMemcpyAsync(h->meta, words, (size_t)(1 + 3 * count) * 4, cudaMemcpyHostToDevice,
@@ -894,10 +915,13 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
     int32_t* segs = h->meta + tile_words(h);
     SegLayout lay = h->seg;
     if (decode) lay.run_min = 1 << 30;
+    // behind the kernel that wrote the tile words the launch overlaps it (and waits for it first)
+    LaunchOrder::Stream key;
+    const bool behind = h->tiles_built && stream_key(stream, &key) && key == h->tiles_stream;
     CUK(h, "meta_group", plora_launch_meta_group(h->meta, segs, lay, h->status, h->tables, h->site_cols, (int)h->sites.size(),
-                                                 h->recs, h->rec_cap, h->prefix, h->pdl && h->tiles_built, as_stream(stream)));
+                                                 h->recs, h->rec_cap, h->prefix, h->pdl && behind, as_stream(stream)));
     h->tiles_built = false;
-    h->pdl_armed = 1;
+    h->order.grouped();
     out->run_min = lay.run_min;
     out->pad_ = 0;
     out->tiles = (uint64_t)(uintptr_t)h->meta;
@@ -962,8 +986,7 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     // at most one per slot plus one per 16 tokens
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
-    const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
-    h->pdl_armed = 2;
+    const auto [pdl, late] = next_launch(h, stream, true);
     // a tile kernel behind the gather kernel runs beside it, provided that the gather kernel releases it only after its own wait
     const bool tiles = has_tiles(h, step, rows);
     if (tiles && !early_x) early = false;
@@ -1015,8 +1038,7 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     if (!y || (y & (f32_out ? 7 : 3)) || (ldy & 1)) return fail(h, PLORA_ERR_ARG, "y must be aligned to two elements and ldy even");
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
-    const bool late = h->pdl_armed == 1, pdl = h->pdl && h->pdl_armed != 0;
-    h->pdl_armed = 2;
+    const auto [pdl, late] = next_launch(h, stream, true);
     int total = 0;
     for (auto& p : site.parts) total += p.rows;
     CUK(h, "site kernel",
@@ -1051,8 +1073,7 @@ int plora_s_reduce(plora_t* h, const plora_hook* hook, const plora_step* step, i
     if (rows < 0 || rows > h->max_tokens) return fail(h, PLORA_ERR_CAPACITY, "more rows than max_tokens");
     const SiteInfo& site = h->sites[(size_t)hook->site];
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
-    const bool pdl = h->pdl && h->pdl_armed == 2;
-    h->pdl_armed = 2;
+    const bool pdl = next_launch(h, stream, false).pdl;
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
@@ -1072,8 +1093,7 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     const SiteInfo& site = h->sites[(size_t)hook->site];
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);  // src/linear.rs:900
     if (work_cap == 0) return PLORA_OK;
-    const bool pdl = h->pdl && h->pdl_armed == 2;
-    h->pdl_armed = 2;
+    const bool pdl = next_launch(h, stream, false).pdl;
     const bool tiles = has_tiles(h, step, rows);
     if (tiles) early = false;  // (as in the shrink)
     CUK(h, "expand",
@@ -1100,8 +1120,7 @@ int plora_fp8_quant_rows(plora_t* h, uint64_t x, int rows, int cols, uint64_t xq
     if (rows == 0) return PLORA_OK;
     // (waits for the kernel before it reads or releases anything: what follows may read launch records at once)
     CUK(h, "fp8 quantise", plora_launch_fp8_quant((const void*)(uintptr_t)x, rows, cols, cols, (void*)(uintptr_t)xq,
-                                                 (float*)(uintptr_t)st, h->pdl && h->pdl_armed != 0, as_stream(stream)));
-    h->pdl_armed = 2;
+                                                 (float*)(uintptr_t)st, next_launch(h, stream, true).pdl, as_stream(stream)));
     return PLORA_OK;
 }
 
@@ -1111,8 +1130,7 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
                       uint64_t w, uint64_t sn, int rows, int width, uint64_t y, int ldy, int f32_out, int work_cap,
                       void* stream) {
     const SiteInfo& site = h->sites[(size_t)hook->site];
-    const bool pdl = h->pdl && h->pdl_armed == 2;
-    h->pdl_armed = 2;
+    const bool pdl = next_launch(h, stream, false).pdl;
     // the kernel reads the long runs' S from plane 0: fold the tile path's planes (the gather tokens' K-split
     // planes are added by the gather expand itself)
     CUK(h, "S reduce (tiles)",
@@ -1186,8 +1204,7 @@ int plora_linear_fp8_fused(plora_t* h, const plora_hook* hook, const plora_step*
         plora_gemm_fits(0, (const void*)(uintptr_t)xq, (const void*)(uintptr_t)wq, (const void*)(uintptr_t)y, ldy, f32_out,
                         site.cols, (int)site.parts.size(), off))
         return gemm_layer(h, hook, step, 0, xq, st, wq, sn, rows, width, y, ldy, f32_out, work_cap, stream);
-    const bool pdl = h->pdl && h->pdl_armed == 2;
-    h->pdl_armed = 2;
+    const bool pdl = next_launch(h, stream, false).pdl;
     CUK(h, "S reduce", plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
@@ -1412,8 +1429,7 @@ int plora_s_exchange(plora_t* h, const plora_hook* hook, const plora_step* step,
     int nblocks = 0;
     int rc = xchg_ctx(h, hook, step, rows, &c, &nblocks);
     if (rc != PLORA_OK) return rc;
-    const bool pdl = h->pdl && h->pdl_armed == 2;
-    h->pdl_armed = 2;
+    const bool pdl = next_launch(h, stream, false).pdl;
     CUK(h, "S exchange", plora_launch_xchg(c, nblocks, pdl, as_stream(stream)));
     return PLORA_OK;
 }
@@ -1432,7 +1448,7 @@ int plora_s_exchange_all_ranks(plora_t* const* hs, const plora_hook* const* hook
         if (rc != PLORA_OK) return rc;
         if (r && nb != nblocks) return fail(h0, PLORA_ERR_ARG, "all-ranks exchange: ranks disagree on the step's shape");
         nblocks = nb;
-        hs[r]->pdl_armed = 0;  // a cooperative launch: the next kernel of each rank starts plain
+        hs[r]->order.reset();  // a cooperative launch: the next kernel of each rank starts plain
     }
     CU(h0, "cudaSetDevice", cudaSetDevice(h0->device));
     PloraXchgCtx* dev = (PloraXchgCtx*)(h0->xchg + h0->xchg_ctx_off);

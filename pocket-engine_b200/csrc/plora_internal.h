@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/plora.h"
+#include "plora_order.h"
 #include "plora_units.h"
 
 // ---- device metadata produced once per step by the grouping kernel ("segs") ----
@@ -216,10 +217,9 @@ struct plora {
     int fused_tile_rows = 1;  // steps with at least this many rows take it (plora_set_fused_tile_rows)
     bool tile_late = true;    // tile kernels run beside the gather kernel launched right before them (PLORA_TILE_LATE=0: behind it)
     bool mma_ok = false;    // the tensor-core tile kernels can run (max_rank <= 128 and the driver entry point exists)
-    // what the kernel before the next launch is: 0 = not one of ours (a plain launch), 1 = the step's grouping (its
-    // launch records must not be read before the dependency wait), 2 = a kernel of the step
-    int pdl_armed = 0;
-    bool tiles_built = false;  // plora_meta_build was the last call that touched the tile words
+    LaunchOrder order;
+    bool tiles_built = false;  // plora_meta_build was the last call that touched the tile words, on this stream:
+    LaunchOrder::Stream tiles_stream = {0, 0};
     // plora_profile_begin / _end: one pair of events per kernel launch while a profile is open
     struct ProfEntry {
         const char* what;
