@@ -1039,14 +1039,14 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
     const auto [pdl, late] = next_launch(h, stream, true);
+    const int release = h->site_release >= 0 && h->site_release <= 4 ? h->site_release : (h->early_x ? 0 : 1);
     int total = 0;
     for (auto& p : site.parts) total += p.rows;
     CUK(h, "site kernel",
        plora_launch_site((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
                          hook->site + 1 < (int)h->sites.size() ? recs_of(h, hook->site + 1) : nullptr,
                          (void*)(uintptr_t)y, ldy, f32_out, (int)site.parts.size(), h->max_rank, total, work_cap,
-                         site.max_clusters, (h->early_x ? 1 : 0) | ((h->site_release >= 0 && h->site_release <= 4 ? h->site_release : (h->early_x ? 0 : 1)) << 1) |
-                             (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
+                         site.max_clusters, (h->early_x ? 1 : 0) | (release << 1) | (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
                          bounds_of(h, hook, rows, ldy), h->status, pdl, as_stream(stream)));
     if (has_tiles(h, step, rows)) {
         CUK(h, "shrink (tile path)",
@@ -1054,7 +1054,8 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
-                                   tile_split(h, rows), h->status, h->pdl, h->tile_late, as_stream(stream)));
+                                   tile_split(h, rows), h->status, h->pdl, tile_shrink_beside(h->tile_late, h->early_x, release, late && pdl),
+                                   as_stream(stream)));
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
                                    tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,

@@ -48,3 +48,8 @@ private:
     std::vector<Stream> past_;  // streams with a launch since
     bool grouped_ = false;
 };
+
+// Whether a layer's tile shrink may run beside the cluster kernel launched right before it, reading x at once: only if that
+// kernel lets it start after its own wait (release 0 is at kernel start), or the caller vouched for x. waits_first: the
+// cluster kernel is the first of its step on the stream and waits before anything else.
+inline bool tile_shrink_beside(bool tile_late, bool early_x, int release, bool waits_first) { return tile_late && (early_x || release != 0 || waits_first); }

@@ -47,5 +47,9 @@ int main() {
     o.grouped();
     for (uint64_t s = 100; s < 200; s++) CHECK(go({s, 0}, true).late);
     CHECK(o.next({100, 0}, true).late && !o.next({199, 0}, true).late);
+    // the tile shrink beside a cluster kernel that lets it start before its own wait
+    CHECK(!tile_shrink_beside(true, false, 0, false));
+    CHECK(tile_shrink_beside(true, false, 0, true) && tile_shrink_beside(true, true, 0, false) && tile_shrink_beside(true, false, 1, false));
+    CHECK(!tile_shrink_beside(false, true, 1, true));
     return 0;
 }
