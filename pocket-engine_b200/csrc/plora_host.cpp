@@ -302,6 +302,9 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
         si.kchunk = next_mult((si.cols + want - 1) / want, 1024);
         si.nsplit = (si.cols + si.kchunk - 1) / si.kchunk;
         h->nsplit_max = std::max(h->nsplit_max, si.nsplit);
+        long long width = 0;
+        for (auto& part : si.parts) width += part.rows;
+        si.exp_most = expand_most(width);
         for (size_t p = 0; p < si.parts.size() && p < PLORA_MAX_PARTS; p++) {
             si.part_off[p] = si.parts[p].off;
             si.part_rows[p] = si.parts[p].rows;
@@ -392,7 +395,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
                 info.push_back(s.cols);
                 info.push_back(s.cluster_ok ? 8 * nsub : 0);
                 info.push_back(s.nsplit);
-                info.push_back(0);
+                info.push_back(s.exp_most);
             }
             if (rc == PLORA_OK)
                 check("upload layer widths", cudaMemcpy(h->site_cols, info.data(), info.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
@@ -1101,7 +1104,7 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
        plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds,
                            reduced ? 1 : site.nsplit, recs_of(h, hook->site), h->rec_cap, expand_units(h, hook->site),
                            (void*)(uintptr_t)y, ldy, f32_out, hook->parts, hook->max_rows, work_cap,
-                           bounds_of(h, hook, rows, ldy), h->status, pdl, early, as_stream(stream)));
+                           site.exp_most, bounds_of(h, hook, rows, ldy), h->status, pdl, early, as_stream(stream)));
     if (tiles)
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
@@ -1149,7 +1152,7 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
         CUK(h, "expand (tokens outside long runs)",
            plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
                                recs_of(h, hook->site), h->rec_cap, expand_units(h, hook->site), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
-                               hook->max_rows, work_cap, bounds_of(h, hook, rows, ldy), h->status, h->pdl, false,
+                               hook->max_rows, work_cap, site.exp_most, bounds_of(h, hook, rows, ldy), h->status, h->pdl, false,
                                as_stream(stream)));
     return PLORA_OK;
 }

@@ -106,6 +106,7 @@ struct PloraSlabMaps {
 
 struct SiteInfo {
     int layer = 0, cols = 0;
+    int exp_most = 1;  // expand_most of the layer's output columns
     int col_heads_start = -1, col_heads_block = 0;
     struct Part {
         std::string module;
@@ -190,7 +191,7 @@ struct plora {
     int rec_cap = 0;
     int32_t* prefix = nullptr;  // device: [sites][unit_words(rec_cap)] units of the gather kernels before every work item of the step
     int32_t* host_meta = nullptr;  // pinned staging for plora_meta_upload
-    int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel, K-splits, 0} (for the launch records)
+    int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel, K-splits, most units of a column} (for the launch records)
     int cap_tiles = 0;
     SegLayout seg;
     int* status = nullptr;  // device status word
@@ -270,7 +271,7 @@ cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, 
                                     int cap_tiles, int* status, cudaStream_t st);
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
 // site_info: per layer {input width, blocks that share a work item's output columns in the cluster kernel (0: none),
-// K-splits of the gather shrink, 0}; prefix: per layer the unit counts of the gather shrink and expand before every item
+// K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
                                     const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
                                     cudaStream_t st);
@@ -326,4 +327,4 @@ cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* r
                                 cudaStream_t st);
 cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, int nsplit, const PloraRec* recs,
                                 int rec_cap, const int* prefix, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
-                                const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st);
+                                int most, const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st);

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 // that layer make one metadata fetch per block. `o` is the record's 16 uint4.
 // Returns the item's units of the few-token kernels (pack_units).
 __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
-                                             int cols, int pieces, int nsplit) {
+                                             int cols, int pieces, int nsplit, int most) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
     const uint4 head = work[0];  // slot, perm start, count, 0
     const int slot = (int)head.x;
@@ -145,7 +145,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
 #pragma unroll
     for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = (int)dw[11 + p], rows[p] = (int)dw[23 + p];
-    return pack_units(expand_item_units(r, rows, (int)head.z), shrink_item_units((int)dw[10], nsplit));
+    return pack_units(expand_item_units(r, rows, (int)head.z, most), shrink_item_units((int)dw[10], nsplit));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
         for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
-            const int cols = site_cols[4 * site], pieces = site_cols[4 * site + 1], nsplit = site_cols[4 * site + 2];
+            const int cols = site_cols[4 * site], pieces = site_cols[4 * site + 1], nsplit = site_cols[4 * site + 2], most = site_cols[4 * site + 3];
             int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
             long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
@@ -414,7 +414,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                 if (w < end) {
                     uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
                     if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
-                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, pieces, nsplit);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, pieces, nsplit, most);
                 }
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
                 if (w < nw) {
@@ -1044,7 +1044,7 @@ template <bool F32>
 __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(const float* __restrict__ S, size_t s_stride, int lds, int nsplit,
                                                                       const PloraRec* __restrict__ recs, int rec_cap,
                                                                       const int* __restrict__ prefix, void* Y, int ldy, int s_pad,
-                                                                      int early, int* __restrict__ status PLORA_BOUNDS_PARAM) {
+                                                                      int most, int early, int* __restrict__ status PLORA_BOUNDS_PARAM) {
     // early != 0: dependents are released at kernel start. No value of y is bound before the dependency wait
     // (the kernel before, the layer's matrix multiply, may still be writing it): only L2 prefetch hints.
     extern __shared__ __align__(128) unsigned char gsm[];
@@ -1083,7 +1083,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
                 continue;
             }
 #endif
-            u += expand_stretch_at(r, rows, cnt, u - pre[1 + w], u1 - u, part, c0, c1);
+            u += expand_stretch_at(r, rows, cnt, most, u - pre[1 + w], u1 - u, part, c0, c1);
             const int rp = __ldcg(&rec.r[part]);
             if (c0 >= c1 || rp > 128) continue;  // (ranks above 128 are read from global memory)
             const bf16* B = reinterpret_cast<const bf16*>(__ldcg(&rec.b[part]));
@@ -1137,7 +1137,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
 #endif
         ExpandUnit un;
         int part;
-        u += expand_stretch_at(srec.r, srec.rows, srec.cnt, u - pre[1 + w], u1 - u, part, un.c0, un.c1);
+        u += expand_stretch_at(srec.r, srec.rows, srec.cnt, most, u - pre[1 + w], u1 - u, part, un.c0, un.c1);
         if (un.c0 < un.c1) {
             un.r = srec.r[part], un.r_off = srec.r_off[part];
             un.ybase = (size_t)srec.off[part];
@@ -1241,12 +1241,12 @@ cudaError_t plora_launch_shrink(const void* x, int ldx, int K, const PloraRec* r
 
 cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, int nsplit, const PloraRec* recs,
                                 int rec_cap, const int* prefix, void* y, int ldy, int f32_out, int parts, int max_rows, int work_cap,
-                                const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st) {
+                                int most, const PloraBounds& bnd, int* status, bool pdl, bool early, cudaStream_t st) {
     (void)bnd;
     const int max_rank = lds / PLORA_MAX_PARTS;
     const int s_pad = ((max_rank + 31) & ~31) * 2 + 16;  // an odd number of 16-byte pieces between the rows of a plane
     const unsigned grid = unit_grid(1 + (long long)work_cap * parts * max_rows * expand_cost(max_rank, PLORA_WORK_TOKENS) / 2048);
     const size_t smem = (size_t)EXP_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)8 * EXP_AHEAD * EXP_Y_BYTES + (size_t)(rec_cap + 2) * sizeof(int);
     return launch_pdl(f32_out ? plora_expand_gather_kernel<true> : plora_expand_gather_kernel<false>, dim3(grid), dim3(GATHER_THREADS), smem, st,
-                      pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
+                      pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, most, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
 }

@@ -26,23 +26,16 @@ PLORA_HD int expand_cost(int r, int cnt) {
 // more columns than EXP_ITEM_MAX) and a share of 64 or more blocks under 2^31.
 #define EXP_ITEM_MAX (1 << 23)
 #define PLORA_MAX_ITEMS 12864
-PLORA_HD long long expand_width(const int* r, const int* rows) {
-    long long width = 0;
-    for (int p = 0; p < PLORA_MAX_PARTS; p++)
-        if (r[p] > 0 && rows[p] > 0) width += rows[p];
-    return width;
-}
-PLORA_HD int expand_col_cost(int r, int cnt, long long width) {
+// ... which limits what a column of a layer this wide may cost (found once, on the host)
+inline int expand_most(long long width) { return width < 1 ? EXP_ITEM_MAX : width < EXP_ITEM_MAX ? (int)(EXP_ITEM_MAX / width) : 1; }
+PLORA_HD int expand_col_cost(int r, int cnt, int most) {
     const int c = expand_cost(r, cnt);
-    if (c * width <= EXP_ITEM_MAX) return c;
-    const int most = (int)(EXP_ITEM_MAX / width);
-    return most < 1 ? 1 : most < c ? most : c;
+    return c < most ? c : most;
 }
-PLORA_HD long long expand_item_units(const int* r, const int* rows, int cnt) {
-    const long long width = expand_width(r, rows);
+PLORA_HD long long expand_item_units(const int* r, const int* rows, int cnt, int most) {
     long long units = 0;
     for (int p = 0; p < PLORA_MAX_PARTS; p++)
-        if (r[p] > 0 && rows[p] > 0) units += (long long)rows[p] * expand_col_cost(r[p], cnt, width);
+        if (r[p] > 0 && rows[p] > 0) units += (long long)rows[p] * expand_col_cost(r[p], cnt, most);
     return units;
 }
 PLORA_HD int shrink_item_units(int rank, int nsplit) { return (rank + SHR_ROWS - 1) / SHR_ROWS * nsplit; }
@@ -69,11 +62,10 @@ PLORA_HD int units_from(long long before, long long first) {
 
 // The block's next stretch: the part of the item that the sum reaches at `local` (into the item), and its columns up to
 // `left` further. Returns how much of the sum that is. Both blocks at a cut round it the same way.
-PLORA_HD int expand_stretch_at(const int* r, const int* rows, int cnt, int local, int left, int& part, int& c0, int& c1) {
-    const long long width = expand_width(r, rows);
+PLORA_HD int expand_stretch_at(const int* r, const int* rows, int cnt, int most, int local, int left, int& part, int& c0, int& c1) {
     for (part = 0; part < PLORA_MAX_PARTS; part++) {
         if (r[part] <= 0 || rows[part] <= 0) continue;
-        const int each = expand_col_cost(r[part], cnt, width), all = rows[part] * each;
+        const int each = expand_col_cost(r[part], cnt, most), all = rows[part] * each;
         if (local < all) {
             const int take = left < all - local ? left : all - local;
             const unsigned grain = EXP_GRAIN * (unsigned)each;

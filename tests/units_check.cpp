@@ -15,16 +15,18 @@ static int fail(const char* what, long long a, long long b) {
 int main(int argc, char** argv) {
     const int items = std::atoi(argv[1]), cnt = std::atoi(argv[2]), blocks = std::atoi(argv[3]), walk = std::atoi(argv[4]);
     int r[PLORA_MAX_PARTS] = {}, rows[PLORA_MAX_PARTS] = {}, rank = 0;
-    for (int p = 0; 5 + 2 * p < argc; p++) r[p] = std::atoi(argv[5 + 2 * p]), rows[p] = std::atoi(argv[6 + 2 * p]), rank += r[p];
+    long long width = 0;
+    for (int p = 0; 5 + 2 * p < argc; p++) r[p] = std::atoi(argv[5 + 2 * p]), rows[p] = std::atoi(argv[6 + 2 * p]), rank += r[p], width += rows[p];
+    const int most = expand_most(width);
     // the grouping kernel's scan
     std::vector<long long> before(items + 1);
     unsigned long long at = 0;
     for (int w = 0; w <= items; w++) {
         before[w] = packed_expand(at);
         if (packed_shrink(at) != w * shrink_item_units(rank, 8)) return fail("shrink units", w, packed_shrink(at));
-        if (w < items) at += pack_units(expand_item_units(r, rows, cnt), shrink_item_units(rank, 8));
+        if (w < items) at += pack_units(expand_item_units(r, rows, cnt, most), shrink_item_units(rank, 8));
     }
-    const long long total = before[items], item = expand_item_units(r, rows, cnt);
+    const long long total = before[items], item = expand_item_units(r, rows, cnt, most);
     if (total != items * item || item > 0x7fffffffLL) return fail("expand units", total, item);
     int last = -1, part0 = 0, col = 0, next = 0;  // where the block before ended: item, part, column; the block after it
     for (int b = 0; b < blocks; b++) {
@@ -39,7 +41,7 @@ int main(int argc, char** argv) {
             while (units_from(before[w + 1], u0) <= u) w++;
             const int local = u - units_from(before[w], u0);
             int part, c0, c1;
-            const int take = expand_stretch_at(r, rows, cnt, local, (int)share - u, part, c0, c1);
+            const int take = expand_stretch_at(r, rows, cnt, most, local, (int)share - u, part, c0, c1);
             if (local < 0 || take <= 0 || c0 < 0 || c1 < c0 || c1 > rows[part]) return fail("stretch", c0, c1);
             if (first) last = w, part0 = part, col = c0, first = false;
             if (last != w || part0 != part) {  // on to the next part, or the next item's first
