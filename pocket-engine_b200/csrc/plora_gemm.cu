@@ -311,9 +311,9 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
         const uint32_t ad_full = at_leader(&sh.ad_full);
         uint32_t apar = 0;
         bool staged = false;  // the adapter operands have been used before
-        bool ok = true;
+        bool ok = true;  // (of this warp: after a wait that ran out it goes on meeting the barriers, and does nothing else)
         int i = 0;
-        for (int t = pair; ok && t < tiles; t += pairs, i++) {
+        for (int t = pair; t < tiles; t += pairs, i++) {
             int m0, n0;
             place(t, m0, n0);
             int part = 0;  // the part the tile's columns lie in
@@ -363,13 +363,16 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             epi_sync_all();
             const int npass = TWO ? sh.npass : 0;
             if (TWO && e == 0) mbar_arrive(&sh.meta);
-            for (int ps = 0; ok && ps < npass; ps++) {
+            for (int ps = 0; ps < npass; ps++) {
                 if (staged) {  // the operands of the pass before are still being read until its MMAs complete
-                    ok = mbar_wait_long(&sh.ad_empty, apar, status);
+                    if (ok) ok = mbar_wait_long(&sh.ad_empty, apar, status);
                     apar ^= 1;
-                    if (!ok) break;
                 }
                 staged = true;
+                if (!ok) {
+                    epi_sync_all();
+                    continue;
+                }
                 const plora_desc& d = table[sh.slot[ps]];
                 const int rc0 = sh.rc0[ps], r = d.r[part], P = sh.rw[ps] >> 3;
                 // eight threads a row, one 16-byte piece of 8 ranks each: rows of B_p for the block's half of the columns
@@ -421,7 +424,10 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             // bytes a row, then a tensor store (clipped at the edges of y by the tensor map)
             const int buf = KIND == 0 ? 0 : i & 1;
             if (ok) ok = mbar_wait_long(&sh.acc_full[buf], (i / NBUF) & 1, status);
-            if (!ok) break;
+            if (!ok) {
+                epi_sync_all();
+                continue;
+            }
             tc_fence_after();
             const int row = m0 + (int)rank * G_BM + wq * 32 + lane;
             constexpr int CW = F32 ? 32 : 64;  // y columns per slot

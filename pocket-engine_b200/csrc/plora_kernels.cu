@@ -485,6 +485,17 @@ __device__ __forceinline__ int find_item(const int* pre, int u) {
 }
 // barrier among the eight warps that compute (the producer warp does not take part)
 __device__ __forceinline__ void gather_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// The barrier behind a unit's waits. A wait that ran out is one warp's; all eight leave for it, or the others would meet the
+// next barrier without it. `gave_up` is only set between a barrier before and this one, and only read behind this one.
+__device__ __forceinline__ bool gather_sync_ok(bool ok, int* gave_up) {
+    if (!ok) *reinterpret_cast<volatile int*>(gave_up) = 1;
+    gather_sync();
+    return *reinterpret_cast<volatile int*>(gave_up) == 0;
+}
+// The producer leaves once the last `stages` of its n copies have landed, whoever still wanted them
+__device__ __forceinline__ void ring_landed(uint64_t* full, int n, int stages, int* status) {
+    for (int m = n > stages ? n - stages : 0; m < n; m++) mbar_wait_long(&full[m % stages], (uint32_t)(m / stages) & 1u, status);
+}
 
 #define GATHER_STAGES 3
 #define GATHER_THREADS 288  // eight computing warps and the producer
@@ -510,6 +521,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
     extern __shared__ __align__(128) unsigned char gsm[];
     __shared__ __align__(16) PloraRec srec[2];
     __shared__ __align__(8) uint64_t full[GATHER_STAGES], empty[GATHER_STAGES];
+    __shared__ int gave_up;
     float* red = reinterpret_cast<float*>(gsm + GATHER_STAGES * SHR_STAGE);  // [8 warps][16][SHR_PAD]
     int* pre = reinterpret_cast<int*>(red + 8 * 16 * SHR_PAD);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -519,6 +531,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 8);
         }
+        gave_up = 0;
         mbar_fence_init();
     }
     bool waited = false;
@@ -580,6 +593,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
                 }
             }
         }
+        ring_landed(full, n, GATHER_STAGES, status);
         if (!waited) pdl_wait();
         return;
     }
@@ -660,7 +674,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
             *reinterpret_cast<float2*>(mine + 8 * i) = make_float2(acc[i][0], acc[i][1]);
             if (two) *reinterpret_cast<float2*>(mine + 8 * SHR_PAD + 8 * i) = make_float2(acc[i][2], acc[i][3]);
         }
-        gather_sync();  // the partials and the next record are there
+        ok = gather_sync_ok(ok, &gave_up);  // the partials and the next record are there
         const bool was = good && ok;
         if (u + 1 < u1) {
             good = fine(srec[at ^ 1], next);
@@ -1050,6 +1064,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
     extern __shared__ __align__(128) unsigned char gsm[];
     __shared__ __align__(16) PloraRec srec;
     __shared__ __align__(8) uint64_t full[EXP_STAGES], empty[EXP_STAGES];
+    __shared__ int gave_up;
     unsigned char* planes = gsm + EXP_STAGES * EXP_PIECE;
     int* pre = reinterpret_cast<int*>(planes + 3 * 16 * (size_t)s_pad + 8 * EXP_AHEAD * EXP_Y_BYTES);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t4 = lane & 3;
@@ -1060,6 +1075,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 8);
         }
+        gave_up = 0;
         mbar_fence_init();
     }
     int u1;  // the block's share is the units 0 .. u1
@@ -1112,6 +1128,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
                 }
             }
         }
+        ring_landed(full, n, EXP_STAGES, status);
         pdl_wait();
         return;
     }
@@ -1157,7 +1174,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
                 ok = at >= 0;
             }
         }
-        gather_sync();  // S and the record are replaced for the next stretch
+        ok = gather_sync_ok(ok, &gave_up);  // S and the record are replaced for the next stretch
     }
     if (!waited) pdl_wait();
 }
