@@ -1013,6 +1013,14 @@ __device__ __noinline__ void expand_wide_rank(const bf16* B, ExpandUnit un, Expa
     }
 }
 
+// The bf16 high part of a sum, and what the lower parts are to hold. A sum whose nearest bf16 would be infinite is rounded
+// towards zero; of an infinite one nothing is left (infinity less itself would be no number).
+__device__ __forceinline__ float high_part(float f) {
+    const float h = __bfloat162float(__float2bfloat16_rn(f));
+    return isinf(h) ? __uint_as_float(__float_as_uint(f) & 0xffff0000u) : h;
+}
+__device__ __forceinline__ float rest_of(float f, float h) { return isinf(h) ? 0.f : f - h; }
+
 // S of an item's part, four values a thread and step: all planes on their way together, added in split order; the bf16
 // planes are filled up with zeros to a multiple of 32 ranks
 __device__ __forceinline__ void expand_stage_s(const ExpandUnit& un, const ExpandStep& st, const PloraRec& rec, int tid) {
@@ -1039,9 +1047,9 @@ __device__ __forceinline__ void expand_stage_s(const ExpandUnit& un, const Expan
         uint32_t w[3][2];
 #pragma unroll
         for (int e = 0; e < 2; e++) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-            const float2 hf = __bfloat1622float2(h);
-            const float m0 = f[2 * e] - hf.x, m1 = f[2 * e + 1] - hf.y;
+            const float2 hf = make_float2(high_part(f[2 * e]), high_part(f[2 * e + 1]));
+            const __nv_bfloat162 h = __floats2bfloat162_rn(hf.x, hf.y);
+            const float m0 = rest_of(f[2 * e], hf.x), m1 = rest_of(f[2 * e + 1], hf.y);
             const __nv_bfloat162 m = __floats2bfloat162_rn(m0, m1);
             const float2 mf = __bfloat1622float2(m);
             const __nv_bfloat162 l = __floats2bfloat162_rn(m0 - mf.x, m1 - mf.y);
