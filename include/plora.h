@@ -333,9 +333,8 @@ int plora_fork(plora_t* h, void* main_stream, void* side_stream);
 int plora_join(plora_t* h, void* main_stream, void* side_stream);
 
 /* Runs of contiguous tokens of one slot at least this long leave the gather kernels for the
- * tensor-core tile kernels (no counterpart in the engine, whose tiles are always 16 tokens). Unless this is called, runs of
- * 64 tokens do, in steps of more than 256 adapter tokens; a line set here holds in steps of every size, so that the kernels
- * which a run takes do not depend on what else is in the step. */
+ * tensor-core tile kernels (no counterpart in the engine, whose tiles are always 16 tokens). 64 unless this is called. The
+ * kernels that a run takes do not depend on what else is in the step. */
 int plora_set_run_min(plora_t* h, int tokens);
 
 /* The tile kernels cut a layer's inputs into a fixed number of ranges (a function of the layer's width and

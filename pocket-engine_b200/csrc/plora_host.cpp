@@ -320,7 +320,6 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
     h->seg.max_slots = max_slots;
     h->seg.max_tokens = max_tokens;
     h->seg.cap_tiles = h->cap_tiles;
-    h->seg.step_min = 0;
     h->seg.run_min = 1 << 30;  // every run takes the gather path unless the tile path can run (set below)
     if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024) {
         delete h;
@@ -402,10 +401,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             if (rc == PLORA_OK && h->max_rank <= 128) h->fp8_ok = plora_fp8_init(h->max_rank) == cudaSuccess;
             if (rc == PLORA_OK && h->mma_ok) h->gemm_ok = plora_gemm_init() == cudaSuccess;
             // runs of 64 or more contiguous tokens of one slot take the tensor-core tile kernels
-            if (h->mma_ok) {
-                h->seg.run_min = PLORA_RUN_MIN_DEFAULT;
-                h->seg.step_min = PLORA_STEP_MIN_DEFAULT;
-            }
+            if (h->mma_ok) h->seg.run_min = PLORA_RUN_MIN_DEFAULT;
             if (const char* e = getenv("PLORA_PDL")) h->pdl = e[0] != '0';
             if (const char* e = getenv("PLORA_FUSED_TILE_ROWS")) h->fused_tile_rows = std::max(1, atoi(e));
             if (const char* e = getenv("PLORA_TILE_LATE")) h->tile_late = e[0] != '0';
@@ -938,9 +934,9 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
 
 // ------------------------------------------------------------------ bracket
 
-// whether a step over `rows` token rows can have tensor-core tiles (its adapter tokens are at most its rows)
+// whether a step over `rows` token rows can have tensor-core tiles
 static bool has_tiles(const plora_t* h, const plora_step* step, int rows) {
-    return h->mma_ok && rows >= step->run_min && rows > h->seg.step_min;
+    return h->mma_ok && rows >= step->run_min;
 }
 
 // How many blocks share the K chunks of one tensor-core tile: enough to fill the SMs when a step has few
@@ -1306,7 +1302,6 @@ int plora_set_run_min(plora_t* h, int tokens) {
     if (!h->mma_ok && tokens < (1 << 30))
         return fail(h, PLORA_ERR_CONFIG, "the tile path needs a device handle and max_rank <= 128");
     h->seg.run_min = tokens;
-    h->seg.step_min = 0;  // the caller's line holds in steps of every size
     return PLORA_OK;
 }
 

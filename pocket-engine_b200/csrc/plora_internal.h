@@ -17,27 +17,16 @@
 // ---- device metadata produced once per step by the grouping kernel ("segs") ----
 // All int32 words. Gather path: tokens of short runs regrouped by slot and cut into work items of at
 // most PLORA_WORK_TOKENS tokens of one slot. Tile path: runs of contiguous tokens of one slot that are
-// at least PLORA_RUN_MIN long, cut into tensor-core tiles of PLORA_MMA_TOKENS tokens, in steps of more than
-// PLORA_STEP_MIN adapter tokens.
+// at least PLORA_RUN_MIN long, cut into tensor-core tiles of PLORA_MMA_TOKENS tokens.
 #define PLORA_WORK_TOKENS 16
 #define PLORA_WORK_WORDS 32
 #define PLORA_MMA_TOKENS 128
 #define PLORA_RUN_MIN_DEFAULT 64
-// A step of few tokens has too few tiles to fill the chip: a tile's shrink is a chain of copies along K that at most 8
-// blocks share (1 at a total rank over 128), and two more kernels per layer have to be launched and waited for.
-// The gather kernels cut the same tokens into items of 16, each over many blocks, and read the slab again for each item
-// (from L2), so their time grows with the tokens. Gather against tile path, us per step of 4 layers (hidden 4096):
-//   tokens            128        199        256        320        384        448        768
-//   rank 16         62 / 76    71 / 88    84 / 87    96 / 101  100 / 106   97 / 100  161 / 129
-//   rank 64         74 / 147  114 / 153  125 / 157  147 / 167  157 / 178  183 / 176  255 / 208
-//   rank 128       104 / 238  130 / 248  143 / 252  168 / 261  181 / 273  201 / 273
-// The one-kernel layers add a tile's term inside the base product, but a gather item's after it. Shrink and layer there:
-//   bf16, rank 16  243 / 247  258 / 250             293 / 277 (384)
-//   bf16, rank 64  250 / 310  274 / 311             327 / 339 (384)
-//   fp8, rank 16    68 / 64    74 / 64               95 / 77 (384)
-//   fp8, rank 64    74 / 87    82 / 86              113 / 102 (384)
-// so the line lies where these still break even over the ranks, not where the separate kernels would.
-#define PLORA_STEP_MIN_DEFAULT 256
+// The line is one of the run alone, in steps of every size: a prompt has the same bits alone and in any company, and in the
+// one-kernel layers its term is added before y is rounded. (One prompt of 64 to 256 tokens alone would be faster through the
+// gather kernels, us per step of 4 layers with hidden 4096, gather against tiles: rank 16 59 / 74 at 128 tokens, 68 / 79 at 199,
+// 84 / 86 at 256; rank 64 77 / 122, 111 / 130, 122 / 135; rank 128 95 / 152, 127 / 160, 140 / 166. Several of them are
+// not: eight of 100 tokens 193 / 130 at rank 16, 308 / 184 at rank 64, 348 / 226 at rank 128.)
 #define PLORA_XCHG_MAX_WORLD 8  // ranks of a tensor-parallel exchange
 
 #define SEG_N_ACT 0    // slots that have gather tokens
@@ -50,8 +39,7 @@
 
 struct SegLayout {
     int max_slots, max_tokens, cap_tiles;
-    int run_min;   // runs at least this long take the tensor-core tile path
-    int step_min;  // provided that the step has more adapter tokens than this
+    int run_min;  // runs at least this long take the tensor-core tile path
     // word offsets
     __host__ __device__ int act() const { return SEG_HDR; }                            // [max_slots] slot ids, ascending
     __host__ __device__ int seg_off() const { return act() + max_slots; }              // [max_slots + 1] by active index

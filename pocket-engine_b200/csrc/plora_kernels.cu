@@ -150,7 +150,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
 
 // ---------------------------------------------------------------------------------------------
 // Regroup the tile words by slot. Runs = maximal ranges of contiguous tokens of one slot. Runs of at
-// least lay.run_min tokens become tensor-core tiles, in steps of more than lay.step_min tokens; the rest are gathered by slot: perm lists their
+// least lay.run_min tokens become tensor-core tiles; the rest are gathered by slot: perm lists their
 // token rows ordered by (slot, position in the tile list), cut into work items of <= 16 tokens.
 //
 // Every block then writes the launch records of its layers (blockIdx.x, blockIdx.x + gridDim.x, ...): each gather work
@@ -264,8 +264,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
         }
 
     // classify runs; tensor-core tiles (none when every run stays under run_min)
-    const int run_min = n_tok > lay.step_min ? lay.run_min : 1 << 30;
-    const bool any_mma = run_min <= n_tok;
+    const bool any_mma = lay.run_min <= n_tok;
     int n_mma = 0;
     for (int base = 0; base < n_runs; base += 1024) {
         const int r = base + tid;
@@ -275,7 +274,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             slot = run_slot[r];
             start = run_start[r];
             if (slot == 0 || len == 0) run_pos[r] = -1;
-            else if (len >= run_min) {
+            else if (len >= lay.run_min) {
                 nm = (len + PLORA_MMA_TOKENS - 1) / PLORA_MMA_TOKENS;
                 run_pos[r] = -1;
             } else {

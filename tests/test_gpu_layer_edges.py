@@ -121,6 +121,7 @@ def test_few_tokens_over_a_wide_layer(pe, kind, rows, widths, f32_out):
         base = x.double() @ w.double().t()
     want = harness.oracle_f64(wl, table, harness.tiles_of(pe, wl), y_base=[base.cpu().numpy().astype(np.float32)])[0]
     y = torch.full((T, N), float("nan"), dtype=torch.float32 if f32_out else torch.bfloat16, device="cuda")
+    loras.set_run_min(1 << 30)  # (a step without long runs; only those take these tiles)
     loras.meta_upload(harness.tiles_of(pe, wl, loras.max_lora_tiles()))
     step = loras.lora_step(loras.max_lora_tiles())
     for _ in range(2):
