@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                                                                  const plora_desc* __restrict__ tables,
                                                                  const int* __restrict__ site_cols, int n_sites,
                                                                  PloraRec* __restrict__ recs, int rec_cap,
-                                                                 int* __restrict__ prefix) {
+                                                                 int* __restrict__ prefix, int expand_grid) {
     extern __shared__ int sm[];
     __shared__ unsigned long long sh[4][33];  // a row per scan in flight: no barrier between one scan and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -407,6 +407,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
             long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
+            long long first_item = 0;  // (thread 0's) units of the first item in the expand
             for (int base = 0; base < end; base += 1024) {
                 const int w = base + tid;
                 unsigned long long units = 0, total = 0;
@@ -415,6 +416,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                     if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
                     else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, pieces, nsplit, most);
                 }
+                if (w == 0) first_item = packed_expand(units);
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
                 if (w < nw) {
                     ps[1 + w] = packed_shrink(at);
@@ -424,7 +426,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             }
             if (tid == 0) {
                 ps[0] = nw;
-                pe[0] = nw;
+                pe[0] = (long long)share_blocks(packed_expand(before), nw, first_item, expand_grid) << 32 | nw;
                 ps[1 + nw] = packed_shrink(before);
                 pe[1] = pe[2 + nw] = packed_expand(before);
             }
@@ -455,15 +457,14 @@ __device__ __forceinline__ int load_prefix(int* pre, const int* __restrict__ src
     return pre[1 + n];
 }
 // The same for the expand, and the block's share [u0, u1) of all units. In shared memory the units before an item are
-// counted from u0. False where the block has no share (no less than about 200 columns per block).
+// counted from u0. False where the block has no share.
 __device__ __forceinline__ bool load_share(int* pre, const int* __restrict__ src, int rec_cap, int& share) {
     const long long* pe = reinterpret_cast<const long long*>(src);
-    const int n = min((int)__ldcg(pe), rec_cap);
-    const long long total = __ldcg(pe + 1);
+    const long long head = __ldcg(pe), total = __ldcg(pe + 1);
+    const int n = min((int)(head & 0xffffffff), rec_cap);
     long long mine = 0;  // (fetched beside the counts that say how many there are)
     if ((int)threadIdx.x <= rec_cap) mine = __ldcg(pe + 2 + threadIdx.x);
-    const long long most = total / 2048;
-    const int blocks = most < 1 ? 1 : most < (long long)gridDim.x ? (int)most : (int)gridDim.x;
+    const int blocks = min((int)(head >> 32), (int)gridDim.x);
     if ((int)blockIdx.x >= blocks || total == 0) return false;
     const long long u0 = share_at(total, blockIdx.x, blocks);
     share = (int)(share_at(total, blockIdx.x + 1, blocks) - u0);
@@ -1245,7 +1246,7 @@ cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayo
     // block repeats the grouping
     const int blocks = recs == nullptr ? 1 : n_sites < 64 ? n_sites : 64;
     return launch_pdl(plora_meta_group_kernel, dim3((unsigned)blocks), dim3(1024), plora_meta_group_smem(lay), st, pdl, tiles, segs, lay,
-                      status, tables, site_cols, n_sites, recs, rec_cap, prefix);
+                      status, tables, site_cols, n_sites, recs, rec_cap, prefix, 2 * g_sms);
 }
 
 // Two blocks per SM walk the units; `bound` is the most units a step of this size can have

@@ -28,6 +28,11 @@ int main(int argc, char** argv) {
     }
     const long long total = before[items], item = expand_item_units(r, rows, cnt, most);
     if (total != items * item || item > 0x7fffffffLL) return fail("expand units", total, item);
+    for (int grid = 1; grid <= 296; grid++) {  // the blocks that a grid gives the step
+        const int n = share_blocks(total, items, item, grid);
+        if (n < 1 || n > grid || (8 * items <= n && n % items != 0) || n < grid - grid / 8 - 1 - (total / 2048 < grid ? grid : 0)) return fail("blocks", grid, n);
+        if (share_blocks(total + 1, items, item, grid) < n) return fail("blocks of unequal items", grid, n);
+    }
     int last = -1, part0 = 0, col = 0, next = 0;  // where the block before ended: item, part, column; the block after it
     for (int b = 0; b < blocks; b++) {
         if (walk && b >= walk && b + walk < blocks && (b < blocks / 2 || b >= blocks / 2 + walk)) continue;
