@@ -973,10 +973,12 @@ __device__ __noinline__ int expand_stretch(unsigned char* pieces, uint64_t* full
     return stg | (int)(par << 8);
 }
 
-// The same for ranks above 128, which no piece holds: the rows of B from global memory, 32 ranks at a time
+// The same for ranks above 128, which no piece holds: the rows of B from global memory, 32 ranks at a time, four such loads
+// of a row on their way together. (With one, each waited for L2 or memory by itself: a layer block at rank 256, 16 tokens of
+// 16 adapters 389 -> 219 us, 2,000 tokens 2900 -> 1950; the CUDA-core kernel before took 291 and 12,200.)
 template <bool F32>
 __device__ __noinline__ void expand_wide_rank(const bf16* B, ExpandUnit un, ExpandStep st, const PloraRec& rec, int warp, int g, int t4) {
-    constexpr int ES = F32 ? 4 : 2, NT = 2;
+    constexpr int ES = F32 ? 4 : 2, NT = 2, AHEAD = 4;
     const bool wide = ((reinterpret_cast<uintptr_t>(st.Y) | ((size_t)st.ldy * ES) | (un.ybase * ES)) & 15) == 0;
     const uint32_t plane = 16u * st.s_pad;
 #pragma unroll 1
@@ -992,20 +994,33 @@ __device__ __noinline__ void expand_wide_rank(const bf16* B, ExpandUnit un, Expa
             float d[NT][4];
 #pragma unroll
             for (int i = 0; i < NT; i++) d[i][0] = d[i][1] = d[i][2] = d[i][3] = 0.f;
-#pragma unroll 1
-            for (int k = 0; k < un.r; k += 32) {
-                const uint32_t o = 2u * k + 16u * t4;
-                const uint4 h = lds128(sp + o), m = lds128(sp + plane + o), l = lds128(sp + 2 * plane + o);
-                const uint32_t al0[4] = {l.x, 0u, l.y, 0u}, ah0[4] = {h.x, m.x, h.y, m.y}, al1[4] = {l.z, 0u, l.w, 0u}, ah1[4] = {h.z, m.z, h.w, m.w};
+            const bf16* row[NT];
 #pragma unroll
-                for (int i = 0; i < NT; i++) {
-                    const int col = min(c + 2 * NT * (g >> 1) + 2 * i + (g & 1), un.c1 - 1);
-                    uint4 b = make_uint4(0u, 0u, 0u, 0u);
-                    if (k + 8 * t4 < un.r) b = __ldg(reinterpret_cast<const uint4*>(B + (size_t)col * un.r + k + 8 * t4));
-                    mma_16816(d[i], al0, b.x, b.y);
-                    mma_16816(d[i], ah0, b.x, b.y);
-                    mma_16816(d[i], al1, b.z, b.w);
-                    mma_16816(d[i], ah1, b.z, b.w);
+            for (int i = 0; i < NT; i++) row[i] = B + (size_t)min(c + 2 * NT * (g >> 1) + 2 * i + (g & 1), un.c1 - 1) * un.r + 8 * t4;
+#pragma unroll 1
+            for (int k0 = 0; k0 < un.r; k0 += 32 * AHEAD) {
+                uint4 b[AHEAD][NT];
+#pragma unroll
+                for (int q = 0; q < AHEAD; q++)
+#pragma unroll
+                    for (int i = 0; i < NT; i++) {
+                        b[q][i] = make_uint4(0u, 0u, 0u, 0u);
+                        if (k0 + 32 * q + 8 * t4 < un.r) b[q][i] = __ldg(reinterpret_cast<const uint4*>(row[i] + k0 + 32 * q));
+                    }
+#pragma unroll
+                for (int q = 0; q < AHEAD; q++) {
+                    const int k = k0 + 32 * q;
+                    if (k >= un.r) break;
+                    const uint32_t o = 2u * k + 16u * t4;
+                    const uint4 h = lds128(sp + o), m = lds128(sp + plane + o), l = lds128(sp + 2 * plane + o);
+                    const uint32_t al0[4] = {l.x, 0u, l.y, 0u}, ah0[4] = {h.x, m.x, h.y, m.y}, al1[4] = {l.z, 0u, l.w, 0u}, ah1[4] = {h.z, m.z, h.w, m.w};
+#pragma unroll
+                    for (int i = 0; i < NT; i++) {
+                        mma_16816(d[i], al0, b[q][i].x, b[q][i].y);
+                        mma_16816(d[i], ah0, b[q][i].x, b[q][i].y);
+                        mma_16816(d[i], al1, b[q][i].z, b[q][i].w);
+                        mma_16816(d[i], ah1, b[q][i].z, b[q][i].w);
+                    }
                 }
             }
             y_store<F32, NT>(y, d, yrow + (size_t)mine * ES, cols, wide);
@@ -1062,7 +1077,8 @@ __device__ __forceinline__ void expand_stage_s(const ExpandUnit& un, const Expan
     }
 }
 
-template <bool F32>
+// WIDE: for registries whose adapters may have ranks above 128 (the call takes registers that the other form has better uses for)
+template <bool F32, bool WIDE>
 __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(const float* __restrict__ S, size_t s_stride, int lds, int nsplit,
                                                                       const PloraRec* __restrict__ recs, int rec_cap,
                                                                       const int* __restrict__ prefix, void* Y, int ldy, int s_pad,
@@ -1109,7 +1125,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
 #endif
             u += expand_stretch_at(r, rows, cnt, most, u - pre[1 + w], u1 - u, part, c0, c1);
             const int rp = __ldcg(&rec.r[part]);
-            if (c0 >= c1 || rp > 128) continue;  // (ranks above 128 are read from global memory)
+            if (c0 >= c1 || (WIDE && rp > 128)) continue;  // (ranks above 128 are read from global memory)
             const bf16* B = reinterpret_cast<const bf16*>(__ldcg(&rec.b[part]));
             const size_t off = (size_t)__ldcg(&rec.off[part]);
             const int pc = expand_piece_cols(rp);
@@ -1168,7 +1184,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
             un.ybase = (size_t)srec.off[part];
             expand_stage_s(un, st, srec, tid);
             gather_sync();
-            if (un.r > 128) {
+            if (WIDE && un.r > 128) {
                 expand_wide_rank<F32>(reinterpret_cast<const bf16*>(srec.b[part]), un, st, srec, warp, g, t4);
             } else {
 #define PLORA_STRETCH(NARROW, KEEP)                                                                                     \
@@ -1233,9 +1249,10 @@ cudaError_t plora_kernels_init(const SegLayout& lay) {
     // The few-token kernels overlap with their neighbours in the stream (programmatic dependent launch), and an SM's
     // split between L1 and shared memory is fixed while any block runs on it: all of them ask for the largest
     // split, so that a block of the next kernel finds room beside the blocks of this one.
-    const void* fns[3] = {reinterpret_cast<const void*>(plora_shrink_gather_kernel), reinterpret_cast<const void*>(plora_expand_gather_kernel<false>),
-                          reinterpret_cast<const void*>(plora_expand_gather_kernel<true>)};
-    for (int i = 0; i < 3 && e == cudaSuccess; i++) e = plora_kernel_shared(fns[i], 220 * 1024);
+    const void* fns[5] = {reinterpret_cast<const void*>(plora_shrink_gather_kernel),
+                          reinterpret_cast<const void*>(plora_expand_gather_kernel<false, false>), reinterpret_cast<const void*>(plora_expand_gather_kernel<true, false>),
+                          reinterpret_cast<const void*>(plora_expand_gather_kernel<false, true>), reinterpret_cast<const void*>(plora_expand_gather_kernel<true, true>)};
+    for (int i = 0; i < 5 && e == cudaSuccess; i++) e = plora_kernel_shared(fns[i], 220 * 1024);
     return e;
 }
 
@@ -1272,6 +1289,8 @@ cudaError_t plora_launch_expand(const float* S, size_t s_stride_elems, int lds, 
     const int s_pad = ((max_rank + 31) & ~31) * 2 + 16;  // an odd number of 16-byte pieces between the rows of a plane
     const unsigned grid = unit_grid(1 + (long long)work_cap * parts * max_rows * expand_cost(max_rank, PLORA_WORK_TOKENS) / 2048);
     const size_t smem = (size_t)EXP_STAGES * EXP_PIECE + (size_t)3 * 16 * s_pad + (size_t)8 * EXP_AHEAD * EXP_Y_BYTES + (size_t)(rec_cap + 2) * sizeof(int);
-    return launch_pdl(f32_out ? plora_expand_gather_kernel<true> : plora_expand_gather_kernel<false>, dim3(grid), dim3(GATHER_THREADS), smem, st,
+    auto* fn = max_rank > 128 ? (f32_out ? plora_expand_gather_kernel<true, true> : plora_expand_gather_kernel<false, true>)
+                              : (f32_out ? plora_expand_gather_kernel<true, false> : plora_expand_gather_kernel<false, false>);
+    return launch_pdl(fn, dim3(grid), dim3(GATHER_THREADS), smem, st,
                       pdl, S, s_stride_elems, lds, nsplit, recs, rec_cap, prefix, y, ldy, s_pad, most, early ? 1 : 0, status PLORA_BOUNDS_ARG(bnd));
 }
