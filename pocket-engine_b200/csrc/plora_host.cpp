@@ -385,11 +385,11 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
                 s.cluster_ok = h->site_ok && plora_site_plan(s.cols, (int)s.parts.size(), h->max_rank, total, &nsub) > 0;
                 if (s.cluster_ok) {
                     s.max_clusters = plora_site_max_clusters(s.cols, (int)s.parts.size(), h->max_rank, total);
-                    // One work item per slot, in no more than a round and a quarter of the clusters that run at once: past that
-                    // the pair of kernels, whose blocks share all items' work evenly, is faster (128 tokens of 48 rank-16
-                    // adapters, four layers: 295 us in clusters, 261 as pairs; of 32 adapters 181 and 216). The rule looks at
-                    // the registry and not at the step, so that a token's result does not depend on its batch.
-                    if (s.max_clusters < nsub || 4 * max_slots * nsub > 5 * s.max_clusters) s.cluster_ok = false;
+                    // Whatever the number of slots: how many of them a step uses is not known here, and a rule on the step
+                    // would let a token's result depend on its batch. Rank 16, two layers, tokens of adapters in 64 slots,
+                    // clusters against the pair of kernels: 1 of 1 50 / 55 us, 8 of 8 60 / 76, 64 of 16 71 / 92, 64 of 32
+                    // 101 / 114; only steps of more than 40 adapters are faster as pairs (64 of 48 147 / 137, 64 of 64 179 / 163).
+                    if (s.max_clusters < nsub) s.cluster_ok = false;
                 }
                 info.push_back(s.cols);
                 info.push_back(s.cluster_ok ? 8 * nsub : 0);

@@ -1,6 +1,6 @@
 """The few-token shrink and expand at the edges of their units: every width of the rank, work items of 1, 8, 9 and 16
-tokens, input ranges and output columns that end inside a unit, more work items than a block keeps counts for, and slot
-counts on both sides of the line between one cluster kernel per layer and the pair."""
+tokens, input ranges and output columns that end inside a unit, more work items than a block keeps counts for, and the
+cluster kernel over steps of fewer and of more adapters than clusters run at once."""
 import pytest
 
 import harness
