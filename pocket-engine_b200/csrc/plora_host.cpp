@@ -7,7 +7,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <system_error>
+#include <exception>
 #include <thread>
 
 #include "plora_internal.h"
@@ -120,9 +120,10 @@ void run_jobs(const std::vector<FillJob>& jobs, size_t values) {
     const size_t want = std::min<size_t>(std::min<size_t>(16, std::max(1u, std::thread::hardware_concurrency())), values / kJobValues + 1);
     std::vector<std::thread> others;
     try {
+        others.reserve(want);
         for (size_t t = 1; t < want; t++) others.emplace_back(work);
-    } catch (const std::system_error&) {
-        // no more threads to be had: the ones that run, this one among them, do the work
+    } catch (const std::exception&) {
+        // no more threads, or memory for them, to be had: the ones that run, this one among them, do the work
     }
     work();
     for (auto& t : others) t.join();
