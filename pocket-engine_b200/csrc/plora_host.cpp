@@ -715,15 +715,17 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
     cudaStream_t st = as_stream(stream);
     uint8_t* base = h->pool + (size_t)(slot - 1) * h->slot_bytes;
     if (a->len > 0) {
-        CU(h, "upload slab", cudaMemcpyAsync(base, a->data, a->len, cudaMemcpyHostToDevice, st));
-        // the buffer may be handed to another adapter once this copy is done; a second stream, or a graph that copies
-        // again on every replay, takes it out of that
+        // The buffer may be handed to another adapter once this copy is done; a second stream, or a graph that copies again on
+        // every replay, takes it out of that. So does a call below that fails: nothing then tells when the copy is done.
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         CU(h, "capture status", cudaStreamIsCapturing(st, &cs));
-        if (cs != cudaStreamCaptureStatusNone || (a->uploaded && a->up_stream != stream)) a->keep_out = true;
-        if (!a->keep_out) {
-            if (!a->buf.used) CU(h, "event", cudaEventCreateWithFlags(&a->buf.used, cudaEventDisableTiming));
+        const bool once = !a->keep_out && cs == cudaStreamCaptureStatusNone && (!a->uploaded || a->up_stream == stream);
+        if (once && !a->buf.used) CU(h, "event", cudaEventCreateWithFlags(&a->buf.used, cudaEventDisableTiming));
+        a->keep_out = true;
+        CU(h, "upload slab", cudaMemcpyAsync(base, a->data, a->len, cudaMemcpyHostToDevice, st));
+        if (once) {
             CU(h, "upload record", cudaEventRecord(a->buf.used, st));
+            a->keep_out = false;
             a->up_stream = stream;
             a->uploaded = true;
         }
