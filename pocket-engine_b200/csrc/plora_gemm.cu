@@ -573,8 +573,11 @@ cudaError_t plora_gemm_init() {
     PLORA_GEMM_INIT(1, false);
     PLORA_GEMM_INIT(1, true);
 #undef PLORA_GEMM_INIT
+    int dev = 0, sms = 0;
+    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(148);
+    cfg.gridDim = dim3((unsigned)(sms & ~1));
     cfg.blockDim = dim3(64 + G_EPI);
     cfg.dynamicSmemBytes = gemm_smem(256, true);
     int n = 0;

@@ -561,285 +561,285 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
     // walk in turn. (Sized for the most tiles a step can have, half of the blocks of a prefill step found none and
     // cost 15 us of 780.)
     for (int tile = blockIdx.z; tile < n_mma; tile += gridDim.z) {
-    const int* mt = segs + lay.mma() + 3 * tile;
-    const int start = mt[0], len = mt[1], slot = mt[2];
-    const plora_desc& d = table[slot];
-    const int r = d.r[p], rows = d.rows[p];
-    if (r == 0 || cb0 * EXP_BN >= rows) continue;
-    const int nblk = min(nb_per_cta, (rows - cb0 * EXP_BN + EXP_BN - 1) / EXP_BN);
-    const int nchunks = min(nblk * CH, (rows - cb0 * EXP_BN + CW - 1) / CW);  // slots this block fills, in column order
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    unsigned char* ring = dsm1k + (size_t)warp * nst * EXP_SLOT_BYTES;  // this warp's slots
-    unsigned char* ops = dsm1k + (size_t)NW * nst * EXP_SLOT_BYTES;
-    ExpandBars& bars = *reinterpret_cast<ExpandBars*>(ops + nbs * (size_t)b_bytes);
-    // warps w and w + 4 read the same 32 lanes of tensor memory (rows 32 (w % 4) ...) and take the even and the odd
-    // slots of the block's columns
-    const int wq = warp & 3, wh = warp >> 2;
-    const int P = r >> 3;
-    const CUtensorMap* ymap = &ymaps.m[p];
-    const CUtensorMap* bmap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].b[p]);
-    // the rows of B of column block nb: r / bw boxes of 64 rows by bw ranks, one after another in stage nb % nbs
-    const int bw = exp_b_width(r);
-    auto load_b = [&](int nb) {
-        const int stg = nb % nbs;
-        mbar_expect_tx(&bars.b_full[stg], (uint32_t)(EXP_BN * r * 2));
-        for (int q = 0; q < r; q += bw)
-            tma_load_2d(ops + (size_t)stg * b_bytes + (size_t)q * EXP_BN * 2, bmap, q, (cb0 + nb) * EXP_BN, &bars.b_full[stg]);
-    };
-
-    if (tid == 0) {
-        auto start_bar = [&](uint64_t* bar, uint32_t count) {
-            if (begun) mbar_inval(bar);
-            mbar_init(bar, count);
+        const int* mt = segs + lay.mma() + 3 * tile;
+        const int start = mt[0], len = mt[1], slot = mt[2];
+        const plora_desc& d = table[slot];
+        const int r = d.r[p], rows = d.rows[p];
+        if (r == 0 || cb0 * EXP_BN >= rows) continue;
+        const int nblk = min(nb_per_cta, (rows - cb0 * EXP_BN + EXP_BN - 1) / EXP_BN);
+        const int nchunks = min(nblk * CH, (rows - cb0 * EXP_BN + CW - 1) / CW);  // slots this block fills, in column order
+        const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+        unsigned char* ring = dsm1k + (size_t)warp * nst * EXP_SLOT_BYTES;  // this warp's slots
+        unsigned char* ops = dsm1k + (size_t)NW * nst * EXP_SLOT_BYTES;
+        ExpandBars& bars = *reinterpret_cast<ExpandBars*>(ops + nbs * (size_t)b_bytes);
+        // warps w and w + 4 read the same 32 lanes of tensor memory (rows 32 (w % 4) ...) and take the even and the odd
+        // slots of the block's columns
+        const int wq = warp & 3, wh = warp >> 2;
+        const int P = r >> 3;
+        const CUtensorMap* ymap = &ymaps.m[p];
+        const CUtensorMap* bmap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].b[p]);
+        // the rows of B of column block nb: r / bw boxes of 64 rows by bw ranks, one after another in stage nb % nbs
+        const int bw = exp_b_width(r);
+        auto load_b = [&](int nb) {
+            const int stg = nb % nbs;
+            mbar_expect_tx(&bars.b_full[stg], (uint32_t)(EXP_BN * r * 2));
+            for (int q = 0; q < r; q += bw)
+                tma_load_2d(ops + (size_t)stg * b_bytes + (size_t)q * EXP_BN * 2, bmap, q, (cb0 + nb) * EXP_BN, &bars.b_full[stg]);
         };
-        start_bar(&bars.done[0], 1);
-        start_bar(&bars.done[1], 1);
-        // the warps that have rows of the tile and a slot in the accumulator's column blocks: the ones of one parity
-        // where a column block is one slot, all where it is two
-        const int live_warps = CH * min(4, (len + 31) / 32);
-        start_bar(&bars.acc_free[0], live_warps);
-        start_bar(&bars.acc_free[1], live_warps);
-        start_bar(&bars.a_full, 32 * NW);
-        for (int i = 0; i < nbs; i++) start_bar(&bars.b_full[i], 1);
-        for (int w = 0; w < NW; w++)
-            for (int i = 0; i < nst; i++) start_bar(&bars.ybar[w][i], 1);
-        mbar_fence_init();
-    }
-    if (warp == NW && !begun) tmem_alloc(&bars.tmem_slot, 256);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = bars.tmem_slot;
-    const bool leader = warp == NW && elect_one();
-    if (leader) {
-        tmap_acquire(bmap);
-        for (int nb = 0; nb < nbs - 2 && nb < nblk; nb++) load_b(nb);  // a slab: it may be fetched before the kernels ahead have finished
-    }
-    if (!begun) {
-        if (!late) pdl_wait();
-        pdl_trigger();
-        begun = true;
-    }
 
-    if (warp == NW) {
-        // ---- B copies (nbs - 2 column blocks ahead) and MMAs (up to two column blocks ahead of the additions)
-        if (leader) {
-            const uint32_t idesc = umma_idesc_bf16(MMA_M, EXP_BN);
-            const uint32_t a_hi = tmem + EXP_TMEM_A, a_lo = a_hi + (uint32_t)(r >> 1);
-            const uint32_t sw = bw == 64 ? 2u : bw == 32 ? 4u : 6u;
-            const uint64_t b0 = umma_desc(smem_u32(ops), 16, (uint32_t)bw * 16u, sw);  // eight rows of a box are bw * 16 bytes
-            bool ok = mbar_wait_long(&bars.a_full, 0, status);  // S staged by the other warps
-            int stg = 0;
-            uint32_t bpar = 0;
-            for (int nb = 0; ok && nb < nblk; nb++) {
-                // the accumulator this block goes to was last read for block nb - 2, whose stage of B is therefore free too
-                if (nb >= 2) ok = mbar_wait_long(&bars.acc_free[nb & 1], ((nb >> 1) - 1) & 1, status);
-                if (!ok) break;
-                if (nb + nbs - 2 < nblk) load_b(nb + nbs - 2);
-                ok = mbar_wait_long(&bars.b_full[stg], bpar, status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t bd = b0 + (uint64_t)((uint32_t)stg * (uint32_t)b_bytes >> 4);
-                const uint32_t acc = tmem + (uint32_t)(nb & 1) * EXP_BN;
-                for (int half = 0; half < 2; half++)
-                    for (int k = 0; k < r; k += 16)
-                        umma_ta(acc, (half ? a_lo : a_hi) + (uint32_t)(k >> 1), bd + (uint64_t)((k / bw) * (EXP_BN * bw * 2 / 16) + (k % bw) / 8),
-                                idesc, (half | k) != 0);
-                umma_commit(&bars.done[nb & 1]);
-                if (++stg == nbs) {
-                    stg = 0;
-                    bpar ^= 1;
-                }
-            }
-            // every MMA has completed before the tensor memory goes back
-            if (ok && nblk >= 1) mbar_wait_long(&bars.done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status);
-            if (ok && nblk >= 2) mbar_wait_long(&bars.done[(nblk - 2) & 1], ((nblk - 2) >> 1) & 1, status);
+        if (tid == 0) {
+            auto start_bar = [&](uint64_t* bar, uint32_t count) {
+                if (begun) mbar_inval(bar);
+                mbar_init(bar, count);
+            };
+            start_bar(&bars.done[0], 1);
+            start_bar(&bars.done[1], 1);
+            // the warps that have rows of the tile and a slot in the accumulator's column blocks: the ones of one parity
+            // where a column block is one slot, all where it is two
+            const int live_warps = CH * min(4, (len + 31) / 32);
+            start_bar(&bars.acc_free[0], live_warps);
+            start_bar(&bars.acc_free[1], live_warps);
+            start_bar(&bars.a_full, 32 * NW);
+            for (int i = 0; i < nbs; i++) start_bar(&bars.b_full[i], 1);
+            for (int w = 0; w < NW; w++)
+                for (int i = 0; i < nst; i++) start_bar(&bars.ybar[w][i], 1);
+            mbar_fence_init();
         }
-        __syncwarp();
-    } else {
-    const int wrow0 = wq * 32;
-    const bool live = wrow0 < len;            // the warp has rows of the tile
-    const bool whole = wrow0 + 32 <= len;     // all its 32 rows are: results go back by tensor store
-    const int ycol0 = d.off[p] + cb0 * EXP_BN;  // first y column of this block's range
-    const uint32_t lane_base = tmem + ((uint32_t)wrow0 << 16);
-    // the warp's i-th slot is slot wh + 2 i of the block's column range
-    const int my_n = (nchunks - wh + WPQ - 1) / WPQ;
-    auto load_y = [&](int i, int at) {        // lane 0 only; `at` = i % nst
-        uint64_t* bar = &bars.ybar[warp][at];
-        mbar_expect_tx(bar, EXP_SLOT_BYTES);
-        tma_load_2d(ring + (size_t)at * EXP_SLOT_BYTES, ymap, ycol0 + (wh + WPQ * i) * CW, start + wrow0, bar);
-    };
-    if (live && lane == 0)
-        for (int i = 0; i < nst && i < my_n; i++) load_y(i, i);
+        if (warp == NW && !begun) tmem_alloc(&bars.tmem_slot, 256);
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        const uint32_t tmem = bars.tmem_slot;
+        const bool leader = warp == NW && elect_one();
+        if (leader) {
+            tmap_acquire(bmap);
+            for (int nb = 0; nb < nbs - 2 && nb < nblk; nb++) load_b(nb);  // a slab: it may be fetched before the kernels ahead have finished
+        }
+        if (!begun) {
+            if (!late) pdl_wait();
+            pdl_trigger();
+            begun = true;
+        }
 
-    // this thread's token row of S, split into a bf16 high part and the bf16 of what is left, into its lane of tensor memory
-    {
-        const int row = tid & 127;
-        const bool valid = row < len;
-        const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
-        const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
-        auto put = [&](int j, const float* f) {
-            uint32_t hi[4], lo[4];
-#pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-                const float2 hf = __bfloat1622float2(h);
-                const __nv_bfloat162 l = __floats2bfloat162_rn(f[2 * e] - hf.x, f[2 * e + 1] - hf.y);
-                hi[e] = *reinterpret_cast<const uint32_t*>(&h);
-                lo[e] = *reinterpret_cast<const uint32_t*>(&l);
+        if (warp == NW) {
+            // ---- B copies (nbs - 2 column blocks ahead) and MMAs (up to two column blocks ahead of the additions)
+            if (leader) {
+                const uint32_t idesc = umma_idesc_bf16(MMA_M, EXP_BN);
+                const uint32_t a_hi = tmem + EXP_TMEM_A, a_lo = a_hi + (uint32_t)(r >> 1);
+                const uint32_t sw = bw == 64 ? 2u : bw == 32 ? 4u : 6u;
+                const uint64_t b0 = umma_desc(smem_u32(ops), 16, (uint32_t)bw * 16u, sw);  // eight rows of a box are bw * 16 bytes
+                bool ok = mbar_wait_long(&bars.a_full, 0, status);  // S staged by the other warps
+                int stg = 0;
+                uint32_t bpar = 0;
+                for (int nb = 0; ok && nb < nblk; nb++) {
+                    // the accumulator this block goes to was last read for block nb - 2, whose stage of B is therefore free too
+                    if (nb >= 2) ok = mbar_wait_long(&bars.acc_free[nb & 1], ((nb >> 1) - 1) & 1, status);
+                    if (!ok) break;
+                    if (nb + nbs - 2 < nblk) load_b(nb + nbs - 2);
+                    ok = mbar_wait_long(&bars.b_full[stg], bpar, status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint64_t bd = b0 + (uint64_t)((uint32_t)stg * (uint32_t)b_bytes >> 4);
+                    const uint32_t acc = tmem + (uint32_t)(nb & 1) * EXP_BN;
+                    for (int half = 0; half < 2; half++)
+                        for (int k = 0; k < r; k += 16)
+                            umma_ta(acc, (half ? a_lo : a_hi) + (uint32_t)(k >> 1), bd + (uint64_t)((k / bw) * (EXP_BN * bw * 2 / 16) + (k % bw) / 8),
+                                    idesc, (half | k) != 0);
+                    umma_commit(&bars.done[nb & 1]);
+                    if (++stg == nbs) {
+                        stg = 0;
+                        bpar ^= 1;
+                    }
+                }
+                // every MMA has completed before the tensor memory goes back
+                if (ok && nblk >= 1) mbar_wait_long(&bars.done[(nblk - 1) & 1], ((nblk - 1) >> 1) & 1, status);
+                if (ok && nblk >= 2) mbar_wait_long(&bars.done[(nblk - 2) & 1], ((nblk - 2) >> 1) & 1, status);
             }
             __syncwarp();
-            tmem_st4(lane_base + EXP_TMEM_A + 4 * j, hi);
-            tmem_st4(lane_base + EXP_TMEM_A + (r >> 1) + 4 * j, lo);
-        };
-        if (s_eff > 1) {
-#pragma unroll 1
-            for (int j = tid >> 7; j < P; j += WPQ) {
-                float v[PLORA_TILE_SPLIT_MAX][8];
-#pragma unroll
-                for (int s = 0; s < PLORA_TILE_SPLIT_MAX; s++) {
-                    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                    if (valid && s < s_eff) {
-                        const float* q = sp + (size_t)s * s_stride + j * 8;
-                        a = __ldcg(reinterpret_cast<const float4*>(q));
-                        b = __ldcg(reinterpret_cast<const float4*>(q + 4));
-                    }
-                    v[s][0] = a.x, v[s][1] = a.y, v[s][2] = a.z, v[s][3] = a.w;
-                    v[s][4] = b.x, v[s][5] = b.y, v[s][6] = b.z, v[s][7] = b.w;
-                }
-                tree_sum<8>(v, s_eff);
-                put(j, v[0]);
-            }
         } else {
-            // four pieces of eight values per round trip
-#pragma unroll 1
-            for (int j0 = tid >> 7; j0 < P; j0 += 4 * WPQ) {
-                float4 f[4][2];
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const int j = j0 + q * WPQ;
-                    f[q][0] = f[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (valid && j < P) {
-                        f[q][0] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
-                        f[q][1] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
-                    }
-                }
-#pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (j0 + q * WPQ < P) put(j0 + q * WPQ, reinterpret_cast<const float*>(f[q]));
-            }
-        }
-        tmem_st_wait();
-        tc_fence_before();
-        mbar_arrive(&bars.a_full);  // S is staged
-    }
+            const int wrow0 = wq * 32;
+            const bool live = wrow0 < len;            // the warp has rows of the tile
+            const bool whole = wrow0 + 32 <= len;     // all its 32 rows are: results go back by tensor store
+            const int ycol0 = d.off[p] + cb0 * EXP_BN;  // first y column of this block's range
+            const uint32_t lane_base = tmem + ((uint32_t)wrow0 << 16);
+            // the warp's i-th slot is slot wh + 2 i of the block's column range
+            const int my_n = (nchunks - wh + WPQ - 1) / WPQ;
+            auto load_y = [&](int i, int at) {        // lane 0 only; `at` = i % nst
+                uint64_t* bar = &bars.ybar[warp][at];
+                mbar_expect_tx(bar, EXP_SLOT_BYTES);
+                tma_load_2d(ring + (size_t)at * EXP_SLOT_BYTES, ymap, ycol0 + (wh + WPQ * i) * CW, start + wrow0, bar);
+            };
+            if (live && lane == 0)
+                for (int i = 0; i < nst && i < my_n; i++) load_y(i, i);
 
-    bool ok = true;
-    int at = 0;             // i % nst
-    uint32_t ypar = 0;      // (i / nst) & 1
+            // this thread's token row of S, split into a bf16 high part and the bf16 of what is left, into its lane of tensor memory
+            {
+                const int row = tid & 127;
+                const bool valid = row < len;
+                const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
+                const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
+                auto put = [&](int j, const float* f) {
+                    uint32_t hi[4], lo[4];
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
+                        const float2 hf = __bfloat1622float2(h);
+                        const __nv_bfloat162 l = __floats2bfloat162_rn(f[2 * e] - hf.x, f[2 * e + 1] - hf.y);
+                        hi[e] = *reinterpret_cast<const uint32_t*>(&h);
+                        lo[e] = *reinterpret_cast<const uint32_t*>(&l);
+                    }
+                    __syncwarp();
+                    tmem_st4(lane_base + EXP_TMEM_A + 4 * j, hi);
+                    tmem_st4(lane_base + EXP_TMEM_A + (r >> 1) + 4 * j, lo);
+                };
+                if (s_eff > 1) {
 #pragma unroll 1
-    for (int i = 0; ok && live && i < my_n; i++) {  // the warp's slots, in column order
-        const int q = wh + WPQ * i, nb = q / CH, ch = q % CH;
-        ok = mbar_wait_long(&bars.done[nb & 1], (nb >> 1) & 1, status);
-        if (!ok) break;
-        tc_fence_after();
-        // 32 accumulator columns at a time: 64 at once leave too few registers, and what spills goes through to L2 beside y;
-        // the accumulator is given back once the last ones are in registers
-        uint32_t v[32];
-        const uint32_t acc = lane_base + (uint32_t)(nb & 1) * EXP_BN + ch * CW;
-        auto fetch = [&](int h) {
-            tmem_ld32(acc + h * 32, v);
-            if (h + 1 == CW / 32) {
+                    for (int j = tid >> 7; j < P; j += WPQ) {
+                        float v[PLORA_TILE_SPLIT_MAX][8];
+#pragma unroll
+                        for (int s = 0; s < PLORA_TILE_SPLIT_MAX; s++) {
+                            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+                            if (valid && s < s_eff) {
+                                const float* q = sp + (size_t)s * s_stride + j * 8;
+                                a = __ldcg(reinterpret_cast<const float4*>(q));
+                                b = __ldcg(reinterpret_cast<const float4*>(q + 4));
+                            }
+                            v[s][0] = a.x, v[s][1] = a.y, v[s][2] = a.z, v[s][3] = a.w;
+                            v[s][4] = b.x, v[s][5] = b.y, v[s][6] = b.z, v[s][7] = b.w;
+                        }
+                        tree_sum<8>(v, s_eff);
+                        put(j, v[0]);
+                    }
+                } else {
+                    // four pieces of eight values per round trip
+#pragma unroll 1
+                    for (int j0 = tid >> 7; j0 < P; j0 += 4 * WPQ) {
+                        float4 f[4][2];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const int j = j0 + q * WPQ;
+                            f[q][0] = f[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (valid && j < P) {
+                                f[q][0] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
+                                f[q][1] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
+                            }
+                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            if (j0 + q * WPQ < P) put(j0 + q * WPQ, reinterpret_cast<const float*>(f[q]));
+                    }
+                }
+                tmem_st_wait();
                 tc_fence_before();
+                mbar_arrive(&bars.a_full);  // S is staged
+            }
+
+            bool ok = true;
+            int at = 0;             // i % nst
+            uint32_t ypar = 0;      // (i / nst) & 1
+#pragma unroll 1
+            for (int i = 0; ok && live && i < my_n; i++) {  // the warp's slots, in column order
+                const int q = wh + WPQ * i, nb = q / CH, ch = q % CH;
+                ok = mbar_wait_long(&bars.done[nb & 1], (nb >> 1) & 1, status);
+                if (!ok) break;
+                tc_fence_after();
+                // 32 accumulator columns at a time: 64 at once leave too few registers, and what spills goes through to L2 beside y;
+                // the accumulator is given back once the last ones are in registers
+                uint32_t v[32];
+                const uint32_t acc = lane_base + (uint32_t)(nb & 1) * EXP_BN + ch * CW;
+                auto fetch = [&](int h) {
+                    tmem_ld32(acc + h * 32, v);
+                    if (h + 1 == CW / 32) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&bars.acc_free[nb & 1]);
+                    }
+                };
+                fetch(0);
+                unsigned char* sl = ring + (size_t)at * EXP_SLOT_BYTES;
+                if (!mbar_wait(&bars.ybar[warp][at], ypar, status)) {
+                    ok = false;
+                    break;
+                }
+                unsigned char* myrow = sl + lane * 128;
+                const int col0 = (cb0 + nb) * EXP_BN + ch * CW;  // first column of the slot within the part
+                const bool mine = wrow0 + lane < len;
+                if (F32) {
+                    float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        float4* yp = reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4));
+                        float4 y = *yp;
+                        y.x += __uint_as_float(v[4 * c]), y.y += __uint_as_float(v[4 * c + 1]);
+                        y.z += __uint_as_float(v[4 * c + 2]), y.w += __uint_as_float(v[4 * c + 3]);
+                        if (whole) {
+                            *yp = y;
+                        } else if (mine) {
+                            if (col0 + 4 * c + 4 <= rows) {
+                                *reinterpret_cast<float4*>(yrow + 4 * c) = y;
+                            } else {
+                                const float e[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+                                for (int k = 0; k < 4; k++)
+                                    if (col0 + 4 * c + k < rows) yrow[4 * c + k] = e[k];
+                            }
+                        }
+                    }
+                } else {
+                    bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+#pragma unroll
+                    for (int c = 0; c < 8; c++) {
+                        if (c == 4) fetch(1);
+                        uint4* yp = reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4));
+                        const uint4 raw = *yp;
+                        float f[8];
+                        unpack8(raw, f);
+                        uint32_t o[4];
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[8 * (c & 3) + 2 * e]),
+                                                                            f[2 * e + 1] + __uint_as_float(v[8 * (c & 3) + 2 * e + 1]));
+                            o[e] = *reinterpret_cast<const uint32_t*>(&b2);
+                        }
+                        if (whole) {
+                            *yp = make_uint4(o[0], o[1], o[2], o[3]);
+                        } else if (mine) {
+                            if (col0 + 8 * c + 8 <= rows) {
+                                *reinterpret_cast<uint4*>(yrow + 8 * c) = make_uint4(o[0], o[1], o[2], o[3]);
+                            } else {
+#pragma unroll
+                                for (int k = 0; k < 4; k++)  // (a part's width is even)
+                                    if (col0 + 8 * c + 2 * k < rows) *reinterpret_cast<uint32_t*>(yrow + 8 * c + 2 * k) = o[k];
+                            }
+                        }
+                    }
+                }
+                if (whole) fence_async_smem();  // the additions above, before the tensor store reads them
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&bars.acc_free[nb & 1]);
-            }
-        };
-        fetch(0);
-        unsigned char* sl = ring + (size_t)at * EXP_SLOT_BYTES;
-        if (!mbar_wait(&bars.ybar[warp][at], ypar, status)) {
-            ok = false;
-            break;
-        }
-        unsigned char* myrow = sl + lane * 128;
-        const int col0 = (cb0 + nb) * EXP_BN + ch * CW;  // first column of the slot within the part
-        const bool mine = wrow0 + lane < len;
-        if (F32) {
-            float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                float4* yp = reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4));
-                float4 y = *yp;
-                y.x += __uint_as_float(v[4 * c]), y.y += __uint_as_float(v[4 * c + 1]);
-                y.z += __uint_as_float(v[4 * c + 2]), y.w += __uint_as_float(v[4 * c + 3]);
-                if (whole) {
-                    *yp = y;
-                } else if (mine) {
-                    if (col0 + 4 * c + 4 <= rows) {
-                        *reinterpret_cast<float4*>(yrow + 4 * c) = y;
-                    } else {
-                        const float e[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            if (col0 + 4 * c + k < rows) yrow[4 * c + k] = e[k];
+                if (lane == 0) {
+                    if (whole) {
+                        tma_store_2d(ymap, ycol0 + q * CW, start + wrow0, sl);
+                        bulk_commit();
+                        if (nst == 1) {  // one slot: wait for this store to have read it, then refill it
+                            bulk_wait_read();
+                            if (i + 1 < my_n) load_y(i + 1, 0);
+                        } else {  // the store before this one has read its slot: refill that slot
+                            bulk_wait_read_1();
+                            if (i >= 1 && i - 1 + nst < my_n) load_y(i - 1 + nst, at == 0 ? nst - 1 : at - 1);
+                        }
+                    } else if (i + nst < my_n) {
+                        load_y(i + nst, at);  // plain stores: the slot is free at once
                     }
                 }
-            }
-        } else {
-            bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
-#pragma unroll
-            for (int c = 0; c < 8; c++) {
-                if (c == 4) fetch(1);
-                uint4* yp = reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4));
-                const uint4 raw = *yp;
-                float f[8];
-                unpack8(raw, f);
-                uint32_t o[4];
-#pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const __nv_bfloat162 b2 = __floats2bfloat162_rn(f[2 * e] + __uint_as_float(v[8 * (c & 3) + 2 * e]),
-                                                                    f[2 * e + 1] + __uint_as_float(v[8 * (c & 3) + 2 * e + 1]));
-                    o[e] = *reinterpret_cast<const uint32_t*>(&b2);
-                }
-                if (whole) {
-                    *yp = make_uint4(o[0], o[1], o[2], o[3]);
-                } else if (mine) {
-                    if (col0 + 8 * c + 8 <= rows) {
-                        *reinterpret_cast<uint4*>(yrow + 8 * c) = make_uint4(o[0], o[1], o[2], o[3]);
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < 4; k++)  // (a part's width is even)
-                            if (col0 + 8 * c + 2 * k < rows) *reinterpret_cast<uint32_t*>(yrow + 8 * c + 2 * k) = o[k];
-                    }
+                if (++at == nst) {
+                    at = 0;
+                    ypar ^= 1;
                 }
             }
+            if (lane == 0) bulk_wait_all();
         }
-        if (whole) fence_async_smem();  // the additions above, before the tensor store reads them
-        __syncwarp();
-        if (lane == 0) {
-            if (whole) {
-                tma_store_2d(ymap, ycol0 + q * CW, start + wrow0, sl);
-                bulk_commit();
-                if (nst == 1) {  // one slot: wait for this store to have read it, then refill it
-                    bulk_wait_read();
-                    if (i + 1 < my_n) load_y(i + 1, 0);
-                } else {  // the store before this one has read its slot: refill that slot
-                    bulk_wait_read_1();
-                    if (i >= 1 && i - 1 + nst < my_n) load_y(i - 1 + nst, at == 0 ? nst - 1 : at - 1);
-                }
-            } else if (i + nst < my_n) {
-                load_y(i + nst, at);  // plain stores: the slot is free at once
-            }
-        }
-        if (++at == nst) {
-            at = 0;
-            ypar ^= 1;
-        }
-    }
-    if (lane == 0) bulk_wait_all();
-    }
-    tc_fence_before();
-    __syncthreads();
+        tc_fence_before();
+        __syncthreads();
     }
     if (!begun) return pdl_exit_idle();
     if (late) pdl_wait();
@@ -968,7 +968,7 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
         for (int nb = 1; nb <= most; nb++) {
             long long groups = 0;
             for (int p = 0; p < parts; p++) groups += ((part_rows[p] + width - 1) / width + nb - 1) / nb;
-            const long long waves = (tiles_est * groups + 2 * 148 - 1) / (2 * 148);
+            const long long waves = (tiles_est * groups + 2 * g_sms - 1) / (2 * g_sms);
             const double cost = (double)waves * (320.0 + (double)nb * width);
             if (cost < best) {
                 best = cost;
