@@ -120,6 +120,10 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     for (int i = 0; i < 7; i++) dv[i] = d[i];
     // Desc: a | b0 b1 | b2 b3 | rank r0 r1 r2 | r3 ro0 ro1 ro2 | ro3 o0 o1 o2 | o3 rows0 rows1 rows2 | rows3 pad
     const uint32_t* dw = reinterpret_cast<const uint32_t*>(dv);
+    int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
+#pragma unroll
+    for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = (int)dw[11 + p], rows[p] = (int)dw[23 + p];
+    const unsigned long long units = pack_units(expand_item_units(r, rows, (int)head.z, most), shrink_item_units((int)dw[10], nsplit));
     o[0] = make_uint4(head.z, head.x, dw[10], (uint32_t)cols);  // cnt, slot, rank, cols
     o[1] = make_uint4(dw[0], dw[1], dw[2], dw[3]);              // a, b[0]
     o[2] = make_uint4(dw[4], dw[5], dw[6], dw[7]);              // b[1], b[2]
@@ -142,10 +146,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     o[10] = work[3];
     o[11] = work[4];
     o[12] = make_uint4(cat[0], cat[1], cat[2], cat[3]);
-    int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
-#pragma unroll
-    for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = (int)dw[11 + p], rows[p] = (int)dw[23 + p];
-    return pack_units(expand_item_units(r, rows, (int)head.z, most), shrink_item_units((int)dw[10], nsplit));
+    return units;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -169,6 +170,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                                                                  PloraRec* __restrict__ recs, int rec_cap,
                                                                  int* __restrict__ prefix, int expand_grid) {
     extern __shared__ int sm[];
+    __shared__ int first_item;  // (thread 0's) units of a layer's first item in the expand
     __shared__ unsigned long long sh[4][33];  // a row per scan in flight: no barrier between one scan and the next
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cap = lay.cap_tiles, S1 = lay.max_slots + 1;
@@ -403,20 +405,19 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
         for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
-            const int cols = site_cols[4 * site], pieces = site_cols[4 * site + 1], nsplit = site_cols[4 * site + 2], most = site_cols[4 * site + 3];
+            const int4 info = reinterpret_cast<const int4*>(site_cols)[site];
             int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
             long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
-            long long first_item = 0;  // (thread 0's) units of the first item in the expand
             for (int base = 0; base < end; base += 1024) {
                 const int w = base + tid;
                 unsigned long long units = 0, total = 0;
                 if (w < end) {
                     uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
-                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
-                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, pieces, nsplit, most);
+                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)info.x);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, info.x, info.y, info.z, info.w);
                 }
-                if (w == 0) first_item = packed_expand(units);
+                if (w == 0) first_item = (int)packed_expand(units);
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
                 if (w < nw) {
                     ps[1 + w] = packed_shrink(at);

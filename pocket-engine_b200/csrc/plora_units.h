@@ -32,10 +32,10 @@ PLORA_HD int expand_col_cost(int r, int cnt, int most) {
     const int c = expand_cost(r, cnt);
     return c < most ? c : most;
 }
-PLORA_HD long long expand_item_units(const int* r, const int* rows, int cnt, int most) {
-    long long units = 0;
+PLORA_HD int expand_item_units(const int* r, const int* rows, int cnt, int most) {
+    int units = 0;
     for (int p = 0; p < PLORA_MAX_PARTS; p++)
-        if (r[p] > 0 && rows[p] > 0) units += (long long)rows[p] * expand_col_cost(r[p], cnt, most);
+        if (r[p] > 0 && rows[p] > 0) units += rows[p] * expand_col_cost(r[p], cnt, most);
     return units;
 }
 PLORA_HD int shrink_item_units(int rank, int nsplit) { return (rank + SHR_ROWS - 1) / SHR_ROWS * nsplit; }
@@ -43,7 +43,7 @@ PLORA_HD int shrink_item_units(int rank, int nsplit) { return (rank + SHR_ROWS -
 // Both kinds of units in one word, for one scan over the items: a step has at most 12,864 x (4 x 512 / 16 rows x 8 splits) =
 // 13.2e6 units of the shrink, under 2^24.
 #define UNIT_SHIFT 24
-PLORA_HD unsigned long long pack_units(long long expand, int shrink) { return ((unsigned long long)expand << UNIT_SHIFT) | (unsigned)shrink; }
+PLORA_HD unsigned long long pack_units(int expand, int shrink) { return ((unsigned long long)expand << UNIT_SHIFT) | (unsigned)shrink; }
 PLORA_HD int packed_shrink(unsigned long long at) { return (int)(at & ((1u << UNIT_SHIFT) - 1)); }
 PLORA_HD long long packed_expand(unsigned long long at) { return (long long)(at >> UNIT_SHIFT); }
 
