@@ -612,8 +612,8 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
     // 256 output columns per tile, or fewer where that makes the rounds of the pairs shorter: a step of few tokens has few
     // tiles, and a round that is nearly empty costs as much as a full one. A step of K costs what it moves into an SM,
     // G_BM rows of x and the block's rows of W, of 128 bytes each. Tiles of 192 columns may span two parts, which adapter
-    // passes do not, so they are for steps without long runs (FP8, 256 tokens, 24,576 columns, shrink and layer: 77.3 -> 74.9 us). Up to 128
-    // tokens of such a step, blocks on their own take tiles of 256 or 192 columns where that costs less: layers too wide for
+    // passes do not, so they are for steps that cannot have long runs: begun as decoding steps, or of fewer
+    // rows (FP8, 256 tokens, 24,576 columns, shrink and layer: 77.3 -> 74.9 us). Up to 128 tokens of such a step, blocks on their own take tiles of 256 or 192 columns where that costs less: layers too wide for
     // one round of pairs. FP8, 24,576 columns: 36 us in two rounds of pairs, 24 in one round of blocks (shrink and layer at
     // 70 tokens: 65 -> 53 us, at 128: 69 -> 57); the bf16 layers of a block at 70 tokens: 238 -> 218 us.
     const int blocks = 2 * g_pairs;

@@ -567,7 +567,8 @@ int plora_adapter_prepare(const plora_t* h, const char* name, const plora_module
     }
     // The slab is bound by the host's memory: 4 bytes in and 2 out per value, once (the zeros of :375 are written where
     // padding is, not under everything). Jobs first, then several threads fill them: an adapter of 9.7 M values took 20
-    // ms on one thread behind a clearing pass over a freshly pinned buffer, and takes about 1 ms.
+    // ms on one thread behind a clearing pass over a freshly pinned buffer, and takes about 1 ms into a buffer that another
+    // adapter left. Without one, locking the pages is most of a load, as it was.
     std::vector<FillJob> jobs;
     std::vector<std::vector<float>> permuted;  // (the buffers stay where they are when the outer vector grows)
     size_t values = 0;
