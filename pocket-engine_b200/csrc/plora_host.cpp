@@ -381,19 +381,20 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             if (rc == PLORA_OK) h->site_ok = plora_site_init() == cudaSuccess;
             std::vector<int32_t> info;
             for (auto& s : h->sites) {
-                int nsub = 1, total = 0;
-                for (auto& p : s.parts) total += p.rows;
-                s.cluster_ok = h->site_ok && plora_site_plan(s.cols, (int)s.parts.size(), h->max_rank, total, &nsub) > 0;
-                if (s.cluster_ok) {
-                    s.max_clusters = plora_site_max_clusters(s.cols, (int)s.parts.size(), h->max_rank, total);
-                    // Whatever the number of slots: how many of them a step uses is not known here, and a rule on the step
-                    // would let a token's result depend on its batch. Rank 16, two layers, tokens of adapters in 64 slots,
-                    // clusters against the pair of kernels: 1 of 1 50 / 55 us, 8 of 8 60 / 76, 64 of 16 71 / 92, 64 of 32
-                    // 101 / 114; only steps of more than 40 adapters are faster as pairs (64 of 48 147 / 137, 64 of 64 179 / 163).
-                    if (s.max_clusters < nsub) s.cluster_ok = false;
-                }
+                // Cluster kernel or pair whatever the number of slots: how many of them a step uses is not known here, and a
+                // rule on the step would let a token's result depend on its batch. Rank 16, two layers, tokens of adapters in 64
+                // slots, clusters against the pair of kernels: 1 of 1 50 / 55 us, 8 of 8 60 / 76, 64 of 16 71 / 92, 64 of 32
+                // 101 / 114; only steps of more than 40 adapters are faster as pairs (64 of 48 147 / 137, 64 of 64 179 / 163).
+                for (auto& o : h->sites)  // (a model's layers are of a few shapes)
+                    if (&o < &s && o.cols == s.cols && o.parts.size() == s.parts.size() && std::equal(o.part_rows, o.part_rows + PLORA_MAX_PARTS, s.part_rows)) {
+                        s.plans = o.plans;
+                        break;
+                    } else if (&o == &s && h->site_ok) {
+                        s.plans = plora_site_plans(s.cols, (int)s.parts.size(), s.part_rows, h->max_rank);
+                        break;
+                    }
                 info.push_back(s.cols);
-                info.push_back(s.cluster_ok ? 8 * nsub : 0);
+                info.push_back(0);
                 info.push_back(s.nsplit);
                 info.push_back(s.exp_most);
             }
@@ -1023,6 +1024,15 @@ int plora_expand_reduced(plora_t* h, const plora_hook* hook, const plora_step* s
     return expand_impl(h, hook, step, rows, y, ldy, f32_out, true, false, stream);
 }
 
+// How the cluster kernel runs a layer: as few column groups as fit, and more of them in steps of few work items, as long as
+// the step's clusters leave half of the device's places to the next layer's.
+static const PloraSitePlan& site_plan(const SiteInfo& site, int work_cap) {
+    const PloraSitePlan* pick = &site.plans[0];
+    for (auto& p : site.plans)
+        if (work_cap * p.nsub <= p.max_clusters / 2) pick = &p;
+    return *pick;
+}
+
 // Shrink and expand of one layer in one call, for callers whose x and y are both ready (after the layer's own
 // matrix multiply): the gather tokens go through the cluster kernel where the layer's shapes fit it.
 int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint64_t x, int rows, uint64_t y, int ldy,
@@ -1031,7 +1041,7 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     if (h->device < 0) return fail(h, PLORA_ERR_CUDA, "layout-only handle: no device");
     if (hook->site < 0 || hook->site >= (int)h->sites.size()) return fail(h, PLORA_ERR_ARG, "hook names no site");
     const SiteInfo& site = h->sites[(size_t)hook->site];
-    if (!site.cluster_ok || h->apply_mode == 0) {
+    if (site.plans.empty() || h->apply_mode == 0) {
         // x and y are both older than the kernel before each launch: fetch them ahead of the dependency waits
         int rc = shrink_impl(h, hook, step, x, rows, true, h->early_x, stream);
         return rc != PLORA_OK ? rc : expand_impl(h, hook, step, rows, y, ldy, f32_out, false, true, stream);
@@ -1042,14 +1052,12 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
     const auto [pdl, late] = next_launch(h, stream, true);
-    const int release = h->site_release >= 0 && h->site_release <= 4 ? h->site_release : (h->early_x ? 0 : 1);
-    int total = 0;
-    for (auto& p : site.parts) total += p.rows;
+    const int release = h->site_release >= 0 && h->site_release <= 3 ? h->site_release : (h->early_x ? 0 : 3);
     CUK(h, "site kernel",
        plora_launch_site((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
                          hook->site + 1 < (int)h->sites.size() ? recs_of(h, hook->site + 1) : nullptr,
-                         (void*)(uintptr_t)y, ldy, f32_out, (int)site.parts.size(), h->max_rank, total, work_cap,
-                         site.max_clusters, (h->early_x ? 1 : 0) | (release << 1) | (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
+                         (void*)(uintptr_t)y, ldy, f32_out, site_plan(site, work_cap), work_cap,
+                         (h->early_x ? 1 : 0) | (release << 1) | (h->prefetch_next ? 16 : 0) | (late && pdl ? 32 : 0),
                          bounds_of(h, hook, rows, ldy), h->status, pdl, as_stream(stream)));
     if (has_tiles(h, step, rows)) {
         CUK(h, "shrink (tile path)",

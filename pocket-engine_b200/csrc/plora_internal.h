@@ -63,7 +63,7 @@ struct alignas(256) PloraRec {
     uint64_t a;
     uint64_t b[PLORA_MAX_PARTS];
     int32_t r[PLORA_MAX_PARTS], r_off[PLORA_MAX_PARTS], off[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
-    int32_t ntot, share;  // output columns over the targeted parts; columns per block of the layer's cluster kernel
+    int32_t ntot, pad1;  // output columns over the targeted parts
     int32_t tok[PLORA_WORK_TOKENS];
     int32_t cat[PLORA_MAX_PARTS];  // where each targeted part starts when the targeted parts are laid end to end
     int32_t pad2[12];
@@ -92,6 +92,23 @@ struct PloraSlabMaps {
     PloraTmap a, a64, b[PLORA_MAX_PARTS];  // a64: A in boxes of 64 rows
 };
 
+// Shared-memory layout of the cluster kernel (one kernel per layer, plora_site.cu)
+struct PloraSiteShape {
+    int kchunk;   // input features per block of the cluster (a multiple of 32)
+    int kb_pad;   // bytes between rows of A in shared memory (64 over a multiple of 128: an operand load meets every bank once)
+    int rc;       // most rows of A one cluster works on (of the parts its columns meet)
+    int sp_pad;   // bytes between rows of a bf16 plane of the summed S
+    int a_bytes;  // shared-memory bytes for the block's rows of A
+    int p_bytes;  // ... for the eight warps' partial sums
+    int r_bytes;  // ... for the partial sums that the cluster's blocks send one another
+    int b_bytes;  // ... for the block's share of B
+};
+// One way to run it: column groups per work item (each is a cluster), and how many such clusters the device runs at once
+struct PloraSitePlan {
+    PloraSiteShape shape;
+    int nsub, smem, max_clusters;
+};
+
 struct SiteInfo {
     int layer = 0, cols = 0;
     int exp_most = 1;  // expand_most of the layer's output columns
@@ -109,8 +126,7 @@ struct SiteInfo {
     int part_off[PLORA_MAX_PARTS] = {0, 0, 0, 0}, part_rows[PLORA_MAX_PARTS] = {0, 0, 0, 0};  // copies of parts[]
     // K-split of the shrink: fixed per site so results do not depend on the batch
     int kchunk = 0, nsplit = 1;
-    bool cluster_ok = false;  // the one-kernel-per-layer cluster path fits this layer's shapes
-    int max_clusters = 0;     // clusters of that kernel the device runs at once
+    std::vector<PloraSitePlan> plans;  // of the one-kernel-per-layer cluster path, by column groups; empty: it does not fit
 };
 
 struct SiteData {  // src/lora.rs:74-79
@@ -179,7 +195,7 @@ struct plora {
     int rec_cap = 0;
     int32_t* prefix = nullptr;  // device: [sites][unit_words(rec_cap)] units of the gather kernels before every work item of the step
     int32_t* host_meta = nullptr;  // pinned staging for plora_meta_upload
-    int32_t* site_cols = nullptr;  // device: per layer {input width, column pieces of the cluster kernel, K-splits, most units of a column} (for the launch records)
+    int32_t* site_cols = nullptr;  // device: per layer {input width, 0, K-splits, most units of a column} (for the launch records)
     int cap_tiles = 0;
     SegLayout seg;
     int* status = nullptr;  // device status word
@@ -258,7 +274,7 @@ __host__ __device__ inline int plora_tile_chunks(int K, int R) {
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st);
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
-// site_info: per layer {input width, blocks that share a work item's output columns in the cluster kernel (0: none),
+// site_info: per layer {input width, 0,
 // K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
                                     const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
@@ -275,11 +291,10 @@ inline cudaError_t plora_kernel_shared(const void* fn, int max_dynamic_bytes) {
 }
 cudaError_t plora_kernels_init(const SegLayout& lay);
 cudaError_t plora_site_init();
-size_t plora_site_plan(int K, int parts, int max_rank, int total_rows, int* nsub);
-int plora_site_max_clusters(int K, int parts, int max_rank, int total_rows);
+std::vector<PloraSitePlan> plora_site_plans(int K, int n_parts, const int* part_rows, int max_rank);
 cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, const PloraRec* next_recs,
-                              void* y, int ldy, int f32_out, int parts, int max_rank, int total_rows, int work_cap,
-                              int max_clusters, int mode, const PloraBounds& bnd, int* status, bool pdl, cudaStream_t st);
+                              void* y, int ldy, int f32_out, const PloraSitePlan& plan, int work_cap, int mode, const PloraBounds& bnd,
+                              int* status, bool pdl, cudaStream_t st);
 cudaError_t plora_mma_init();
 cudaError_t plora_fp8_init(int max_rank);
 cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, bool pdl, cudaStream_t stream);

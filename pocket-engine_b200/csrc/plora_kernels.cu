@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 // that layer make one metadata fetch per block. `o` is the record's 16 uint4.
 // Returns the item's units of the few-token kernels (pack_units).
 __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
-                                             int cols, int pieces, int nsplit, int most) {
+                                             int cols, int nsplit, int most) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
     const uint4 head = work[0];  // slot, perm start, count, 0
     const int slot = (int)head.x;
@@ -131,16 +131,14 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     o[4] = make_uint4(dw[13], dw[14], dw[15], dw[16]);          // r[2], r[3], r_off[0], r_off[1]
     o[5] = make_uint4(dw[17], dw[18], dw[19], dw[20]);          // r_off[2], r_off[3], off[0], off[1]
     o[6] = make_uint4(dw[21], dw[22], dw[23], dw[24]);          // off[2], off[3], rows[0], rows[1]
-    // the slot's output columns over its targeted parts laid end to end, and the even share of them that
-    // one block of the layer's cluster kernel expands
+    // the slot's output columns over its targeted parts laid end to end
     uint32_t cat[PLORA_MAX_PARTS], ntot = 0;
 #pragma unroll
     for (int p = 0; p < PLORA_MAX_PARTS; p++) {
         cat[p] = ntot;
         if ((int)dw[11 + p] > 0) ntot += dw[23 + p];
     }
-    const uint32_t share = pieces > 0 ? (((ntot + pieces - 1) / pieces + 1) & ~1u) : 0u;
-    o[7] = make_uint4(dw[25], dw[26], ntot, share);             // rows[2], rows[3], ntot, share
+    o[7] = make_uint4(dw[25], dw[26], ntot, 0u);                // rows[2], rows[3], ntot
     o[8] = work[1];                                             // the token rows
     o[9] = work[2];
     o[10] = work[3];
@@ -415,7 +413,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                 if (w < end) {
                     uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
                     if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)info.x);
-                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, info.x, info.y, info.z, info.w);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, info.x, info.z, info.w);
                 }
                 if (w == 0) first_item = (int)packed_expand(units);
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);

@@ -5,30 +5,42 @@
 // lora_shrink + lora_expand pair of src/kernels/lora.cuh:23-126 when x and y are both ready at the call (after
 // the layer's own matrix multiply).
 //
-// Order of events in a block, chosen so that nothing that can be known early waits for anything:
-//   1. (when the caller vouched for x) the next kernel of the stream is released at once;
-//   2. one fetch of the work item's launch record (descriptor and token rows, written once per step);
-//   3. bulk async copies of the block's rows of A and of its share of B into shared memory, L2 prefetch hints
+// A layer is a chain of latencies from the dependency wait to the last store of y, and everything that can be known early is
+// done before that wait. Order of events in a block:
+//   1. one fetch of the work item's launch record (descriptor and token rows, written once per step);
+//   2. bulk async copies of the block's inputs of the rows of A and of its share of B into shared memory, L2 prefetch hints
 //      for the x and y lines it will touch (and, when asked for, an L2 prefetch of the same work item's slabs of
-//      the next layer);
-//   4. the dependency wait (the kernel before, typically the layer's matrix multiply, wrote y);
-//   5. x into shared memory, shrink, release of the next kernel of the stream (its prologue, steps 2 and 3, then
-//      overlaps this kernel's exchange and expand), exchange, expand, y read-modify-write.
-// Nothing before step 4 binds a value of x or y, unless the caller vouched for x (early_x). The release point was
-// measured: released at kernel start, the next layer's blocks take the places that this layer's own late clusters
-// need (a B200 holds about 33 clusters of this kernel, two neighbouring layers can need 48) and sit in their wait.
+//      the next layer); addresses and predicates of the loads to come; A has landed;
+//   3. the dependency wait (the kernel before, typically the layer's matrix multiply, wrote y);
+//   4. x from L2 straight into operand registers, y of the first two steps of columns behind it; the next kernel of the stream
+//      is released (its steps 1 and 2 then overlap the rest of this one);
+//   5. shrink, exchange (the summed partials are stored into all eight blocks, with their own completion), expand.
+// Nothing before step 3 binds a value of x or y, unless the caller vouched for x (early_x; the next kernel is then released at
+// once). Cycles from the wait to the end of a block, one token of rank 16: 5,100 with the parts and shares walked after the wait, 3,300
+// so; one layer then takes 2.9 us against 4.8 (x through bulk copies, partials fetched from the other blocks, y and S in
+// tiles of 8 tokens), 64 tokens of 16 adapters 5.2 against 7.0. The release point, one token / 64 tokens, us per 16 layers: at kernel
+// start 57 / 96, after the loads 57 / 95, after the shrink 69 / 106.
+//
+// Column groups: a cluster loads and multiplies the rows of A of the parts its columns meet, no others. A step of many work items
+// takes as few groups as fit, since a B200 holds 33 clusters of such blocks; one of few items takes more, up to a
+// step of columns per warp: one token over 24,576 columns goes to 96 blocks instead of 16.
 //
 // Arithmetic: tiles of the warp-level tensor-core instruction (m16n8k16, bf16 in, f32 accumulate), the shape the
-// engine's own kernels use for their 16-token tiles; here a tile carries 8 tokens, and in the expand its other 8
-// rows carry a second term of S (plora_tiles.cuh). On the CUDA cores the step is bound by
+// engine's own kernels use for their 16-token tiles; here the shrink has 16 rows of A by 8 tokens in a tile, the expand four tokens'
+// three terms of S by 8 columns (plora_tiles.cuh). On the CUDA cores the step is bound by
 // instruction issue (one conversion per bf16 element plus one multiply-add per token), not by memory; a 128-row
 // tcgen05 tile would spend 1/8 or less of its rows on a work item. The f32 intermediate enters the expand as
 // three bf16 terms (high, middle, low part), whose products with bf16 B are exact in f32, so no precision is
 // given up against an f32 multiply-add chain.
+//
+// No registers spill, and none may: these kernels leave L1 no room, so a spilled value comes back from L2 (300 bytes of them
+// doubled the time of a layer).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <type_traits>
+#include <vector>
 
 #include "plora_internal.h"
 #include "plora_device.cuh"
@@ -38,6 +50,7 @@
 #define SITE_THREADS 256
 #define SITE_WARPS PLORA_TILE_WARPS
 #define SITE_TOK 8  // tokens per pass over a work item
+#define SITE_SMEM (112 * 1024)  // two blocks per SM: half of 228 KB, less the 1 KB the system keeps per block and the static part
 
 namespace {
 
@@ -47,51 +60,54 @@ __device__ __forceinline__ uint32_t cluster_rank() {
     return r;
 }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// a float at the same shared-memory offset in block `rank` of the cluster
-__device__ __forceinline__ float ld_peer_f32(const float* p, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
-    float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
-    return v;
-}
 
-struct SiteShape {
-    int kchunk;    // input features per block of the cluster (a multiple of 8)
-    int kb_pad;    // bytes between rows of the A and x tiles in shared memory (an odd number of 16-byte pieces)
-    int rmax;      // floats per partial S row in shared memory (parts * max_rank)
-    int sp_pad;    // bytes between rows of a bf16 plane of the summed S
-    int aw_bytes;  // shared-memory bytes for the block's A rows, reused for the warps' partial sums
-    int g_rows;    // rows of A per group (64, or all of them when there are fewer)
-    int g_stride;  // bytes between groups: room for g_rows rows of A and for the 8 warps' partials of those rows
-    int x_bytes;   // ... for the tokens' x chunks
-    int b_bytes;   // ... for the block's share of B
-    int nsub;      // column groups per work item (grid y): each is one cluster
+// a block's columns of one part, which it expands in one go
+struct alignas(16) Seg {
+    int r, ncols, boff, soff;  // ranks, columns; bytes to its rows of B and to the first of its ranks in a row of S
+    long long ycol;            // first column of y
+    int fast, pad;             // y rows that move in pieces of 4 columns, 16-byte aligned every eighth
 };
 
-// this block's share [lo, hi) of each part's output columns, and where its rows of B start in shared memory
-struct Share {
-    int lo[PLORA_MAX_PARTS], hi[PLORA_MAX_PARTS], boff[PLORA_MAX_PARTS];
-};
+// Columns per block when `pieces` blocks share `ntot` output columns: in eights, so that y moves in whole pieces
+__host__ __device__ inline int site_share(int ntot, int pieces) { return ((ntot + pieces - 1) / pieces + 7) & ~7; }
 
 // The slot's output columns, over the targeted parts laid end to end (rec.cat, rec.ntot), are cut into even shares of
-// rec.share columns, one per block of the cluster kernel. Run by lanes 0..3 of one warp, lane p for part p.
-__device__ __forceinline__ void column_share(const PloraRec& rec, int piece, int p, Share& s) {
-    const int c_lo = min(rec.ntot, piece * rec.share), c_hi = min(rec.ntot, c_lo + rec.share);
+// `share` columns, one per block of the layer's clusters. One warp: lane p finds what of part p falls into the block's share, and
+// asks for its rows of B.
+__device__ __forceinline__ void block_segs(const PloraRec& rec, int share, int piece, int ja, const void* Y, int ldy, int esize, int lane, Seg* segs,
+                                           int* n_segs, unsigned char* Bs, uint64_t* bar) {
+    const int p = lane & (PLORA_MAX_PARTS - 1);
+    const int c_lo = min(rec.ntot, piece * share), c_hi = min(rec.ntot, c_lo + share);
     const int lo = max(c_lo, rec.cat[p]) - rec.cat[p];
-    int hi = rec.r[p] > 0 ? min(c_hi, rec.cat[p] + rec.rows[p]) - rec.cat[p] : 0;
-    hi = hi > lo ? hi : lo;
-    const int bytes = (hi - lo) * rec.r[p] * 2;
+    const int hi = rec.r[p] > 0 ? min(c_hi, rec.cat[p] + rec.rows[p]) - rec.cat[p] : 0;
+    const int ncols = max(0, hi - lo), bytes = ncols * rec.r[p] * 2;
     // where the part's rows of B start in shared memory: the bytes of the parts before it
-    int off = 0;
+    int off = 0, total = 0;
 #pragma unroll
-    for (int q = 0; q < PLORA_MAX_PARTS - 1; q++) {
-        const int b = __shfl_sync(0xfu, bytes, q);
+    for (int q = 0; q < PLORA_MAX_PARTS; q++) {
+        const int b = __shfl_sync(0xffffffffu, bytes, q);
         if (q < p) off += b;
+        total += b;
     }
-    s.lo[p] = lo;
-    s.hi[p] = hi;
-    s.boff[p] = off;
+    const unsigned have = __ballot_sync(0xffffffffu, lane < PLORA_MAX_PARTS && ncols > 0);
+    if (lane == 0) {
+        *n_segs = __popc(have);
+        if (have == 0) segs[0] = Seg{};
+        if (total > 0) mbar_expect_tx(bar, (uint32_t)total);
+    }
+    __syncwarp();
+    if (lane < PLORA_MAX_PARTS && ncols > 0) {
+        bulk_g2s(Bs + off, reinterpret_cast<const bf16*>(rec.b[p]) + (size_t)lo * rec.r[p], (uint32_t)bytes, bar);
+        Seg s;
+        s.r = rec.r[p];
+        s.ncols = ncols;
+        s.boff = off;
+        s.soff = (rec.r_off[p] - ja) * 2;
+        s.ycol = (long long)rec.off[p] + lo;
+        s.fast = (ncols & 7) == 0 && ((reinterpret_cast<uintptr_t>(Y) | ((size_t)ldy * esize) | (size_t)(s.ycol * esize)) & 15) == 0;
+        s.pad = 0;
+        segs[__popc(have & ((1u << lane) - 1u))] = s;
+    }
 }
 
 // L2 prefetch of this block's eighth of `bytes` at `base` (both multiples of 16), 32 KB per request, one warp
@@ -104,12 +120,14 @@ __device__ __forceinline__ void prefetch_eighth(uint64_t base, uint64_t bytes, u
     }
 }
 
-// remote arrival on the same barrier in block `rank` of the cluster, releasing this thread's (and, through the
-// block barrier before it, the block's) shared-memory writes to the cluster
-__device__ __forceinline__ void mbar_arrive_peer(uint64_t* bar, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(bar)), "r"(rank));
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(a) : "memory");
+// 16 bytes to the same shared-memory offset in block `rank` of the cluster, counted on the same barrier there
+__device__ __forceinline__ void st_async_peer(const void* p, float4 v, const uint64_t* bar, uint32_t rank) {
+    uint32_t a, m;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(m) : "r"(smem_u32(bar)), "r"(rank));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(a),
+                 "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)), "r"(m)
+                 : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
     uint32_t ok;
@@ -131,51 +149,80 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // "my reads of your shared memory are done": no memory ordering is asked of the arrival itself
 __device__ __forceinline__ void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 
-// The shrink's inner loop for one warp: n 16-wide steps, SITE_WARPS steps apart, over PAIRS pairs of 8-row tiles of A
-template <int PAIRS>
-__device__ __forceinline__ void shrink_steps(float (&acc)[8][4], uint32_t xs_w, uint32_t as_w, uint32_t kb_pad, int n) {
-#pragma unroll 2
-    for (int i = 0; i < n; i++) {
-        uint32_t xa[4];
-        ldmatrix_x4(xa, xs_w + (uint32_t)i * (SITE_WARPS * 32u));
+#define SITE_XSTEPS 8  // steps of 32 inputs per warp whose x is held in registers at a time
+
+// The shrink's inner loop for one warp: acc (16 rows of A x 8 tokens per tile) += A . x over the steps of 32 inputs whose x is
+// in registers. Rows of A are the multiply's 16-row operand and tokens its 8 columns. Its 16 input slots may be permuted freely as
+// long as both operands agree: lane t of four holds inputs 8 t .. 8 t + 7 of a step, two multiplies' worth, as one
+// 16-byte piece of either. a0: this lane's row and piece of the first of n steps; the lane has inputs in the first `mine` of them.
+template <int TILES>
+__device__ __forceinline__ void shrink_steps(float (&acc)[2][4], const uint4 (&xr)[SITE_XSTEPS], uint32_t a0, uint32_t kb_pad, int n, int mine) {
+    // A step's rows of A are fetched before the multiplies of the step before (those of the first while x is on its way), and its
+    // two multiplies of a tile go to accumulators of their own: half as long a chain of dependent multiplies.
+    float odd[TILES][4];
 #pragma unroll
-        for (int pr = 0; pr < PAIRS; pr++) {
-            uint32_t bb[4];
-            ldmatrix_x4(bb, as_w + (uint32_t)(pr * 16) * kb_pad + (uint32_t)i * (SITE_WARPS * 32u));
-            mma_16816(acc[2 * pr], xa, bb[0], bb[1]);
-            mma_16816(acc[2 * pr + 1], xa, bb[2], bb[3]);
+    for (int i = 0; i < TILES; i++) odd[i][0] = odd[i][1] = odd[i][2] = odd[i][3] = 0.f;
+    uint4 lo[TILES], hi[TILES];
+    auto fetch = [&](int s) {
+#pragma unroll
+        for (int i = 0; i < TILES; i++) {
+            const uint32_t at = a0 + (uint32_t)(i * 16) * kb_pad + (uint32_t)s * (SITE_WARPS * 64u);
+            lo[i] = hi[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (s < mine) {  // (shared memory behind the inputs may hold anything)
+                lo[i] = lds128(at);
+                hi[i] = lds128(at + 8u * kb_pad);
+            }
         }
+    };
+    fetch(0);
+#pragma unroll
+    for (int s = 0; s < SITE_XSTEPS; s++) {
+        if (s >= n) break;
+        uint32_t m[TILES][2][4];
+#pragma unroll
+        for (int i = 0; i < TILES; i++) {
+            m[i][0][0] = lo[i].x, m[i][0][1] = hi[i].x, m[i][0][2] = lo[i].y, m[i][0][3] = hi[i].y;
+            m[i][1][0] = lo[i].z, m[i][1][1] = hi[i].z, m[i][1][2] = lo[i].w, m[i][1][3] = hi[i].w;
+        }
+        if (s + 1 < SITE_XSTEPS) fetch(s + 1);
+#pragma unroll
+        for (int i = 0; i < TILES; i++) mma_16816(acc[i], m[i][0], xr[s].x, xr[s].y);
+#pragma unroll
+        for (int i = 0; i < TILES; i++) mma_16816(odd[i], m[i][1], xr[s].z, xr[s].w);
     }
+#pragma unroll
+    for (int i = 0; i < TILES; i++)
+#pragma unroll
+        for (int e = 0; e < 4; e++) acc[i][e] += odd[i][e];
 }
 
 template <bool F32>
 __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THREADS, 2)
     plora_site_gather_kernel(const bf16* __restrict__ X, int ldx, int K, const PloraRec* __restrict__ recs, int rec_cap,
-                             const PloraRec* __restrict__ next_recs, void* Y, int ldy, SiteShape sh, int mode,
+                             const PloraRec* __restrict__ next_recs, void* Y, int ldy, PloraSiteShape sh, int mode,
                              int* __restrict__ status PLORA_BOUNDS_PARAM) {
     extern __shared__ __align__(128) unsigned char dsm[];
-    __shared__ __align__(8) uint64_t bars[4];  // A rows, x chunks, B rows, the cluster's partials
+    __shared__ __align__(8) uint64_t bars[3];  // A rows, B rows, the cluster's partials
     __shared__ PloraRec srec;
-    __shared__ Share sshare;
+    __shared__ __align__(16) Seg segs[PLORA_MAX_PARTS];
+    __shared__ int n_segs;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t crank = cluster_rank();
-    // A rows in groups of g_rows: group q at q * g_stride, its rows kb_pad apart. Once a group's rows are used up,
-    // the warps' partial sums of those rows [warp][16][g_rows] take their place.
-    unsigned char* As = dsm;
-    unsigned char* Xs = As + sh.aw_bytes;                   // x chunks [8][kb_pad]
-    unsigned char* Bs = Xs + sh.x_bytes;                    // this block's rows of B, part after part
-    float* Sp = reinterpret_cast<float*>(Bs + sh.b_bytes);  // this block's partial S [16][rmax]
-    // the summed S as three bf16 planes [16][sp_pad] (high, middle, low term) and a fourth plane that stays zero
-    unsigned char* S3 = reinterpret_cast<unsigned char*>(Sp + PLORA_WORK_TOKENS * sh.rmax);
-    const uint32_t plane_bytes = PLORA_WORK_TOKENS * (uint32_t)sh.sp_pad;
+    unsigned char* As = dsm;                                                 // this block's inputs of the cluster's rows of A, kb_pad apart
+    float* Ps = reinterpret_cast<float*>(As + sh.a_bytes);                   // the warps' partial sums [warp][token][rc + 4]
+    float* Rs = reinterpret_cast<float*>(As + sh.a_bytes + sh.p_bytes);      // the blocks' partial sums [block][token][rc]
+    unsigned char* Bs = As + sh.a_bytes + sh.p_bytes + sh.r_bytes;           // this block's rows of B, part after part
+    // the summed S as three bf16 planes [8][sp_pad] (high, middle, low term) and a fourth plane that stays zero
+    unsigned char* S3 = Bs + sh.b_bytes;
+    const uint32_t plane_bytes = SITE_TOK * (uint32_t)sh.sp_pad;
     for (uint32_t i = tid * 16u; i < plane_bytes; i += SITE_THREADS * 16u)
         *reinterpret_cast<uint4*>(S3 + 3u * plane_bytes + i) = make_uint4(0u, 0u, 0u, 0u);
     // The kernels after this one may start their prologues now: before their own waits they touch slabs and
     // launch records only (and x, where their caller vouched for it); every store of the path comes after a
     // wait, and every grid waits for its predecessor before it completes.
     // mode: bit 0 = the caller vouched for x; bits 1-3 = when the next kernel of the stream is released (0: at
-    // once, 1: after the shrink, 2: after the exchange); bit 4 = ask L2 for the next layer's slabs too
-    const int early_x = mode & 1, release_at = (mode >> 1) & 7;  // (3, 4: after the wait, after A and x landed)
+    // once, 1: after the shrink, 2: after the exchange, 3: after the loads of x and y); bit 4 = ask L2 for the next layer's slabs too
+    const int early_x = mode & 1, release_at = (mode >> 1) & 7;
     // bit 5 = the kernel before is the step's grouping, which writes the records: nothing is read, and nothing
     // released, before the dependency wait (the launch itself overlaps the grouping)
     const bool late = (mode & 32) != 0;
@@ -184,11 +231,10 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
     if (tid == 0) {
         mbar_init(&bars[0], 1);
         mbar_init(&bars[1], 1);
-        mbar_init(&bars[2], 1);
-        mbar_init(&bars[3], SITE_CLUSTER);  // one arrival per block of the cluster
+        mbar_init(&bars[2], 1);  // this block's own arrival; the bytes of all eight blocks' partials complete it
         mbar_fence_init();
     }
-    cluster_arrive_relaxed();  // the barriers exist (published by the init fence); met before the first remote arrival
+    cluster_arrive_relaxed();  // the barriers exist (published by the init fence); met before the first remote store
     bool met = false, waited = false, hints = true;
     if (late) {
         pdl_wait();
@@ -198,28 +244,23 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
             triggered = true;
         }
     }
-    uint32_t ph_ax = 0, ph_b = 0, ph_s = 0;  // barrier phases (each flips only when its barrier was used)
-    bool alive = true;                       // false once a bounded wait ran out: keep meeting the cluster, do no more work
+    uint32_t ph_a = 0, ph_b = 0, ph_s = 0;  // barrier phases (each flips only when its barrier was used)
+    bool alive = true;                      // false once a bounded wait ran out: keep meeting the cluster, do no more work
     const int k0 = (int)crank * sh.kchunk;
     const int klen = max(0, min(sh.kchunk, K - k0));
     const uint32_t kbytes = (uint32_t)klen * 2u;
-    const int nks = (klen + 15) >> 4;  // 16-wide steps over this block's inputs (a half step reads zeros)
     const int esize = F32 ? 4 : 2;
     // fragment coordinates of the tensor-core tile: this lane holds rows g and g + 8, columns 2 t and 2 t + 1
-    const int g = lane >> 2, t2 = (lane & 3) * 2;
-    // row and 16-byte piece this lane names in a four-matrix load: A-side (16 rows x 16 inputs) and B-side (two
-    // 8-row tiles x 16 inputs)
-    const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_piece = lane >> 4;
-    const int b_row = (lane & 7) + (lane >> 4) * 8, b_piece = (lane >> 3) & 1;
-    // (the x tile has 8 rows: rows 8-15 of the multiply's token tile repeat them and their results are dropped)
-    const uint32_t xs_lane = smem_u32(Xs) + (uint32_t)(a_row & 7) * (uint32_t)sh.kb_pad + (uint32_t)a_piece * 16u;
-    const uint32_t as_lane = smem_u32(As) + (uint32_t)b_row * (uint32_t)sh.kb_pad + (uint32_t)b_piece * 16u;
-    const uint32_t s3_lane = smem_u32(S3) + (uint32_t)a_row * (uint32_t)sh.sp_pad + (uint32_t)a_piece * 16u;
+    const int g = lane >> 2, t4 = lane & 3, t2 = t4 * 2;
+    // shrink: warp q takes the steps of 32 inputs q, q + 8, ...; a lane has no inputs in a last one that ends before its piece
+    const int w_steps = (((klen + 31) >> 5) - warp + SITE_WARPS - 1) / SITE_WARPS;
+    const int w_mine = ((klen - 8 * t4 + 31) >> 5) - warp > 0 ? (((klen - 8 * t4 + 31) >> 5) - warp + SITE_WARPS - 1) / SITE_WARPS : 0;
+    const uint32_t a_lane = smem_u32(As) + (uint32_t)g * (uint32_t)sh.kb_pad + (uint32_t)warp * 64u + (uint32_t)t4 * 16u;
     for (int w = blockIdx.z; w < rec_cap; w += gridDim.z) {
         // ---- the one metadata fetch: the record's 208 live bytes into shared memory
         if (tid < 13) reinterpret_cast<uint4*>(&srec)[tid] = __ldg(reinterpret_cast<const uint4*>(recs + w) + tid);
         __syncthreads();
-        const int cnt = srec.cnt, R = srec.rank;
+        const int cnt = srec.cnt;
         if (cnt == 0) break;  // end of the list: the same decision in every block of the cluster
 #ifdef PLORA_BOUNDS
         if (!rec_in_bounds(srec, bnd, K) || srec.cols != K) {  // the same decision in every block that reads this record
@@ -228,52 +269,44 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
             continue;
         }
 #endif
-        if (R == 0) {         // the slot's adapter skips this layer
+        // the rows of A of the parts that the cluster's columns meet: [ja, ja + R)
+        const int share = site_share(srec.ntot, SITE_CLUSTER * (int)gridDim.y);
+        const int c_lo = (int)blockIdx.y * SITE_CLUSTER * share, c_hi = min(srec.ntot, c_lo + SITE_CLUSTER * share);
+        int ja = srec.rank, jb = 0;
+#pragma unroll
+        for (int p = 0; p < PLORA_MAX_PARTS; p++)
+            if (srec.r[p] > 0 && srec.cat[p] < c_hi && srec.cat[p] + srec.rows[p] > c_lo) {
+                ja = min(ja, srec.r_off[p]);
+                jb = max(jb, srec.r_off[p] + srec.r[p]);
+            }
+        const int R = jb - ja;
+        if (R <= 0) {  // the slot's adapter skips this layer, or its columns end before this cluster's: the same in every block
             __syncthreads();
             continue;
         }
-        // the work item's tokens, 8 at a time (a decoding batch rarely has more of one slot): the x tile has 8 rows,
-        // which is what lets the layers with the longest inputs keep their whole share of B in one block
+        // quads of a token's partial sums, and the factor that divides by their number (exact for the at most 512 quads)
+        const int nq = R >> 2;
+        const uint32_t inv = (65536u + (uint32_t)nq - 1u) / (uint32_t)nq;
+        // the work item's tokens, 8 at a time (a decoding batch rarely has more of one slot)
         for (int t0 = 0; t0 < cnt; t0 += SITE_TOK) {
             const int cn = min(SITE_TOK, cnt - t0);
             const int* tok = srec.tok + t0;
-            // warp 1: the block's share of the output columns (lane p takes part p), then the copies of its rows of B
-            if (warp == 1 && t0 == 0) {
-                if (lane < PLORA_MAX_PARTS) column_share(srec, (int)blockIdx.y * SITE_CLUSTER + (int)crank, lane, sshare);
-                __syncwarp();
-                if (lane == 0) {
-                    uint32_t total = 0;
-    #pragma unroll
-                    for (int p = 0; p < PLORA_MAX_PARTS; p++)
-                        total += (uint32_t)(sshare.hi[p] - sshare.lo[p]) * (uint32_t)srec.r[p] * 2u;
-                    if (total > 0) {
-                        mbar_expect_tx(&bars[2], total);
-    #pragma unroll
-                        for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-                            const uint32_t bytes = (uint32_t)(sshare.hi[p] - sshare.lo[p]) * (uint32_t)srec.r[p] * 2u;
-                            if (bytes > 0)
-                                bulk_g2s(Bs + sshare.boff[p],
-                                         reinterpret_cast<const bf16*>(srec.b[p]) + (size_t)sshare.lo[p] * srec.r[p], bytes, &bars[2]);
-                        }
-                    }
+            // ---- slab requests (before the dependency wait)
+            if (t0 == 0) {  // (a second pass finds the slabs in place)
+                // the block's inputs of the rows of A, one bulk copy per row. The copies of the lanes of one warp are issued
+                // one after another, so the rows go round the warps: row r is lane r / 8 of warp r % 8. (The barrier's one
+                // arrival carries the whole byte count; copies that land before it only run the count down early.)
+                if (klen > 0) {
+                    const bf16* A = reinterpret_cast<const bf16*>(srec.a) + (size_t)ja * K + k0;
+                    if (tid == 0) mbar_expect_tx(&bars[0], (uint32_t)R * kbytes);
+                    for (int r = warp + SITE_WARPS * lane; r < R; r += SITE_THREADS)
+                        bulk_g2s(As + (size_t)r * sh.kb_pad, A + (size_t)r * K, kbytes, &bars[0]);
                 }
+                // warp 1: the block's share of the output columns (lane p takes part p), and the copies of its rows of B
+                if (warp == 1) block_segs(srec, share, (int)blockIdx.y * SITE_CLUSTER + (int)crank, ja, Y, ldy, esize, lane, segs, &n_segs, Bs, &bars[1]);
+                __syncthreads();  // the share is known to every warp
             }
-            // ---- slab requests (before the dependency wait): the block's rows of A, one bulk copy per row. The copies
-            // of the lanes of one warp are issued one after another, so the rows go round the warps: row r is lane
-            // r / 8 of warp r % 8. (The barrier's one arrival carries the whole byte count; copies that land before it
-            // only run the count down early.)
-            if (klen > 0) {
-                const bf16* A = reinterpret_cast<const bf16*>(srec.a) + k0;
-                if (tid == 0) mbar_expect_tx(&bars[0], (uint32_t)R * kbytes);
-                for (int r = warp + SITE_WARPS * lane; r < R; r += SITE_THREADS)
-                    bulk_g2s(As + (size_t)(r >> 6) * sh.g_stride + (size_t)(r & 63) * sh.kb_pad, A + (size_t)r * K, kbytes, &bars[0]);
-            }
-            // a half step at the end of the rows multiplies zeros
-            if ((klen & 15) != 0)
-                for (int r = tid; r < R + SITE_TOK; r += SITE_THREADS)
-                    *reinterpret_cast<uint4*>((r < R ? As + (size_t)(r >> 6) * sh.g_stride + (size_t)(r & 63) * sh.kb_pad
-                                                     : Xs + (size_t)(r - R) * sh.kb_pad) + kbytes) = make_uint4(0u, 0u, 0u, 0u);
-            __syncthreads();  // the share is known to every warp
+            const int nseg = n_segs;
             // ---- hints: the x and y lines this block will touch, and the next layer's slabs of this work item
             if (hints && warp >= 2) {
                 const int t1 = tid - 64, n1 = SITE_THREADS - 64;
@@ -284,15 +317,13 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                         prefetch_l2(reinterpret_cast<const unsigned char*>(X + (size_t)tok[t] * ldx + k0) + (size_t)l * 128);
                     }
                 }
-    #pragma unroll 1
-                for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-                    const int ncol = sshare.hi[p] - sshare.lo[p];
-                    if (ncol <= 0) continue;
-                    const size_t len = (size_t)ncol * esize;
+#pragma unroll 1
+                for (int q = 0; q < nseg; q++) {
+                    const size_t len = (size_t)segs[q].ncols * esize;
                     const int lines = (int)((len + 127) / 128) + 1;
                     for (int i = t1; i < cn * lines; i += n1) {
                         const int t = i / lines, l = i - t * lines;
-                        const size_t start = ((size_t)tok[t] * ldy + srec.off[p] + sshare.lo[p]) * esize;
+                        const size_t start = ((size_t)tok[t] * ldy + segs[q].ycol) * esize;
                         const size_t at = (start & ~(size_t)127) + (size_t)l * 128;
                         if (at < start + len) prefetch_l2(reinterpret_cast<const unsigned char*>(Y) + at);
                     }
@@ -307,7 +338,7 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                     const int4 head = __ldg(reinterpret_cast<const int4*>(nr));  // cn, slot, rank, cols
                     if (head.x > 0 && head.z > 0) {
                         prefetch_eighth(__ldg(&nr->a), (uint64_t)head.z * (uint64_t)head.w * 2u, crank, lane);
-    #pragma unroll 1
+#pragma unroll 1
                         for (int p = 0; p < PLORA_MAX_PARTS; p++) {
                             const int rp = __ldg(&nr->r[p]);
                             if (rp > 0) prefetch_eighth(__ldg(&nr->b[p]), (uint64_t)__ldg(&nr->rows[p]) * (uint64_t)rp * 2u, crank, lane);
@@ -316,119 +347,124 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                 }
             }
             hints = false;
+            // ---- everything that the rest of the pass will need and that is known by now: where this lane's x is (the token of
+            // column g of the multiply), and its y of the first two steps of the block's first columns
+            const bf16* xrow = X + (size_t)(g < cn ? tok[g] : 0) * ldx + k0 + warp * 32 + 8 * t4;
+            const int x_steps = g < cn ? w_mine : 0;
+            const Seg first = segs[0];  // (of zeros where the block has no columns)
+            const int qtok = g & 3;     // the token whose y this lane moves (of the first four), and its columns of a step
+            const int qcol = warp * 32 + 8 * t4 + 4 * (g >> 2);
+            const bool ahead = first.fast != 0 && qtok < cn;
+            const unsigned char* yahead = reinterpret_cast<const unsigned char*>(Y) + ((size_t)(ahead ? tok[qtok] : 0) * ldy + first.ycol + qcol) * esize;
+            const bool ahead0 = ahead && qcol < first.ncols, ahead1 = ahead && qcol + SITE_WARPS * 32 < first.ncols;
+            if (klen > 0 && t0 == 0) {
+                if (alive) alive = mbar_wait(&bars[0], ph_a, status);
+                ph_a ^= 1;
+            }
             if (!waited && !early_x) {
                 pdl_wait();
                 waited = true;
+            }
+            // ---- x straight into operand registers, all steps at once
+            uint4 xr[SITE_XSTEPS];
+            auto load_x = [&](int s0) {
+#pragma unroll
+                for (int s = 0; s < SITE_XSTEPS; s++) {
+                    xr[s] = make_uint4(0u, 0u, 0u, 0u);
+                    if (s0 + s < x_steps) xr[s] = __ldcg(reinterpret_cast<const uint4*>(xrow + (size_t)(s0 + s) * (SITE_WARPS * 32)));
+                }
+            };
+            load_x(0);
+            // ... and y, on its way while the shrink and the exchange run
+            YQuad<F32> y0, y1;
+            y0.clear();
+            y1.clear();
+            const bool fetched = waited;
+            if (fetched) {
+                if (ahead0) y0.load(yahead);
+                if (ahead1) y1.load(yahead + SITE_WARPS * 32 * esize);
             }
             if (!triggered && release_at == 3) {
                 pdl_trigger();
                 triggered = true;
             }
-            // y of this lane's first expand step (first part of the share), on its way while the shrink and the exchange run
-            uint4 pre0 = make_uint4(0u, 0u, 0u, 0u), pre1 = pre0;
-            int pre_part = -1;
-            if (waited) {
-    #pragma unroll
-                for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-                    if (pre_part < 0 && srec.r[p] > 0 && sshare.hi[p] > sshare.lo[p]) {
-                        pre_part = p;
-                        const size_t ybase = (size_t)srec.off[p] + sshare.lo[p];
-                        const int ncols = sshare.hi[p] - sshare.lo[p];
-                        const bool fast = cn <= 8 && (ncols & 7) == 0 &&
-                                          ((reinterpret_cast<uintptr_t>(Y) | ((size_t)ldy * esize) | (ybase * esize)) & 15) == 0;
-                        const int c = warp * 32 + 8 * (lane & 3);
-                        if (fast && g < cn && c < ncols) {
-                            const unsigned char* yp = reinterpret_cast<const unsigned char*>(Y) + ((size_t)tok[g] * ldy + ybase + c) * esize;
-                            pre0 = __ldcg(reinterpret_cast<const uint4*>(yp));
-                            if (F32) pre1 = __ldcg(reinterpret_cast<const uint4*>(yp) + 1);
+            // ---- shrink over this block's eighth of the inputs, 32 rows of A at a time
+            for (int j0 = 0; j0 < R; j0 += 32) {
+                float acc[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+                const int tiles = min(2, (R - j0) >> 4);
+                for (int s0 = 0; alive && s0 < w_steps; s0 += SITE_XSTEPS) {
+                    if (s0 > 0 || (j0 > 0 && w_steps > SITE_XSTEPS)) load_x(s0);  // (else still in registers)
+                    const uint32_t a0 = a_lane + (uint32_t)j0 * (uint32_t)sh.kb_pad + (uint32_t)s0 * (SITE_WARPS * 64u);
+                    if (tiles == 1) shrink_steps<1>(acc, xr, a0, (uint32_t)sh.kb_pad, w_steps - s0, w_mine - s0);
+                    else shrink_steps<2>(acc, xr, a0, (uint32_t)sh.kb_pad, w_steps - s0, w_mine - s0);
+                }
+                float* wp = Ps + (size_t)warp * SITE_TOK * (sh.rc + 4) + j0 + g;
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    if (i < tiles) {
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            if (t2 + e < cn) {
+                                wp[(t2 + e) * (sh.rc + 4) + i * 16] = acc[i][e];
+                                wp[(t2 + e) * (sh.rc + 4) + i * 16 + 8] = acc[i][2 + e];
+                            }
                         }
                     }
                 }
             }
-            // ---- shrink over this block's eighth of the inputs: warp q takes the 16-wide steps q, q + 8, ...
-            if (klen > 0) {
-                if (warp == 0) {
-                    if (lane == 0) mbar_expect_tx(&bars[1], (uint32_t)cn * kbytes);
-                    __syncwarp();
-                    if (lane < cn) bulk_g2s(Xs + (size_t)lane * sh.kb_pad, X + (size_t)tok[lane] * ldx + k0, kbytes, &bars[1]);
-                }
-                if (alive) alive = mbar_wait(&bars[0], ph_ax, status) && mbar_wait(&bars[1], ph_ax, status);
-                ph_ax ^= 1;
-            }
-            if (!triggered && release_at == 4) {
-                pdl_trigger();
-                triggered = true;
-            }
-            // rows of A in groups of 64 (8 tiles of 8): 32 accumulators per lane
-            for (int j0 = 0; j0 < R; j0 += 64) {
-                float acc[8][4];
-    #pragma unroll
-                for (int i = 0; i < 8; i++) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
-                const int pairs = min(4, (R - j0) >> 4);  // 16-row pairs of tiles in this group
-                const uint32_t grp = (uint32_t)(j0 >> 6) * (uint32_t)sh.g_stride;
-                if (alive && klen > 0) {
-                    const uint32_t xs_w = xs_lane + (uint32_t)warp * 32u, as_w = as_lane + grp + (uint32_t)warp * 32u;
-                    const int n = (nks - warp + SITE_WARPS - 1) / SITE_WARPS;  // this warp's steps
-                    if (pairs == 1) shrink_steps<1>(acc, xs_w, as_w, (uint32_t)sh.kb_pad, n);
-                    else if (pairs == 2) shrink_steps<2>(acc, xs_w, as_w, (uint32_t)sh.kb_pad, n);
-                    else if (pairs == 3) shrink_steps<3>(acc, xs_w, as_w, (uint32_t)sh.kb_pad, n);
-                    else shrink_steps<4>(acc, xs_w, as_w, (uint32_t)sh.kb_pad, n);
-                }
-                __syncthreads();  // every warp is through with this group's rows of A: their place takes the partials
-                float* wp = reinterpret_cast<float*>(As + grp) + (size_t)warp * PLORA_WORK_TOKENS * sh.g_rows + t2;
-    #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (i < 2 * pairs) {
-                        if (g < cn) *reinterpret_cast<float2*>(wp + g * sh.g_rows + i * 8) = make_float2(acc[i][0], acc[i][1]);
-                    }
-                }
-            }
+            if (tid == 0) mbar_expect_tx(&bars[2], (uint32_t)(SITE_CLUSTER * cn * R * 4));
             __syncthreads();
-            // the eight warps' partials, added in warp order: warp q takes the token rows q, q + 8
-            for (int t = warp; t < cn; t += SITE_WARPS) {
-                for (int j = lane; j < R; j += 32) {
-                    const float* p = reinterpret_cast<const float*>(As + (size_t)(j >> 6) * sh.g_stride) + t * sh.g_rows + (j & 63);
-                    float acc = p[0];
-    #pragma unroll
-                    for (int q = 1; q < SITE_WARPS; q++) acc += p[(size_t)q * PLORA_WORK_TOKENS * sh.g_rows];
-                    Sp[t * sh.rmax + j] = acc;
-                }
-            }
             if (!triggered && release_at == 1) {
                 pdl_trigger();
                 triggered = true;
             }
-            // ---- the eight partials meet: every block tells every block that its Sp is written, then reads all
-            // eight and adds them in block order
-            __syncthreads();
             if (!met) {
                 cluster_wait();  // everybody's barriers exist
                 met = true;
             }
-            if (tid < SITE_CLUSTER) mbar_arrive_peer(&bars[3], (uint32_t)tid);
-            if (alive) alive = mbar_wait_cluster(&bars[3], ph_s, status);
-            ph_s ^= 1;
-            for (int t = warp; t < cn; t += SITE_WARPS) {
-                for (int j = lane; j < R; j += 32) {
-                    const float* p = Sp + t * sh.rmax + j;
-                    float v[SITE_CLUSTER];
-    #pragma unroll
-                    for (int q = 0; q < SITE_CLUSTER; q++) v[q] = ld_peer_f32(p, q);
-                    float acc = v[0];
-    #pragma unroll
-                    for (int q = 1; q < SITE_CLUSTER; q++) acc += v[q];
-                    // three bf16 terms whose sum is the f32 value
-                    const bf16 hi = __float2bfloat16_rn(acc);
-                    const float r1 = acc - __bfloat162float(hi);
-                    const bf16 mid = __float2bfloat16_rn(r1);
-                    const bf16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-                    unsigned char* s3 = S3 + (size_t)t * sh.sp_pad + (size_t)j * 2;
-                    *reinterpret_cast<bf16*>(s3) = hi;
-                    *reinterpret_cast<bf16*>(s3 + plane_bytes) = mid;
-                    *reinterpret_cast<bf16*>(s3 + 2 * plane_bytes) = lo;
+            // ---- the eight warps' partials are added in warp order, four rows of a token at a time, and every sum goes to all
+            // eight blocks at once: a store that arrives with its own completion takes one way through the cluster, where an
+            // arrival, a wait and a remote load took three
+            for (int i = tid; i < cn * nq * SITE_CLUSTER; i += SITE_THREADS) {
+                const int q = i >> 3, t = (int)(((uint32_t)q * inv) >> 16), j = 4 * (q - t * nq);
+                const float* p = Ps + (size_t)t * (sh.rc + 4) + j;
+                float4 v = *reinterpret_cast<const float4*>(p);
+#pragma unroll
+                for (int u = 1; u < SITE_WARPS; u++) {
+                    const float4 b = *reinterpret_cast<const float4*>(p + (size_t)u * SITE_TOK * (sh.rc + 4));
+                    v.x += b.x, v.y += b.y, v.z += b.z, v.w += b.w;
                 }
+                st_async_peer(Rs + (size_t)(crank * SITE_TOK + t) * sh.rc + j, v, &bars[2], (uint32_t)(i & 7));
             }
-            cluster_arrive_relaxed();  // my reads of the others' partials are done
+            if (nseg > 0 && t0 == 0) {  // (a later pass finds the rows of B in place)
+                if (alive) alive = mbar_wait(&bars[1], ph_b, status);
+                ph_b ^= 1;
+            }
+            if (alive) alive = mbar_wait_cluster(&bars[2], ph_s, status);
+            ph_s ^= 1;
+            // added in block order, as three bf16 terms whose sum is the f32 value
+            for (int i = tid; i < 2 * cn * nq; i += SITE_THREADS) {
+                const int t = (int)(((uint32_t)(i >> 1) * inv) >> 16), j = 2 * (i - 2 * t * nq);
+                const float* p = Rs + (size_t)t * sh.rc + j;
+                float2 v = *reinterpret_cast<const float2*>(p);
+#pragma unroll
+                for (int q = 1; q < SITE_CLUSTER; q++) {
+                    const float2 b = *reinterpret_cast<const float2*>(p + (size_t)q * SITE_TOK * sh.rc);
+                    v.x += b.x, v.y += b.y;
+                }
+                const __nv_bfloat162 hi = __floats2bfloat162_rn(v.x, v.y);
+                const float2 hf = __bfloat1622float2(hi);
+                const float2 r1 = make_float2(v.x - hf.x, v.y - hf.y);
+                const __nv_bfloat162 mid = __floats2bfloat162_rn(r1.x, r1.y);
+                const float2 mf = __bfloat1622float2(mid);
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(r1.x - mf.x, r1.y - mf.y);
+                unsigned char* s3 = S3 + (size_t)t * sh.sp_pad + (size_t)j * 2;
+                *reinterpret_cast<__nv_bfloat162*>(s3) = hi;
+                *reinterpret_cast<__nv_bfloat162*>(s3 + plane_bytes) = mid;
+                *reinterpret_cast<__nv_bfloat162*>(s3 + 2 * plane_bytes) = lo;
+            }
             if (!triggered) {
                 pdl_trigger();
                 triggered = true;
@@ -438,42 +474,36 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                 waited = true;
             }
             __syncthreads();
+            cluster_arrive_relaxed();  // (every warp behind its reads of Rs) the others may send the next pass's partials
             // ---- expand over this block's share of the output columns
-            bool okb = true;
-            {
-                int total = 0;
-    #pragma unroll
-                for (int p = 0; p < PLORA_MAX_PARTS; p++) total += sshare.hi[p] - sshare.lo[p];
-                if (total > 0 && t0 == 0) {  // (a later pass finds the rows of B in place)
-                    if (alive) okb = mbar_wait(&bars[2], ph_b, status);
-                    ph_b ^= 1;
-                }
-            }
-            if (!okb) alive = false;
             if (alive) {
-                const int tok0 = g < cn ? tok[g] : -1, tok1 = g + 8 < cn ? tok[g + 8] : -1;
-    #pragma unroll 1
-                for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-                    const int r = srec.r[p];
-                    const int lo = sshare.lo[p], hi = sshare.hi[p];
-                    if (r == 0 || hi <= lo) continue;
-                    const uint32_t s3_part = s3_lane + (uint32_t)srec.r_off[p] * 2u;
-                    const uint32_t bs_lane = smem_u32(Bs) + (uint32_t)sshare.boff[p] + (uint32_t)b_row * (uint32_t)r * 2u + (uint32_t)b_piece * 16u;
-                    const size_t ybase = (size_t)srec.off[p] + lo;
-                    // fast form: at most 8 tokens, and y rows that move in 16-byte pieces
-                    const bool fast = cn <= 8 && ((hi - lo) & 7) == 0 && ((reinterpret_cast<uintptr_t>(Y) | ((size_t)ldy * esize) | (ybase * esize)) & 15) == 0;
-                    if (fast) {
+#pragma unroll 1
+                for (int q = 0; q < nseg; q++) {
+                    const Seg sg = segs[q];
+                    const uint32_t s3 = smem_u32(S3) + (uint32_t)sg.soff, b = smem_u32(Bs) + (uint32_t)sg.boff;
+                    if (sg.fast) {
+#pragma unroll 1
+                        for (int q0 = 0; q0 < cn; q0 += 4) {  // four tokens at a time
+                            const bool have = fetched && q == 0 && q0 == 0;
+                            const int nt = min(4, cn - q0);
+                            const uint32_t sq = s3 + (uint32_t)q0 * (uint32_t)sh.sp_pad;
+                            if (sg.r == 16) expand_quads<R16, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
+                            else if (sg.r == 32) expand_quads<R32, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
+                            else if (sg.r & 16) expand_quads<ODD, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
+                            else expand_quads<EVEN, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
+                        }
+                    } else {
+                        // row and 16-byte piece this lane names in a four-matrix load of S (16 rows, the upper 8 repeating the lower
+                        // ones, whose results are dropped) and of B (two 8-row tiles x 16 inputs)
+                        const uint32_t s3_lane = s3 + (uint32_t)(lane & 7) * (uint32_t)sh.sp_pad + (uint32_t)(lane >> 4) * 16u;
+                        const uint32_t bs_lane = b + (uint32_t)((lane & 7) + (lane >> 4) * 8) * (uint32_t)sg.r * 2u + (uint32_t)((lane >> 3) & 1) * 16u;
                         const int tk = g < cn ? tok[g] : -1;
-                        const uint32_t s3p = smem_u32(S3) + (uint32_t)srec.r_off[p] * 2u, bsp = smem_u32(Bs) + (uint32_t)sshare.boff[p];
-                        const bool pre = p == pre_part;
-                        if (r == 16) expand_fast<1, F32>(s3p, (uint32_t)sh.sp_pad, plane_bytes, bsp, r, hi - lo, Y, ldy, ybase, tk, warp, lane, pre, pre0, pre1);
-                        else if (r == 32) expand_fast<2, F32>(s3p, (uint32_t)sh.sp_pad, plane_bytes, bsp, r, hi - lo, Y, ldy, ybase, tk, warp, lane, pre, pre0, pre1);
-                        else expand_fast<0, F32>(s3p, (uint32_t)sh.sp_pad, plane_bytes, bsp, r, hi - lo, Y, ldy, ybase, tk, warp, lane, pre, pre0, pre1);
-                    } else if (r == 16) expand_part<1, F32>(s3_part, plane_bytes, bs_lane, r, hi - lo, Y, ldy, ybase, tok0, tok1, warp, t2);
-                    else expand_part<0, F32>(s3_part, plane_bytes, bs_lane, r, hi - lo, Y, ldy, ybase, tok0, tok1, warp, t2);
+                        if (sg.r == 16) expand_part<1, F32>(s3_lane, plane_bytes, bs_lane, sg.r, sg.ncols, Y, ldy, sg.ycol, tk, -1, warp, t2);
+                        else expand_part<0, F32>(s3_lane, plane_bytes, bs_lane, sg.r, sg.ncols, Y, ldy, sg.ycol, tk, -1, warp, t2);
+                    }
                 }
             }
-            cluster_wait();   // nobody reads my partials any more: they may be overwritten (or the block may leave)
+            cluster_wait();   // nobody reads what this block sent any more
             __syncthreads();  // shared memory is reused by the next pass or work item
         }
     }
@@ -484,51 +514,56 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
     if (!waited && (blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
 }
 
-struct Plan {
-    SiteShape sh;
-    size_t smem;
-};
-
-// Shared-memory plan for `nsub` column groups
-Plan plan_for(int K, int parts, int max_rank, int total_rows, int nsub) {
-    Plan pl;
-    SiteShape& s = pl.sh;
-    s.kchunk = (((K + SITE_CLUSTER - 1) / SITE_CLUSTER) + 7) & ~7;
-    const int pieces = s.kchunk / 8;                          // 16-byte pieces per row
-    s.kb_pad = s.kchunk * 2 + ((pieces + 1) % 2 ? 16 : 32);   // an odd number of pieces between rows
-    s.rmax = parts * max_rank;
-    s.sp_pad = (s.rmax + 8) * 2;
-    s.g_rows = s.rmax < 64 ? s.rmax : 64;
-    const size_t a = (size_t)s.g_rows * s.kb_pad, wsum = (size_t)SITE_WARPS * PLORA_WORK_TOKENS * s.g_rows * 4;
-    s.g_stride = (int)(((a > wsum ? a : wsum) + 127) & ~(size_t)127);
-    s.aw_bytes = s.g_stride * ((s.rmax + 63) / 64);
-    s.x_bytes = (int)(((size_t)SITE_TOK * s.kb_pad + 127) & ~(size_t)127);
-    const int share = ((total_rows + nsub * SITE_CLUSTER - 1) / (nsub * SITE_CLUSTER) + 1) & ~1;
+PloraSiteShape shape_for(int K, int n_parts, const int* part_rows, int max_rank, int nsub) {
+    PloraSiteShape s;
+    s.kchunk = ((K + SITE_CLUSTER - 1) / SITE_CLUSTER + 31) & ~31;
+    s.kb_pad = ((s.kchunk * 2 + 127) & ~127) + 64;
+    // Whichever parts an adapter targets: the most of them that one cluster's columns meet, and the widest share
+    int most = 1, wide = 0;
+    for (int set = 1; set < 1 << n_parts; set++) {
+        int ntot = 0;
+        for (int p = 0; p < n_parts; p++)
+            if (set >> p & 1) ntot += part_rows[p];
+        const int share = site_share(ntot, SITE_CLUSTER * nsub);
+        wide = std::max(wide, share);
+        for (int y = 0; y < nsub; y++) {
+            const int lo = y * SITE_CLUSTER * share, hi = std::min(ntot, lo + SITE_CLUSTER * share);
+            int met = 0, at = 0;
+            for (int p = 0; p < n_parts; p++) {
+                if (!(set >> p & 1)) continue;
+                met += at < hi && at + part_rows[p] > lo;
+                at += part_rows[p];
+            }
+            most = std::max(most, met);
+        }
+    }
+    s.rc = most * max_rank;
+    s.sp_pad = (s.rc + 8) * 2;
+    s.a_bytes = s.rc * s.kb_pad;
+    s.p_bytes = SITE_WARPS * SITE_TOK * (s.rc + 4) * 4;
+    s.r_bytes = SITE_CLUSTER * SITE_TOK * s.rc * 4;
     // the tile loads of the last columns of a part may run up to 31 rows past the share
-    s.b_bytes = (int)((((size_t)share + 32 * parts) * max_rank * 2 + 127) & ~(size_t)127);
-    s.nsub = nsub;
-    pl.smem = (size_t)s.aw_bytes + s.x_bytes + s.b_bytes + (size_t)PLORA_WORK_TOKENS * s.rmax * 4 +
-              (size_t)4 * PLORA_WORK_TOKENS * s.sp_pad;
-    return pl;
+    s.b_bytes = ((wide + 32 * n_parts) * max_rank * 2 + 127) & ~127;
+    return s;
+}
+
+int shape_smem(const PloraSiteShape& s) { return s.a_bytes + s.p_bytes + s.r_bytes + s.b_bytes + 4 * SITE_TOK * s.sp_pad; }
+
+// the clusters of such blocks that the device runs at once (0 on failure)
+int clusters_at_once(int smem) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(SITE_CLUSTER, 1, 16);
+    cfg.blockDim = dim3(SITE_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, plora_site_gather_kernel<false>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return n;
 }
 
 }  // namespace
-
-// Plan of the cluster kernel for one layer: the fewest column groups (1, 2 or 4) with which two blocks share an
-// SM (one SM cannot take a whole cluster of 8, and a B200 has room for only 15 clusters of 8 at one block per
-// SM). Returns the dynamic shared memory per block, 0 when nothing fits: such a layer takes the shrink / expand pair, which
-// is faster there (13 tokens of 8 adapters at rank 32, four layers: 240 us with one block per SM, 150 as pairs).
-size_t plora_site_plan(int K, int parts, int max_rank, int total_rows, int* nsub) {
-    if (parts * max_rank > 256) return 0;  // the shrink keeps at most 4 x 64 rows of A in flight per pass
-    for (int n = 1; n <= 4; n *= 2) {
-        const Plan pl = plan_for(K, parts, max_rank, total_rows, n);
-        if (pl.smem <= 111 * 1024) {
-            *nsub = n;
-            return pl.smem;
-        }
-    }
-    return 0;
-}
 
 cudaError_t plora_site_init() {
     // The split of an SM's memory between L1 and shared memory is fixed while any block runs on it. Layers of
@@ -545,39 +580,40 @@ cudaError_t plora_site_init() {
     return e;
 }
 
-// How many clusters of the layer's plan the device runs at once (0 on failure)
-int plora_site_max_clusters(int K, int parts, int max_rank, int total_rows) {
-    int nsub = 1;
-    const size_t smem = plora_site_plan(K, parts, max_rank, total_rows, &nsub);
-    if (smem == 0) return 0;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SITE_CLUSTER, (unsigned)nsub, 16);
-    cfg.blockDim = dim3(SITE_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, plora_site_gather_kernel<false>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
+// Plans of the cluster kernel for one layer, by column groups per work item: those with which two blocks share an SM (one SM
+// cannot take a whole cluster of 8, and a B200 has room for only 15 clusters of 8 at one block per SM). Empty when
+// nothing fits: such a layer takes the shrink / expand pair, which is faster there (13 tokens of 8 adapters at rank 32,
+// four layers: 240 us with one block per SM, 150 as pairs).
+std::vector<PloraSitePlan> plora_site_plans(int K, int n_parts, const int* part_rows, int max_rank) {
+    std::vector<PloraSitePlan> out;
+    int total = 0;
+    for (int p = 0; p < n_parts; p++) total += part_rows[p];
+    for (int nsub : {1, 2, 3, 4, 6, 8, 12, 16}) {
+        if (nsub > 4 && out.empty()) break;  // (as few clusters as that run at once, and every group reads x again)
+        PloraSitePlan pl;
+        pl.shape = shape_for(K, n_parts, part_rows, max_rank, nsub);
+        if (pl.shape.rc > 256 || shape_smem(pl.shape) > SITE_SMEM) continue;
+        pl.nsub = nsub;
+        pl.smem = shape_smem(pl.shape);
+        pl.max_clusters = clusters_at_once(pl.smem);
+        if (pl.max_clusters < nsub) continue;
+        out.push_back(pl);
+        if (site_share(total, SITE_CLUSTER * nsub) <= SITE_WARPS * 32) break;  // every warp has one step of columns
     }
-    return n;
+    return out;
 }
 
 cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, const PloraRec* next_recs,
-                              void* y, int ldy, int f32_out, int parts, int max_rank, int total_rows, int work_cap,
-                              int max_clusters, int mode, const PloraBounds& bnd, int* status, bool pdl, cudaStream_t st) {
+                              void* y, int ldy, int f32_out, const PloraSitePlan& plan, int work_cap, int mode, const PloraBounds& bnd,
+                              int* status, bool pdl, cudaStream_t st) {
     (void)bnd;
-    int nsub = 1;
-    const size_t smem = plora_site_plan(K, parts, max_rank, total_rows, &nsub);
-    if (smem == 0) return cudaErrorInvalidValue;
-    const Plan pl = plan_for(K, parts, max_rank, total_rows, nsub);
     // one wave: work items beyond the clusters the device runs at once are walked in a loop, so that every block
     // of the grid starts (and releases the next kernel) at once
-    int z = work_cap < PLORA_REC_TERM ? work_cap : PLORA_REC_TERM;
-    if (max_clusters >= nsub && z > max_clusters / nsub) z = max_clusters / nsub;
+    const int z = std::min(std::min(work_cap, PLORA_REC_TERM), std::max(1, plan.max_clusters / plan.nsub));
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(SITE_CLUSTER, (unsigned)nsub, (unsigned)z);
+    cfg.gridDim = dim3(SITE_CLUSTER, (unsigned)plan.nsub, (unsigned)z);
     cfg.blockDim = dim3(SITE_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.dynamicSmemBytes = (size_t)plan.smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -586,7 +622,7 @@ cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* rec
     cfg.numAttrs = pdl ? 1 : 0;
     if (f32_out)
         return cudaLaunchKernelEx(&cfg, plora_site_gather_kernel<true>, reinterpret_cast<const bf16*>(x), ldx, K, recs, rec_cap,
-                                  next_recs, y, ldy, pl.sh, mode, status PLORA_BOUNDS_ARG(bnd));
+                                  next_recs, y, ldy, plan.shape, mode, status PLORA_BOUNDS_ARG(bnd));
     return cudaLaunchKernelEx(&cfg, plora_site_gather_kernel<false>, reinterpret_cast<const bf16*>(x), ldx, K, recs, rec_cap,
-                              next_recs, y, ldy, pl.sh, mode, status PLORA_BOUNDS_ARG(bnd));
+                              next_recs, y, ldy, plan.shape, mode, status PLORA_BOUNDS_ARG(bnd));
 }
