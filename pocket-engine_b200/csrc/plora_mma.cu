@@ -14,6 +14,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "plora_internal.h"
 #include "plora_device.cuh"
@@ -33,9 +34,10 @@ __device__ __forceinline__ void umma_ta(uint32_t d, uint32_t a, uint64_t b, uint
         "r"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
-// 4 consecutive columns of this warp's 32 lanes; to be followed by tmem_st_wait
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t (&v)[4]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3])
+// 8 consecutive columns of this warp's 32 lanes; to be followed by tmem_st_wait
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
@@ -66,6 +68,8 @@ __device__ __forceinline__ void tree_sum(float (&v)[PLORA_TILE_SPLIT_MAX][W], in
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+
+__device__ __forceinline__ float4 add4(const float4& a, const float4& b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
     const uint32_t n = valid ? 16u : 0u;  // a zero source size fills the 16 bytes with zeros
@@ -536,6 +540,13 @@ struct ExpandBars {
     uint32_t tmem_slot;
 };
 
+// barrier of the two warps that share a quarter of the tile's rows
+__device__ __forceinline__ void pair_sync(int quarter) {
+    if (quarter == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+    else if (quarter == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+    else if (quarter == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+    else asm volatile("bar.sync 4, 64;" ::: "memory");
+}
 __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 
 template <bool F32>
@@ -563,8 +574,9 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
     for (int tile = blockIdx.z; tile < n_mma; tile += gridDim.z) {
         const int* mt = segs + lay.mma() + 3 * tile;
         const int start = mt[0], len = mt[1], slot = mt[2];
+        // (all that the block needs of the descriptor at once: fetched where it is used, each field is one more way to L2)
         const plora_desc& d = table[slot];
-        const int r = d.r[p], rows = d.rows[p];
+        const int r = __ldg(&d.r[p]), rows = __ldg(&d.rows[p]), y_off = __ldg(&d.off[p]), r_off = __ldg(&d.r_off[p]), rank = __ldg(&d.rank);
         if (r == 0 || cb0 * EXP_BN >= rows) continue;
         const int nblk = min(nb_per_cta, (rows - cb0 * EXP_BN + EXP_BN - 1) / EXP_BN);
         const int nchunks = min(nblk * CH, (rows - cb0 * EXP_BN + CW - 1) / CW);  // slots this block fills, in column order
@@ -575,7 +587,6 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         // warps w and w + 4 read the same 32 lanes of tensor memory (rows 32 (w % 4) ...) and take the even and the odd
         // slots of the block's columns
         const int wq = warp & 3, wh = warp >> 2;
-        const int P = r >> 3;
         const CUtensorMap* ymap = &ymaps.m[p];
         const CUtensorMap* bmap = reinterpret_cast<const CUtensorMap*>(&smaps[slot].b[p]);
         // the rows of B of column block nb: r / bw boxes of 64 rows by bw ranks, one after another in stage nb % nbs
@@ -628,7 +639,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                 const uint32_t a_hi = tmem + EXP_TMEM_A, a_lo = a_hi + (uint32_t)(r >> 1);
                 const uint32_t sw = bw == 64 ? 2u : bw == 32 ? 4u : 6u;
                 const uint64_t b0 = umma_desc(smem_u32(ops), 16, (uint32_t)bw * 16u, sw);  // eight rows of a box are bw * 16 bytes
-                bool ok = mbar_wait_long(&bars.a_full, 0, status);  // S staged by the other warps
+                bool ok = mbar_wait(&bars.a_full, 0, status);  // S staged by the other warps
                 int stg = 0;
                 uint32_t bpar = 0;
                 for (int nb = 0; ok && nb < nblk; nb++) {
@@ -660,7 +671,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             const int wrow0 = wq * 32;
             const bool live = wrow0 < len;            // the warp has rows of the tile
             const bool whole = wrow0 + 32 <= len;     // all its 32 rows are: results go back by tensor store
-            const int ycol0 = d.off[p] + cb0 * EXP_BN;  // first y column of this block's range
+            const int ycol0 = y_off + cb0 * EXP_BN;  // first y column of this block's range
             const uint32_t lane_base = tmem + ((uint32_t)wrow0 << 16);
             // the warp's i-th slot is slot wh + 2 i of the block's column range
             const int my_n = (nchunks - wh + WPQ - 1) / WPQ;
@@ -669,69 +680,90 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                 mbar_expect_tx(bar, EXP_SLOT_BYTES);
                 tma_load_2d(ring + (size_t)at * EXP_SLOT_BYTES, ymap, ycol0 + (wh + WPQ * i) * CW, start + wrow0, bar);
             };
+            // (the last slot of the ring is the staging buffer of S first)
+            const int early_y = nst - 1;
             if (live && lane == 0)
-                for (int i = 0; i < nst && i < my_n; i++) load_y(i, i);
+                for (int i = 0; i < early_y && i < my_n; i++) load_y(i, i);
 
-            // this thread's token row of S, split into a bf16 high part and the bf16 of what is left, into its lane of tensor memory
+            // The quarter's 32 rows of S, 32 ranks at a time: each of its two warps fetches 16 rows, a row's 128 bytes by eight lanes, adds
+            // up the planes and leaves the sums in shared memory; there every lane finds its own row, split into a bf16 high part (the
+            // first warp) and the bf16 of what is left (the second), and puts it into its lane of tensor memory. With a row
+            // per lane from the start, each load touched 32 lines of L1 for 16 bytes each: 7,500 to 16,000 cycles to here, now
+            // 4,000 to 8,000 (512 mixed tokens: 186 -> 172 us a step; eight prompts of 2048: 784 -> 760).
             {
-                const int row = tid & 127;
-                const bool valid = row < len;
-                const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
-                const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
-                auto put = [&](int j, const float* f) {
-                    uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int e = 0; e < 4; e++) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(f[2 * e], f[2 * e + 1]);
-                        const float2 hf = __bfloat1622float2(h);
-                        const __nv_bfloat162 l = __floats2bfloat162_rn(f[2 * e] - hf.x, f[2 * e + 1] - hf.y);
-                        hi[e] = *reinterpret_cast<const uint32_t*>(&h);
-                        lo[e] = *reinterpret_cast<const uint32_t*>(&l);
-                    }
-                    __syncwarp();
-                    tmem_st4(lane_base + EXP_TMEM_A + 4 * j, hi);
-                    tmem_st4(lane_base + EXP_TMEM_A + (r >> 1) + 4 * j, lo);
-                };
-                if (s_eff > 1) {
+                const int s_eff = min(ksplit, plora_tile_chunks(K, rank));  // planes the shrink wrote for this slot
+                const float* sq = S + (size_t)(start + wrow0) * lds + r_off;
 #pragma unroll 1
-                    for (int j = tid >> 7; j < P; j += WPQ) {
-                        float v[PLORA_TILE_SPLIT_MAX][8];
+                for (int k0 = 0; k0 < r; k0 += 32) {
+                    unsigned char* buf = dsm1k + (size_t)((wq + (k0 & 32 ? 4 : 0)) * nst + nst - 1) * EXP_SLOT_BYTES;
+                    const int lpr = r - k0 >= 32 ? 8 : 4, rpi = 32 / lpr;  // lanes of a row, rows of an instruction
+                    const int row0 = 16 * wh + lane / lpr, piece = lane % lpr;
+                    auto fetch = [&](auto count, int i0) {  // `count` instructions' rows from the i0-th on, all of them on their way together
+                        constexpr int N = decltype(count)::value;
+                        float4 sum[N];
+                        const float* from[N];
 #pragma unroll
-                        for (int s = 0; s < PLORA_TILE_SPLIT_MAX; s++) {
-                            float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-                            if (valid && s < s_eff) {
-                                const float* q = sp + (size_t)s * s_stride + j * 8;
-                                a = __ldcg(reinterpret_cast<const float4*>(q));
-                                b = __ldcg(reinterpret_cast<const float4*>(q + 4));
-                            }
-                            v[s][0] = a.x, v[s][1] = a.y, v[s][2] = a.z, v[s][3] = a.w;
-                            v[s][4] = b.x, v[s][5] = b.y, v[s][6] = b.z, v[s][7] = b.w;
-                        }
-                        tree_sum<8>(v, s_eff);
-                        put(j, v[0]);
-                    }
-                } else {
-                    // four pieces of eight values per round trip
-#pragma unroll 1
-                    for (int j0 = tid >> 7; j0 < P; j0 += 4 * WPQ) {
-                        float4 f[4][2];
+                        for (int i = 0; i < N; i++) from[i] = sq + (size_t)(row0 + (i0 + i) * rpi) * lds + k0 + 4 * piece;
+                        for (int s0 = 0; s0 < s_eff; s0 += 4) {
+                            float4 v[N == 4 ? 1 : 4][N];
 #pragma unroll
-                        for (int q = 0; q < 4; q++) {
-                            const int j = j0 + q * WPQ;
-                            f[q][0] = f[q][1] = make_float4(0.f, 0.f, 0.f, 0.f);
-                            if (valid && j < P) {
-                                f[q][0] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8));
-                                f[q][1] = __ldcg(reinterpret_cast<const float4*>(sp + j * 8 + 4));
+                            for (int u = 0; u < (N == 4 ? 1 : 4); u++)
+#pragma unroll
+                                for (int i = 0; i < N; i++) {
+                                    v[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                                    if (s0 + u < s_eff && wrow0 + row0 + (i0 + i) * rpi < len)
+                                        v[u][i] = __ldcg(reinterpret_cast<const float4*>(from[i] + (size_t)(s0 + u) * s_stride));
+                                }
+#pragma unroll
+                            for (int i = 0; i < N; i++) {  // a balanced tree over the 1, 2, 4 or 8 planes
+                                float4 t = v[0][i];
+                                if (N != 4) {
+                                    t = add4(t, v[N == 4 ? 0 : 1][i]);
+                                    if (s_eff > 2) t = add4(t, add4(v[N == 4 ? 0 : 2][i], v[N == 4 ? 0 : 3][i]));
+                                }
+                                sum[i] = s0 == 0 ? t : add4(sum[i], t);
                             }
                         }
 #pragma unroll
-                        for (int q = 0; q < 4; q++)
-                            if (j0 + q * WPQ < P) put(j0 + q * WPQ, reinterpret_cast<const float*>(f[q]));
+                        for (int i = 0; i < N; i++) {
+                            const int row = row0 + (i0 + i) * rpi;
+                            if (row < 16 * wh + 16) *reinterpret_cast<float4*>(buf + row * 128 + ((piece ^ (row & 7)) << 4)) = sum[i];
+                        }
+                    };
+                    if (s_eff == 1) {
+                        fetch(std::integral_constant<int, 4>(), 0);
+                    } else {
+                        fetch(std::integral_constant<int, 2>(), 0);
+                        if (lpr == 8) fetch(std::integral_constant<int, 2>(), 2);
+                    }
+                    pair_sync(wq);  // (the buffer of the ranks before stays: the next ones go to the other warp's slot)
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        if (k0 + 16 * h < r) {
+                            uint32_t w[8];
+#pragma unroll
+                            for (int c = 0; c < 4; c++) {
+                                const float4 f = *reinterpret_cast<const float4*>(buf + lane * 128 + (((4 * h + c) ^ (lane & 7)) << 4));
+                                __nv_bfloat162 a = __floats2bfloat162_rn(f.x, f.y), b = __floats2bfloat162_rn(f.z, f.w);
+                                if (wh == 1) {
+                                    const float2 af = __bfloat1622float2(a), bf = __bfloat1622float2(b);
+                                    a = __floats2bfloat162_rn(f.x - af.x, f.y - af.y);
+                                    b = __floats2bfloat162_rn(f.z - bf.x, f.w - bf.y);
+                                }
+                                w[2 * c] = *reinterpret_cast<const uint32_t*>(&a);
+                                w[2 * c + 1] = *reinterpret_cast<const uint32_t*>(&b);
+                            }
+                            __syncwarp();
+                            tmem_st8(lane_base + EXP_TMEM_A + (wh == 1 ? (uint32_t)(r >> 1) : 0u) + (uint32_t)((k0 + 16 * h) >> 1), w);
+                        }
                     }
                 }
                 tmem_st_wait();
                 tc_fence_before();
                 mbar_arrive(&bars.a_full);  // S is staged
+                fence_async_smem();         // the staging buffers, read and written, before the copies of y into them
+                pair_sync(wq);
+                if (live && lane == 0 && early_y < my_n) load_y(early_y, early_y);
             }
 
             bool ok = true;
@@ -765,7 +797,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                 const int col0 = (cb0 + nb) * EXP_BN + ch * CW;  // first column of the slot within the part
                 const bool mine = wrow0 + lane < len;
                 if (F32) {
-                    float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+                    float* yrow = reinterpret_cast<float*>(Y) + (size_t)(start + wrow0 + lane) * ldy + y_off + col0;
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
                         float4* yp = reinterpret_cast<float4*>(myrow + ((c ^ (lane & 7)) << 4));
@@ -786,7 +818,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
                         }
                     }
                 } else {
-                    bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + d.off[p] + col0;
+                    bf16* yrow = reinterpret_cast<bf16*>(Y) + (size_t)(start + wrow0 + lane) * ldy + y_off + col0;
 #pragma unroll
                     for (int c = 0; c < 8; c++) {
                         if (c == 4) fetch(1);
