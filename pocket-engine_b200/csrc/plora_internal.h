@@ -259,14 +259,17 @@ cudaError_t plora_launch_xchg_all_ranks(const PloraXchgCtx* ctxs_dev, int world,
 // its own tensor-memory accumulator, inputs in order) and then added as a balanced binary tree. The count is a
 // function of the site and of the slot's total rank only, so a token's result never depends on the batch; a
 // launch may hand the chunks to 1, 2, 4 or 8 blocks (each an aligned subtree, one plane of S per block, the
-// planes tree-summed by the reader) and every such choice gives the same bits. At most 256 accumulator
-// columns per block, so that two blocks share an SM's tensor memory, and at least 8 steps of 64 inputs per chunk.
+// planes tree-summed by the reader) and every such choice gives the same bits. At most the 512 accumulator
+// columns of an SM for all of a tile's chunks (where they go to several blocks, each holds its own only), and at least 8 steps of
+// 64 inputs per chunk. With 256 of them, ranges of K were twice as long at total ranks over 32: 1,545 ragged tokens of ranks 16 to
+// 64 275 us a step, 261 so; 512 mixed tokens of rank 32 172 and 167; eight prompts of 2048 tokens, whose tiles are one
+// block each, 760 and 761.
 #define PLORA_TILE_SPLIT_MAX 8
 __host__ __device__ inline int plora_tile_cols(int R) { return R <= 32 ? 32 : R <= 64 ? 64 : R <= 128 ? 128 : R <= 256 ? 256 : 512; }
 __host__ __device__ inline int plora_tile_chunks(int K, int R) {
     const int nk = (K + 63) / 64, rc = plora_tile_cols(R);
     int c = PLORA_TILE_SPLIT_MAX;
-    while (c > 1 && (c * 8 > nk || c * rc > 256)) c >>= 1;
+    while (c > 1 && (c * 8 > nk || c * rc > 512)) c >>= 1;
     return c;
 }
 
