@@ -732,8 +732,8 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
             a->uploaded = true;
         }
     }
-    // The slot's column of the descriptor tables [sites][max_slots + 1], and of the tile path's views of the stacked A, in one
-    // kernel (:616-621 copies entry by entry; at 4.6 us per 112-byte copy the 32 layers' entries of an
+    // The slot's column of the descriptor tables [sites][max_slots + 1], and of the tile path's views of the stacked A:
+    // one strided copy each (:616-621 copies entry by entry; at 4.6 us per 112-byte copy the 32 layers' entries of an
     // eight-layer model took as long as 16 MB of slab).
     const size_t stride = (size_t)h->max_slots + 1, n = h->sites.size();
     bool maps = false;
@@ -746,8 +746,13 @@ int plora_upload(plora_t* h, int slot, uint32_t id, void* stream) {
             maps = true;
         }
     }
-    CUK(h, "upload descriptors",
-        plora_launch_upload_column(h->tables, h->host_tables, maps ? h->smaps : nullptr, h->host_smaps, (int)n, (int)stride, slot, st));
+    CU(h, "upload descriptors",
+       cudaMemcpy2DAsync(h->tables + slot, stride * sizeof(plora_desc), h->host_tables + slot, stride * sizeof(plora_desc),
+                         sizeof(plora_desc), n, cudaMemcpyHostToDevice, st));
+    if (maps)
+        CU(h, "upload slab tensor maps",
+           cudaMemcpy2DAsync(h->smaps + slot, stride * sizeof(PloraSlabMaps), h->host_smaps + slot, stride * sizeof(PloraSlabMaps),
+                             sizeof(PloraSlabMaps), n, cudaMemcpyHostToDevice, st));
     return PLORA_OK;
 }
 

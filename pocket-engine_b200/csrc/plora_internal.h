@@ -274,9 +274,6 @@ __host__ __device__ inline int plora_tile_chunks(int K, int R) {
 }
 
 // ---- kernel launchers (plora_kernels.cu); each returns a cudaError_t from the launch ----
-// One slot's column of the descriptor tables and, unless null, of the tensor maps, from their pinned mirrors
-cudaError_t plora_launch_upload_column(plora_desc* tables, const plora_desc* host_tables, PloraSlabMaps* maps, const PloraSlabMaps* host_maps,
-                                       int n_sites, int stride, int slot, cudaStream_t st);
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st);
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).

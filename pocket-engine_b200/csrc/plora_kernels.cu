@@ -59,19 +59,6 @@ __device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long
 }
 
 // ---------------------------------------------------------------------------------------------
-// One slot's column of the descriptor tables and of the tensor maps, a block per layer, read from their pinned mirrors over the bus. (As
-// two strided copies behind the slab's they took 10.8 us of the stream an upload, a copy's start each; so 5 to 6.)
-__global__ void __launch_bounds__(64) plora_upload_column_kernel(plora_desc* __restrict__ tables, const plora_desc* host_tables,
-                                                                  PloraSlabMaps* __restrict__ maps, const PloraSlabMaps* host_maps, int stride, int slot) {
-    constexpr int DESC = sizeof(plora_desc) / 16, MAPS = sizeof(PloraSlabMaps) / 16;
-    static_assert(sizeof(plora_desc) % 16 == 0 && DESC + MAPS <= 64, "a piece of 16 bytes per thread");
-    const size_t at = (size_t)blockIdx.x * (size_t)stride + (size_t)slot;
-    const int i = threadIdx.x;
-    if (i < DESC) reinterpret_cast<uint4*>(tables + at)[i] = __ldcv(reinterpret_cast<const uint4*>(host_tables + at) + i);
-    else if (i - DESC < MAPS && maps != nullptr) reinterpret_cast<uint4*>(maps + at)[i - DESC] = __ldcv(reinterpret_cast<const uint4*>(host_maps + at) + (i - DESC));
-}
-
-// ---------------------------------------------------------------------------------------------
 // Tile words from the step's sequences: for each sequence in order with a slot, chunks of 16 tokens
 // (start, len, slot); word 0 is the count. One block, of a thread per sequence where there are fewer than 1024.
 __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __restrict__ cu,
@@ -140,6 +127,9 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w, int slot,
                                              int cnt, int cols, int nsplit, int most) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
+    uint4 tok[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) tok[i] = work[1 + i];
     const uint4* d = reinterpret_cast<const uint4*>(table + slot);  // 112 bytes: a, b[4], rank, r, r_off, off, rows
     uint4 dv[7];
 #pragma unroll
@@ -166,7 +156,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     }
     o[7] = make_uint4(dw[25], dw[26], ntot, 0u);                // rows[2], rows[3], ntot
 #pragma unroll
-    for (int i = 0; i < 4; i++) o[8 + i] = work[1 + i];         // the token rows (fetched here: ahead of the rest they spilled registers)
+    for (int i = 0; i < 4; i++) o[8 + i] = tok[i];              // the token rows
     o[12] = make_uint4(cat[0], cat[1], cat[2], cat[3]);
     return units;
 }
@@ -1270,12 +1260,6 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
     return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
 }  // namespace
-
-cudaError_t plora_launch_upload_column(plora_desc* tables, const plora_desc* host_tables, PloraSlabMaps* maps, const PloraSlabMaps* host_maps,
-                                       int n_sites, int stride, int slot, cudaStream_t st) {
-    plora_upload_column_kernel<<<n_sites, 64, 0, st>>>(tables, host_tables, maps, host_maps, stride, slot);
-    return cudaGetLastError();
-}
 
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st) {
