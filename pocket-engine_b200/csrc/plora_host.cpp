@@ -1142,20 +1142,22 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
                       uint64_t w, uint64_t sn, int rows, int width, uint64_t y, int ldy, int f32_out, int work_cap,
                       void* stream) {
     const SiteInfo& site = h->sites[(size_t)hook->site];
-    const bool pdl = next_launch(h, stream, false).pdl;
-    // the kernel reads the long runs' S from plane 0: fold the tile path's planes (the gather tokens' K-split
-    // planes are added by the gather expand itself)
-    CUK(h, "S reduce (tiles)",
-       plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, 1,
-                             (const int32_t*)(uintptr_t)step->segs, h->seg, (const plora_desc*)(uintptr_t)hook->table, 0,
-                             has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0, tile_split(h, rows),
-                             site.cols, pdl, as_stream(stream)));
+    bool pdl = next_launch(h, stream, false).pdl;
+    // the kernel reads the long runs' S from plane 0: fold the tile path's planes, where a tile was more than one block's (the gather
+    // tokens' K-split planes are added by the gather expand itself)
+    if (has_tiles(h, step, rows) && tile_split(h, rows) > 1) {
+        CUK(h, "S reduce (tiles)",
+           plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, 1,
+                                 (const int32_t*)(uintptr_t)step->segs, h->seg, (const plora_desc*)(uintptr_t)hook->table, 0,
+                                 std::max(1, rows / 64), tile_split(h, rows), site.cols, pdl, as_stream(stream)));
+        pdl = h->pdl;
+    }
     CUK(h, "fused layer (tensor-core adapter term)",
        plora_launch_gemm_fused(kind, (const void*)(uintptr_t)x, (const float*)(uintptr_t)st, (const void*)(uintptr_t)w,
                                (const float*)(uintptr_t)sn, rows, width, site.cols, (const int32_t*)(uintptr_t)step->segs,
                                h->seg, (const plora_desc*)(uintptr_t)hook->table, (int)site.parts.size(), site.part_off,
                                site.part_rows, (const float*)(uintptr_t)step->s, step->lds, (void*)(uintptr_t)y, ldy, f32_out,
-                               has_tiles(h, step, rows), h->status, h->pdl, as_stream(stream)));
+                               has_tiles(h, step, rows), h->status, pdl, as_stream(stream)));
     if (work_cap > 0)
         CUK(h, "expand (tokens outside long runs)",
            plora_launch_expand((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.nsplit,
