@@ -142,7 +142,7 @@ struct GemmShared {
 // rows of W per block; the adapter operands are the pairs' only
 __host__ __device__ constexpr int gemm_w_rows(int bn, bool two) { return two ? bn / 2 : bn; }
 __host__ __device__ constexpr size_t gemm_stage_bytes(int bn, bool two) { return G_BM * G_BKB + gemm_w_rows(bn, two) * G_BKB; }
-__host__ __device__ constexpr size_t gemm_operands(int bn, bool two) { return two && bn <= 256 ? 2 * G_AOP + (size_t)bn / 2 * G_RC * 2 : 0; }
+__host__ __device__ constexpr size_t gemm_operands(int bn, bool two) { return two ? 2 * G_AOP + (size_t)bn / 2 * G_RC * 2 : 0; }
 constexpr size_t gemm_smem(int bn, bool two) {
     return 1024 + G_STAGES * gemm_stage_bytes(bn, two) + gemm_operands(bn, two) + G_EPI_WARPS * G_SLOT + bn * sizeof(float);
 }
@@ -161,14 +161,11 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
     constexpr uint32_t STAGE = (uint32_t)gemm_stage_bytes(BN, TWO);
     constexpr int BLOCKS = TWO ? 2 : 1, TM = BLOCKS * G_BM;  // blocks and tokens of a tile
     constexpr int WR = gemm_w_rows(BN, TWO);
-    // A tile of 384 columns is two multiplies of 192 side by side, over the same x: for decoding steps, which have no adapter passes
-    constexpr bool DUAL = BN > 256, PASSES = TWO && !DUAL;
-    constexpr int UN = DUAL ? BN / 2 : BN;          // columns of a multiply
     constexpr int HALF = BN == 192 ? 128 : BN / 2;  // columns of the first four epilogue warps (whole slots of 64)
-    constexpr int NBUF = KIND == 0 || DUAL ? 1 : 2;               // accumulators of the base product
-    constexpr bool SHARED = KIND == 1 && BN > 128 && !DUAL;        // the adapter term uses the other one of them
+    constexpr int NBUF = KIND == 0 ? 1 : 2;               // accumulators of the base product
+    constexpr bool SHARED = KIND == 1 && BN > 128;        // the adapter term uses the other one of them
     // first column of the adapter term of a tile whose base product is in accumulator `buf`
-    auto ad_col = [](int buf) { return (uint32_t)(KIND == 0 || DUAL ? BN : SHARED ? (buf ^ 1) * BN : (2 + buf) * BN); };
+    auto ad_col = [](int buf) { return (uint32_t)(KIND == 0 ? BN : SHARED ? (buf ^ 1) * BN : (2 + buf) * BN); };
     constexpr int KEL = KIND == 0 ? G_BKB : G_BKB / 2;    // elements of K per step
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = TWO ? pair_rank() : 0;
@@ -229,9 +226,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                     if (TWO) {
                         const uint32_t bar = at_leader(&sh.full[stg]);
                         tma_load_2d_pair(xs, &xmap, ks * KEL, m0 + (int)rank * G_BM, bar);
-#pragma unroll
-                        for (int u = 0; u < BN / UN; u++)
-                            tma_load_2d_pair(xs + G_BM * G_BKB + u * (UN / 2) * G_BKB, &wmap, ks * KEL, n0 + u * UN + (int)rank * (UN / 2), bar);
+                        tma_load_2d_pair(xs + G_BM * G_BKB, &wmap, ks * KEL, n0 + (int)rank * WR, bar);
                     } else {
                         tma_load_2d(xs, &xmap, ks * KEL, m0, &sh.full[stg]);
                         tma_load_2d(xs + G_BM * G_BKB, &wmap, ks * KEL, n0, &sh.full[stg]);
@@ -248,15 +243,15 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
             // M TM, N BN, f32 accumulator, K-major operands; kind::f16 carries the bf16 formats in bits 7 and 10
-            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
-            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(UN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24) : idesc_ad;
+            const uint32_t idesc_ad = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+            const uint32_t idesc = KIND == 0 ? (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24) : idesc_ad;
             const uint64_t dx0 = umma_desc(smem_u32(ring), 16, 1024, 2), dw0 = umma_desc(smem_u32(ring) + G_BM * G_BKB, 16, 1024, 2);
             int stg = 0, i = 0;
             uint32_t par = 0, apar = 0;  // parities of the stages and of the adapter operands
             int before = 0;              // passes of the tile before
             bool ok = true;
             for (int t = pair; ok && t < tiles; t += pairs, i++) {
-                const int buf = NBUF == 1 ? 0 : i & 1;
+                const int buf = KIND == 0 ? 0 : i & 1;
                 const uint32_t acc = tmem + (uint32_t)buf * BN, ad = tmem + ad_col(buf);
                 // Whoever last had this tile's accumulator has been read: the tile NBUF before, or the one before, whose
                 // adapter term was in it (its warps have then read the earlier tile too). The adapter term's needs no wait of
@@ -264,7 +259,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                 if (SHARED && before > 0) ok = mbar_wait_long(&sh.acc_empty[buf ^ 1], (i - 1) / NBUF & 1, status);
                 else if (i >= NBUF) ok = mbar_wait_long(&sh.acc_empty[buf], (i / NBUF - 1) & 1, status);
                 tc_fence_after();
-                int npass = PASSES ? -1 : 0, ps = 0;  // npass: not known before the other warps have written the list
+                int npass = TWO ? -1 : 0, ps = 0;  // npass: not known before the other warps have written the list
                 auto pass = [&]() {
                     tc_fence_after();
                     const int rw = sh.rw[ps];
@@ -283,11 +278,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                     const uint64_t dx = dx0 + (uint64_t)((uint32_t)stg * STAGE >> 4), dw = dw0 + (uint64_t)((uint32_t)stg * STAGE >> 4);
 #pragma unroll
                     for (int kk = 0; kk < G_BKB / 32; kk++) {
-                        if (TWO) {
-#pragma unroll
-                            for (int u = 0; u < BN / UN; u++)
-                                pair_umma<KIND>(acc + u * UN, dx + 2 * kk, dw + u * (UN / 2 * G_BKB / 16) + 2 * kk, idesc, (ks | kk) != 0);
-                        }
+                        if (TWO) pair_umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
                         else umma<KIND>(acc, dx + 2 * kk, dw + 2 * kk, idesc, (ks | kk) != 0);
                     }
                     if (TWO) pair_commit(&sh.empty[stg]);
@@ -296,14 +287,14 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                         stg = 0;
                         par ^= 1;
                     }
-                    if (PASSES && npass < 0 && mbar_test(&sh.meta, i & 1)) npass = sh.npass;
-                    if (PASSES && ps < npass && mbar_test(&sh.ad_full, apar)) pass();
+                    if (TWO && npass < 0 && mbar_test(&sh.meta, i & 1)) npass = sh.npass;
+                    if (TWO && ps < npass && mbar_test(&sh.ad_full, apar)) pass();
                 }
-                if (PASSES && ok && npass < 0) {
+                if (TWO && ok && npass < 0) {
                     ok = mbar_wait_long(&sh.meta, i & 1, status);
                     npass = ok ? sh.npass : 0;
                 }
-                while (PASSES && ok && ps < npass) {
+                while (TWO && ok && ps < npass) {
                     ok = mbar_wait_long(&sh.ad_full, apar, status);
                     if (ok) pass();
                 }
@@ -331,7 +322,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
                 if (q < parts.n && n0 >= parts.off[q]) part = q;
             const int n_local = n0 - parts.off[part] + (int)rank * WR;  // this block's first row of B_p
             // ---- the tile's adapter passes: tensor-core tiles of the grouping that meet the pair's rows
-            if (PASSES && ew == 0) {
+            if (TWO && ew == 0) {
                 const int n_mma = segs[SEG_N_MMA];
                 const int* ml = segs + lay.mma();
                 // the first tile that ends after the first row: 32 probes a round
@@ -370,8 +361,8 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             if (KIND == 0)
                 for (int c = e; c < BN; c += G_EPI) sn_s[c] = n0 + c < N ? sn[n0 + c] : 0.f;
             epi_sync_all();
-            const int npass = PASSES ? sh.npass : 0;
-            if (PASSES && e == 0) mbar_arrive(&sh.meta);
+            const int npass = TWO ? sh.npass : 0;
+            if (TWO && e == 0) mbar_arrive(&sh.meta);
             for (int ps = 0; ps < npass; ps++) {
                 if (staged) {  // the operands of the pass before are still being read until its MMAs complete
                     if (ok) ok = mbar_wait_long(&sh.ad_empty, apar, status);
@@ -431,7 +422,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             }
             // ---- epilogue: the warp's 32 rows of its half of the columns, scaled and added, into a swizzled slot of 128
             // bytes a row, then a tensor store (clipped at the edges of y by the tensor map)
-            const int buf = NBUF == 1 ? 0 : i & 1;
+            const int buf = KIND == 0 ? 0 : i & 1;
             if (ok) ok = mbar_wait_long(&sh.acc_full[buf], (i / NBUF) & 1, status);
             if (!ok) {
                 epi_sync_all();
@@ -572,7 +563,6 @@ cudaError_t plora_gemm_init() {
     cudaError_t e;
     auto init = [](auto* kernel, size_t smem) { return plora_kernel_shared(reinterpret_cast<const void*>(kernel), (int)smem); };
 #define PLORA_GEMM_INIT(KIND, F32)                                                                                                         \
-    if ((e = init(plora_gemm_fused_kernel<KIND, F32, 384, true>, gemm_smem(384, true)))) return e;   \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 256, true>, gemm_smem(256, true)))) return e;   \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 192, true>, gemm_smem(192, true)))) return e;   \
     if ((e = init(plora_gemm_fused_kernel<KIND, F32, 128, true>, gemm_smem(128, true)))) return e;   \
@@ -623,9 +613,7 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
     // tiles, and a round that is nearly empty costs as much as a full one. A step of K costs what it moves into an SM,
     // G_BM rows of x and the block's rows of W, of 128 bytes each. Tiles of 192 columns may span two parts, which adapter
     // passes do not, so they are for steps that cannot have long runs: begun as decoding steps, or of fewer
-    // rows (FP8, 256 tokens, 24,576 columns, shrink and layer: 77.3 -> 74.9 us). With more than 128 tokens such a step may take two
-    // multiplies of 192 columns a tile over the same x: what x costs an SM is paid once for 384 columns, and 28,416 of them are one
-    // round (256 tokens, 24,576 columns: 39.4 -> 31.9 us). Up to 128 tokens of such a step, blocks on their own take tiles of 256 or 192 columns where that costs less: layers too wide for
+    // rows (FP8, 256 tokens, 24,576 columns, shrink and layer: 77.3 -> 74.9 us). Up to 128 tokens of such a step, blocks on their own take tiles of 256 or 192 columns where that costs less: layers too wide for
     // one round of pairs. FP8, 24,576 columns: 36 us in two rounds of pairs, 24 in one round of blocks (shrink and layer at
     // 70 tokens: 65 -> 53 us, at 128: 69 -> 57); the bf16 layers of a block at 70 tokens: 238 -> 218 us.
     const int blocks = 2 * g_pairs;
@@ -642,7 +630,6 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
         best = cost;
     };
     consider(256, true);
-    if (!tiles && T > G_BM) consider(384, true);
     if (!tiles) consider(192, true);
     consider(128, true);
     if (!tiles && T <= G_BM) {
@@ -650,7 +637,7 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
         consider(192, false);
     }
     if (!encode2d(&xmap, dt, x, (uint64_t)K, (uint64_t)T, (uint64_t)K * el, G_BKB / el, G_BM)) return cudaErrorInvalidValue;
-    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)(gemm_w_rows(bn, two) / (bn > 256 ? 2 : 1)))) return cudaErrorInvalidValue;
+    if (!encode2d(&wmap, dt, w, (uint64_t)K, (uint64_t)N, (uint64_t)K * el, G_BKB / el, (uint32_t)gemm_w_rows(bn, two))) return cudaErrorInvalidValue;
     if (!encode2d(&ymap, f32_out ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, y, (uint64_t)N,
                   (uint64_t)T, (uint64_t)ldy * (f32_out ? 4 : 2), f32_out ? 32 : 64, 32))
         return cudaErrorInvalidValue;
@@ -668,8 +655,7 @@ cudaError_t plora_launch_gemm_fused(int kind, const void* x, const float* st_, c
                           status);
     };
 #define PLORA_GEMM_LAUNCH(KIND, F32)                                                  \
-    return two ? launch(bn == 384   ? plora_gemm_fused_kernel<KIND, F32, 384, true>   \
-                        : bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, true>   \
+    return two ? launch(bn == 256   ? plora_gemm_fused_kernel<KIND, F32, 256, true>   \
                         : bn == 192 ? plora_gemm_fused_kernel<KIND, F32, 192, true>   \
                                     : plora_gemm_fused_kernel<KIND, F32, 128, true>)  \
                : launch(bn == 256 ? plora_gemm_fused_kernel<KIND, F32, 256, false>    \

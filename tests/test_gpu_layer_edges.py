@@ -136,12 +136,3 @@ def test_few_tokens_over_a_wide_layer(pe, kind, rows, widths, f32_out):
     mx, mn = harness.tolerance(got, want)
     assert (mx <= 1e-3 and mn <= 1e-4) if f32_out else (mx <= 4e-2 and mn <= 4e-3), (mx, mn)
     loras.close()
-
-
-@pytest.mark.parametrize("f32_out", [True, False])
-@pytest.mark.parametrize("kind", ["bf16", "fp8"])
-@pytest.mark.parametrize("rows,widths", [([256], [28416]), ([129], [14600]), ([100, 100], [18944, 18952])])
-def test_pairs_with_two_multiplies_a_tile(pe, kind, rows, widths, f32_out):
-    """129 to 256 tokens over layers that tiles of 384 columns take in one round or in two: the last tile whole, ending inside its first
-    multiply, and spanning parts."""
-    test_few_tokens_over_a_wide_layer(pe, kind, rows, widths, f32_out)
