@@ -138,16 +138,6 @@ __device__ __forceinline__ void pdl_exit_idle() {
     if ((blockIdx.x | blockIdx.y | blockIdx.z) == 0) pdl_wait();
 }
 
-// A layer's tile kernels follow its gather kernels, run beside them, and start only once those have waited. Where the step has no
-// gather tokens at all, that would put the launch and the first fetches of every tile kernel behind the kernel before: a gather
-// kernel that finds its list of items empty (so do all its blocks, and all the step's gather kernels) releases at once, and
-// a tile kernel that finds no items in the step waits by itself. Eight prompts of 2048 tokens, one block of
-// layers: 759 -> 739 us.
-__device__ __forceinline__ void pdl_exit_empty() {
-    pdl_trigger();
-    pdl_exit_idle();
-}
-
 // Hints that the 128-byte line holding `p` will be read soon: the line is brought into L2, no value is bound,
 // so it is safe on memory an earlier kernel may still be writing.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }

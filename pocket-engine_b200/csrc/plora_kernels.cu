@@ -493,15 +493,14 @@ __device__ __forceinline__ int load_prefix(int* pre, const int* __restrict__ src
     return pre[1 + n];
 }
 // The same for the expand, and the block's share [u0, u1) of all units. In shared memory the units before an item are
-// counted from u0. False where the block has no share; `none`: the step has no items.
-__device__ __forceinline__ bool load_share(int* pre, const int* __restrict__ src, int rec_cap, int& share, bool& none) {
+// counted from u0. False where the block has no share.
+__device__ __forceinline__ bool load_share(int* pre, const int* __restrict__ src, int rec_cap, int& share) {
     const long long* pe = reinterpret_cast<const long long*>(src);
     const long long head = __ldcg(pe), total = __ldcg(pe + 1);
     const int n = min((int)(head & 0xffffffff), rec_cap);
     long long mine = 0;  // (fetched beside the counts that say how many there are)
     if ((int)threadIdx.x <= rec_cap) mine = __ldcg(pe + 2 + threadIdx.x);
     const int blocks = min((int)(head >> 32), (int)gridDim.x);
-    none = n == 0;
     if ((int)blockIdx.x >= blocks || total == 0) return false;
     const long long u0 = share_at(total, blockIdx.x, blocks);
     share = (int)(share_at(total, blockIdx.x + 1, blocks) - u0);
@@ -580,8 +579,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_shrink_gather_kernel(
     const int total = load_prefix(pre, prefix, rec_cap);  // (its barrier publishes the ring's as well)
     const int u0 = (int)((long long)total * blockIdx.x / gridDim.x), u1 = (int)((long long)total * (blockIdx.x + 1) / gridDim.x);
     if (u0 >= u1) {
-        if (!waited && pre[0] == 0) pdl_exit_empty();
-        else if (!waited) pdl_exit_idle();
+        if (!waited) pdl_exit_idle();
         return;
     }
     // a unit's place: its item, its split and first row (units of an item go split by split, so that the rows of A of a split
@@ -1141,8 +1139,7 @@ __global__ void __launch_bounds__(GATHER_THREADS, 2) plora_expand_gather_kernel(
         mbar_fence_init();
     }
     int u1;  // the block's share is the units 0 .. u1
-    bool none;
-    if (!load_share(pre, prefix, rec_cap, u1, none)) return none ? pdl_exit_empty() : pdl_exit_idle();  // (its barrier publishes the ring's as well)
+    if (!load_share(pre, prefix, rec_cap, u1)) return pdl_exit_idle();  // (its barrier publishes the ring's as well)
     const int w0 = find_item(pre, 0);
     if (warp == 8) {
         // ---- copies of B, and hints for y

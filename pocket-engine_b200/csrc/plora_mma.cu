@@ -131,7 +131,6 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     __shared__ int s_fail;
     const int tile = blockIdx.z;
     const int n_mma = segs[SEG_N_MMA];
-    const bool beside = late && segs[SEG_N_WORK] > 0;  // (without items the kernel before has released this one at once: pdl_exit_empty)
     const int* mt = segs + lay.mma() + 3 * tile;
     const int start = mt[0], len = mt[1], slot = mt[2];
     if (tile >= n_mma) return pdl_exit_idle();
@@ -173,7 +172,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     const uint32_t a_box_bytes = (uint32_t)R * 128u;
     // the slab's rows arrive as one box of R rows, or two of R / 2 when R is over the 256-row limit of a box
     const int nbox = R > 256 ? 2 : 1, box_rows = R / nbox;
-    if (!beside) pdl_wait();  // x comes from the kernels before
+    if (!late) pdl_wait();  // x comes from the kernels before
     pdl_trigger();
 
     if (warp == 0) {
@@ -257,7 +256,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     // everyone: the accumulators are complete once the last commit has arrived
     bool ok = mbar_wait_long(&acc_bar, 0, status);
     __syncthreads();
-    if (beside) pdl_wait();  // before any store, and on every path: this grid must outlast the ones before it
+    if (late) pdl_wait();  // before any store, and on every path: this grid must outlast the ones before it
     if (ok && !s_fail) {
         tc_fence_after();
         const int row = tid;
@@ -566,7 +565,6 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
     constexpr int CW = F32 ? 32 : 64;     // y columns per slot
     constexpr int CH = EXP_BN / CW;       // slots per column block
     constexpr int NW = EXP_WARPS, WPQ = NW / 4;
-    const bool beside = late && segs[SEG_N_WORK] > 0;  // (as in the shrink)
     const int n_mma = segs[SEG_N_MMA], p = blockIdx.y, cb0 = blockIdx.x * nb_per_cta;
     bool begun = false;  // the block has waited for the kernels before it and holds tensor memory
     // The grid is as deep as a step of full tiles needs; a step of many short runs has more tiles, which the blocks then
@@ -628,7 +626,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             for (int nb = 0; nb < nbs - 2 && nb < nblk; nb++) load_b(nb);  // a slab: it may be fetched before the kernels ahead have finished
         }
         if (!begun) {
-            if (!beside) pdl_wait();
+            if (!late) pdl_wait();
             pdl_trigger();
             begun = true;
         }
@@ -875,7 +873,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
         __syncthreads();
     }
     if (!begun) return pdl_exit_idle();
-    if (beside) pdl_wait();
+    if (late) pdl_wait();
     if ((threadIdx.x >> 5) == NW) tmem_dealloc(reinterpret_cast<ExpandBars*>(dsm1k + (size_t)NW * nst * EXP_SLOT_BYTES + nbs * (size_t)b_bytes)->tmem_slot, 256);
 }
 

@@ -261,13 +261,7 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
         if (tid < 13) reinterpret_cast<uint4*>(&srec)[tid] = __ldg(reinterpret_cast<const uint4*>(recs + w) + tid);
         __syncthreads();
         const int cnt = srec.cnt;
-        if (cnt == 0) {  // end of the list: the same decision in every block of the cluster
-            if (w == 0 && !triggered && !waited) {  // an empty one: a tile kernel behind this one then waits by itself (plora_device.cuh)
-                pdl_trigger();
-                triggered = true;
-            }
-            break;
-        }
+        if (cnt == 0) break;  // end of the list: the same decision in every block of the cluster
 #ifdef PLORA_BOUNDS
         if (!rec_in_bounds(srec, bnd, K) || srec.cols != K) {  // the same decision in every block that reads this record
             if (tid == 0) atomicMax(status, PLORA_ERR_ARG);
