@@ -322,7 +322,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
     h->seg.max_tokens = max_tokens;
     h->seg.cap_tiles = h->cap_tiles;
     h->seg.run_min = 1 << 30;  // every run takes the gather path unless the tile path can run (set below)
-    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024 + 3 * (size_t)(max_slots + 1) * sizeof(int)) {
+    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024) {
         delete h;
         return fail(nullptr, PLORA_ERR_CAPACITY,
                     "limits: max_slots <= 1023, max_rank <= 512, and max_tokens/16 + max_seqs tiles must fit the "
@@ -923,7 +923,7 @@ int plora_step_begin(plora_t* h, int max_tiles, int decode, void* stream, plora_
     LaunchOrder::Stream key;
     const bool behind = h->tiles_built && stream_key(stream, &key) && key == h->tiles_stream;
     CUK(h, "meta_group", plora_launch_meta_group(h->meta, segs, lay, h->status, h->tables, h->site_cols, (int)h->sites.size(),
-                                                 h->recs, h->rec_cap, h->prefix, max_tiles, h->pdl && behind, as_stream(stream)));
+                                                 h->recs, h->rec_cap, h->prefix, h->pdl && behind, as_stream(stream)));
     h->tiles_built = false;
     h->order.grouped();
     out->run_min = lay.run_min;

@@ -278,10 +278,9 @@ cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, 
                                     int cap_tiles, int* status, cudaStream_t st);
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
 // site_info: per layer {input width, 0,
-// K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item;
-// tiles_hint: about how many tiles the step has (any number is right, more of them take more rounds)
+// K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, int tiles_hint, bool pdl,
+                                    const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
                                     cudaStream_t st);
 // Dynamic shared-memory limit of a kernel together with a request for the largest shared-memory split of the SM.
 // Kernels of this library overlap with their neighbours in the stream (programmatic dependent launch); an SM's

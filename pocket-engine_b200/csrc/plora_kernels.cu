@@ -10,8 +10,6 @@
 // the partials in split order, so S needs no zeroing and the result is reproducible bit for bit.
 #include <cuda_bf16.h>
 
-#include <algorithm>
-
 #include "plora_internal.h"
 #include "plora_device.cuh"
 #include "plora_tc.cuh"
@@ -20,7 +18,7 @@
 
 namespace {
 
-// Exclusive scan of one 64-bit word per thread over a block of whole warps (several counts packed into one word are
+// Exclusive scan of one 64-bit word per thread over a block of 1024 threads (several counts packed into one word are
 // scanned together). `sh` holds 33 words; it may be used again after the next __syncthreads().
 __device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long v, unsigned long long& total, unsigned long long* sh) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -32,18 +30,8 @@ __device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long
     }
     if (lane == 31) sh[warp] = incl;
     __syncthreads();
-    if (blockDim.x <= 12 * 32) {  // few warps: each adds up the ones before it by itself
-        unsigned long long before = 0;
-        total = 0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); q++) {
-            const unsigned long long t = sh[q];
-            if (q < warp) before += t;
-            total += t;
-        }
-        return incl - v + before;
-    }
     if (warp == 0) {
-        const unsigned long long t = lane < (int)(blockDim.x >> 5) ? sh[lane] : 0ull;
+        const unsigned long long t = sh[lane];
         unsigned long long ti = t;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -60,18 +48,17 @@ __device__ __forceinline__ unsigned long long block_scan_excl(unsigned long long
 
 // ---------------------------------------------------------------------------------------------
 // Tile words from the step's sequences: for each sequence in order with a slot, chunks of 16 tokens
-// (start, len, slot); word 0 is the count. One block, of a thread per sequence where there are fewer than 1024.
+// (start, len, slot); word 0 is the count. One block of 1024 threads.
 __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __restrict__ cu,
                                                                  const int* __restrict__ seq_slot, int n_seqs,
                                                                  int* __restrict__ tiles, int cap_tiles,
                                                                  int* __restrict__ status) {
     __shared__ unsigned long long sh[33];
-    __shared__ int s_first[1024], s_start[1024], s_n[1024], s_slot[1024], n_long;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt_all = blockDim.x;
+    __shared__ int s_first[1024], s_start[1024], s_n[1024], s_slot[1024];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     pdl_trigger();  // the grouping kernel waits for this grid before it reads a word
-    if (tid == 0) n_long = 0;  // (the scan's barriers come before it is counted)
     int carry = 0;
-    for (int base = 0; base < n_seqs; base += nt_all) {
+    for (int base = 0; base < n_seqs; base += 1024) {
         const int i = base + tid;
         int start = 0, n = 0, slot = 0, nt = 0;
         if (i < n_seqs) {
@@ -83,30 +70,28 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
         }
         unsigned long long total;
         const int excl = (int)block_scan_excl((unsigned long long)nt, total, sh);
-        // a sequence's first tile by its own thread, the others by a warp
-        auto put = [&](int idx, int at, int left, int s) {
-            if (idx < cap_tiles) {
-                tiles[1 + 3 * idx] = at;
-                tiles[2 + 3 * idx] = min(left, PLORA_TILE);
-                tiles[3 + 3 * idx] = s;
-            }
-        };
-        if (nt > 0) put(carry + excl, start, n, slot);
-        if (nt > 1) {
-            const int q = atomicAdd(&n_long, 1);
-            s_first[q] = carry + excl;
-            s_start[q] = start;
-            s_n[q] = n;
-            s_slot[q] = slot;
-        }
+        s_first[tid] = carry + excl;
+        s_start[tid] = start;
+        s_n[tid] = n;
+        s_slot[tid] = slot;
         __syncthreads();
-        for (int q = warp; q < n_long; q += nt_all >> 5) {
-            const int qn = s_n[q], qt = (qn + PLORA_TILE - 1) / PLORA_TILE;
-            for (int k = 1 + lane; k < qt; k += 32) put(s_first[q] + k, s_start[q] + k * PLORA_TILE, qn - k * PLORA_TILE, s_slot[q]);
+        const int here = min(1024, n_seqs - base);
+        for (int q = warp; q < here; q += 32) {
+            const int qs = s_slot[q];
+            if (qs == 0) continue;
+            const int qn = s_n[q], q0 = s_start[q], qf = s_first[q];
+            const int qt = (qn + PLORA_TILE - 1) / PLORA_TILE;
+            for (int k = lane; k < qt; k += 32) {
+                const int idx = qf + k;
+                if (idx < cap_tiles) {
+                    tiles[1 + 3 * idx] = q0 + k * PLORA_TILE;
+                    tiles[2 + 3 * idx] = min(qn - k * PLORA_TILE, PLORA_TILE);
+                    tiles[3 + 3 * idx] = qs;
+                }
+            }
         }
         carry += (int)total;
         __syncthreads();
-        if (tid == 0) n_long = 0;
     }
     if (tid == 0) {
         if (carry > cap_tiles) {
@@ -121,15 +106,14 @@ __global__ void __launch_bounds__(1024) plora_meta_tiles_kernel(const int* __res
 // ---------------------------------------------------------------------------------------------
 #define SHR_PAD 20  // floats between the token rows of a warp's partial
 
-// One launch record: gather work item w (`cnt` tokens of a slot) resolved against one layer's descriptor table, so that the kernels of
+// One launch record: gather work item w resolved against one layer's descriptor table, so that the kernels of
 // that layer make one metadata fetch per block. `o` is the record's 16 uint4.
 // Returns the item's units of the few-token kernels (pack_units).
-__device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w, int slot,
-                                             int cnt, int cols, int nsplit, int most) {
+__device__ __forceinline__ unsigned long long write_record(uint4* o, const int* segs, const SegLayout& lay, const plora_desc* table, int w,
+                                             int cols, int nsplit, int most) {
     const uint4* work = reinterpret_cast<const uint4*>(segs + lay.work() + PLORA_WORK_WORDS * w);
-    uint4 tok[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) tok[i] = work[1 + i];
+    const uint4 head = work[0];  // slot, perm start, count, 0
+    const int slot = (int)head.x;
     const uint4* d = reinterpret_cast<const uint4*>(table + slot);  // 112 bytes: a, b[4], rank, r, r_off, off, rows
     uint4 dv[7];
 #pragma unroll
@@ -139,8 +123,8 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
     int r[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
 #pragma unroll
     for (int p = 0; p < PLORA_MAX_PARTS; p++) r[p] = (int)dw[11 + p], rows[p] = (int)dw[23 + p];
-    const unsigned long long units = pack_units(expand_item_units(r, rows, cnt, most), shrink_item_units((int)dw[10], nsplit));
-    o[0] = make_uint4((uint32_t)cnt, (uint32_t)slot, dw[10], (uint32_t)cols);  // cnt, slot, rank, cols
+    const unsigned long long units = pack_units(expand_item_units(r, rows, (int)head.z, most), shrink_item_units((int)dw[10], nsplit));
+    o[0] = make_uint4(head.z, head.x, dw[10], (uint32_t)cols);  // cnt, slot, rank, cols
     o[1] = make_uint4(dw[0], dw[1], dw[2], dw[3]);              // a, b[0]
     o[2] = make_uint4(dw[4], dw[5], dw[6], dw[7]);              // b[1], b[2]
     o[3] = make_uint4(dw[8], dw[9], dw[11], dw[12]);            // b[3], r[0], r[1]
@@ -155,8 +139,10 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
         if ((int)dw[11 + p] > 0) ntot += dw[23 + p];
     }
     o[7] = make_uint4(dw[25], dw[26], ntot, 0u);                // rows[2], rows[3], ntot
-#pragma unroll
-    for (int i = 0; i < 4; i++) o[8 + i] = tok[i];              // the token rows
+    o[8] = work[1];                                             // the token rows
+    o[9] = work[2];
+    o[10] = work[3];
+    o[11] = work[4];
     o[12] = make_uint4(cat[0], cat[1], cat[2], cat[3]);
     return units;
 }
@@ -166,17 +152,15 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
 // least lay.run_min tokens become tensor-core tiles; the rest are gathered by slot: perm lists their
 // token rows ordered by (slot, position in the tile list), cut into work items of <= 16 tokens.
 //
-// Every block but the first then writes the launch records of its layers (every gridDim.x - 1 of them): each gather work
+// Every block then writes the launch records of its layers (blockIdx.x, blockIdx.x + gridDim.x, ...): each gather work
 // item resolved against the layer's descriptor table. The list of a layer ends with records whose cnt is 0.
 //
 // The kernel is a chain of latencies (fetch, scans, fetch of the descriptors), not of bytes. So the blocks do not
 // share the grouping, which would take a grid-wide wait: each of them does all of it, with the same result, and writes
-// the regrouped rows and work items that it will read back itself (the same words from every block); block 0 writes, in place of
-// records, what only later kernels read. Counts that are scanned together share one 64-bit scan. A block has a thread per tile or slot
-// of the step (plora_launch_meta_group): every warp runs all of this code, and with 32 of them the issue of it was a good part of the
-// time. Tile words and grouping, us from the first launch to the end: 230 of 256 sequences over 64 adapters, one layer 14.3 -> 10.9;
-// 512 tokens over 32 adapters, four layers 14.7 -> 10.3; the grouping of one token over 16 layers 6.6 -> 4.8. What is left there is
-// mostly the records themselves: uncoalesced 16-byte pieces, on one SM per layer.
+// the regrouped rows and work items that it will read back itself (the same words from every block); block 0 also
+// writes what only later kernels read. Counts that are scanned together share one 64-bit scan. One block wrote the
+// records of all layers before: 9 us for a single token over 16 layers, 13 us for 64 tokens, 19-27 us for a prefill
+// step, against what bench.py reports as meta_us now.
 __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __restrict__ tiles, int* __restrict__ segs,
                                                                  SegLayout lay, int* __restrict__ status,
                                                                  const plora_desc* __restrict__ tables,
@@ -186,7 +170,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     extern __shared__ int sm[];
     __shared__ int first_item;  // (thread 0's) units of a layer's first item in the expand
     __shared__ unsigned long long sh[4][33];  // a row per scan in flight: no barrier between one scan and the next
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x, nw_all = nt >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cap = lay.cap_tiles, S1 = lay.max_slots + 1;
     const bool first = blockIdx.x == 0;
     int* run_tok = sm;  // [cap + 1]: tokens of the runs before; the length of run r is run_tok[r + 1] - run_tok[r]
@@ -196,18 +180,12 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     int* cnt = run_pos + cap;
     int* seg_base = cnt + S1;
     int* fill = seg_base + S1;
-    int* act_slot = fill + S1;   // by active index, ascending: the slot, its first work item, its gather tokens
-    int* act_work = act_slot + S1;
-    int* act_cnt = act_work + S1;
-    int* whist = act_cnt + S1;   // [warps][S1]
+    int* whist = fill + S1;  // [32][S1]
 
-    int4 info = make_int4(0, 0, 0, 0);
-    const int my_site = (int)blockIdx.x - 1, site_step = (int)gridDim.x - 1;  // the layers whose records this block writes
-    if (recs != nullptr && my_site >= 0 && my_site < n_sites) info = reinterpret_cast<const int4*>(site_cols)[my_site];
     // what needs no tile word, under the wait for the kernel before (the tile words, or the step before, which may
     // still be reading the metadata)
-    for (int i = tid; i < S1; i += nt) cnt[i] = fill[i] = seg_base[i] = 0;
-    for (int i = tid; i < nw_all * S1; i += nt) whist[i] = 0;
+    for (int i = tid; i < S1; i += 1024) cnt[i] = fill[i] = seg_base[i] = 0;
+    for (int i = tid; i < 32 * S1; i += 1024) whist[i] = 0;
     pdl_trigger();  // (the first kernel of the step waits for this grid before it reads a record)
     pdl_wait();
 
@@ -225,12 +203,12 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
         bad = true;
     }
     if (first)
-        for (int i = tid; i < lay.max_tokens; i += nt) segs[lay.tslot() + i] = 0;
+        for (int i = tid; i < lay.max_tokens; i += 1024) segs[lay.tslot() + i] = 0;
     __syncthreads();
 
     // runs
     int n_runs = 0, n_tok = 0;
-    for (int base = 0, it = 0; base < n_tiles; base += nt, it ^= 1) {
+    for (int base = 0; base < n_tiles; base += 1024) {
         const int i = base + tid;
         int head = 0, start = 0, len = 0, slot = 0;
         if (i < n_tiles) {
@@ -257,16 +235,14 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
                 slot = 0;
                 len = 0;
                 start = 0;
-            } else if (recs != nullptr && my_site >= 0 && my_site < n_sites) {
-                // the descriptor this block will resolve first (112 bytes over one line or two)
-                const unsigned char* d = reinterpret_cast<const unsigned char*>(tables + (size_t)my_site * (size_t)S1 + slot);
-                prefetch_l2(d);
-                prefetch_l2(d + sizeof(plora_desc) - 1);
+            } else if (recs != nullptr && blockIdx.x < (unsigned)n_sites) {
+                // the descriptor this block will resolve first
+                prefetch_l2(tables + (size_t)blockIdx.x * (size_t)S1 + slot);
             }
             head = i == 0 || !(pslot == slot && ps + pl == start);
         }
         unsigned long long total;
-        const unsigned long long excl = block_scan_excl(((unsigned long long)head << 32) | (unsigned)len, total, sh[it]);
+        const unsigned long long excl = block_scan_excl(((unsigned long long)head << 32) | (unsigned)len, total, sh[(base >> 10) & 1]);
         const int rid = n_runs + (int)(excl >> 32);
         if (head) {
             run_start[rid] = start;
@@ -280,7 +256,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     __syncthreads();
     // the slot of every token row: 16 lanes a tile
     if (first)
-        for (int i = tid; i < 16 * n_tiles; i += nt) {
+        for (int i = tid; i < 16 * n_tiles; i += 1024) {
             const int t = i >> 4, k = i & 15;
             const int start = tiles[1 + 3 * t], len = tiles[2 + 3 * t], slot = tiles[3 + 3 * t];
             if (slot >= 0 && slot <= lay.max_slots && len >= 1 && len <= PLORA_TILE && start >= 0 && start + len <= lay.max_tokens && k < len)
@@ -290,7 +266,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     // classify runs; tensor-core tiles (none when every run stays under run_min)
     const bool any_mma = lay.run_min <= n_tok;
     int n_mma = 0;
-    for (int base = 0, it = 2; base < n_runs; base += nt, it ^= 1) {
+    for (int base = 0; base < n_runs; base += 1024) {
         const int r = base + tid;
         int nm = 0, len = 0, slot = 0, start = 0;
         if (r < n_runs) {
@@ -308,7 +284,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
         }
         if (any_mma) {
             unsigned long long total;
-            const int excl = (int)block_scan_excl((unsigned long long)nm, total, sh[it]);
+            const int excl = (int)block_scan_excl((unsigned long long)nm, total, sh[2 + ((base >> 10) & 1)]);
             int* mma = segs + lay.mma();
             for (int q = 0; first && q < nm; q++) {
                 const int at = n_mma + excl + q;
@@ -350,9 +326,6 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             for (int q = 0; q < nw; q++)
                 *reinterpret_cast<int4*>(work + PLORA_WORK_WORDS * (woff + q)) =
                     make_int4(s, off + q * PLORA_WORK_TOKENS, min(PLORA_WORK_TOKENS, c - q * PLORA_WORK_TOKENS), 0);
-            act_slot[aidx] = s;
-            act_work[aidx] = woff;
-            act_cnt[aidx] = c;
             cnt[s] = woff;  // from here on: the slot's first work item
         }
         if (first && tid == 0 && !over) segs[lay.seg_off() + n_act] = n_gather;
@@ -361,7 +334,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
 
     // stable position of every gather run inside its slot's segment: the weights of the same slot in the lanes below,
     // in the warps below (whist), and in the rounds of 1024 runs before (fill)
-    for (int base = 0; base < n_runs; base += nt) {
+    for (int base = 0; base < n_runs; base += 1024) {
         const int r = base + tid;
         int key = 0, w = 0;
         if (r < n_runs && run_pos[r] == -2) {
@@ -369,7 +342,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             w = run_tok[r + 1] - run_tok[r];
         }
         if (base > 0) {
-            for (int i = tid; i < nw_all * S1; i += nt) whist[i] = 0;
+            for (int i = tid; i < 32 * S1; i += 1024) whist[i] = 0;
             __syncthreads();
         }
         const unsigned peers = __match_any_sync(0xffffffffu, key);
@@ -391,11 +364,11 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
             for (int q = 0; q < warp; q++) pre += whist[q * S1 + key];
             run_pos[r] = seg_base[key] + fill[key] + pre + sum;
         }
-        if (base + nt < n_runs) {
+        if (base + 1024 < n_runs) {
             __syncthreads();
-            for (int s = tid; s < S1; s += nt) {
+            for (int s = tid; s < S1; s += 1024) {
                 int tot = 0;
-                for (int q = 0; q < nw_all; q++) tot += whist[q * S1 + s];
+                for (int q = 0; q < 32; q++) tot += whist[q * S1 + s];
                 fill[s] += tot;
             }
             __syncthreads();
@@ -405,7 +378,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     // perm, and the same token rows inside the work items (each thread reads back the positions it wrote)
     int* perm = segs + lay.perm();
     int* work = segs + lay.work();
-    for (int r = tid; r < n_runs; r += nt) {
+    for (int r = tid; r < n_runs; r += 1024) {
         const int pos = run_pos[r];
         if (pos < 0) continue;
         const int start = run_start[r], len = run_tok[r + 1] - run_tok[r], slot = run_slot[r];
@@ -427,33 +400,23 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
         segs[SEG_STATUS] = any_bad ? PLORA_ERR_ARG : 0;
     }
     // launch records (the barrier above made the work items, written by other threads of this block, visible)
-    if (recs != nullptr && my_site >= 0) {
+    if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
-        for (int site = my_site; site < n_sites; site += site_step) {
-            if (site != my_site) info = reinterpret_cast<const int4*>(site_cols)[site];
+        for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
+            const int4 info = reinterpret_cast<const int4*>(site_cols)[site];
             int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
             long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
-            for (int base = 0, it = 0; base < end; base += nt, it ^= 1) {
+            for (int base = 0; base < end; base += 1024) {
                 const int w = base + tid;
                 unsigned long long units = 0, total = 0;
                 if (w < end) {
                     uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
-                    if (w >= nw) {
-                        o[0] = make_uint4(0u, 0u, 0u, (uint32_t)info.x);
-                    } else {
-                        int lo = 0, hi = n_act;  // the item's slot: from shared memory, where its own words would come back from L2
-                        while (hi - lo > 1) {
-                            const int mid = (lo + hi) >> 1;
-                            if (act_work[mid] <= w) lo = mid;
-                            else hi = mid;
-                        }
-                        units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, act_slot[lo],
-                                             min(PLORA_WORK_TOKENS, act_cnt[lo] - (w - act_work[lo]) * PLORA_WORK_TOKENS), info.x, info.z, info.w);
-                    }
+                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)info.x);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, info.x, info.z, info.w);
                 }
                 if (w == 0) first_item = (int)packed_expand(units);
-                const unsigned long long at = before + block_scan_excl(units, total, sh[it]);
+                const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
                 if (w < nw) {
                     ps[1 + w] = packed_shrink(at);
                     pe[2 + w] = packed_expand(at);
@@ -1263,13 +1226,12 @@ cudaError_t launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t 
 
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st) {
-    const int threads = n_seqs > 992 ? 1024 : n_seqs <= 64 ? 64 : (n_seqs + 31) / 32 * 32;
-    plora_meta_tiles_kernel<<<1, threads, 0, st>>>(cu, seq_slot, n_seqs, tiles, cap_tiles, status);
+    plora_meta_tiles_kernel<<<1, 1024, 0, st>>>(cu, seq_slot, n_seqs, tiles, cap_tiles, status);
     return cudaGetLastError();
 }
 
 size_t plora_meta_group_smem(const SegLayout& lay) {
-    return (size_t)(4 * lay.cap_tiles + 1 + 6 * (lay.max_slots + 1) + 32 * (lay.max_slots + 1)) * sizeof(int);
+    return (size_t)(4 * lay.cap_tiles + 1 + 3 * (lay.max_slots + 1) + 32 * (lay.max_slots + 1)) * sizeof(int);
 }
 
 // One-time function attributes (dynamic shared memory above 48 KB). Called from plora_create, never from
@@ -1294,15 +1256,12 @@ cudaError_t plora_kernels_init(const SegLayout& lay) {
 }
 
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
-                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, int* prefix, int tiles_hint, bool pdl,
+                                    const int32_t* site_cols, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
                                     cudaStream_t st) {
-    // the first block, and one per layer up to 64: past that a block has more than one layer's records to write, and every further
+    // a block per layer, up to 64: past that a block has more than one layer's records to write, and every further
     // block repeats the grouping
-    const int blocks = recs == nullptr ? 1 : 1 + std::min(n_sites, 64);
-    // a thread per tile and per slot, no more than there are of either
-    const int want = std::max(std::min(tiles_hint, lay.cap_tiles), lay.max_slots + 1);
-    const int threads = want > 992 ? 1024 : want <= 128 ? 128 : (want + 31) / 32 * 32;
-    return launch_pdl(plora_meta_group_kernel, dim3((unsigned)blocks), dim3((unsigned)threads), plora_meta_group_smem(lay), st, pdl, tiles, segs, lay,
+    const int blocks = recs == nullptr ? 1 : n_sites < 64 ? n_sites : 64;
+    return launch_pdl(plora_meta_group_kernel, dim3((unsigned)blocks), dim3(1024), plora_meta_group_smem(lay), st, pdl, tiles, segs, lay,
                       status, tables, site_cols, n_sites, recs, rec_cap, prefix, 2 * g_sms);
 }
 
