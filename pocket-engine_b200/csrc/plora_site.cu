@@ -196,6 +196,9 @@ __device__ __forceinline__ void shrink_steps(float (&acc)[2][4], const uint4 (&x
         for (int e = 0; e < 4; e++) acc[i][e] += odd[i][e];
 }
 
+template <RankWalk W>
+using Walk = std::integral_constant<RankWalk, W>;
+
 template <bool F32>
 __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THREADS, 2)
     plora_site_gather_kernel(const bf16* __restrict__ X, int ldx, int K, const PloraRec* __restrict__ recs, int rec_cap,
@@ -481,25 +484,25 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                 for (int q = 0; q < nseg; q++) {
                     const Seg sg = segs[q];
                     const uint32_t s3 = smem_u32(S3) + (uint32_t)sg.soff, b = smem_u32(Bs) + (uint32_t)sg.boff;
+                    auto expand = [&](auto walk, auto whole, int q0) {  // four tokens at a time
+                        expand_quads<decltype(walk)::value, F32, decltype(whole)::value>(s3 + (uint32_t)q0 * (uint32_t)sh.sp_pad, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r,
+                                                                                         sg.ncols, Y, ldy, sg.ycol, tok + q0, min(4, cn - q0), warp, lane,
+                                                                                         fetched && q == 0 && q0 == 0, y0, y1);
+                    };
                     if (sg.fast) {
 #pragma unroll 1
-                        for (int q0 = 0; q0 < cn; q0 += 4) {  // four tokens at a time
-                            const bool have = fetched && q == 0 && q0 == 0;
-                            const int nt = min(4, cn - q0);
-                            const uint32_t sq = s3 + (uint32_t)q0 * (uint32_t)sh.sp_pad;
-                            if (sg.r == 16) expand_quads<R16, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
-                            else if (sg.r == 32) expand_quads<R32, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
-                            else if (sg.r & 16) expand_quads<ODD, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
-                            else expand_quads<EVEN, F32>(sq, (uint32_t)sh.sp_pad, plane_bytes, b, sg.r, sg.ncols, Y, ldy, sg.ycol, tok + q0, nt, warp, lane, have, y0, y1);
+                        for (int q0 = 0; q0 < cn; q0 += 4) {
+                            if (sg.r == 16) expand(Walk<R16>(), std::true_type(), q0);
+                            else if (sg.r == 32) expand(Walk<R32>(), std::true_type(), q0);
+                            else if (sg.r & 16) expand(Walk<ODD>(), std::true_type(), q0);
+                            else expand(Walk<EVEN>(), std::true_type(), q0);
                         }
                     } else {
-                        // row and 16-byte piece this lane names in a four-matrix load of S (16 rows, the upper 8 repeating the lower
-                        // ones, whose results are dropped) and of B (two 8-row tiles x 16 inputs)
-                        const uint32_t s3_lane = s3 + (uint32_t)(lane & 7) * (uint32_t)sh.sp_pad + (uint32_t)(lane >> 4) * 16u;
-                        const uint32_t bs_lane = b + (uint32_t)((lane & 7) + (lane >> 4) * 8) * (uint32_t)sg.r * 2u + (uint32_t)((lane >> 3) & 1) * 16u;
-                        const int tk = g < cn ? tok[g] : -1;
-                        if (sg.r == 16) expand_part<1, F32>(s3_lane, plane_bytes, bs_lane, sg.r, sg.ncols, Y, ldy, sg.ycol, tk, -1, warp, t2);
-                        else expand_part<0, F32>(s3_lane, plane_bytes, bs_lane, sg.r, sg.ncols, Y, ldy, sg.ycol, tk, -1, warp, t2);
+#pragma unroll 1
+                        for (int q0 = 0; q0 < cn; q0 += 4) {
+                            if (sg.r & 16) expand(Walk<ODD>(), std::false_type(), q0);
+                            else expand(Walk<EVEN>(), std::false_type(), q0);
+                        }
                     }
                 }
             }

@@ -1,7 +1,8 @@
 """The cluster kernel of plora_apply over its column groups: steps of few work items take more of them (each loads and multiplies
 only the rows of A of the parts its columns meet), with the same bits as in a step of many; ranks that its expand walks 16
 and 32 at a time; one to nine tokens of an adapter (groups of four, passes of eight); inputs that end inside a block's share,
-inside a step of 32 and inside a warp's round; shares of columns that are no multiple of a step."""
+inside a step of 32 and inside a warp's round; shares of columns that are no multiple of a step, and parts whose widths are no
+multiples of 8, where rows of y move in pairs of columns and which shares end in one depends on the number of groups."""
 import numpy as np
 import pytest
 
@@ -16,11 +17,18 @@ SITES = [
     (17416, [("d", 264)]),                        # more than eight steps of 32 inputs for a warp
     (8, [("t", 40)]),
 ]
+UNEVEN = [
+    (4096, [("a", 4100)]),                        # one to three groups, each of them with an odd last share
+    (2048, [("a", 1030), ("b", 2050)]),
+    (1024, [("g", 6148), ("u", 6148)]),           # the second part's rows of y start at a multiple of 4
+    (5120, [("q", 2054), ("k", 1030), ("v", 518)]),
+]
+SETS = {"whole": SITES, "uneven": UNEVEN}
 
 
-def workload(pe, ranks, rows, slots):
+def workload(pe, ranks, rows, slots, which=SITES):
     from pocket_engine_b200 import workloads
-    sites = [pe.Site.fused(i, cols, mods) for i, (cols, mods) in enumerate(SITES)]
+    sites = [pe.Site.fused(i, cols, mods) for i, (cols, mods) in enumerate(which)]
     return workloads.Workload("groups", sites, ranks, 1.0, rows, slots, 41)
 
 
@@ -34,15 +42,25 @@ def test_groups(pe, ranks, f32_out):
 
 
 @pytest.mark.parametrize("f32_out", [True, False])
-def test_bits_whatever_the_number_of_groups(pe, f32_out):
+@pytest.mark.parametrize("ranks", [[32, 16], [48]], ids=str)
+def test_uneven_widths(pe, ranks, f32_out):
+    for n in (1, 3, 5, 9):
+        rows = [n] + [1] * (len(ranks) - 1)
+        wl = workload(pe, ranks, rows, [1 + i for i in range(len(rows))], UNEVEN)
+        harness.run_and_check(pe, wl, f32_out=f32_out, meta="device", fused="cluster")
+
+
+@pytest.mark.parametrize("f32_out", [True, False])
+@pytest.mark.parametrize("which", sorted(SETS))
+def test_bits_whatever_the_number_of_groups(pe, which, f32_out):
     ranks = [16, 16, 32, 8]
     rows, slots = [1] * 40, [1 + i % 4 for i in range(40)]
-    wl = workload(pe, ranks, rows, slots)
-    n = len(SITES)
+    wl = workload(pe, ranks, rows, slots, SETS[which])
+    n = len(SETS[which])
     xs, ys = [wl.x_bits(i) for i in range(n)], [wl.y_base(i) for i in range(n)]
 
     def run(first, count):
-        w = workload(pe, ranks, rows[first:first + count], slots[first:first + count])
+        w = workload(pe, ranks, rows[first:first + count], slots[first:first + count], SETS[which])
         loras = harness.product_registry(pe, w)
         got = harness.run_gpu(pe, loras, w, f32_out, meta="device", fused="cluster", xs=[x[first:first + count] for x in xs],
                               y_base=[y[first:first + count] for y in ys])
