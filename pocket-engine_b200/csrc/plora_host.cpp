@@ -381,10 +381,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             if (rc == PLORA_OK) h->site_ok = plora_site_init() == cudaSuccess;
             std::vector<int32_t> info;
             for (auto& s : h->sites) {
-                // Cluster kernel or pair whatever the number of slots: how many of them a step uses is not known here, and a
-                // rule on the step would let a token's result depend on its batch. Rank 16, two layers, tokens of adapters in 64
-                // slots, clusters against the pair of kernels: 1 of 1 50 / 55 us, 8 of 8 60 / 76, 64 of 16 71 / 92, 64 of 32
-                // 101 / 114; only steps of more than 40 adapters are faster as pairs (64 of 48 147 / 137, 64 of 64 179 / 163).
+                // cluster kernel or pair whatever the number of slots: how many of them a step uses is not known here
                 for (auto& o : h->sites)  // (a model's layers are of a few shapes)
                     if (&o < &s && o.cols == s.cols && o.parts.size() == s.parts.size() && std::equal(o.part_rows, o.part_rows + PLORA_MAX_PARTS, s.part_rows)) {
                         s.plans = o.plans;

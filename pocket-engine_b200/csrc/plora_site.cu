@@ -583,14 +583,38 @@ cudaError_t plora_site_init() {
     return e;
 }
 
+// Whether the cluster kernel or the shrink / expand pair is the better one for a layer that the cluster kernel could run. It may
+// depend on the layer and the largest rank alone: a rule on the step would let a token's result depend on its batch.
+// Column groups make ever larger layers fit, but each group repeats the shrink, and 33 clusters run at a time: such layers are faster as
+// clusters in steps of few items and slower in steps of many. The line is drawn where a block's inputs of all parts' rows of A
+// (every 64 of them at least the eight warps' sums over them), eight tokens of x, its columns of B out of four groups and S leave
+// no room for two blocks per SM. Beyond it, four layers, clusters / pairs in us for 1, 8, 16 and 64 tokens of as many adapters and
+// 128 tokens of 8:
+//   4096 -> 2 x 12288, rank 32   25 / 35   39 / 51   65 / 63   205 / 139   87 / 74
+//   2048 -> 2 x 6144,  rank 48   25 / 35   37 / 50   62 / 61   193 / 133   77 / 70
+//   1024 -> 2 x 3072,  rank 64   26 / 33   38 / 40   60 / 49   183 /  98   77 / 51
+// Within it the most clusters lose is (3072 -> 3072, rank 64)  25 / 35   31 / 40   49 / 48   148 /  85   69 / 53,
+// and most layers gain throughout (4096 -> 4096, rank 16       23 / 32   25 / 35   25 / 40    52 /  63   41 / 44).
+bool clusters_pay(int K, int n_parts, int total, int max_rank) {
+    const int rows = n_parts * max_rank, kchunk = ((K + SITE_CLUSTER - 1) / SITE_CLUSTER + 7) & ~7;
+    const size_t pitch = (size_t)kchunk * 2 + (kchunk / 8 % 2 ? 32 : 16), in64 = std::min(rows, 64);
+    const size_t a = (std::max(in64 * pitch, in64 * SITE_WARPS * PLORA_WORK_TOKENS * 4) + 127) / 128 * 128 * (size_t)((rows + 63) / 64);
+    const size_t x = (SITE_TOK * pitch + 127) / 128 * 128;
+    const size_t share = (((size_t)total + 4 * SITE_CLUSTER - 1) / (4 * SITE_CLUSTER) + 1) / 2 * 2;
+    const size_t b = ((share + 32 * n_parts) * max_rank * 2 + 127) / 128 * 128;
+    const size_t s = (size_t)PLORA_WORK_TOKENS * rows * 4 + (size_t)4 * PLORA_WORK_TOKENS * (rows + 8) * 2;
+    return rows <= 256 && a + x + b + s <= 111 * 1024;
+}
+
 // Plans of the cluster kernel for one layer, by column groups per work item: those with which two blocks share an SM (one SM
-// cannot take a whole cluster of 8, and a B200 has room for only 15 clusters of 8 at one block per SM). Empty when
-// nothing fits: such a layer takes the shrink / expand pair, which is faster there (13 tokens of 8 adapters at rank 32,
-// four layers: 240 us with one block per SM, 150 as pairs).
+// cannot take a whole cluster of 8, and a B200 has room for only 15 clusters of 8 at one block per SM). Empty where nothing
+// fits (13 tokens of 8 adapters at rank 32, four layers: 240 us with one block per SM, 150 as pairs) or clusters do not pay: such
+// a layer takes the shrink / expand pair.
 std::vector<PloraSitePlan> plora_site_plans(int K, int n_parts, const int* part_rows, int max_rank) {
     std::vector<PloraSitePlan> out;
     int total = 0;
     for (int p = 0; p < n_parts; p++) total += part_rows[p];
+    if (!clusters_pay(K, n_parts, total, max_rank)) return out;
     for (int nsub : {1, 2, 3, 4, 6, 8, 12, 16}) {
         if (nsub > 4 && out.empty()) break;  // (as few clusters as that run at once, and every group reads x again)
         PloraSitePlan pl;

@@ -71,3 +71,18 @@ def test_bits_whatever_the_number_of_groups(pe, which, f32_out):
     for first, count in ((0, 1), (1, 1), (2, 1), (3, 1), (4, 7)):
         for got, all_rows in zip(run(first, count), together):
             assert np.array_equal(got, all_rows[first:first + count]), (first, count)
+
+
+# layers that the cluster kernel could run, in three or four column groups, and in which it is the slower one for steps of many items
+BEYOND = [(32, 4096, [("g", 12288), ("u", 12288)]), (48, 2048, [("g", 6144), ("u", 6144)]), (64, 1024, [("g", 3072), ("u", 3072)])]
+
+
+@pytest.mark.parametrize("rank,cols,mods", BEYOND, ids=lambda v: str(v) if isinstance(v, int) else "")
+def test_layers_beyond_the_line_run_as_pairs(pe, rank, cols, mods):
+    wl = workload(pe, [rank], [3], [1], [(cols, mods)])
+    got = []
+    for form in ("cluster", "early"):
+        loras = harness.product_registry(pe, wl)
+        got.append(harness.run_gpu(pe, loras, wl, True, meta="device", fused=form))
+        loras.close()
+    assert np.array_equal(got[0][0], got[1][0])
