@@ -110,10 +110,10 @@ __global__ void __launch_bounds__(256) plora_fp8_quant_rows_kernel(const bf16* _
     }
 }
 
-// The same, a warp per row of up to 256 P inputs, all of them on their way at once (P pieces of 8 per lane): for steps of more rows than the
-// kernel above runs at once. There a block's 8 KB are on their way for a third of its time and eight blocks share an SM, 64 KB;
-// here it is three times as much and nobody waits at a block's barrier. The maximum is taken over pairs of bf16. 16384 rows of 4096:
-// 53 -> 48 us.
+// The same, a warp per row of up to 256 P inputs, all of them on their way at once (P pieces of 8 per lane): for steps of many rows
+// (plora_launch_fp8_quant). In the kernel above a block's 8 KB are on their way for a third of its time and eight blocks share an SM, 64 KB;
+// here it is three times as much and nobody waits at a block's barrier. The maximum is taken over pairs of bf16. 16384 rows of 4096
+// inputs: 43.7 -> 39.8 us, 5.1 TB/s.
 template <int P>
 __global__ void __launch_bounds__(64, P > 16 ? 10 : 12) plora_fp8_quant_warp_kernel(const bf16* __restrict__ X, int rows, int ldx, int K, uint8_t* __restrict__ Xq,
                                                                   float* __restrict__ st) {
@@ -590,8 +590,6 @@ int fused_ring_bytes() {
 
 }  // namespace
 
-static int g_fp8_sms = 148;  // SMs of the device the kernels were set up for
-
 cudaError_t plora_fp8_init(int max_rank) {
     if (!g_encode) {
         void* fn = nullptr;
@@ -612,9 +610,6 @@ cudaError_t plora_fp8_init(int max_rank) {
     if (e0 == cudaSuccess) e0 = plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_quant_warp_kernel<8>), 0);
     if (e0 == cudaSuccess) e0 = plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_quant_warp_kernel<16>), 0);
     if (e0 == cudaSuccess) e0 = plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_quant_warp_kernel<20>), 0);
-    int dev = 0;
-    if (e0 == cudaSuccess) e0 = cudaGetDevice(&dev);
-    if (e0 == cudaSuccess) e0 = cudaDeviceGetAttribute(&g_fp8_sms, cudaDevAttrMultiProcessorCount, dev);
     if (e0 == cudaSuccess) e0 = plora_kernel_shared(reinterpret_cast<const void*>(plora_s_reduce_kernel), 0);
     if (e0 != cudaSuccess) return e0;
     cudaError_t e = plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_fused_kernel<false>), smem);
@@ -622,12 +617,18 @@ cudaError_t plora_fp8_init(int max_rank) {
     return plora_kernel_shared(reinterpret_cast<const void*>(plora_fp8_fused_kernel<true>), smem);
 }
 
-cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, bool pdl, cudaStream_t stream) {
+cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, int sms, bool pdl, cudaStream_t stream) {
     // two pieces of 8 inputs per thread where 256 threads are more than that needs, up to four beyond
     const int pieces = (K + 7) / 8, threads = std::min(256, std::max(32, (pieces / 2 + 31) / 32 * 32)), nv = (pieces + threads - 1) / threads;
-    // a warp per row where the rows are more than the blocks that run at once (eight on an SM), up to 5120 inputs
+    // A warp per row in steps of many rows: over 48 for every SM, six rounds of the kernel above. In fewer, its blocks of many threads
+    // are through their few rounds sooner. Not where the loads of a lane that are not there (9 to 14 pieces in the kernel of 16)
+    // cost what the others gain. us per call, block / warp, rows of 2048, 2560, 4096, 5120 inputs:
+    //   1600 rows   4.4 / 4.2   4.5 / 5.1   6.1 / 6.4   7.6 / 10.0
+    //   3200        5.8 / 5.5   7.1 / 8.4   10.6 / 10.8  13.0 / 13.4
+    //   8192        12.4 / 11.5  15.1 / 16.3  23.3 / 22.4  29.7 / 27.3
+    //   16384       22.7 / 20.3  27.6 / 28.3  43.7 / 39.8  57.0 / 49.5
     const int per = (pieces + 31) / 32;
-    if (per <= 20 && rows > 8 * g_fp8_sms) {
+    if ((per <= 8 || (per > 14 && per <= 20)) && rows > 48 * sms) {
         auto* fn = per <= 8 ? plora_fp8_quant_warp_kernel<8> : per <= 16 ? plora_fp8_quant_warp_kernel<16> : plora_fp8_quant_warp_kernel<20>;
         return launch_pdl(fn, dim3((unsigned)((rows + 1) / 2)), dim3(64), 0, stream, pdl, reinterpret_cast<const bf16*>(x), rows, ldx, K,
                           reinterpret_cast<uint8_t*>(xq), st);

@@ -1129,7 +1129,7 @@ int plora_fp8_quant_rows(plora_t* h, uint64_t x, int rows, int cols, uint64_t xq
     if (rows == 0) return PLORA_OK;
     // (waits for the kernel before it reads or releases anything: what follows may read launch records at once)
     CUK(h, "fp8 quantise", plora_launch_fp8_quant((const void*)(uintptr_t)x, rows, cols, cols, (void*)(uintptr_t)xq,
-                                                 (float*)(uintptr_t)st, next_launch(h, stream, true).pdl, as_stream(stream)));
+                                                 (float*)(uintptr_t)st, h->sm_count, next_launch(h, stream, true).pdl, as_stream(stream)));
     return PLORA_OK;
 }
 

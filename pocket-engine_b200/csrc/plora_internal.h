@@ -300,7 +300,7 @@ cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* rec
                               int* status, bool pdl, cudaStream_t st);
 cudaError_t plora_mma_init();
 cudaError_t plora_fp8_init(int max_rank);
-cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, bool pdl, cudaStream_t stream);
+cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void* xq, float* st, int sms, bool pdl, cudaStream_t stream);
 cudaError_t plora_launch_s_reduce(float* S, size_t s_stride_elems, int lds, int nsplit, const int32_t* segs,
                                   SegLayout lay, const plora_desc* table, int work_cap, int tile_cap, int tile_split,
                                   int K, bool pdl, cudaStream_t st);
