@@ -1049,7 +1049,8 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
     int work_cap = std::min(std::min(step->max_tiles, rows), h->max_slots + rows / PLORA_WORK_TOKENS);
     if (work_cap == 0) return PLORA_OK;
     const auto [pdl, late] = next_launch(h, stream, true);
-    const int release = h->site_release >= 0 && h->site_release <= 3 ? h->site_release : (h->early_x ? 0 : 3);
+    // (4, once A and x have landed: x goes straight into the shrink's registers, so the shrink's end is the first such point)
+    const int release = h->site_release == 4 ? 1 : h->site_release >= 0 && h->site_release <= 3 ? h->site_release : (h->early_x ? 0 : 3);
     CUK(h, "site kernel",
        plora_launch_site((const void*)(uintptr_t)x, site.cols, site.cols, recs_of(h, hook->site), h->rec_cap,
                          hook->site + 1 < (int)h->sites.size() ? recs_of(h, hook->site + 1) : nullptr,
