@@ -127,7 +127,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 
 // Programmatic dependent launch. Every kernel of the path waits for the kernels before it and only then
 // lets the next one start its prologue, so a prologue may read anything written two or more kernels back
-// (slabs, descriptors, the step's grouping) but nothing the kernel right before it writes.
+// (slabs, descriptors, the step's grouping) but nothing the kernel right before it writes. What that one writes is read after the
+// wait, and not by __ldg or through a const __restrict__ pointer: those say that nobody writes the memory while the kernel lives, and the
+// compiler may move such a load above the wait.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -64,12 +64,12 @@ __global__ void __launch_bounds__(256) plora_fp8_quant_rows_kernel(const bf16* _
 #pragma unroll
         for (int i = 0; i < (NV > 0 ? NV : 1); i++) {
             const int k = ((int)threadIdx.x + i * nt) * 8;
-            keep[i] = k < K ? *reinterpret_cast<const uint4*>(x + k) : make_uint4(0u, 0u, 0u, 0u);
+            keep[i] = k < K ? __ldcg(reinterpret_cast<const uint4*>(x + k)) : make_uint4(0u, 0u, 0u, 0u);
         }
 #pragma unroll
         for (int i = 0; i < (NV > 0 ? NV : 1); i++) scan(keep[i]);
     } else {
-        for (int k = threadIdx.x * 8; k < K; k += nt * 8) scan(*reinterpret_cast<const uint4*>(x + k));
+        for (int k = threadIdx.x * 8; k < K; k += nt * 8) scan(__ldcg(reinterpret_cast<const uint4*>(x + k)));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(256) plora_fp8_quant_rows_kernel(const bf16* _
         *reinterpret_cast<uint2*>(q + k) = make_uint2(w[0], w[1]);
     };
     if (!plain) {
-        for (int k = threadIdx.x * 8; k < K; k += nt * 8) put(*reinterpret_cast<const uint4*>(x + k), k, [&](float v) { return __fdiv_rn(v, s); });
+        for (int k = threadIdx.x * 8; k < K; k += nt * 8) put(__ldcg(reinterpret_cast<const uint4*>(x + k)), k, [&](float v) { return __fdiv_rn(v, s); });
         return;
     }
     auto quotient = [&](float v) {
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(256) plora_fp8_quant_rows_kernel(const bf16* _
             if (k < K) put(keep[i], k, quotient);
         }
     } else {
-        for (int k = threadIdx.x * 8; k < K; k += nt * 8) put(*reinterpret_cast<const uint4*>(x + k), k, quotient);
+        for (int k = threadIdx.x * 8; k < K; k += nt * 8) put(__ldcg(reinterpret_cast<const uint4*>(x + k)), k, quotient);
     }
 }
 
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(64, P > 16 ? 10 : 12) plora_fp8_quant_warp_ker
 #pragma unroll
     for (int i = 0; i < P; i++) {
         const int k = (i * 32 + lane) * 8;
-        v[i] = k < K ? *reinterpret_cast<const uint4*>(x + k) : make_uint4(0u, 0u, 0u, 0u);
+        v[i] = k < K ? __ldcg(reinterpret_cast<const uint4*>(x + k)) : make_uint4(0u, 0u, 0u, 0u);
     }
     __nv_bfloat162 most = __floats2bfloat162_rn(0.f, 0.f);
     auto scan = [&](uint32_t w) { most = __hmax2(most, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&w))); };
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(64, P > 16 ? 10 : 12) plora_fp8_quant_warp_ker
             });
     } else {
 #pragma unroll 1
-        for (int k = lane * 8; k < K; k += 256) put(*reinterpret_cast<const uint4*>(x + k), k, [&](float u) { return __fdiv_rn(u, s); });
+        for (int k = lane * 8; k < K; k += 256) put(__ldcg(reinterpret_cast<const uint4*>(x + k)), k, [&](float u) { return __fdiv_rn(u, s); });
     }
 }
 
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(224) plora_fp8_fused_kernel(const __grid_const
         tc_fence_after();
         const int q4 = warp & 3;  // this warp's quarter of the 128 tensor-memory lanes
         const int lrow = q4 * 32 + lane;
-        const float srow_scale = (m0 + lrow) < T ? st[m0 + lrow] : 0.f;
+        const float srow_scale = (m0 + lrow) < T ? __ldcg(st + m0 + lrow) : 0.f;
         if (ok) {
 #pragma unroll
             for (int cc = 0; cc < F8_BN; cc += 32) {

@@ -432,7 +432,7 @@ __global__ void __cluster_dims__(TWO ? 2 : 1, 1, 1) __launch_bounds__(64 + G_EPI
             const int row = m0 + (int)rank * G_BM + wq * 32 + lane;
             constexpr int CW = F32 ? 32 : 64;  // y columns per slot
             const int c0 = (ew >> 2) * HALF, groups = (ew >> 2 ? BN - HALF : HALF) / 32;
-            const float srow = KIND == 0 ? (row < T ? st[row] : 0.f) : 1.f;
+            const float srow = KIND == 0 ? (row < T ? __ldcg(st + row) : 0.f) : 1.f;
             const uint32_t lanes = tmem + ((uint32_t)(wq * 32) << 16) + (uint32_t)c0;
             const uint32_t base = lanes + (uint32_t)buf * BN, ad = lanes + ad_col(buf);
             constexpr int NW = F32 ? 32 : 16;  // words of 32 columns

@@ -161,7 +161,7 @@ __device__ __forceinline__ unsigned long long write_record(uint4* o, const int* 
 // writes what only later kernels read. Counts that are scanned together share one 64-bit scan. One block wrote the
 // records of all layers before: 9 us for a single token over 16 layers, 13 us for 64 tokens, 19-27 us for a prefill
 // step, against what bench.py reports as meta_us now.
-__global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __restrict__ tiles, int* __restrict__ segs,
+__global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* tiles, int* __restrict__ segs,
                                                                  SegLayout lay, int* __restrict__ status,
                                                                  const plora_desc* __restrict__ tables,
                                                                  const int* __restrict__ site_cols, int n_sites,
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* __res
     pdl_trigger();  // (the first kernel of the step waits for this grid before it reads a record)
     pdl_wait();
 
-    // the first tile words are fetched together with their count
+    // the first tile words are fetched together with their count (`tiles` is not __restrict__: its writer may run when this kernel begins)
     int w0 = 0, w1 = 0, w2 = 0;
     if (tid < cap) {
         w0 = tiles[1 + 3 * tid];

@@ -201,8 +201,8 @@ using Walk = std::integral_constant<RankWalk, W>;
 
 template <bool F32>
 __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THREADS, 2)
-    plora_site_gather_kernel(const bf16* __restrict__ X, int ldx, int K, const PloraRec* __restrict__ recs, int rec_cap,
-                             const PloraRec* __restrict__ next_recs, void* Y, int ldy, PloraSiteShape sh, int mode,
+    plora_site_gather_kernel(const bf16* __restrict__ X, int ldx, int K, const PloraRec* recs, int rec_cap,
+                             const PloraRec* next_recs, void* Y, int ldy, PloraSiteShape sh, int mode,
                              int* __restrict__ status PLORA_BOUNDS_PARAM) {
     extern __shared__ __align__(128) unsigned char dsm[];
     __shared__ __align__(8) uint64_t bars[3];  // A rows, B rows, the cluster's partials
@@ -261,7 +261,7 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
     const uint32_t a_lane = smem_u32(As) + (uint32_t)g * (uint32_t)sh.kb_pad + (uint32_t)warp * 64u + (uint32_t)t4 * 16u;
     for (int w = blockIdx.z; w < rec_cap; w += gridDim.z) {
         // ---- the one metadata fetch: the record's 208 live bytes into shared memory
-        if (tid < 13) reinterpret_cast<uint4*>(&srec)[tid] = __ldg(reinterpret_cast<const uint4*>(recs + w) + tid);
+        if (tid < 13) reinterpret_cast<uint4*>(&srec)[tid] = reinterpret_cast<const uint4*>(recs + w)[tid];
         __syncthreads();
         const int cnt = srec.cnt;
         if (cnt == 0) break;  // end of the list: the same decision in every block of the cluster
@@ -338,13 +338,13 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                 const PloraRec* nr = next_recs + w;
                 if (crank == 0 && lane < 2) prefetch_l2(reinterpret_cast<const unsigned char*>(nr) + 128 * lane);
                 if (mode & 16) {
-                    const int4 head = __ldg(reinterpret_cast<const int4*>(nr));  // cn, slot, rank, cols
+                    const int4 head = __ldcg(reinterpret_cast<const int4*>(nr));  // cn, slot, rank, cols
                     if (head.x > 0 && head.z > 0) {
-                        prefetch_eighth(__ldg(&nr->a), (uint64_t)head.z * (uint64_t)head.w * 2u, crank, lane);
+                        prefetch_eighth(__ldcg(&nr->a), (uint64_t)head.z * (uint64_t)head.w * 2u, crank, lane);
 #pragma unroll 1
                         for (int p = 0; p < PLORA_MAX_PARTS; p++) {
-                            const int rp = __ldg(&nr->r[p]);
-                            if (rp > 0) prefetch_eighth(__ldg(&nr->b[p]), (uint64_t)__ldg(&nr->rows[p]) * (uint64_t)rp * 2u, crank, lane);
+                            const int rp = __ldcg(&nr->r[p]);
+                            if (rp > 0) prefetch_eighth(__ldcg(&nr->b[p]), (uint64_t)__ldcg(&nr->rows[p]) * (uint64_t)rp * 2u, crank, lane);
                         }
                     }
                 }
