@@ -322,7 +322,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
     h->seg.max_tokens = max_tokens;
     h->seg.cap_tiles = h->cap_tiles;
     h->seg.run_min = 1 << 30;  // every run takes the gather path unless the tile path can run (set below)
-    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > 201 * 1024) {
+    if (max_slots > 1023 || h->max_rank > 512 || plora_meta_group_smem(h->seg) > PLORA_GROUP_SMEM_MAX) {
         delete h;
         return fail(nullptr, PLORA_ERR_CAPACITY,
                     "limits: max_slots <= 1023, max_rank <= 512, and max_tokens/16 + max_seqs tiles must fit the "
@@ -376,7 +376,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             if (rc == PLORA_OK) check("zero unit counts", cudaMemset(h->prefix, 0, prefix_bytes));
             if (rc == PLORA_OK) check("zero launch records", cudaMemset(h->recs, 0, rec_bytes));
             check("alloc status", cudaMalloc((void**)&h->status, 64));
-            check("kernel attributes", plora_kernels_init(h->seg));
+            check("kernel attributes", plora_kernels_init());
             if (rc == PLORA_OK && h->max_rank <= 128) h->mma_ok = plora_mma_init() == cudaSuccess;
             if (rc == PLORA_OK) h->site_ok = plora_site_init() == cudaSuccess;
             std::vector<int32_t> info;

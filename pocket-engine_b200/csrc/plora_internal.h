@@ -276,6 +276,7 @@ __host__ __device__ inline int plora_tile_chunks(int K, int R) {
 // ---- kernel launchers (plora_kernels.cu); each returns a cudaError_t from the launch ----
 cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, int n_seqs, int32_t* tiles,
                                     int cap_tiles, int* status, cudaStream_t st);
+#define PLORA_GROUP_SMEM_MAX (201 * 1024)  // shared memory that the grouping kernel may take: the limit of a handle's slots and tiles
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
 // site_info: per layer {input width, 0,
 // K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item
@@ -292,7 +293,7 @@ inline cudaError_t plora_kernel_shared(const void* fn, int max_dynamic_bytes) {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
     return e;
 }
-cudaError_t plora_kernels_init(const SegLayout& lay);
+cudaError_t plora_kernels_init();
 cudaError_t plora_site_init();
 std::vector<PloraSitePlan> plora_site_plans(int K, int n_parts, const int* part_rows, int max_rank);
 cudaError_t plora_launch_site(const void* x, int ldx, int K, const PloraRec* recs, int rec_cap, const PloraRec* next_recs,

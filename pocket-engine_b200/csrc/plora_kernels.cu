@@ -1238,12 +1238,11 @@ size_t plora_meta_group_smem(const SegLayout& lay) {
 // the launch path, so launches stay legal inside a stream capture.
 static int g_sms = 148;  // SMs of the device the kernels were set up for
 
-cudaError_t plora_kernels_init(const SegLayout& lay) {
+cudaError_t plora_kernels_init() {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&g_sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(plora_meta_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)plora_meta_group_smem(lay) > 48 * 1024 ? (int)plora_meta_group_smem(lay)
-                                                                                       : 48 * 1024);
+    // (the limit belongs to the kernel, not to a handle: the most that any handle may need)
+    cudaError_t e = cudaFuncSetAttribute(plora_meta_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PLORA_GROUP_SMEM_MAX);
     if (e != cudaSuccess) return e;
     // The few-token kernels overlap with their neighbours in the stream (programmatic dependent launch), and an SM's
     // split between L1 and shared memory is fixed while any block runs on it: all of them ask for the largest
