@@ -248,7 +248,9 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
         }
     }
     uint32_t ph_a = 0, ph_b = 0, ph_s = 0;  // barrier phases (each flips only when its barrier was used)
-    bool alive = true;                      // false once a bounded wait ran out: keep meeting the cluster, do no more work
+    // false once a bounded wait ran out: the block goes on meeting the cluster and waiting for what is still on its way into its shared
+    // memory (copies of its own, the other blocks' partials), which must not arrive after it has left, and does no more work
+    bool alive = true;
     const int k0 = (int)crank * sh.kchunk;
     const int klen = max(0, min(sh.kchunk, K - k0));
     const uint32_t kbytes = (uint32_t)klen * 2u;
@@ -361,7 +363,7 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
             const unsigned char* yahead = reinterpret_cast<const unsigned char*>(Y) + ((size_t)(ahead ? tok[qtok] : 0) * ldy + first.ycol + qcol) * esize;
             const bool ahead0 = ahead && qcol < first.ncols, ahead1 = ahead && qcol + SITE_WARPS * 32 < first.ncols;
             if (klen > 0 && t0 == 0) {
-                if (alive) alive = mbar_wait(&bars[0], ph_a, status);
+                alive = mbar_wait(&bars[0], ph_a, status) && alive;
                 ph_a ^= 1;
             }
             if (!waited && !early_x) {
@@ -442,10 +444,10 @@ __global__ void __cluster_dims__(SITE_CLUSTER, 1, 1) __launch_bounds__(SITE_THRE
                 st_async_peer(Rs + (size_t)(crank * SITE_TOK + t) * sh.rc + j, v, &bars[2], (uint32_t)(i & 7));
             }
             if (nseg > 0 && t0 == 0) {  // (a later pass finds the rows of B in place)
-                if (alive) alive = mbar_wait(&bars[1], ph_b, status);
+                alive = mbar_wait(&bars[1], ph_b, status) && alive;
                 ph_b ^= 1;
             }
-            if (alive) alive = mbar_wait_cluster(&bars[2], ph_s, status);
+            alive = mbar_wait_cluster(&bars[2], ph_s, status) && alive;
             ph_s ^= 1;
             // added in block order, as three bf16 terms whose sum is the f32 value
             for (int i = tid; i < 2 * cn * nq; i += SITE_THREADS) {
