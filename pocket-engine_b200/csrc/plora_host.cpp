@@ -370,7 +370,7 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
             h->rec_cap = std::min(h->cap_tiles, max_slots + max_tokens / PLORA_WORK_TOKENS) + 1;
             const size_t rec_bytes = sizeof(PloraRec) * h->sites.size() * (size_t)h->rec_cap;
             check("alloc launch records", cudaMalloc((void**)&h->recs, rec_bytes));
-            check("alloc layer widths", cudaMalloc((void**)&h->site_cols, 4 * h->sites.size() * sizeof(int32_t)));
+            check("alloc layer widths", cudaMalloc((void**)&h->site_cols, 3 * h->sites.size() * sizeof(int32_t)));
             const size_t prefix_bytes = h->sites.size() * (size_t)unit_words(h->rec_cap) * sizeof(int32_t);
             check("alloc unit counts", cudaMalloc((void**)&h->prefix, prefix_bytes));
             if (rc == PLORA_OK) check("zero unit counts", cudaMemset(h->prefix, 0, prefix_bytes));
@@ -391,7 +391,6 @@ int plora_create(const plora_site* sites, int n_sites, int base_gguf, int key_he
                         break;
                     }
                 info.push_back(s.cols);
-                info.push_back(0);
                 info.push_back(s.nsplit);
                 info.push_back(s.exp_most);
             }

@@ -63,7 +63,7 @@ struct alignas(256) PloraRec {
     uint64_t a;
     uint64_t b[PLORA_MAX_PARTS];
     int32_t r[PLORA_MAX_PARTS], r_off[PLORA_MAX_PARTS], off[PLORA_MAX_PARTS], rows[PLORA_MAX_PARTS];
-    int32_t ntot, pad1;  // output columns over the targeted parts
+    int32_t ntot, pad1;  // output columns over the targeted parts (the token rows start at a piece of 16 bytes)
     int32_t tok[PLORA_WORK_TOKENS];
     int32_t cat[PLORA_MAX_PARTS];  // where each targeted part starts when the targeted parts are laid end to end
     int32_t pad2[12];
@@ -195,7 +195,7 @@ struct plora {
     int rec_cap = 0;
     int32_t* prefix = nullptr;  // device: [sites][unit_words(rec_cap)] units of the gather kernels before every work item of the step
     int32_t* host_meta = nullptr;  // pinned staging for plora_meta_upload
-    int32_t* site_cols = nullptr;  // device: per layer {input width, 0, K-splits, most units of a column} (for the launch records)
+    int32_t* site_cols = nullptr;  // device: per layer {input width, K-splits, most units of a column} (for the launch records)
     int cap_tiles = 0;
     SegLayout seg;
     int* status = nullptr;  // device status word
@@ -278,8 +278,8 @@ cudaError_t plora_launch_meta_tiles(const int32_t* cu, const int32_t* seq_slot, 
                                     int cap_tiles, int* status, cudaStream_t st);
 #define PLORA_GROUP_SMEM_MAX (201 * 1024)  // shared memory that the grouping kernel may take: the limit of a handle's slots and tiles
 // Groups the step's tiles by slot and writes the launch records of every layer (recs may be null: grouping only).
-// site_info: per layer {input width, 0,
-// K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the unit counts of the gather shrink and expand before every item
+// site_info: per layer {input width, K-splits of the gather shrink, most units of a column in the gather expand}; prefix: per layer the
+// unit counts of the gather shrink and expand before every item
 cudaError_t plora_launch_meta_group(const int32_t* tiles, int32_t* segs, SegLayout lay, int* status, const plora_desc* tables,
                                     const int32_t* site_info, int n_sites, PloraRec* recs, int rec_cap, int* prefix, bool pdl,
                                     cudaStream_t st);

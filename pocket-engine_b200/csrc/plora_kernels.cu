@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* tiles
     if (recs != nullptr) {
         const int nw = min(n_work, rec_cap - 1), end = min(rec_cap, nw + PLORA_REC_TERM);
         for (int site = blockIdx.x; site < n_sites; site += gridDim.x) {
-            const int4 info = reinterpret_cast<const int4*>(site_cols)[site];
+            const int cols = site_cols[3 * site], nsplit = site_cols[3 * site + 1], most = site_cols[3 * site + 2];
             int* ps = prefix + (size_t)site * (size_t)unit_words(rec_cap);
             long long* pe = reinterpret_cast<long long*>(ps + unit_expand(rec_cap));
             unsigned long long before = 0;
@@ -412,8 +412,8 @@ __global__ void __launch_bounds__(1024) plora_meta_group_kernel(const int* tiles
                 unsigned long long units = 0, total = 0;
                 if (w < end) {
                     uint4* o = reinterpret_cast<uint4*>(recs + (size_t)site * (size_t)rec_cap + w);
-                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)info.x);
-                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, info.x, info.z, info.w);
+                    if (w >= nw) o[0] = make_uint4(0u, 0u, 0u, (uint32_t)cols);
+                    else units = write_record(o, segs, lay, tables + (size_t)site * (size_t)S1, w, cols, nsplit, most);
                 }
                 if (w == 0) first_item = (int)packed_expand(units);
                 const unsigned long long at = before + block_scan_excl(units, total, sh[(base >> 10) & 1]);
