@@ -262,8 +262,9 @@ cudaError_t plora_launch_xchg_all_ranks(const PloraXchgCtx* ctxs_dev, int world,
 // planes tree-summed by the reader) and every such choice gives the same bits. At most the 512 accumulator
 // columns of an SM for all of a tile's chunks (where they go to several blocks, each holds its own only), and at least 8 steps of
 // 64 inputs per chunk. With 256 of them, ranges of K were twice as long at total ranks over 32: 1,545 ragged tokens of ranks 16 to
-// 64 275 us a step, 261 so; 512 mixed tokens of rank 32 172 and 167; eight prompts of 2048 tokens, whose tiles are one
-// block each, 760 and 761.
+// 64 277 us a step, 262 so; 512 mixed tokens of rank 32 176 and 169; eight prompts of 2048 tokens, whose tiles are one
+// block each, 765 and 768. Slower so: steps of two to three dozen runs of 64 to 80 tokens at total ranks over 128 (30 of 64, rank 64: 9 %),
+// which have twice the tiles that their rows let the host expect, and whose blocks then take two rounds.
 #define PLORA_TILE_SPLIT_MAX 8
 __host__ __device__ inline int plora_tile_cols(int R) { return R <= 32 ? 32 : R <= 64 ? 64 : R <= 128 ? 128 : R <= 256 ? 256 : 512; }
 __host__ __device__ inline int plora_tile_chunks(int K, int R) {

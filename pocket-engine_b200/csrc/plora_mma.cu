@@ -548,7 +548,7 @@ __device__ __forceinline__ void pair_sync(int quarter) {
 }
 __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
 
-template <bool F32>
+template <bool F32, bool HIGH>
 __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kernel(const float* __restrict__ S, size_t s_stride, int lds, int K,
                                                                 int ksplit, const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table,
@@ -688,73 +688,98 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             // up the planes and leaves the sums in shared memory; there every lane finds its own row, split into a bf16 high part (the
             // first warp) and the bf16 of what is left (the second), and puts it into its lane of tensor memory. With a row
             // per lane from the start, each load touched 32 lines of L1 for 16 bytes each: 7,500 to 16,000 cycles to here, now
-            // 4,000 to 8,000 (512 mixed tokens: 186 -> 172 us a step; eight prompts of 2048: 784 -> 760).
+            // 4,000 to 8,000 (one prompt of 199 tokens: 157 -> 133 us a step, 512 mixed tokens 194 -> 167, eight prompts of 2048 792 -> 765).
+            // HIGH (registries of ranks over 64): where S is one plane, 64 ranks at a time through both buffers, where it is two, both planes at
+            // once. With one way to L2 per 32 ranks, one run of 64 tokens of rank 128 over four layers of 1024 inputs took 93 us (88 with a row
+            // per lane), 88 so; four prompts of 2048 tokens of rank 128 562 -> 546. Not for the others: the longer code costs more at a
+            // block's start than it gives (the prompt of 199 tokens of rank 16: 133 -> 139).
             {
                 const int s_eff = min(ksplit, plora_tile_chunks(K, rank));  // planes the shrink wrote for this slot
                 const float* sq = S + (size_t)(start + wrow0) * lds + r_off;
+                auto buffer = [&](int k) { return dsm1k + (size_t)((wq + (k & 32 ? 4 : 0)) * nst + nst - 1) * EXP_SLOT_BYTES; };
 #pragma unroll 1
-                for (int k0 = 0; k0 < r; k0 += 32) {
-                    unsigned char* buf = dsm1k + (size_t)((wq + (k0 & 32 ? 4 : 0)) * nst + nst - 1) * EXP_SLOT_BYTES;
-                    const int lpr = r - k0 >= 32 ? 8 : 4, rpi = 32 / lpr;  // lanes of a row, rows of an instruction
-                    const int row0 = 16 * wh + lane / lpr, piece = lane % lpr;
-                    auto fetch = [&](auto count, int i0) {  // `count` instructions' rows from the i0-th on, all of them on their way together
-                        constexpr int N = decltype(count)::value;
-                        float4 sum[N];
-                        const float* from[N];
+                for (int k0 = 0; k0 < r;) {
+                    const bool wide = HIGH && s_eff == 1 && r - k0 >= 64;
+                    const int ls = r - k0 >= 32 ? 3 : 2, rpi = 32 >> ls;  // 1 << ls lanes of a row, rows of an instruction
+                    const int row0 = 16 * wh + (lane >> ls), piece = lane & ((1 << ls) - 1);
+                    // G groups of 32 ranks, U planes and N instructions' rows from the i0-th on, all of them on their way together
+                    auto fetch = [&](auto g_, auto u_, auto n_, int i0) {
+                        constexpr int G = decltype(g_)::value, U = decltype(u_)::value, N = decltype(n_)::value;
+                        float4 sum[G][N];
+                        const float* from = sq + (size_t)(row0 + i0 * rpi) * lds + k0 + 4 * piece;
+                        for (int s0 = 0; s0 < (U == 4 ? s_eff : U); s0 += U) {  // (U = 1, 2: as many planes as there are)
+                            float4 v[U][G][N];
 #pragma unroll
-                        for (int i = 0; i < N; i++) from[i] = sq + (size_t)(row0 + (i0 + i) * rpi) * lds + k0 + 4 * piece;
-                        for (int s0 = 0; s0 < s_eff; s0 += 4) {
-                            float4 v[N == 4 ? 1 : 4][N];
+                            for (int u = 0; u < U; u++)
 #pragma unroll
-                            for (int u = 0; u < (N == 4 ? 1 : 4); u++)
+                                for (int i = 0; i < N; i++)
 #pragma unroll
-                                for (int i = 0; i < N; i++) {
-                                    v[u][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-                                    if (s0 + u < s_eff && wrow0 + row0 + (i0 + i) * rpi < len)
-                                        v[u][i] = __ldcg(reinterpret_cast<const float4*>(from[i] + (size_t)(s0 + u) * s_stride));
+                                    for (int j = 0; j < G; j++) {
+                                        v[u][j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+                                        if ((U < 4 || s0 + u < s_eff) && wrow0 + row0 + (i0 + i) * rpi < len)
+                                            v[u][j][i] = __ldcg(reinterpret_cast<const float4*>(from + (size_t)(s0 + u) * s_stride + i * rpi * lds + 32 * j));
+                                    }
+#pragma unroll
+                            for (int j = 0; j < G; j++)
+#pragma unroll
+                                for (int i = 0; i < N; i++) {  // a balanced tree over the 1, 2, 4 or 8 planes
+                                    float4 t = v[0][j][i];
+                                    if (U > 1) t = add4(t, v[U > 1 ? 1 : 0][j][i]);
+                                    if (U > 2 && (HIGH || s_eff > 2)) t = add4(t, add4(v[U > 2 ? 2 : 0][j][i], v[U > 2 ? 3 : 0][j][i]));
+                                    sum[j][i] = s0 == 0 ? t : add4(sum[j][i], t);
                                 }
-#pragma unroll
-                            for (int i = 0; i < N; i++) {  // a balanced tree over the 1, 2, 4 or 8 planes
-                                float4 t = v[0][i];
-                                if (N != 4) {
-                                    t = add4(t, v[N == 4 ? 0 : 1][i]);
-                                    if (s_eff > 2) t = add4(t, add4(v[N == 4 ? 0 : 2][i], v[N == 4 ? 0 : 3][i]));
-                                }
-                                sum[i] = s0 == 0 ? t : add4(sum[i], t);
-                            }
                         }
 #pragma unroll
-                        for (int i = 0; i < N; i++) {
-                            const int row = row0 + (i0 + i) * rpi;
-                            if (row < 16 * wh + 16) *reinterpret_cast<float4*>(buf + row * 128 + ((piece ^ (row & 7)) << 4)) = sum[i];
+                        for (int j = 0; j < G; j++)
+#pragma unroll
+                            for (int i = 0; i < N; i++) {
+                                const int row = row0 + (i0 + i) * rpi;
+                                if (row < 16 * wh + 16) *reinterpret_cast<float4*>(buffer(k0 + 32 * j) + row * 128 + ((piece ^ (row & 7)) << 4)) = sum[j][i];
+                            }
+                    };
+                    const std::integral_constant<int, 1> one;
+                    const std::integral_constant<int, 2> two;
+                    const std::integral_constant<int, 4> four;
+                    if constexpr (HIGH) {
+                        if (wide) fetch(two, one, four, 0);
+                        else if (s_eff == 2) fetch(one, two, four, 0);
+                    }
+                    if (s_eff == 1 && !wide) {
+                        fetch(one, one, four, 0);
+                    } else if (s_eff > (HIGH ? 2 : 1)) {
+                        fetch(one, four, two, 0);
+                        if (ls == 3) fetch(one, four, two, 2);
+                    }
+                    pair_sync(wq);
+                    auto put = [&](int k) {
+                        const unsigned char* buf = buffer(k);
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            if (k + 16 * h < r) {
+                                uint32_t w[8];
+#pragma unroll
+                                for (int c = 0; c < 4; c++) {
+                                    const float4 f = *reinterpret_cast<const float4*>(buf + lane * 128 + (((4 * h + c) ^ (lane & 7)) << 4));
+                                    __nv_bfloat162 a = __floats2bfloat162_rn(f.x, f.y), b = __floats2bfloat162_rn(f.z, f.w);
+                                    if (wh == 1) {
+                                        const float2 af = __bfloat1622float2(a), bf = __bfloat1622float2(b);
+                                        a = __floats2bfloat162_rn(f.x - af.x, f.y - af.y);
+                                        b = __floats2bfloat162_rn(f.z - bf.x, f.w - bf.y);
+                                    }
+                                    w[2 * c] = *reinterpret_cast<const uint32_t*>(&a);
+                                    w[2 * c + 1] = *reinterpret_cast<const uint32_t*>(&b);
+                                }
+                                __syncwarp();
+                                tmem_st8(lane_base + EXP_TMEM_A + (wh == 1 ? (uint32_t)(r >> 1) : 0u) + (uint32_t)((k + 16 * h) >> 1), w);
+                            }
                         }
                     };
-                    if (s_eff == 1) {
-                        fetch(std::integral_constant<int, 4>(), 0);
-                    } else {
-                        fetch(std::integral_constant<int, 2>(), 0);
-                        if (lpr == 8) fetch(std::integral_constant<int, 2>(), 2);
-                    }
-                    pair_sync(wq);  // (the buffer of the ranks before stays: the next ones go to the other warp's slot)
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        if (k0 + 16 * h < r) {
-                            uint32_t w[8];
-#pragma unroll
-                            for (int c = 0; c < 4; c++) {
-                                const float4 f = *reinterpret_cast<const float4*>(buf + lane * 128 + (((4 * h + c) ^ (lane & 7)) << 4));
-                                __nv_bfloat162 a = __floats2bfloat162_rn(f.x, f.y), b = __floats2bfloat162_rn(f.z, f.w);
-                                if (wh == 1) {
-                                    const float2 af = __bfloat1622float2(a), bf = __bfloat1622float2(b);
-                                    a = __floats2bfloat162_rn(f.x - af.x, f.y - af.y);
-                                    b = __floats2bfloat162_rn(f.z - bf.x, f.w - bf.y);
-                                }
-                                w[2 * c] = *reinterpret_cast<const uint32_t*>(&a);
-                                w[2 * c + 1] = *reinterpret_cast<const uint32_t*>(&b);
-                            }
-                            __syncwarp();
-                            tmem_st8(lane_base + EXP_TMEM_A + (wh == 1 ? (uint32_t)(r >> 1) : 0u) + (uint32_t)((k0 + 16 * h) >> 1), w);
-                        }
+                    put(k0);  // (the buffer of the ranks before stays: the next ones go to the other warp's slot)
+                    k0 += 32;
+                    if (wide) {
+                        put(k0);
+                        k0 += 32;
+                        if (k0 < r) pair_sync(wq);  // both buffers have been read
                     }
                 }
                 tmem_st_wait();
@@ -906,8 +931,10 @@ cudaError_t plora_mma_init() {
     if (e != cudaSuccess) return e;
     e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_mma_kernel<true>), 172 * 1024);
     if (e != cudaSuccess) return e;
-    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false>), EXP_TMA_SMEM))) return e;
-    return plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true>), EXP_TMA_SMEM);
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false, false>), EXP_TMA_SMEM))) return e;
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true, false>), EXP_TMA_SMEM))) return e;
+    if ((e = plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<false, true>), EXP_TMA_SMEM))) return e;
+    return plora_kernel_shared(reinterpret_cast<const void*>(plora_expand_tma_kernel<true, true>), EXP_TMA_SMEM);
 }
 
 namespace {
@@ -1034,7 +1061,9 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
             const int nb_per_cta = per_cta(EXP_BN, 32);
             const dim3 grid((unsigned)(((max_rows + EXP_BN - 1) / EXP_BN + nb_per_cta - 1) / nb_per_cta), (unsigned)parts,
                             (unsigned)std::min(tile_cap, (rows_total + MMA_M - 1) / MMA_M + 4));
-            return launch_pdl(f32_out ? plora_expand_tma_kernel<true> : plora_expand_tma_kernel<false>, grid, dim3(32 * (EXP_WARPS + 1)),
+            auto* fn = max_rank > 64 ? (f32_out ? plora_expand_tma_kernel<true, true> : plora_expand_tma_kernel<false, true>)
+                                     : (f32_out ? plora_expand_tma_kernel<true, false> : plora_expand_tma_kernel<false, false>);
+            return launch_pdl(fn, grid, dim3(32 * (EXP_WARPS + 1)),
                               smem_tma, st, pdl, S, s_stride_elems, lds, K, tile_split, segs, lay, table, smaps, maps, y, ldy,
                               nb_per_cta, b_bytes, nbs, nst, late && pdl ? 1 : 0, status);
         }

@@ -14,6 +14,8 @@ CASES = [
     ("one-column-block", [64], [80], 64, [("a", 8)]),
     # total ranks of 384 and 144 whose rows of A go to several blocks, the last of which has 16; and too many tiles for that
     ("rank-groups", [300, 70], [128, 48], 1032, [("a", 64), ("b", 40), ("c", 8)]),
+    # registries with ranks over 64 stage S in another form: four planes of a rank of 96, eight of a rank of 16 (one and two planes above)
+    ("planes-of-high-ranks", [200, 90], [96, 16], 4096, [("a", 72)]),
     ("rank-groups-no-room", [128] * 60, [96, 16], 520, [("a", 64), ("b", 40)]),
 ]
 
