@@ -1,8 +1,7 @@
 """The cluster kernel of plora_apply over its column groups: steps of few work items take more of them (each loads and multiplies
 only the rows of A of the parts its columns meet), with the same bits as in a step of many; ranks that its expand walks 16
 and 32 at a time; one to nine tokens of an adapter (groups of four, passes of eight); inputs that end inside a block's share,
-inside a step of 32 and inside a warp's round; shares of columns that are no multiple of a step, and parts whose widths are no
-multiples of 8, where rows of y move in pairs of columns and which shares end in one depends on the number of groups."""
+inside a step of 32 and inside a warp's round; shares of columns that are no multiple of a step."""
 import numpy as np
 import pytest
 
@@ -17,18 +16,11 @@ SITES = [
     (17416, [("d", 264)]),                        # more than eight steps of 32 inputs for a warp
     (8, [("t", 40)]),
 ]
-UNEVEN = [
-    (4096, [("a", 4100)]),                        # one to three groups, each of them with an odd last share
-    (2048, [("a", 1030), ("b", 2050)]),
-    (1024, [("g", 6148), ("u", 6148)]),           # the second part's rows of y start at a multiple of 4
-    (5120, [("q", 2054), ("k", 1030), ("v", 518)]),
-]
-SETS = {"whole": SITES, "uneven": UNEVEN}
 
 
-def workload(pe, ranks, rows, slots, which=SITES):
+def workload(pe, ranks, rows, slots):
     from pocket_engine_b200 import workloads
-    sites = [pe.Site.fused(i, cols, mods) for i, (cols, mods) in enumerate(which)]
+    sites = [pe.Site.fused(i, cols, mods) for i, (cols, mods) in enumerate(SITES)]
     return workloads.Workload("groups", sites, ranks, 1.0, rows, slots, 41)
 
 
@@ -42,25 +34,15 @@ def test_groups(pe, ranks, f32_out):
 
 
 @pytest.mark.parametrize("f32_out", [True, False])
-@pytest.mark.parametrize("ranks", [[32, 16], [48]], ids=str)
-def test_uneven_widths(pe, ranks, f32_out):
-    for n in (1, 3, 5, 9):
-        rows = [n] + [1] * (len(ranks) - 1)
-        wl = workload(pe, ranks, rows, [1 + i for i in range(len(rows))], UNEVEN)
-        harness.run_and_check(pe, wl, f32_out=f32_out, meta="device", fused="cluster")
-
-
-@pytest.mark.parametrize("f32_out", [True, False])
-@pytest.mark.parametrize("which", sorted(SETS))
-def test_bits_whatever_the_number_of_groups(pe, which, f32_out):
+def test_bits_whatever_the_number_of_groups(pe, f32_out):
     ranks = [16, 16, 32, 8]
     rows, slots = [1] * 40, [1 + i % 4 for i in range(40)]
-    wl = workload(pe, ranks, rows, slots, SETS[which])
-    n = len(SETS[which])
+    wl = workload(pe, ranks, rows, slots)
+    n = len(SITES)
     xs, ys = [wl.x_bits(i) for i in range(n)], [wl.y_base(i) for i in range(n)]
 
     def run(first, count):
-        w = workload(pe, ranks, rows[first:first + count], slots[first:first + count], SETS[which])
+        w = workload(pe, ranks, rows[first:first + count], slots[first:first + count])
         loras = harness.product_registry(pe, w)
         got = harness.run_gpu(pe, loras, w, f32_out, meta="device", fused="cluster", xs=[x[first:first + count] for x in xs],
                               y_base=[y[first:first + count] for y in ys])
@@ -71,18 +53,3 @@ def test_bits_whatever_the_number_of_groups(pe, which, f32_out):
     for first, count in ((0, 1), (1, 1), (2, 1), (3, 1), (4, 7)):
         for got, all_rows in zip(run(first, count), together):
             assert np.array_equal(got, all_rows[first:first + count]), (first, count)
-
-
-# layers that the cluster kernel could run, in three or four column groups, and in which it is the slower one for steps of many items
-BEYOND = [(32, 4096, [("g", 12288), ("u", 12288)]), (48, 2048, [("g", 6144), ("u", 6144)]), (64, 1024, [("g", 3072), ("u", 3072)])]
-
-
-@pytest.mark.parametrize("rank,cols,mods", BEYOND, ids=lambda v: str(v) if isinstance(v, int) else "")
-def test_layers_beyond_the_line_run_as_pairs(pe, rank, cols, mods):
-    wl = workload(pe, [rank], [3], [1], [(cols, mods)])
-    got = []
-    for form in ("cluster", "early"):
-        loras = harness.product_registry(pe, wl)
-        got.append(harness.run_gpu(pe, loras, wl, True, meta="device", fused=form))
-        loras.close()
-    assert np.array_equal(got[0][0], got[1][0])

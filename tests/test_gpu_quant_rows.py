@@ -1,6 +1,5 @@
-"""Row quantisation of so many rows that a warp takes each (widths up to 2048 and from 3592 to 5120; a block each beyond and between): every
-number of pieces a lane may hold, rows that end inside a lane's pieces, an odd number of rows, rows at the edge of the f32 range, all
-zeros, infinities and no numbers."""
+"""Row quantisation of more rows than run as blocks at once, a warp per row: every number of pieces a lane may hold, rows that end inside
+a lane's pieces, an odd number of rows, rows at the edge of the f32 range, all zeros, infinities and no numbers."""
 import numpy as np
 import pytest
 
@@ -9,10 +8,10 @@ import harness
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cols", [8, 264, 2048, 2056, 3592, 4096, 4104, 5120, 5128])
+@pytest.mark.parametrize("cols", [8, 264, 2048, 2056, 4096, 4104, 5120, 5128])
 def test_many_rows(pe, oracle, cols):
     import torch
-    n = 48 * torch.cuda.get_device_properties(0).multi_processor_count + 3
+    n = 1187
     rng = np.random.default_rng(cols)
     scale = np.array([1, 1e-3, 30, 1e-36, 3e38, 0, 1e-19], np.float32)[np.arange(n) % 7][:, None]
     x = np.clip(rng.standard_normal((n, cols), dtype=np.float32), -1, 1) * scale
