@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(128) plora_s_reduce_kernel(float* __restrict__
         if (tile >= segs[SEG_N_MMA]) return pdl_exit_idle();
         const int* mt = segs + lay.mma() + 3 * tile;
         const int start = mt[0], len = mt[1], rank = table[mt[2]].rank;
-        const int s_eff = rank ? min(tile_split, plora_tile_chunks(K, rank)) : 1;
+        const int s_eff = rank ? plora_tile_blocks(tile_split & (PLORA_TILE_RSPLIT - 1), tile_split / PLORA_TILE_FIT, segs[SEG_N_MMA], K, rank) : 1;
         if (s_eff <= 1) return pdl_exit_idle();
         pdl_wait();
         pdl_trigger();
@@ -641,7 +641,7 @@ cudaError_t plora_launch_fp8_quant(const void* x, int rows, int ldx, int K, void
 cudaError_t plora_launch_s_reduce(float* S, size_t s_stride_elems, int lds, int nsplit, const int32_t* segs,
                                   SegLayout lay, const plora_desc* table, int work_cap, int tile_cap, int tile_split,
                                   int K, bool pdl, cudaStream_t st) {
-    if (tile_split <= 1) tile_cap = 0;
+    if ((tile_split & (PLORA_TILE_RSPLIT - 1)) <= 1) tile_cap = 0;
     if (nsplit <= 1 && tile_cap == 0) return cudaSuccess;
     if (work_cap + tile_cap == 0) return cudaSuccess;
     return launch_pdl(plora_s_reduce_kernel, dim3((unsigned)(work_cap + tile_cap)), dim3(128), 0, st, pdl, S, s_stride_elems,

@@ -941,13 +941,19 @@ static bool has_tiles(const plora_t* h, const plora_step* step, int rows) {
 }
 
 // How many blocks share the K chunks of one tensor-core tile: enough to fill the SMs when a step has few
-// tiles (prompt chunks inside a decode batch), one when there are plenty. Any value gives the same bits.
-static int tile_split(const plora_t* h, int rows) {
-    if (h->tile_split_force) return h->tile_split_force;
-    const int est = std::max(1, rows / PLORA_MMA_TOKENS);
-    int s = 1;
-    while (s < PLORA_TILE_SPLIT_MAX && 2 * s * est <= h->sm_count) s <<= 1;
-    return s;
+// tiles (prompt chunks inside a decode batch), one when there are plenty; whether the rows of A go to several blocks too; and how
+// many tiles have room so (plora_tile_blocks). Any value gives the same bits.
+static int tile_split(const plora_t* h, const plora_hook* hook, int rows) {
+    const int est = std::max(1, rows / PLORA_MMA_TOKENS), rank = hook->parts * h->max_rank;
+    int s = h->tile_split_force;
+    if (s == 0)
+        for (s = 1; s < PLORA_TILE_SPLIT_MAX && 2 * s * est <= h->sm_count;) s <<= 1;
+    const int groups = (rank + PLORA_TILE_GROUP - 1) / PLORA_TILE_GROUP;
+    int blocks = std::min(s, plora_tile_chunks(h->sites[(size_t)hook->site].cols, rank));
+    const bool rsplit = groups > 1 && est * blocks * groups <= h->sm_count;
+    if (rsplit) blocks *= groups;
+    const int fit = h->tile_split_force ? INT32_MAX / PLORA_TILE_FIT - 1 : h->sm_count / blocks;
+    return s + (rsplit ? PLORA_TILE_RSPLIT : 0) + fit * PLORA_TILE_FIT;
 }
 
 static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* step, uint64_t x, int rows, bool early,
@@ -1001,7 +1007,7 @@ static int shrink_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
-                                   tile_split(h, rows), h->status, h->pdl, h->tile_late && (!early || early_x),
+                                   tile_split(h, hook, rows), h->status, h->pdl, h->tile_late && (!early || early_x),
                                    as_stream(stream)));
     return PLORA_OK;
 }
@@ -1062,11 +1068,11 @@ int plora_apply(plora_t* h, const plora_hook* hook, const plora_step* step, uint
                                    h->seg, (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (float*)(uintptr_t)step->s,
                                    (size_t)(step->s_stride / 4), step->lds, hook->parts * h->max_rank, std::max(1, rows / 64),
-                                   tile_split(h, rows), h->status, h->pdl, tile_shrink_beside(h->tile_late, h->early_x, release, late && pdl),
+                                   tile_split(h, hook, rows), h->status, h->pdl, tile_shrink_beside(h->tile_late, h->early_x, release, late && pdl),
                                    as_stream(stream)));
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
-                                   tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
+                                   tile_split(h, hook, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
                                    (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
@@ -1087,7 +1093,7 @@ int plora_s_reduce(plora_t* h, const plora_hook* hook, const plora_step* step, i
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
                                             has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0,
-                                            tile_split(h, rows), site.cols, pdl, as_stream(stream)));
+                                            tile_split(h, hook, rows), site.cols, pdl, as_stream(stream)));
     return PLORA_OK;
 }
 
@@ -1113,7 +1119,7 @@ static int expand_impl(plora_t* h, const plora_hook* hook, const plora_step* ste
     if (tiles)
         CUK(h, "expand (tile path)",
            plora_launch_expand_mma((const float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, site.cols,
-                                   reduced ? 1 : tile_split(h, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
+                                   reduced ? 1 : tile_split(h, hook, rows), (const int32_t*)(uintptr_t)step->segs, h->seg,
                                    (const plora_desc*)(uintptr_t)hook->table,
                                    h->smaps + (size_t)hook->site * (size_t)(h->max_slots + 1), (void*)(uintptr_t)y, ldy, f32_out, hook->parts,
                                    site.part_off, site.part_rows, rows, hook->max_rows, std::max(1, rows / 64), h->status,
@@ -1142,11 +1148,11 @@ static int gemm_layer(plora_t* h, const plora_hook* hook, const plora_step* step
     bool pdl = next_launch(h, stream, false).pdl;
     // the kernel reads the long runs' S from plane 0: fold the tile path's planes, where a tile was more than one block's (the gather
     // tokens' K-split planes are added by the gather expand itself)
-    if (has_tiles(h, step, rows) && tile_split(h, rows) > 1) {
+    if (has_tiles(h, step, rows) && (tile_split(h, hook, rows) & (PLORA_TILE_RSPLIT - 1)) > 1) {
         CUK(h, "S reduce (tiles)",
            plora_launch_s_reduce((float*)(uintptr_t)step->s, (size_t)(step->s_stride / 4), step->lds, 1,
                                  (const int32_t*)(uintptr_t)step->segs, h->seg, (const plora_desc*)(uintptr_t)hook->table, 0,
-                                 std::max(1, rows / 64), tile_split(h, rows), site.cols, pdl, as_stream(stream)));
+                                 std::max(1, rows / 64), tile_split(h, hook, rows), site.cols, pdl, as_stream(stream)));
         pdl = h->pdl;
     }
     CUK(h, "fused layer (tensor-core adapter term)",
@@ -1220,7 +1226,7 @@ int plora_linear_fp8_fused(plora_t* h, const plora_hook* hook, const plora_step*
                                             (const int32_t*)(uintptr_t)step->segs, h->seg,
                                             (const plora_desc*)(uintptr_t)hook->table, work_cap,
                                             has_tiles(h, step, rows) ? std::max(1, rows / 64) : 0,
-                                            tile_split(h, rows), site.cols, pdl, as_stream(stream)));
+                                            tile_split(h, hook, rows), site.cols, pdl, as_stream(stream)));
     CUK(h, "fused fp8 layer",
        plora_launch_fp8_fused((const void*)(uintptr_t)xq, (const float*)(uintptr_t)st, (const void*)(uintptr_t)wq,
                               (const float*)(uintptr_t)sn, rows, width, site.cols, (const int32_t*)(uintptr_t)step->segs,
@@ -1418,7 +1424,7 @@ static int xchg_ctx(plora_t* h, const plora_hook* hook, const plora_step* step, 
     c->lay = h->seg;
     c->table = (const plora_desc*)(uintptr_t)hook->table;
     c->work_cap = work_cap;
-    c->tile_split = tile_split(h, rows);
+    c->tile_split = tile_split(h, hook, rows);
     c->K = site.cols;
     c->world = h->xchg_world;
     c->rank = h->xchg_rank;

@@ -263,8 +263,7 @@ cudaError_t plora_launch_xchg_all_ranks(const PloraXchgCtx* ctxs_dev, int world,
 // columns of an SM for all of a tile's chunks (where they go to several blocks, each holds its own only), and at least 8 steps of
 // 64 inputs per chunk. With 256 of them, ranges of K were twice as long at total ranks over 32: 1,545 ragged tokens of ranks 16 to
 // 64 277 us a step, 262 so; 512 mixed tokens of rank 32 176 and 169; eight prompts of 2048 tokens, whose tiles are one
-// block each, 765 and 768. Slower so: steps of two to three dozen runs of 64 to 80 tokens at total ranks over 128 (30 of 64, rank 64: 9 %),
-// which have twice the tiles that their rows let the host expect, and whose blocks then take two rounds.
+// block each, 765 and 768.
 #define PLORA_TILE_SPLIT_MAX 8
 __host__ __device__ inline int plora_tile_cols(int R) { return R <= 32 ? 32 : R <= 64 ? 64 : R <= 128 ? 128 : R <= 256 ? 256 : 512; }
 __host__ __device__ inline int plora_tile_chunks(int K, int R) {
@@ -272,6 +271,20 @@ __host__ __device__ inline int plora_tile_chunks(int K, int R) {
     int c = PLORA_TILE_SPLIT_MAX;
     while (c > 1 && (c * 8 > nk || c * rc > 512)) c >>= 1;
     return c;
+}
+// How many blocks share a tile's chunks in a launch: at most `most`, which the host made of the step's rows, and half as many where
+// the step has more tiles than `fit`, for which that many blocks (of the largest rank) are one round. The host takes a tile for
+// 128 rows; runs of 64 to 80 are up to twice as many tiles, whose blocks would take a second round. (One comparison, since anything
+// more shows at the start of a block.) Four layers of 4096 -> 4096 + 1024 + 1024, 24 runs of 72 tokens of rank 16 168 -> 151 us,
+// 30 of 64 179 -> 162, of rank 64 256 -> 245; steps within `fit` 0.2 to 0.5 % slower (15 tiles of rank 64 162.8 -> 163.2), 24 runs of
+// rank 64, which just fit, 1.5 %.
+// In one word for the launches: `most`, PLORA_TILE_RSPLIT where the rows of A go to several blocks too, `fit` times PLORA_TILE_FIT.
+#define PLORA_TILE_RSPLIT 16
+#define PLORA_TILE_FIT 32
+#define PLORA_TILE_GROUP 64  // rows of A per block where these go to several
+__host__ __device__ inline int plora_tile_blocks(int most, int fit, int n_tiles, int K, int R) {
+    const int chunks = plora_tile_chunks(K, R), s = most < chunks ? most : chunks;
+    return s > 1 && n_tiles > fit ? s >> 1 : s;
 }
 
 // ---- kernel launchers (plora_kernels.cu); each returns a cudaError_t from the launch ----

@@ -108,7 +108,7 @@ __device__ __forceinline__ void tmap_acquire(const CUtensorMap* map) {
 // (RSPLIT); x is then read again for each group, from L2, which a step with tiles for every SM could not afford. The sums of
 // an element stay the same. 300 tokens, 4 layers: rank 64 169 -> 149 us, rank 128 262 -> 183 us; 2,000 tokens of one
 // adapter: rank 64 228 -> 213 us, rank 128 327 -> 259 us.
-#define SHR_GROUP 64
+#define SHR_GROUP PLORA_TILE_GROUP
 
 template <bool RSPLIT>
 __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_constant__ CUtensorMap xmap,
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
                                                                 const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table,
                                                                 float* __restrict__ S, size_t s_stride, int lds,
-                                                                int ksplit, int nstage, int stage_bytes, int sub,
+                                                                int ksplit, int fit, int nstage, int stage_bytes, int sub,
                                                                 int late, int* __restrict__ status) {
     // late != 0: the kernel launched right before this one is the same layer's gather shrink, whose blocks let
     // this grid start only after they have themselves waited for the kernels before (or whose caller vouches
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(128) plora_shrink_mma_kernel(const __grid_cons
     const int R_out = RSPLIT ? min(SHR_GROUP, R_all - r0) : R_all;
     if (R_out <= 0) return pdl_exit_idle();
     const int n_chunks = plora_tile_chunks(K, R_all);
-    const int s_eff = min(ksplit, n_chunks);
+    const int s_eff = plora_tile_blocks(ksplit, fit, n_mma, K, R_all);
     if ((int)blockIdx.x >= s_eff) return pdl_exit_idle();
     const int n_acc = n_chunks / s_eff;  // accumulators (chunks) of this block
     const CUtensorMap* amap = reinterpret_cast<const CUtensorMap*>(RSPLIT ? &smaps[slot].a64 : &smaps[slot].a);
@@ -310,7 +310,7 @@ __device__ __forceinline__ void load_rows_f32(float2 (&raw)[32], const float* y,
 
 template <bool F32>
 __global__ void __launch_bounds__(128) plora_expand_mma_kernel(const float* __restrict__ S, size_t s_stride, int lds,
-                                                                int K, int ksplit,
+                                                                int K, int ksplit, int fit,
                                                                 const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table, void* Y,
                                                                 int ldy, int nb_per_cta, int op_bytes,
@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(128) plora_expand_mma_kernel(const float* __re
         const int row = tid;
         const bool valid = row < len;
         const float* sp = S + (size_t)(start + (valid ? row : 0)) * lds + d.r_off[p];
-        const int s_eff = min(ksplit, plora_tile_chunks(K, d.rank));  // planes the shrink wrote for this slot
+        const int s_eff = plora_tile_blocks(ksplit, fit, n_mma, K, d.rank);  // planes the shrink wrote for this slot
         unsigned char* ahi = Ahi + (size_t)(row >> 3) * sbo + (row & 7) * 16;
         unsigned char* alo = Alo + (size_t)(row >> 3) * sbo + (row & 7) * 16;
         for (int j = 0; j < P; j++) {
@@ -550,7 +550,7 @@ __device__ __forceinline__ void bulk_wait_read_1() { asm volatile("cp.async.bulk
 
 template <bool F32, bool HIGH>
 __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kernel(const float* __restrict__ S, size_t s_stride, int lds, int K,
-                                                                int ksplit, const int* __restrict__ segs, SegLayout lay,
+                                                                int ksplit, int fit, const int* __restrict__ segs, SegLayout lay,
                                                                 const plora_desc* __restrict__ table,
                                                                 const PloraSlabMaps* __restrict__ smaps,
                                                                 const __grid_constant__ ExpandYMaps ymaps, void* Y, int ldy,
@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(32 * (EXP_WARPS + 1), 2) plora_expand_tma_kern
             // per lane), 88 so; four prompts of 2048 tokens of rank 128 562 -> 546. Not for the others: the longer code costs more at a
             // block's start than it gives (the prompt of 199 tokens of rank 16: 133 -> 139).
             {
-                const int s_eff = min(ksplit, plora_tile_chunks(K, rank));  // planes the shrink wrote for this slot
+                const int s_eff = plora_tile_blocks(ksplit, fit, n_mma, K, rank);  // planes the shrink wrote for this slot
                 const float* sq = S + (size_t)(start + wrow0) * lds + r_off;
                 auto buffer = [&](int k) { return dsm1k + (size_t)((wq + (k & 32 ? 4 : 0)) * nst + nst - 1) * EXP_SLOT_BYTES; };
 #pragma unroll 1
@@ -995,8 +995,7 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return cudaErrorInvalidValue;
     const int groups = (max_rank_total + SHR_GROUP - 1) / SHR_GROUP;
-    const int blocks = std::max(1, rows / MMA_M) * std::min(tile_split, plora_tile_chunks(K, max_rank_total));
-    const bool rsplit = groups > 1 && blocks * groups <= g_sms;
+    const bool rsplit = (tile_split & PLORA_TILE_RSPLIT) != 0;
     int stage_bytes = SHR_X_BYTES + (((rsplit ? SHR_GROUP : max_rank_total) * 128 + 1023) / 1024) * 1024;
     // two steps of 64 inputs per stage where at least three such stages fit
     const int sub = 3 * 2 * stage_bytes <= 190 * 1024 ? 2 : 1;
@@ -1006,8 +1005,8 @@ cudaError_t plora_launch_shrink_mma(const void* x, int rows, int ldx, int K, con
     if (nstage < 2) return cudaErrorInvalidValue;
     const size_t smem = (size_t)nstage * stage_bytes + 1024;
     return launch_pdl(rsplit ? plora_shrink_mma_kernel<true> : plora_shrink_mma_kernel<false>,
-                      dim3((unsigned)tile_split, rsplit ? (unsigned)groups : 1, (unsigned)tile_cap), dim3(128), smem, st, pdl, map, smaps, K, segs, lay, table, S, s_stride_elems, lds, tile_split,
-                      nstage, stage_bytes, sub, late && pdl ? 1 : 0, status);
+                      dim3((unsigned)(tile_split & (PLORA_TILE_RSPLIT - 1)), rsplit ? (unsigned)groups : 1, (unsigned)tile_cap), dim3(128), smem, st, pdl, map, smaps, K, segs, lay, table, S, s_stride_elems, lds,
+                      tile_split & (PLORA_TILE_RSPLIT - 1), tile_split / PLORA_TILE_FIT, nstage, stage_bytes, sub, late && pdl ? 1 : 0, status);
 }
 
 cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int lds, int K, int tile_split,
@@ -1064,7 +1063,7 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
             auto* fn = max_rank > 64 ? (f32_out ? plora_expand_tma_kernel<true, true> : plora_expand_tma_kernel<false, true>)
                                      : (f32_out ? plora_expand_tma_kernel<true, false> : plora_expand_tma_kernel<false, false>);
             return launch_pdl(fn, grid, dim3(32 * (EXP_WARPS + 1)),
-                              smem_tma, st, pdl, S, s_stride_elems, lds, K, tile_split, segs, lay, table, smaps, maps, y, ldy,
+                              smem_tma, st, pdl, S, s_stride_elems, lds, K, tile_split & (PLORA_TILE_RSPLIT - 1), tile_split / PLORA_TILE_FIT, segs, lay, table, smaps, maps, y, ldy,
                               nb_per_cta, b_bytes, nbs, nst, late && pdl ? 1 : 0, status);
         }
     }
@@ -1076,7 +1075,7 @@ cudaError_t plora_launch_expand_mma(const float* S, size_t s_stride_elems, int l
     if (smem < 48 * 1024) smem = 48 * 1024;
     if (f32_out)
         return launch_pdl(plora_expand_mma_kernel<true>, grid, dim3(128), smem, st, pdl, S, s_stride_elems, lds, K,
-                          tile_split, segs, lay, table, y, ldy, nb_per_cta, op_bytes, status);
+                          tile_split & (PLORA_TILE_RSPLIT - 1), tile_split / PLORA_TILE_FIT, segs, lay, table, y, ldy, nb_per_cta, op_bytes, status);
     return launch_pdl(plora_expand_mma_kernel<false>, grid, dim3(128), smem, st, pdl, S, s_stride_elems, lds, K,
-                      tile_split, segs, lay, table, y, ldy, nb_per_cta, op_bytes, status);
+                      tile_split & (PLORA_TILE_RSPLIT - 1), tile_split / PLORA_TILE_FIT, segs, lay, table, y, ldy, nb_per_cta, op_bytes, status);
 }

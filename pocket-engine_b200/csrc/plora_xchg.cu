@@ -89,7 +89,7 @@ __device__ void xchg_body(const PloraXchgCtx& c, int w, int nblocks) {
         start = mt[0];
         cnt = mt[1];
         rank_cols = c.table[mt[2]].rank;
-        nplanes = rank_cols ? min(c.tile_split, plora_tile_chunks(c.K, rank_cols)) : 1;
+        nplanes = rank_cols ? plora_tile_blocks(c.tile_split & (PLORA_TILE_RSPLIT - 1), c.tile_split / PLORA_TILE_FIT, c.segs[SEG_N_MMA], c.K, rank_cols) : 1;
         tree = true;
     }
     const bool live = cnt > 0 && rank_cols > 0;
