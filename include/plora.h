@@ -341,7 +341,7 @@ int plora_set_run_min(plora_t* h, int tokens);
  * the adapter's rank alone), accumulate each on its own and add the results as a balanced tree, so that a
  * token's result does not depend on what else is in the batch. `blocks` = 1, 2, 4 or 8 fixes how many thread
  * blocks share the ranges of one 128-token tile; 0 (the default) lets the library choose from the step's row
- * count. Every value gives bit-identical results. No counterpart in the engine. */
+ * count and its tiles. Every value gives bit-identical results. No counterpart in the engine. */
 int plora_set_tile_split(plora_t* h, int blocks);
 
 /* No counterpart in pocket-engine. One layer's adapter application (shrink, then expand, straight from the

@@ -611,7 +611,10 @@ bool clusters_pay(int K, int n_parts, int total, int max_rank) {
 // Plans of the cluster kernel for one layer, by column groups per work item: those with which two blocks share an SM (one SM
 // cannot take a whole cluster of 8, and a B200 has room for only 15 clusters of 8 at one block per SM). Empty where nothing
 // fits (13 tokens of 8 adapters at rank 32, four layers: 240 us with one block per SM, 150 as pairs) or clusters do not pay: such
-// a layer takes the shrink / expand pair.
+// a layer takes the shrink / expand pair. What does not fit at rank 64 and 4096 inputs are the partial sums of eight tokens; four tokens
+// a pass would, but then the pair is the better one from 16 items on. Four layers, clusters so / pairs in us, steps as above:
+//   4096 -> 4096, rank 64        27 / 35   39 / 42   61 / 47   197 /  97   95 / 51
+//   4096 -> 1024, rank 64        25 / 34   27 / 38   29 / 40    71 /  80   67 / 47
 std::vector<PloraSitePlan> plora_site_plans(int K, int n_parts, const int* part_rows, int max_rank) {
     std::vector<PloraSitePlan> out;
     int total = 0;
